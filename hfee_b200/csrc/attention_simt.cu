@@ -17,6 +17,8 @@
 // leading dimensions of the cached keys (a latent cache: one vector per token serves as key and as value).
 // Reference: hostfog/hfee internal/llm/forward.go:146-178 (scores scaled after the
 // dot, softmax over 0..pos, weighted sum of values), internal/ggml/ops.go:136-150.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -26,7 +28,12 @@ constexpr int MAX_HD = 640;      // key size
 constexpr int MAX_VD = 512;      // value size
 constexpr int GATE_NONE = 0, GATE_ELEMENT = 1, GATE_PER_HEAD = 2;
 
-template <typename T, bool SIGMOID>
+// Bound by the latency of its loads (a warp walks its keys alone): the key of a lane is read 16 bytes at a time where VEC says
+// that keys start on 16-byte boundaries, and the values of VALUES_AHEAD keys are requested together; DPL, the value dimensions
+// a lane owns, is the smallest that covers the value size.  The order of every sum is the one described above.
+constexpr int VALUES_AHEAD = 8;
+
+template <typename T, bool SIGMOID, int DPL, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k_pool,
                       const T* __restrict__ v_pool, PagedCache cache, PagedCache vcache, int vd,
@@ -38,7 +45,7 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
                       const float* __restrict__ sink, int keep_first, float softcap) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float q_s[WARPS][MAX_HD];
+  __shared__ __align__(16) float q_s[WARPS][MAX_HD];
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   long long task = (long long)blockIdx.x * WARPS + warp;
   if (task >= (long long)n * heads) return;
@@ -56,7 +63,6 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
   for (int d = lane; d < hd; d += 32) q_s[warp][d] = to_f32<T>(qrow[d]);
   __syncwarp();
 
-  constexpr int DPL = MAX_VD / 32;     // output dims per lane
   float o[DPL];
 #pragma unroll
   for (int j = 0; j < DPL; ++j) o[j] = 0.f;
@@ -69,10 +75,23 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
     const int end = base < kept ? kept - 1 : pos;            // last key of the range this block of 32 lies in
     int key = base + lane;
     float s = -INFINITY;
+    long long v_at = 0;
     if (key <= end) {
       const T* kr = k_pool + paged_offset(cache, slot, key, kvh);
+      v_at = paged_offset(vcache, slot, key, kvh);
       float acc = 0.f;
-      for (int d = 0; d < hd; ++d) acc = fmaf(q_s[warp][d], to_f32<T>(kr[d]), acc);
+      if constexpr (VEC) {
+#pragma unroll 8
+        for (int d = 0; d < hd; d += 4) {
+          const float4 kv = *(const float4*)(kr + d), qv = *(const float4*)(q_s[warp] + d);
+          acc = fmaf(qv.x, kv.x, acc);
+          acc = fmaf(qv.y, kv.y, acc);
+          acc = fmaf(qv.z, kv.z, acc);
+          acc = fmaf(qv.w, kv.w, acc);
+        }
+      } else {
+        for (int d = 0; d < hd; ++d) acc = fmaf(q_s[warp][d], to_f32<T>(kr[d]), acc);
+      }
       s = acc * scale;
       if (softcap > 0.f) s = softcap * tanhf(s / softcap);
       if (dist_r1 != nullptr) s -= r1 * log1pf(r2 * (float)(pos - key));
@@ -90,13 +109,23 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
       m = m_new;
     }
     int count = min(32, end + 1 - base);
-    for (int t = 0; t < count; ++t) {
-      float pt = __shfl_sync(0xffffffffu, p, t);
-      const T* vr = v_pool + paged_offset(vcache, slot, base + t, kvh);
+    for (int t0 = 0; t0 < count; t0 += VALUES_AHEAD) {
+      float v[VALUES_AHEAD][DPL];
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) {
-        int d = lane + 32 * j;
-        if (d < vd) o[j] = fmaf(pt, to_f32<T>(vr[d]), o[j]);
+      for (int t = 0; t < VALUES_AHEAD; ++t) {
+        const T* vr = v_pool + __shfl_sync(0xffffffffu, v_at, min(t0 + t, count - 1));
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) {
+          const int d = lane + 32 * j;
+          v[t][j] = t0 + t < count && d < vd ? to_f32<T>(vr[d]) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < VALUES_AHEAD; ++t) {
+        if (t0 + t >= count) break;
+        const float pt = __shfl_sync(0xffffffffu, p, t0 + t);
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) o[j] = fmaf(pt, v[t][j], o[j]);
       }
     }
     const bool front = base < kept;
@@ -121,23 +150,40 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
 }  // namespace
 
 namespace {
-template <typename T>
-void launch_simt(const void* q, int ld_q, const void* k_pool, const void* v_pool, const PagedCache& c, const PagedCache& vc,
-                 int vd, const int* positions,
-                 const int* slot_of_token, void* out, int ld_o, int n, int heads, float scale, int window, int chunk,
-                 int sigmoid, const float* head_scale, const float* head_bias, const void* gate, long long ld_gate,
-                 int gate_mode, const float* dist_r1, const float* dist_r2, float out_scale, const float* sink, int keep_first,
-                 float softcap, cudaStream_t stream) {
+template <typename T, bool SIGMOID, int DPL, bool VEC>
+void launch_one(const void* q, int ld_q, const void* k_pool, const void* v_pool, const PagedCache& c, const PagedCache& vc,
+                int vd, const int* positions, const int* slot_of_token, void* out, int ld_o, int n, int heads, float scale,
+                int window, int chunk, const float* head_scale, const float* head_bias, const void* gate, long long ld_gate,
+                int gate_mode, const float* dist_r1, const float* dist_r2, float out_scale, const float* sink, int keep_first,
+                float softcap, cudaStream_t stream) {
   long long tasks = (long long)n * heads;
   unsigned blocks = (unsigned)((tasks + WARPS - 1) / WARPS);
-  if (sigmoid)
-    hfee_launch(attention_simt_kernel<T, true>, dim3(blocks), dim3(WARPS * 32), 0, stream, (const T*)q, ld_q, (const T*)k_pool,
-                (const T*)v_pool, c, vc, vd, positions, slot_of_token, (T*)out, ld_o, n, heads, scale, window, chunk, head_scale,
-                head_bias, (const T*)gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first, softcap);
-  else
-    hfee_launch(attention_simt_kernel<T, false>, dim3(blocks), dim3(WARPS * 32), 0, stream, (const T*)q, ld_q, (const T*)k_pool,
-                (const T*)v_pool, c, vc, vd, positions, slot_of_token, (T*)out, ld_o, n, heads, scale, window, chunk, head_scale,
-                head_bias, (const T*)gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first, softcap);
+  hfee_launch(attention_simt_kernel<T, SIGMOID, DPL, VEC>, dim3(blocks), dim3(WARPS * 32), 0, stream, (const T*)q, ld_q, (const T*)k_pool,
+              (const T*)v_pool, c, vc, vd, positions, slot_of_token, (T*)out, ld_o, n, heads, scale, window, chunk, head_scale,
+              head_bias, (const T*)gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first, softcap);
+}
+
+template <typename T, bool SIGMOID, typename... Args>
+void launch_weights(const void* q, int ld_q, const void* k_pool, const void* v_pool, const PagedCache& c, const PagedCache& vc, int vd,
+                    Args... args) {
+  const bool vec = sizeof(T) == 4 && c.head_dim % 4 == 0 && (uintptr_t)k_pool % 16 == 0;
+  auto with = [&](auto dpl) {
+    constexpr int DPL = decltype(dpl)::value;
+    if constexpr (sizeof(T) == 4) {
+      if (vec) return launch_one<T, SIGMOID, DPL, true>(q, ld_q, k_pool, v_pool, c, vc, vd, args...);
+    }
+    launch_one<T, SIGMOID, DPL, false>(q, ld_q, k_pool, v_pool, c, vc, vd, args...);
+  };
+  if (vd <= 64) with(std::integral_constant<int, 2>{});
+  else if (vd <= 128) with(std::integral_constant<int, 4>{});
+  else if (vd <= 256) with(std::integral_constant<int, 8>{});
+  else with(std::integral_constant<int, MAX_VD / 32>{});
+}
+
+template <typename T, typename... Args>
+void launch_simt(int sigmoid, Args... args) {
+  if (sigmoid) launch_weights<T, true>(args...);
+  else launch_weights<T, false>(args...);
 }
 }  // namespace
 
@@ -183,12 +229,12 @@ HFEE_API int hfee_attention_simt_capped(const void* q, int ld_q, const void* k_p
     make_paged_cache(&vc, block_table, max_pages, page_size, kv_heads, value_dim);
   }
   if (dtype == HFEE_F32)
-    launch_simt<float>(q, ld_q, k_pool, v_pool, c, vc, value_dim, positions, slot_of_token, out, ld_o, n, heads, scale,
-                       window, chunk, weights, head_scale, head_bias, gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first,
+    launch_simt<float>(weights, q, ld_q, k_pool, v_pool, c, vc, value_dim, positions, slot_of_token, out, ld_o, n, heads, scale,
+                       window, chunk, head_scale, head_bias, gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first,
                        softcap, stream);
   else if (dtype == HFEE_BF16)
-    launch_simt<__nv_bfloat16>(q, ld_q, k_pool, v_pool, c, vc, value_dim, positions, slot_of_token, out, ld_o, n, heads,
-                               scale, window, chunk, weights, head_scale, head_bias, gate, ld_gate, gate_mode, dist_r1, dist_r2,
+    launch_simt<__nv_bfloat16>(weights, q, ld_q, k_pool, v_pool, c, vc, value_dim, positions, slot_of_token, out, ld_o, n, heads,
+                               scale, window, chunk, head_scale, head_bias, gate, ld_gate, gate_mode, dist_r1, dist_r2,
                                out_scale, sink, keep_first, softcap, stream);
   else
     return hfee_fail(HFEE_ERR_ARG, "attention_simt: unknown dtype %d", dtype);

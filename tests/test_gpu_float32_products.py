@@ -1,0 +1,44 @@
+"""The float32 product's kernels (a warp per 16 rows of the weights, three tile sizes, the general kernel) add in one order:
+every output element is the same bits whichever of them runs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from hfee_b200.kernels import ops as o
+    o.library()
+    return o
+
+
+def _shifted(t):
+    """The same rows one float off a 16-byte boundary: only the general kernel takes them."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + 1, device=t.device)
+    wide[:, 1:] = t
+    return wide[:, 1:]
+
+
+# token counts around every change of kernel (2, 4, 8, 16) and of tile (32, 64, 128), widths around a warp's 16 rows and a
+# tile's 64 and 128, depths below, at and past a piece of 64 and of 32
+@pytest.mark.parametrize("n,k", [(1, 4), (16, 60), (17, 64), (130, 100), (2500, 36), (300, 2052), (20000, 8)])
+def test_every_kernel_gives_the_same_bits(ops, n, k):
+    g = torch.Generator().manual_seed(n + k)
+    w = torch.randn(n, k, generator=g).cuda()
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 65, 129, 700):
+        a = torch.randn(m, k, generator=g).cuda()
+        plain = torch.empty(m, n, device="cuda")
+        ops.gemm_simt(_shifted(a), _shifted(w), plain)
+        # k additions of rounded products: at most (k + 1) 2^-24 of the sum of magnitudes
+        ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+        assert ((plain.double() - ref).abs() <= (k + 1) * 2.0 ** -24 * size).all()
+        out = torch.full((m, n + 3), 7.0, device="cuda")
+        ops.gemm_simt(a, w, out[:, :n])
+        assert torch.equal(out[:, :n], plain) and (out[:, n:] == 7.0).all(), m
+        acc = torch.ones(m, n, device="cuda")
+        ops.gemm_simt(a, w, acc, accumulate=True)
+        assert torch.equal(acc, 1.0 + plain), m
+        narrow = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        ops.gemm_simt(a, w, narrow)
+        assert torch.equal(narrow, plain.bfloat16()), m
