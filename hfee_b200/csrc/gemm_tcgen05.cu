@@ -48,14 +48,14 @@ template <int BN> struct TileCfg {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int W_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + W_BYTES;
-  static constexpr int EPI_BYTES = EPI_WARPS * 32 * 128;        // accumulate epilogue: a 32 x 32 float chunk per warp
+  static constexpr int EPI_BYTES = EPI_WARPS * 32 * 128;        // a 32 x 32 float chunk per warp
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + EPI_BYTES;      // + slack to align the base to 1024
 };
 
 template <int BN, int EPI, typename TOut>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-               const __grid_constant__ CUtensorMap map_c, int reduce_by_tma,
+               const __grid_constant__ CUtensorMap map_c, int c_by_tma,
                TOut* __restrict__ C, long long ldc, int M, int N, int K, int* __restrict__ status,
                float* __restrict__ sk_parts, int* __restrict__ sk_flags, const RopeEpi rope,
                const int* __restrict__ tile_group, int group_rows) {
@@ -272,28 +272,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
         const int col0 = n0 + ch * 32;
-        if constexpr (EPI == EPI_ACCUM) {
-          if (reduce_by_tma) {
-            // The chunk goes to shared memory (thread = row, 128 bytes, in the 128-byte swizzle the
-            // tensor map of C expects) and from there into C by a bulk tensor reduction: the addition
-            // happens in the memory system, nothing of C is read here, and rows or columns beyond the
-            // matrix are clipped by the copy.
+        if constexpr (EPI == EPI_ACCUM || EPI == EPI_STORE || EPI == EPI_RELU2) {
+          if (c_by_tma) {
+            // through shared memory and by a bulk tensor copy or reduction: an addition happens in the memory
+            // system, nothing of C is read here, and rows or columns beyond the matrix are clipped by the copy
             const int row0 = m0 + quad * 32;
             if (row0 >= M || col0 >= N) continue;                      // the same for the whole warp
+            if constexpr (EPI == EPI_RELU2) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const float t = fmaxf(__uint_as_float(v[j]), 0.f);
+                v[j] = __float_as_uint(t * t);
+              }
+            }
             unsigned char* cs = epi_stage + (warp - 2) * 4096;
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the previous chunk has left the buffer
             __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<uint4*>(cs + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                  make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            stage_chunk((TOut*)nullptr, cs, lane, v);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(reinterpret_cast<uint64_t>(&map_c)), "r"(col0), "r"(row0), "r"(smem_u32(cs)) : "memory");
-              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
+            if (lane == 0) tma_store_2d<EPI == EPI_ACCUM>(&map_c, col0, row0, cs);
             continue;
           }
         }
@@ -400,9 +398,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   }
 
-  if constexpr (EPI == EPI_ACCUM) {
-    // bulk reductions of this thread are complete (not merely read out of shared memory) before the CTA ends
-    if (reduce_by_tma && warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if constexpr (EPI == EPI_ACCUM || EPI == EPI_STORE || EPI == EPI_RELU2) {
+    // bulk copies of this thread are complete (not merely read out of shared memory) before the CTA ends
+    if (c_by_tma && warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -434,32 +432,17 @@ int plan_stream_k(long long tiles, int k_blocks, int sms, long long workspace_fl
   return (int)ctas;
 }
 
-// Tensor map of the float32 output for the bulk reduction of 32 x 32 chunks (128-byte rows, swizzled).
-int make_map_c(CUtensorMap* map, void* base, long long rows, long long cols, long long ld) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05: the driver has no cuTensorMapEncodeTiled");
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  cuuint32_t box[2] = {32, 32};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05: cuTensorMapEncodeTiled (output) failed with %d", (int)r);
-  return HFEE_OK;
-}
-
 template <int BN, int EPI, typename TOut>
 int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* C, long long ldc, int M, int N, int K, int* status,
            float* workspace, long long workspace_floats, int* flags, cudaStream_t stream, const RopeEpi& rope = RopeEpi{},
            const int* tile_group = nullptr, int group_rows = 0) {
   using Cfg = TileCfg<BN>;
-  // accumulate: by bulk tensor reduction when C can have a tensor map (16-byte aligned base and pitch)
   CUtensorMap mc = ma;
-  int reduce_by_tma = 0;
-  if (EPI == EPI_ACCUM && (uintptr_t)C % 16 == 0 && ldc % 4 == 0) {
-    int rc = make_map_c(&mc, C, M, N, ldc);
+  int c_by_tma = 0;
+  if ((EPI == EPI_ACCUM || EPI == EPI_STORE || EPI == EPI_RELU2) && mappable_out(C, N, ldc, sizeof(TOut))) {
+    int rc = make_map_out(&mc, C, M, N, ldc, sizeof(TOut));
     if (rc != HFEE_OK) return rc;
-    reduce_by_tma = 1;
+    c_by_tma = 1;
   }
   static bool configured = false;
   if (!configured) {
@@ -472,7 +455,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* C, long long ldc,
   long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int sk_ctas = (workspace && flags) ? plan_stream_k(tiles, (K + BK - 1) / BK, sms, workspace_floats, BN) : 0;
   dim3 grid((unsigned)(sk_ctas ? sk_ctas : (tiles < sms ? tiles : sms)));          // one CTA per SM
-  hfee_launch(gemm_tc_kernel<BN, EPI, TOut>, dim3(grid), dim3(TC_THREADS), Cfg::SMEM, stream, ma, mw, mc, reduce_by_tma, (TOut*)C, ldc, M, N, K, status,
+  hfee_launch(gemm_tc_kernel<BN, EPI, TOut>, dim3(grid), dim3(TC_THREADS), Cfg::SMEM, stream, ma, mw, mc, c_by_tma, (TOut*)C, ldc, M, N, K, status,
               sk_ctas ? workspace : (float*)nullptr, sk_ctas ? flags : (int*)nullptr, rope, tile_group, group_rows);
   return hfee_check_launch("gemm_tcgen05");
 }
@@ -617,28 +600,25 @@ HFEE_API int hfee_gemm_tcgen05_rope(const void* A, long long lda, const void* W,
   HFEE_REQUIRE(make_paged_cache(&rope.cache, block_table, max_pages, page_size, kv_heads, head_dim),
                "gemm_tcgen05_rope: page_size %d must be a power of two", page_size);
   rope.heads = heads; rope.kv_heads = kv_heads; rope.head_dim = head_dim; rope.interleaved = interleaved;
-  // tiles of whole heads: 256 columns, or 128 where those fill the SMs better
+  // Tiles of whole heads, of the kind whose rounds take least: percent of a round of 128 x 256 tiles, as in ops.py (tile_choice);
+  // 192 columns are three 64-dim heads.  The benchmark model's q/k/v product at 2,048 tokens: 128 pair tiles of 256 x 192 are two
+  // rounds, as are 96 of 256 x 256 (prompt pass 3.69 against 3.76 ms).
   const int sms = hfee_sm_count();
-  const long long tiles_256 = (long long)((M + BM - 1) / BM) * ((N + 255) / 256);
-  // pairs of CTAs on tiles of 256 x 256 where those make two rounds or more (the q/k/v product of the
-  // benchmark model at 2,048 tokens has 96 of them for 74 pairs: the single-CTA tiles fill the SMs better)
-  if (sms > 0 && M > BM && (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256) >= 2 * (sms / 2))
-    return hfee_gemm_pair_rope(A, lda, W, ldw, M, N, K, rope, 256, status, stream);
-  if (sms > 0 && M > BM && head_dim == 64 && N % 192 == 0) {
-    // pairs on tiles of 256 x 192 (three heads) where those fill their rounds to four fifths or more: the
-    // q/k/v product of the benchmark model at 2,048 tokens has 128 of them for 74 pairs (prompt pass 3.76 -> 3.69 ms)
-    const long long pairs = sms / 2, tiles = (long long)((M + 2 * BM - 1) / (2 * BM)) * (N / 192);
-    const long long rounds = (tiles + pairs - 1) / pairs;
-    if (tiles * 5 >= rounds * pairs * 4) return hfee_gemm_pair_rope(A, lda, W, ldw, M, N, K, rope, 192, status, stream);
+  if (sms < 2) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05_rope: cannot ask the device for its number of SMs");
+  auto cost = [&](int rows, int cols, int units, int percent) {
+    const long long tiles = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols);
+    return (tiles + units - 1) / units * percent;
+  };
+  int bn = 256, pairs = 0;
+  long long best = cost(BM, 256, sms, 100);
+  auto consider = [&](long long c, int block, int two) { if (c < best) { best = c; bn = block; pairs = two; } };
+  consider(cost(BM, 128, sms, 72), 128, 0);
+  if (head_dim == 64 && N % 192 == 0) consider(cost(BM, 192, sms, 86), 192, 0);
+  if (M > BM) {
+    consider(cost(2 * BM, 256, sms / 2, 85), 256, 1);
+    if (head_dim == 64 && N % 192 == 0) consider(cost(2 * BM, 192, sms / 2, 70), 192, 1);
   }
-  int bn = tiles_256 >= 96 || sms <= 0 ? 256 : 128;
-  if (bn == 256 && head_dim == 64 && sms > 0) {
-    // three heads wide where that saves a round of tiles (16 x 12 tiles of 256 are two rounds on 148 SMs
-    // with the second a third full; 16 x 16 tiles of 192 are two rounds of three quarters the work)
-    const long long m_tiles = (M + BM - 1) / BM;
-    const long long rounds_192 = (m_tiles * ((N + 191) / 192) + sms - 1) / sms, rounds_256 = (tiles_256 + sms - 1) / sms;
-    if (rounds_192 * 192 * 105 < rounds_256 * 256 * 100) bn = 192;
-  }
+  if (pairs) return hfee_gemm_pair_rope(A, lda, W, ldw, M, N, K, rope, bn, status, stream);
   CUtensorMap ma, mw;
   int rc = make_map(&ma, A, M, K, lda, BM);
   if (rc != HFEE_OK) return rc;

@@ -84,7 +84,7 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
 template <int BN, int EPI, typename TOut>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                 const __grid_constant__ CUtensorMap map_c, int reduce_by_tma,
+                 const __grid_constant__ CUtensorMap map_c, int c_by_tma,
                  TOut* __restrict__ C, long long ldc, int M, int N, int K, int* __restrict__ status, const RopeEpi rope) {
   constexpr int BNH = PairCfg<BN>::BNH, STAGE_BYTES = PairCfg<BN>::STAGE_BYTES;
   extern __shared__ unsigned char smem_dyn[];
@@ -200,26 +200,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         tc_ld32(tmem_base + buf * BN + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ch * 32), v);
         tc_wait_ld();
         const int col0 = n0 + ch * 32;
-        if constexpr (EPI == EPI_ACCUM) {
-          if (reduce_by_tma) {
-            // the chunk goes to shared memory (thread = row, 128 bytes, in the swizzle the tensor map of C
-            // expects) and from there into C by a bulk tensor reduction, which clips at the matrix's edges
+        if constexpr (EPI == EPI_ACCUM || EPI == EPI_STORE || EPI == EPI_RELU2) {
+          if (c_by_tma) {
+            // through shared memory and by a bulk tensor copy or reduction: an addition happens in the memory
+            // system, nothing of C is read here, and rows or columns beyond the matrix are clipped by the copy
             const int row0 = m0 + quad * 32;
             if (row0 >= M || col0 >= N) continue;                      // the same for the whole warp
-            unsigned char* cs = epi_stage + (warp - 2) * 4096;
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            __syncwarp();
+            if constexpr (EPI == EPI_RELU2) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<uint4*>(cs + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                  make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+              for (int j = 0; j < 32; ++j) {
+                const float t = fmaxf(__uint_as_float(v[j]), 0.f);
+                v[j] = __float_as_uint(t * t);
+              }
+            }
+            unsigned char* cs = epi_stage + (warp - 2) * 4096;
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the previous chunk has left the buffer
+            __syncwarp();
+            stage_chunk((TOut*)nullptr, cs, lane, v);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(reinterpret_cast<uint64_t>(&map_c)), "r"(col0), "r"(row0), "r"(smem_u32(cs)) : "memory");
-              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
+            if (lane == 0) tma_store_2d<EPI == EPI_ACCUM>(&map_c, col0, row0, cs);
             continue;
           }
         }
@@ -308,9 +308,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   }
 
-  if constexpr (EPI == EPI_ACCUM) {
-    // bulk reductions of this thread are complete (not merely read out of shared memory) before the CTA ends
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if constexpr (EPI == EPI_ACCUM || EPI == EPI_STORE || EPI == EPI_RELU2) {
+    // bulk copies of this thread are complete (not merely read out of shared memory) before the CTA ends
+    if (c_by_tma && warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   // Neither CTA leaves, or frees tensor memory, while the other may still signal its barriers or its
   // MMAs read this CTA's shared memory.
@@ -328,28 +328,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
 }
 
-int make_map_c(CUtensorMap* map, void* base, long long rows, long long cols, long long ld) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05_pair: the driver has no cuTensorMapEncodeTiled");
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  cuuint32_t box[2] = {32, 32};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05_pair: cuTensorMapEncodeTiled (output) failed with %d", (int)r);
-  return HFEE_OK;
-}
-
 template <int BN, int EPI, typename TOut>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C, long long ldc, int M, int N, int K, int* status,
                 cudaStream_t stream, const RopeEpi& rope = RopeEpi{}) {
   CUtensorMap mc = ma;
-  int reduce_by_tma = 0;
-  if (EPI == EPI_ACCUM && (uintptr_t)C % 16 == 0 && ldc % 4 == 0) {
-    int rc = make_map_c(&mc, C, M, N, ldc);
+  int c_by_tma = 0;
+  if ((EPI == EPI_ACCUM || EPI == EPI_STORE || EPI == EPI_RELU2) && mappable_out(C, N, ldc, sizeof(TOut))) {
+    int rc = make_map_out(&mc, C, M, N, ldc, sizeof(TOut));
     if (rc != HFEE_OK) return rc;
-    reduce_by_tma = 1;
+    c_by_tma = 1;
   }
   static bool configured = false;
   if (!configured) {
@@ -379,7 +366,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C, long long
     attr[2].val.sharedMemCarveout = (unsigned int)carve;
     cfg.numAttrs = 3;
   }
-  cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, EPI, TOut>, ma, mw, mc, reduce_by_tma, (TOut*)C, ldc, M, N, K, status, rope);
+  cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, EPI, TOut>, ma, mw, mc, c_by_tma, (TOut*)C, ldc, M, N, K, status, rope);
   return hfee_check_launch("gemm_tcgen05_pair");
 }
 
@@ -387,10 +374,12 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C, long long
 
 // As hfee_gemm_tcgen05 (A, W bfloat16, 16-byte aligned, leading dimensions multiples of 8; epilogue 0
 // store, 1 accumulate into float32 C, 2 SwiGLU with a bfloat16 C of N/2 columns) with pairs of CTAs on
-// tiles of 256 x 256.  `status` (device int, may be null) is set to 4 if a CTA gave up waiting.
+// tiles of 256 x 256, or, with epilogue 0 and block_n = 192, of 256 x 192.  `status` (device int, may be null) is
+// set to 4 if a CTA gave up waiting.
 HFEE_API int hfee_gemm_tcgen05_pair(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
-                                    int out_dtype, int epilogue, int M, int N, int K, int* status, cudaStream_t stream) {
+                                    int out_dtype, int epilogue, int M, int N, int K, int block_n, int* status, cudaStream_t stream) {
   if (M == 0 || N == 0) return HFEE_OK;
+  HFEE_REQUIRE(block_n == 256 || (block_n == 192 && epilogue == EPI_STORE), "gemm_tcgen05_pair: no tiles of %d columns for epilogue %d", block_n, epilogue);
   HFEE_REQUIRE(M > 0 && N > 0 && K > 0 && K % 8 == 0, "gemm_tcgen05_pair: K=%d must be a positive multiple of 8", K);
   HFEE_REQUIRE(lda % 8 == 0 && ldw % 8 == 0 && lda >= K && ldw >= K,
                "gemm_tcgen05_pair: leading dimensions (%lld, %lld) must be multiples of 8 and at least K", lda, ldw);
@@ -401,7 +390,7 @@ HFEE_API int hfee_gemm_tcgen05_pair(const void* A, long long lda, const void* W,
   CUtensorMap ma, mw;
   int rc = make_map(&ma, A, M, K, lda, BM);
   if (rc != HFEE_OK) return rc;
-  rc = make_map(&mw, W, N, K, ldw, 128);
+  rc = make_map(&mw, W, N, K, ldw, block_n / 2);
   if (rc != HFEE_OK) return rc;
   if (epilogue == EPI_ACCUM) {
     if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_tcgen05_pair: accumulate needs a float32 output");
@@ -416,6 +405,10 @@ HFEE_API int hfee_gemm_tcgen05_pair(const void* A, long long lda, const void* W,
   if (epilogue == EPI_RELU2) {
     HFEE_REQUIRE(out_dtype == HFEE_BF16, "gemm_tcgen05_pair: the relu^2 epilogue writes bfloat16");
     return launch_pair<256, EPI_RELU2, __nv_bfloat16>(ma, mw, C, ldc, M, N, K, status, stream);
+  }
+  if (block_n == 192) {
+    if (out_dtype == HFEE_BF16) return launch_pair<192, EPI_STORE, __nv_bfloat16>(ma, mw, C, ldc, M, N, K, status, stream);
+    return launch_pair<192, EPI_STORE, float>(ma, mw, C, ldc, M, N, K, status, stream);
   }
   if (out_dtype == HFEE_BF16) return launch_pair<256, EPI_STORE, __nv_bfloat16>(ma, mw, C, ldc, M, N, K, status, stream);
   return launch_pair<256, EPI_STORE, float>(ma, mw, C, ldc, M, N, K, status, stream);

@@ -114,6 +114,38 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// A chunk of 32 rows (one per lane) x 32 columns of an accumulator on its way to C: into shared memory in the swizzle the
+// tensor map of C (make_map_out) expects, 128-byte rows of float32 or 64-byte rows of bfloat16, and from there by one bulk
+// tensor copy, which writes whole rows' pieces and clips at the matrix's edges.  Stored by the lanes themselves the chunk is
+// 32 rows x 16 bytes per instruction.
+__device__ __forceinline__ void stage_chunk(float*, unsigned char* cs, int lane, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<uint4*>(cs + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+__device__ __forceinline__ void stage_chunk(__nv_bfloat16*, unsigned char* cs, int lane, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(v[8 * j + 2 * i]), __uint_as_float(v[8 * j + 2 * i + 1]));
+      o[i] = *reinterpret_cast<uint32_t*>(&p);
+    }
+    *reinterpret_cast<uint4*>(cs + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+template <bool ADD>
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src) {
+  if constexpr (ADD)
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(src)) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(src)) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 bf16) in the
 // 128-byte swizzle: 8-row groups 1024 bytes apart (stride offset), leading offset 1 (unused
 // for swizzled K-major), descriptor version 1, layout type 2 (SWIZZLE_128B).
@@ -156,6 +188,26 @@ inline int make_map(CUtensorMap* map, const void* base, long long rows, long lon
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05: cuTensorMapEncodeTiled failed with %d", (int)r);
+  return HFEE_OK;
+}
+
+// Whether bulk copies can write C [.., cols] of pitch ld: 16-byte aligned base and pitch, and whole 16-byte pieces in a row (the
+// copy clips at those, not at elements: with 4 bfloat16 columns the next 4 were overwritten).
+inline bool mappable_out(const void* base, long long cols, long long ld, int elem_bytes) {
+  return (uintptr_t)base % 16 == 0 && ld * elem_bytes % 16 == 0 && cols * elem_bytes % 16 == 0;
+}
+// Tensor map of the output for bulk stores and reductions of 32 x 32 chunks (stage_chunk).
+inline int make_map_out(CUtensorMap* map, void* base, long long rows, long long cols, long long ld, int elem_bytes) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05: the driver has no cuTensorMapEncodeTiled");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld * elem_bytes)};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t elem[2] = {1, 1};
+  CUresult r = fn(map, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides,
+                  box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, elem_bytes == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05: cuTensorMapEncodeTiled (output) failed with %d", (int)r);
   return HFEE_OK;
 }
 

@@ -6,6 +6,7 @@ CUDA device of compute capability 10.x and the built library they raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -35,7 +36,7 @@ _SIGNATURES = {
     "hfee_gemm_stream_norm": [_P, _L, _P, _P, _F, _I, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
     "hfee_gemm_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _L, _P, _P],
     "hfee_gemm_tcgen05_stream_k": [_I, _I, _I, _I, _L],
-    "hfee_gemm_tcgen05_pair": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _P],
+    "hfee_gemm_tcgen05_pair": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
     "hfee_gemm_tcgen05_rope": [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "hfee_gemm_tcgen05_rope_supports": [_I, _I],
     "hfee_gemm_skinny": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
@@ -501,22 +502,11 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
     n = w.shape[0]
     assert w.shape[1] == k and a.dtype == w.dtype == torch.bfloat16
     assert tuple(out.shape) == (m, n // 2 if epilogue in EPI_GATED else n)
-    tiles_256 = 0
     if block_n is None:
-        # wide tiles need a third less shared-memory feed per flop (a 128-wide tile's feed rate is at
-        # the L2 -> shared-memory limit); narrow ones fill the SMs when there are few tiles.  Measured
-        # at M = N = 2048 (128 wide tiles on 148 SMs): K = 8192 takes 61 us wide, 95 us narrow.
-        tiles_256 = -(-m // 128) * -(-n // 256)
-        block_n = 256 if tiles_256 >= 96 else 128
-        # 192 wide where that saves a round of tiles: 16 x 12 tiles of 256 are two rounds on 148 SMs
-        # with the second a third full, 16 x 16 tiles of 192 are two rounds of three quarters the work
-        if block_n == 256 and n % 192 == 0:
-            rounds = lambda bn: -(-(-(-m // 128) * -(-n // bn)) // sm_count())
-            if rounds(192) * 192 * 1.05 < rounds(256) * 256:
-                block_n = 192
-    if USE_PAIRS and block_n == 256 and m > 128 and tiles_256 >= 96 and (epilogue != EPI_STORE or n * k >= PAIR_STORE_MIN):
-        gemm_tcgen05_pair(a, w, out, epilogue)
-        return
+        pairs, block_n = tile_choice(m, n, sm_count(), USE_PAIRS, epilogue == EPI_STORE)
+        if pairs:
+            gemm_tcgen05_pair(a, w, out, epilogue, block_n)
+            return
     if stream_k is None:
         stream_k = USE_STREAM_K
     ws, flags = _stream_k_workspace() if stream_k else (None, None)
@@ -526,23 +516,42 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
                                  _stream()), lib)
 
 
-# Two CTAs on a tile of 256 x 256 (cta_group::2) where the single-CTA kernel would take tiles of
-# 128 x 256: measured at 2,048 tokens, gate/up of the benchmark model 102 -> 90 us (1,527 TFLOP/s), down
-# projection 57 -> 50 us, output projection 16.6 -> 17.0 us.
 USE_PAIRS = True
-PAIR_STORE_MIN = 1 << 62        # plain stores: the single-CTA kernel until measured otherwise
+# What a round of tiles takes, one on every SM (or pair of SMs), against a round of single-CTA tiles of 128 x 256.  Measured
+# with one round of each (us at K = 2,048 / 8,192 / 14,336): 128 x 128 13.5 / 40 / 64, 128 x 256 17.6 / 56 / 92, pairs of CTAs on
+# 256 x 256 16.4 / 47 / 72; tiles of 192 columns take 0.8 of those of 256 plus their fixed part.
+ROUND_128, ROUND_192, ROUND_256, ROUND_PAIR_192, ROUND_PAIR_256 = 0.72, 0.86, 1.0, 0.70, 0.85
 
 
-def gemm_tcgen05_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE) -> None:
+@functools.lru_cache(maxsize=4096)
+def tile_choice(m: int, n: int, sms: int, pairs: bool, store: bool):
+    """(pairs of CTAs?, columns of a tile) of the tcgen05 product of m rows and n columns: the kind whose rounds of tiles take
+    least, so a kind that leaves its last round nearly empty gives way to one that does not.  564 rows x 4,096 columns x K = 14,336:
+    160 tiles of 128 x 128 are two rounds on 148 SMs (190 us), 48 pair tiles one (70 us); 1,100 x 4,096 x 4,096: 80 pair tiles are
+    two rounds of 74 (44 us), 144 single tiles one (31 us).  Pairs need more than 128 rows; tiles of 192 columns are taken where
+    they divide the columns (by pairs only in plain stores)."""
+    rounds = lambda rows, cols, units: -(-(-(-m // rows) * -(-n // cols)) // units)
+    kinds = [(rounds(128, 256, sms) * ROUND_256, False, 256), (rounds(128, 128, sms) * ROUND_128, False, 128)]
+    if n % 192 == 0:
+        kinds.append((rounds(128, 192, sms) * ROUND_192, False, 192))
+    if pairs and m > 128 and sms > 1:
+        kinds.append((rounds(256, 256, sms // 2) * ROUND_PAIR_256, True, 256))
+        if n % 192 == 0 and store:
+            kinds.append((rounds(256, 192, sms // 2) * ROUND_PAIR_192, True, 192))
+    return min(kinds)[1:]
+
+
+def gemm_tcgen05_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE, block_n: int = 256) -> None:
     """:func:`gemm_tcgen05` with two CTAs on each tile of 256 x 256 (``cta_group::2``): each CTA loads
-    its own 128 rows of ``a`` and half of the tile's rows of ``w``.  Epilogues as in :func:`gemm_stream`."""
+    its own 128 rows of ``a`` and half of the tile's rows of ``w``.  Epilogues as in :func:`gemm_stream`; a plain store also
+    takes tiles of 256 x 192 (``block_n``)."""
     lib = library()
     m, k = a.shape
     n = w.shape[0]
     assert w.shape[1] == k and a.dtype == w.dtype == torch.bfloat16
     assert tuple(out.shape) == (m, n // 2 if epilogue in EPI_GATED else n)
     _check(lib.hfee_gemm_tcgen05_pair(a.data_ptr(), _rows(a, "gemm a"), w.data_ptr(), _rows(w, "gemm w"), out.data_ptr(),
-                                      _rows(out, "gemm out"), _dt(out), epilogue, m, n, k, _status().data_ptr(),
+                                      _rows(out, "gemm out"), _dt(out), epilogue, m, n, k, block_n, _status().data_ptr(),
                                       _stream()), lib)
 
 
