@@ -1,10 +1,10 @@
 // Causal grouped-query attention over the paged cache on the CUDA cores, float32
-// arithmetic, for any head size: one warp per (token, query head).
+// arithmetic, for any head size: one block of threads per (token, query head).
 //
 // The keys a token sees are the positions lo..pos of its own request, lo = 0 or
-// pos+1-window.  They are visited in blocks of 32 counted from lo with an online
-// softmax, so the result at a position depends neither on how the tokens were cut
-// into steps nor on which pages hold them.  This kernel is the attention of the
+// pos+1-window.  They are taken in blocks of 32 counted from lo, which go to PARTS parts in turn, each with an online
+// softmax of its own, and the parts are put together in their order, so the result at a position depends
+// neither on how the tokens were cut into steps nor on which pages hold them.  This kernel is the attention of the
 // true 32-bit path and the fallback of the bfloat16 path.
 //
 // Options beside the plain softmax over a causal window: `chunk` > 0 hides every key whose
@@ -23,17 +23,20 @@
 
 namespace {
 
-constexpr int WARPS = 4;
+constexpr int PARTS = 8;         // results that are put together: block b of 32 keys goes to part b mod PARTS
 constexpr int MAX_HD = 640;      // key size
 constexpr int MAX_VD = 512;      // value size
 constexpr int GATE_NONE = 0, GATE_ELEMENT = 1, GATE_PER_HEAD = 2;
 
-// Bound by the latency of its loads (a warp walks its keys alone): the key of a lane is read 16 bytes at a time where VEC says
-// that keys start on 16-byte boundaries, and the values of VALUES_AHEAD keys are requested together; DPL, the value dimensions
-// a lane owns, is the smallest that covers the value size.  The order of every sum is the one described above.
+// Bound by the latency of its loads: a block of 32 keys is one trip for the keys (a lane's key is read 16 bytes at a time where
+// VEC says that keys start on 16-byte boundaries) and the values of VALUES_AHEAD keys at a time, the first of them requested with
+// the keys.  A decode step has few (token, head) pairs, so the parts of one pair run side by side in eight warps (two
+// tokens behind prompts of 150: 15 us a layer, with one warp a pair 52); the many pairs of a prompt portion have two warps each,
+// since most of eight would have nothing to do.  DPL, the value dimensions a lane owns, is the smallest that covers
+// the value size.
 constexpr int VALUES_AHEAD = 8;
 
-template <typename T, bool SIGMOID, int DPL, bool VEC>
+template <typename T, bool SIGMOID, int DPL, bool VEC, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k_pool,
                       const T* __restrict__ v_pool, PagedCache cache, PagedCache vcache, int vd,
@@ -45,11 +48,10 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
                       const float* __restrict__ sink, int keep_first, float softcap) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ __align__(16) float q_s[WARPS][MAX_HD];
+  __shared__ __align__(16) float q_s[MAX_HD];
+  __shared__ float o_s[PARTS][DPL * 32], m_s[PARTS], l_s[PARTS];
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long task = (long long)blockIdx.x * WARPS + warp;
-  if (task >= (long long)n * heads) return;
-  int i = (int)(task / heads), h = (int)(task % heads);
+  int i = blockIdx.x / heads, h = blockIdx.x % heads;
   int hd = cache.head_dim;
   int kvh = h / (heads / cache.kv_heads);
   int pos = positions[i], slot = slot_of_token[i];
@@ -60,77 +62,100 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
   const float r1 = dist_r1 != nullptr ? dist_r1[h] : 0.f, r2 = dist_r1 != nullptr ? dist_r2[h] : 0.f;
 
   const T* qrow = q + (long long)i * ld_q + (long long)h * hd;
-  for (int d = lane; d < hd; d += 32) q_s[warp][d] = to_f32<T>(qrow[d]);
-  __syncwarp();
-
-  float o[DPL];
-#pragma unroll
-  for (int j = 0; j < DPL; ++j) o[j] = 0.f;
-  // a sink is one more term exp(sink[h]) of the denominator that has no key and no value
-  float m = (!SIGMOID && sink != nullptr) ? sink[h] : -INFINITY, l = (!SIGMOID && sink != nullptr) ? 1.f : 0.f;
+  for (int d = threadIdx.x; d < hd; d += WARPS * 32) q_s[d] = to_f32<T>(qrow[d]);
+  __syncthreads();
 
   // the first keep_first positions stay visible behind the window: they are visited first, [0, kept), then [lo, pos]
   const int kept = min(keep_first, lo);
-  for (int base = kept > 0 ? 0 : lo; base <= pos;) {
-    const int end = base < kept ? kept - 1 : pos;            // last key of the range this block of 32 lies in
-    int key = base + lane;
-    float s = -INFINITY;
-    long long v_at = 0;
-    if (key <= end) {
-      const T* kr = k_pool + paged_offset(cache, slot, key, kvh);
-      v_at = paged_offset(vcache, slot, key, kvh);
-      float acc = 0.f;
-      if constexpr (VEC) {
-#pragma unroll 8
-        for (int d = 0; d < hd; d += 4) {
-          const float4 kv = *(const float4*)(kr + d), qv = *(const float4*)(q_s[warp] + d);
-          acc = fmaf(qv.x, kv.x, acc);
-          acc = fmaf(qv.y, kv.y, acc);
-          acc = fmaf(qv.z, kv.z, acc);
-          acc = fmaf(qv.w, kv.w, acc);
-        }
-      } else {
-        for (int d = 0; d < hd; ++d) acc = fmaf(q_s[warp][d], to_f32<T>(kr[d]), acc);
-      }
-      s = acc * scale;
-      if (softcap > 0.f) s = softcap * tanhf(s / softcap);
-      if (dist_r1 != nullptr) s -= r1 * log1pf(r2 * (float)(pos - key));
-    }
-    float p;
-    if constexpr (SIGMOID) {
-      p = key <= end ? 1.f / (1.f + expf(-(s * h_scale + h_bias))) : 0.f;
-    } else {
-      float m_new = fmaxf(m, warp_max(s));
-      p = key <= end ? expf(s - m_new) : 0.f;
-      float alpha = expf(m - m_new);          // exp(-inf) = 0 on the first block
-      l = l * alpha + warp_sum(p);
+  const int front_blocks = (kept + 31) / 32, blocks = front_blocks + (pos - lo) / 32 + 1;
+  const int parts = min(PARTS, blocks);
+  float o[DPL], m = 0.f, l = 0.f;
+  for (int part = warp; part < parts; part += WARPS) {
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) o[j] *= alpha;
-      m = m_new;
-    }
-    int count = min(32, end + 1 - base);
-    for (int t0 = 0; t0 < count; t0 += VALUES_AHEAD) {
+    for (int j = 0; j < DPL; ++j) o[j] = 0.f;
+    // a sink is one more term exp(sink[h]) of the denominator that has no key and no value
+    const bool sunk = !SIGMOID && sink != nullptr && part == 0;
+    m = sunk ? sink[h] : -INFINITY;
+    l = sunk ? 1.f : 0.f;
+    for (int block = part; block < blocks; block += PARTS) {
+      const bool front = block < front_blocks;
+      const int base = front ? block * 32 : lo + (block - front_blocks) * 32;
+      const int end = front ? kept - 1 : pos;                  // last key of the range this block of 32 lies in
+      const int count = min(32, end + 1 - base);
+      const int key = base + lane;
+      const long long k_at = key <= end ? paged_offset(cache, slot, key, kvh) : 0, v_at = key <= end ? paged_offset(vcache, slot, key, kvh) : 0;
       float v[VALUES_AHEAD][DPL];
+      auto request = [&](int t0) {
 #pragma unroll
-      for (int t = 0; t < VALUES_AHEAD; ++t) {
-        const T* vr = v_pool + __shfl_sync(0xffffffffu, v_at, min(t0 + t, count - 1));
+        for (int t = 0; t < VALUES_AHEAD; ++t) {
+          const T* vr = v_pool + __shfl_sync(0xffffffffu, v_at, min(t0 + t, count - 1));
 #pragma unroll
-        for (int j = 0; j < DPL; ++j) {
-          const int d = lane + 32 * j;
-          v[t][j] = t0 + t < count && d < vd ? to_f32<T>(vr[d]) : 0.f;
+          for (int j = 0; j < DPL; ++j) {
+            const int d = lane + 32 * j;
+            v[t][j] = t0 + t < count && d < vd ? to_f32<T>(vr[d]) : 0.f;
+          }
+        }
+      };
+      request(0);
+      float s = -INFINITY;
+      if (key <= end) {
+        const T* kr = k_pool + k_at;
+        float acc = 0.f;
+        if constexpr (VEC) {
+#pragma unroll 8
+          for (int d = 0; d < hd; d += 4) {
+            const float4 kv = *(const float4*)(kr + d), qv = *(const float4*)(q_s + d);
+            acc = fmaf(qv.x, kv.x, acc);
+            acc = fmaf(qv.y, kv.y, acc);
+            acc = fmaf(qv.z, kv.z, acc);
+            acc = fmaf(qv.w, kv.w, acc);
+          }
+        } else {
+          for (int d = 0; d < hd; ++d) acc = fmaf(q_s[d], to_f32<T>(kr[d]), acc);
+        }
+        s = acc * scale;
+        if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+        if (dist_r1 != nullptr) s -= r1 * log1pf(r2 * (float)(pos - key));
+      }
+      float p;
+      if constexpr (SIGMOID) {
+        p = key <= end ? 1.f / (1.f + expf(-(s * h_scale + h_bias))) : 0.f;
+      } else {
+        float m_new = fmaxf(m, warp_max(s));
+        p = key <= end ? expf(s - m_new) : 0.f;
+        float alpha = expf(m - m_new);          // exp(-inf) = 0 on the first block
+        l = l * alpha + warp_sum(p);
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) o[j] *= alpha;
+        m = m_new;
+      }
+      for (int t0 = 0; t0 < count; t0 += VALUES_AHEAD) {
+        if (t0 > 0) request(t0);
+#pragma unroll
+        for (int t = 0; t < VALUES_AHEAD; ++t) {
+          if (t0 + t >= count) break;
+          const float pt = __shfl_sync(0xffffffffu, p, t0 + t);
+#pragma unroll
+          for (int j = 0; j < DPL; ++j) o[j] = fmaf(pt, v[t][j], o[j]);
         }
       }
-#pragma unroll
-      for (int t = 0; t < VALUES_AHEAD; ++t) {
-        if (t0 + t >= count) break;
-        const float pt = __shfl_sync(0xffffffffu, p, t0 + t);
-#pragma unroll
-        for (int j = 0; j < DPL; ++j) o[j] = fmaf(pt, v[t][j], o[j]);
-      }
     }
-    const bool front = base < kept;
-    base += 32;
-    if (front && base >= kept) base = lo;
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) o_s[part][lane + 32 * j] = o[j];
+    if (lane == 0) { m_s[part] = m; l_s[part] = l; }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  m = m_s[0];
+  for (int w = 1; w < parts; ++w) m = fmaxf(m, m_s[w]);
+  l = 0.f;
+#pragma unroll
+  for (int j = 0; j < DPL; ++j) o[j] = 0.f;
+  for (int w = 0; w < parts; ++w) {
+    const float share = SIGMOID ? 1.f : expf(m_s[w] - m);
+    l += l_s[w] * share;
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) o[j] = fmaf(o_s[w][lane + 32 * j], share, o[j]);
   }
   T* orow = out + (long long)i * ld_o + (long long)h * vd;
   float inv = (SIGMOID ? 1.f : 1.f / l) * out_scale;
@@ -156,11 +181,14 @@ void launch_one(const void* q, int ld_q, const void* k_pool, const void* v_pool,
                 int window, int chunk, const float* head_scale, const float* head_bias, const void* gate, long long ld_gate,
                 int gate_mode, const float* dist_r1, const float* dist_r2, float out_scale, const float* sink, int keep_first,
                 float softcap, cudaStream_t stream) {
-  long long tasks = (long long)n * heads;
-  unsigned blocks = (unsigned)((tasks + WARPS - 1) / WARPS);
-  hfee_launch(attention_simt_kernel<T, SIGMOID, DPL, VEC>, dim3(blocks), dim3(WARPS * 32), 0, stream, (const T*)q, ld_q, (const T*)k_pool,
-              (const T*)v_pool, c, vc, vd, positions, slot_of_token, (T*)out, ld_o, n, heads, scale, window, chunk, head_scale,
-              head_bias, (const T*)gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first, softcap);
+  auto run = [&](auto warps) {
+    constexpr int WARPS = decltype(warps)::value;
+    hfee_launch(attention_simt_kernel<T, SIGMOID, DPL, VEC, WARPS>, dim3((unsigned)n * (unsigned)heads), dim3(WARPS * 32), 0, stream, (const T*)q,
+                ld_q, (const T*)k_pool, (const T*)v_pool, c, vc, vd, positions, slot_of_token, (T*)out, ld_o, n, heads, scale, window, chunk,
+                head_scale, head_bias, (const T*)gate, ld_gate, gate_mode, dist_r1, dist_r2, out_scale, sink, keep_first, softcap);
+  };
+  if ((long long)n * heads <= 8LL * hfee_sm_count()) run(std::integral_constant<int, 8>{});      // a full SM holds eight such blocks
+  else run(std::integral_constant<int, 2>{});
 }
 
 template <typename T, bool SIGMOID, typename... Args>

@@ -45,9 +45,10 @@ extern "C" int hfee_sm_count();
 int hfee_pdl_enabled();
 int hfee_carveout();
 
+// carve: the split between shared memory and L1 to ask for (percent), below 0 for the driver's choice.
 template <typename... KArgs, typename... Args>
-cudaError_t hfee_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                        Args&&... args) {
+cudaError_t hfee_launch_carved(int carve, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -58,13 +59,17 @@ cudaError_t hfee_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
   attr[0].val.programmaticStreamSerializationAllowed = hfee_pdl_enabled();
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const int carve = hfee_carveout();
   if (carve >= 0) {
     attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
     attr[1].val.sharedMemCarveout = (unsigned int)carve;
     cfg.numAttrs = 2;
   }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t hfee_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                        Args&&... args) {
+  return hfee_launch_carved(hfee_carveout(), kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 
 // Paged cache addressing shared by every kernel that touches the cache.

@@ -2,9 +2,13 @@
 //
 // This is the matrix product of the true 32-bit path (no tensor cores, no
 // reduced-precision mode) and the fallback of the bfloat16 path for shapes the
-// tensor-core kernels refuse.  Every output element is the sum over k = 0..K-1 in
-// that order, whatever M is and whichever of the kernels below runs, so a row's result does
-// not depend on the batch.
+// tensor-core kernels refuse.  Every output element is summed in one order, whatever M is and whichever of
+// the kernels below runs, so a row's result does not depend on the batch: K is cut into segments of SEG, a segment is
+// two chains of fused multiply-adds, over its even and over its odd k, and the segments' sums (even + odd) are added in their
+// order.  One chain over all of K would take 4 clocks for each k (17 us at K = 8,192, whatever the number of warps); segments
+// can run side by side, the sums of shorter chains are closer to the exact ones, and two neighbouring k lie as the pair that
+// the packed multiply-add takes: single FFMA issue at half of the rate on this chip (a 64-row tile that did nothing else stopped at
+// 29 TFLOP/s).
 //
 // Three kernels.  float32 operands whose rows start on 16-byte boundaries take `gemm_rows_kernel` (at most
 // ROWS_MAX_M tokens) or `gemm_tiles_kernel` (more); bfloat16 operands and other alignments take `gemm_simt_kernel`.
@@ -16,6 +20,7 @@
 namespace {
 
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, THREADS = 256;
+constexpr int SEG = 512;        // k of a segment; a multiple of every kernel's piece of K
 
 template <typename T>
 __device__ __forceinline__ float load_guarded(const T* p, long long ld, int r, int c, int rows, int cols) {
@@ -34,11 +39,11 @@ gemm_simt_kernel(const TIn* __restrict__ A, long long lda, const TIn* __restrict
   int tid = threadIdx.x;
   int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   int tr = tid / (BN / TN), tc = tid % (BN / TN);   // 16 x 16 thread grid
-  float acc[TM][TN];
+  float acc[2][TM][TN], sum[TM][TN];    // of this segment (even and odd k), of the segments before it
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = sum[i][j] = 0.f;
 
   // each thread stages 4 consecutive k of one row of A and one row of W
   int lr = tid / (BK / 4), lk = (tid % (BK / 4)) * 4;   // 64 rows x 4 groups
@@ -59,9 +64,14 @@ gemm_simt_kernel(const TIn* __restrict__ A, long long lda, const TIn* __restrict
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
     }
     __syncthreads();
+    if ((k0 + BK) % SEG == 0 || k0 + BK >= K)
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) { sum[i][j] += acc[0][i][j] + acc[1][i][j]; acc[0][i][j] = acc[1][i][j] = 0.f; }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -72,8 +82,8 @@ gemm_simt_kernel(const TIn* __restrict__ A, long long lda, const TIn* __restrict
       int c = n0 + tc * TN + j;
       if (c >= N) continue;
       long long o = (long long)r * ldc + c;
-      if constexpr (ACCUM) C[o] = to_f32<TOut>(C[o]) + acc[i][j];
-      else C[o] = from_f32<TOut>(acc[i][j]);
+      if constexpr (ACCUM) C[o] = to_f32<TOut>(C[o]) + sum[i][j];
+      else C[o] = from_f32<TOut>(sum[i][j]);
     }
   }
 }
@@ -82,236 +92,285 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Two float32 multiply-adds, of the low and of the high halves.
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float halves(unsigned long long v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// A decode step of the 32-bit path.  Bound by the bytes of W (each read once) and, for long rows, by the chain of K
-// dependent additions that one output is (4 clocks each: 17 us at K = 8,192): so an output is one lane's, and what is
-// left to do is to keep the loads running.  One warp per CTA owns 16 rows of W (lane & 15) and two groups of TPL tokens
-// (lane >> 4), and has its own ring of STAGES pieces [16 rows + tokens][KT], filled by 16-byte asynchronous copies; N =
-// 2,048 then gives 128 SMs a warp each, N = 16,384 seven.  Rows are KT + 4 floats apart, so that eight lanes' 16-byte
-// reads fall into different banks.  W does not depend on the kernel in front: its first pieces are requested before the
-// wait for it.  Llama-3.2-1B layer sizes at two tokens: o + down projection 74 us a layer against 797 us with the general
-// kernel's 64-row tiles.
-template <int TPL, int KT, int STAGES, typename TOut, bool ACCUM>
-__global__ void __launch_bounds__(32)
+// A decode step of the 32-bit path, bound by the bytes of W (each read once).  A CTA owns 16 rows of W; its warps take the
+// segments of K in turn, each with its own ring of STAGES pieces [16 rows + tokens][KT] that 16-byte asynchronous copies fill,
+// and lane l sums row l & 15 with TPL tokens (l >> 4, l >> 4 + 2, ..).  After every round of one segment a warp the sums meet in
+// shared memory and warp 0 adds them in the segments' order.  Rows are KT + 4 floats apart, so that eight lanes' 16-byte reads
+// fall into different banks.  W does not depend on the kernel in front: its first pieces are requested before the wait for it.
+// 1B layer sizes at two tokens, a warp for each segment against one for all of K: o + down projection 23.6 against 73 us a layer
+// (the chain of 8,192 additions alone is 17; the bytes 13), q/k/v + gate/up 39 against 53 us (25).
+constexpr int ROWS_KT = 32, ROWS_STAGES = 4;
+
+template <int TPL, int WARPS, typename TOut, bool ACCUM>
+__global__ void __launch_bounds__(WARPS * 32)
 gemm_rows_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw,
                  TOut* __restrict__ C, long long ldc, int M, int N, int K) {
-  constexpr int LD = KT + 4, CHUNKS = KT / 4, STAGE = (16 + 2 * TPL) * LD;
-  extern __shared__ __align__(16) float ring[];
-  const int lane = threadIdx.x, row = lane & 15, g = lane >> 4;
-  const int n0 = blockIdx.x * 16, steps = (K + KT - 1) / KT;
+  constexpr int KT = ROWS_KT, STAGES = ROWS_STAGES, LD = KT + 4, CHUNKS = KT / 4, STAGE = (16 + 2 * TPL) * LD, PIECES = SEG / KT;
+  extern __shared__ __align__(16) float rows_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane & 15, g = lane >> 4;
+  float* ring = rows_smem + warp * (STAGES * STAGE);
+  float* parts = rows_smem + WARPS * (STAGES * STAGE);            // [2][WARPS][TPL][32]
+  const int n0 = blockIdx.x * 16;
+  const int rounds = (K + SEG * WARPS - 1) / (SEG * WARPS), steps = rounds * PIECES;
 
+  auto first_k = [&](int step) { return ((step / PIECES) * WARPS + warp) * SEG + (step % PIECES) * KT; };
   auto load_w = [&](int step) {
     float* dst = ring + (step % STAGES) * STAGE;
+    const int k0 = first_k(step);
 #pragma unroll
     for (int i = 0; i < 16 * CHUNKS / 32; ++i) {
       const int c = lane + 32 * i, r = c / CHUNKS, k = (c % CHUNKS) * 4;
-      if (step * KT + k < K) cp_async16(dst + r * LD + k, W + (long long)min(n0 + r, N - 1) * ldw + step * KT + k);
+      if (k0 + k < K) cp_async16(dst + r * LD + k, W + (long long)min(n0 + r, N - 1) * ldw + k0 + k);
     }
   };
-#pragma unroll 1
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < steps) load_w(s);
-    cp_async_commit();
-  }
-  pdl_wait();
-  pdl_launch_dependents();
-  for (int s = 0; s < min(STAGES - 1, steps); ++s)
+  auto load_a = [&](int step) {
+    float* dst = ring + (step % STAGES) * STAGE + 16 * LD;
+    const int k0 = first_k(step);
     for (int c = lane; c < M * CHUNKS; c += 32) {
       const int r = c / CHUNKS, k = (c % CHUNKS) * 4;
-      if (s * KT + k < K)
-        *(float4*)(ring + s * STAGE + (16 + r) * LD + k) = *(const float4*)(A + (long long)r * lda + s * KT + k);
+      if (k0 + k < K) cp_async16(dst + r * LD + k, A + (long long)r * lda + k0 + k);
     }
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) load_w(s);
+  pdl_wait();
+  pdl_launch_dependents();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    load_a(s);
+    cp_async_commit();
+  }
 
-  float acc[TPL];
+  unsigned long long acc[TPL];
+  float sum[TPL];
 #pragma unroll
-  for (int t = 0; t < TPL; ++t) acc[t] = 0.f;
+  for (int t = 0; t < TPL; ++t) { acc[t] = 0; sum[t] = 0.f; }
   auto four = [&](const float* wr, const float* xr, int k) {
-    const float4 w = *(const float4*)(wr + k);
-    float4 x[TPL];
+    const ulonglong2 w = *(const ulonglong2*)(wr + k);
+    ulonglong2 x[TPL];
 #pragma unroll
-    for (int t = 0; t < TPL; ++t) x[t] = *(const float4*)(xr + 2 * t * LD + k);
+    for (int t = 0; t < TPL; ++t) x[t] = *(const ulonglong2*)(xr + 2 * t * LD + k);
 #pragma unroll
-    for (int t = 0; t < TPL; ++t) acc[t] = fmaf(x[t].x, w.x, acc[t]);
+    for (int t = 0; t < TPL; ++t) fma2(acc[t], x[t].x, w.x);
 #pragma unroll
-    for (int t = 0; t < TPL; ++t) acc[t] = fmaf(x[t].y, w.y, acc[t]);
-#pragma unroll
-    for (int t = 0; t < TPL; ++t) acc[t] = fmaf(x[t].z, w.z, acc[t]);
-#pragma unroll
-    for (int t = 0; t < TPL; ++t) acc[t] = fmaf(x[t].w, w.w, acc[t]);
+    for (int t = 0; t < TPL; ++t) fma2(acc[t], x[t].y, w.y);
   };
 #pragma unroll 1
   for (int step = 0; step < steps; ++step) {
     cp_async_wait<STAGES - 2>();
     __syncwarp();                               // this piece is everybody's; the piece before it has been read by all
-    const int next = step + STAGES - 1;
-    if (next < steps) {
-      load_w(next);
-      float* dst = ring + (next % STAGES) * STAGE + 16 * LD;
-      for (int c = lane; c < M * CHUNKS; c += 32) {
-        const int r = c / CHUNKS, k = (c % CHUNKS) * 4;
-        if (next * KT + k < K) cp_async16(dst + r * LD + k, A + (long long)r * lda + next * KT + k);
-      }
+    if (step + STAGES - 1 < steps) {
+      load_w(step + STAGES - 1);
+      load_a(step + STAGES - 1);
     }
     cp_async_commit();
     const float* wr = ring + (step % STAGES) * STAGE + row * LD;
     const float* xr = ring + (step % STAGES) * STAGE + (16 + g) * LD;
-    const int left = K - step * KT;
+    const int left = K - first_k(step);
     if (left >= KT) {
 #pragma unroll
       for (int k = 0; k < KT; k += 4) four(wr, xr, k);
     } else {
       for (int k = 0; k < left; k += 4) four(wr, xr, k);
     }
+    if (step % PIECES == PIECES - 1) {          // the round's segments are done; the buffer before last is free again by now
+      const int round = step / PIECES;
+      float* mine = parts + (round & 1) * (WARPS * TPL * 32);
+#pragma unroll
+      for (int t = 0; t < TPL; ++t) { mine[(warp * TPL + t) * 32 + lane] = halves(acc[t]); acc[t] = 0; }
+      __syncthreads();
+      if (warp == 0)
+        for (int w = 0; w < WARPS && (round * WARPS + w) * SEG < K; ++w)
+#pragma unroll
+          for (int t = 0; t < TPL; ++t) sum[t] += mine[(w * TPL + t) * 32 + lane];
+    }
   }
   const int n = n0 + row;
+  if (warp != 0 || n >= N) return;
 #pragma unroll
   for (int t = 0; t < TPL; ++t) {
     const int m = g + 2 * t;
-    if (m >= M || n >= N) continue;
+    if (m >= M) continue;
     const long long o = (long long)m * ldc + n;
-    if constexpr (ACCUM) C[o] = to_f32<TOut>(C[o]) + acc[t];
-    else C[o] = from_f32<TOut>(acc[t]);
+    if constexpr (ACCUM) C[o] = to_f32<TOut>(C[o]) + sum[t];
+    else C[o] = from_f32<TOut>(sum[t]);
   }
 }
 
-// Prompts of the 32-bit path, bound by the FFMA rate (128 a clock and SM).  A thread owns TM x TN outputs whose rows and
-// columns lie RG and CG apart, so that a warp's 16-byte reads (four k at once) touch 4 and 8 neighbouring rows of the
-// tiles, KT + 4 floats apart: no bank is hit twice, and 8 reads feed 64 FFMA.  Tiles come in by 16-byte asynchronous
-// copies STAGES - 1 blocks ahead.  M tiles run fastest over the grid, so that a W tile is read from L2 by its row tiles.
-// The four products of a 1B layer at 278 tokens: 1,220 us.
-template <int BM_, int BN_, int TM_, int TN_, typename TOut, bool ACCUM>
-__global__ void __launch_bounds__((BM_ / TM_) * (BN_ / TN_))
+// Prompts of the 32-bit path, bound by the FFMA rate (128 a clock and SM) and, right behind it, by shared memory, which gives a
+// lane 4 bytes a clock: a thread with a x b outputs needs a + b floats for a b / 4 clocks of FFMA, so 8 x 8 is the smallest
+// square that keeps up (4 x 4 stopped at 42 % of the rate).  A warp owns a whole tile of 32 x 64 outputs over one segment of K,
+// with its own ring of pieces filled by 16-byte asynchronous copies, and the four warps of a CTA take the segments of the same
+// tile in turn: short prompts have few tiles, and this way each fills an SM's four schedulers.  After every round the sums of
+// the four meet in shared memory, a quarter of the outputs at a time, and are added in the segments' order; each warp keeps
+// the running sums of its quarter.  The next pair of k is read while one is multiplied, and two CTAs share an SM, for which the
+// launch asks for all of its shared memory: with the step's carve-out one CTA fits, and its four warps stop at 25 TFLOP/s.
+// The four products of a 1B layer at 285 tokens: 954 us, with tiles of 32 x 64 and 4 x 4 a thread 1,220.  8 x 16 a thread spills.
+// A thread's rows lie 4 and its columns 8 apart, rows of a piece KT + 4 floats: no bank is hit
+// twice.  M tiles run fastest over the grid, so that a W tile is read from L2 by its row tiles.
+constexpr int TILE_M = 32, TILE_N = 64, TILE_KT = 16, TILE_STAGES = 3, TILE_WARPS = 4;
+constexpr int TILE_LD = TILE_KT + 4, TILE_STAGE = (TILE_M + TILE_N) * TILE_LD;
+constexpr int TILES_SMEM = (TILE_WARPS * TILE_STAGES * TILE_STAGE + TILE_WARPS * 16 * 32) * 4;
+
+template <typename TOut, bool ACCUM>
+__global__ void __launch_bounds__(TILE_WARPS * 32, 2)
 gemm_tiles_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W, long long ldw,
                   TOut* __restrict__ C, long long ldc, int M, int N, int K, int m_tiles) {
-  constexpr int KT = 32, STAGES = 3, LD = KT + 4, CHUNKS = KT / 4, RG = BM_ / TM_, CG = BN_ / TN_, NT = RG * CG;
-  constexpr int STAGE = (BM_ + BN_) * LD;
-  static_assert(RG % 4 == 0 && CG % 8 == 0 && (BM_ * CHUNKS) % NT == 0 && (BN_ * CHUNKS) % NT == 0, "tile");
-  extern __shared__ __align__(16) float ring[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tr = (warp / (CG / 8)) * 4 + (lane >> 3), tc = (warp % (CG / 8)) * 8 + (lane & 7);
-  const int m0 = (blockIdx.x % m_tiles) * BM_, n0 = (blockIdx.x / m_tiles) * BN_;
-  const int steps = (K + KT - 1) / KT;
-  auto load_rows = [&](const float* src, long long ld, int first, int rows, int step, float* dst, auto count) {
+  constexpr int KT = TILE_KT, STAGES = TILE_STAGES, LD = TILE_LD, STAGE = TILE_STAGE, CHUNKS = KT / 4, PIECES = SEG / KT, WARPS = TILE_WARPS;
+  extern __shared__ __align__(16) float tiles_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tr = lane >> 3, tc = lane & 7;
+  float* ring = tiles_smem + warp * (STAGES * STAGE);
+  float* parts = tiles_smem + WARPS * (STAGES * STAGE);           // [WARPS][16][32]
+  const int m0 = (blockIdx.x % m_tiles) * TILE_M, n0 = (blockIdx.x / m_tiles) * TILE_N;
+  const int rounds = (K + SEG * WARPS - 1) / (SEG * WARPS), steps = rounds * PIECES;
+
+  auto first_k = [&](int step) { return ((step / PIECES) * WARPS + warp) * SEG + (step % PIECES) * KT; };
+  const int lr = lane / CHUNKS, lk = (lane % CHUNKS) * 4;          // 8 rows of a piece an instruction
+  auto load_w = [&](int step) {
+    float* dst = ring + (step % STAGES) * STAGE + (TILE_M + lr) * LD + lk;
+    const int k = first_k(step) + lk;
+    if (k < K)
 #pragma unroll
-    for (int i = 0; i < decltype(count)::value * CHUNKS / NT; ++i) {
-      const int c = tid + NT * i, r = c / CHUNKS, k = (c % CHUNKS) * 4;
-      if (step * KT + k < K) cp_async16(dst + r * LD + k, src + (long long)min(first + r, rows - 1) * ld + step * KT + k);
-    }
+      for (int i = 0; i < TILE_N / 8; ++i) cp_async16(dst + i * 8 * LD, W + (long long)min(n0 + lr + i * 8, N - 1) * ldw + k);
   };
-  auto load_w = [&](int s) { load_rows(W, ldw, n0, N, s, ring + (s % STAGES) * STAGE + BM_ * LD, std::integral_constant<int, BN_>{}); };
-  auto load_a = [&](int s) { load_rows(A, lda, m0, M, s, ring + (s % STAGES) * STAGE, std::integral_constant<int, BM_>{}); };
-  for (int s = 0; s < min(STAGES - 1, steps); ++s) load_w(s);
+  auto load_a = [&](int step) {
+    float* dst = ring + (step % STAGES) * STAGE + lr * LD + lk;
+    const int k = first_k(step) + lk;
+    if (k < K)
+#pragma unroll
+      for (int i = 0; i < TILE_M / 8; ++i) cp_async16(dst + i * 8 * LD, A + (long long)min(m0 + lr + i * 8, M - 1) * lda + k);
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) load_w(s);
   pdl_wait();
   pdl_launch_dependents();
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < steps) load_a(s);
+    load_a(s);
     cp_async_commit();
   }
-  float acc[TM_][TN_];
+  unsigned long long acc[8][8];
+  float sum[16];                                // sum: this warp's quarter, acc's rows 2 warp and 2 warp + 1 of every lane
 #pragma unroll
-  for (int i = 0; i < TM_; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < TN_; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) sum[e] = 0.f;
 #pragma unroll 1
   for (int step = 0; step < steps; ++step) {
     cp_async_wait<STAGES - 2>();
-    __syncthreads();
+    __syncwarp();
     if (step + STAGES - 1 < steps) {
       load_w(step + STAGES - 1);
       load_a(step + STAGES - 1);
     }
     cp_async_commit();
     const float* as = ring + (step % STAGES) * STAGE + tr * LD;
-    const float* ws = ring + (step % STAGES) * STAGE + (BM_ + tc) * LD;
-    const int count = min(KT, K - step * KT);
-#pragma unroll 2
-    for (int k = 0; k < count; k += 4) {
-      float4 a[TM_], b[TN_];
+    const float* ws = ring + (step % STAGES) * STAGE + (TILE_M + tc) * LD;
+    unsigned long long a[2][8], b[2][8];          // the pairs of k being multiplied and the next ones
+    auto read = [&](int buf, int k) {
 #pragma unroll
-      for (int i = 0; i < TM_; ++i) a[i] = *(const float4*)(as + i * RG * LD + k);
+      for (int i = 0; i < 8; ++i) a[buf][i] = *(const unsigned long long*)(as + i * 4 * LD + k);
 #pragma unroll
-      for (int j = 0; j < TN_; ++j) b[j] = *(const float4*)(ws + j * CG * LD + k);
+      for (int j = 0; j < 8; ++j) b[buf][j] = *(const unsigned long long*)(ws + j * 8 * LD + k);
+    };
+    auto multiply = [&](int buf) {
 #pragma unroll
-      for (int i = 0; i < TM_; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < TN_; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+        for (int j = 0; j < 8; ++j) fma2(acc[i][j], a[buf][i], b[buf][j]);
+    };
+    const int left = K - first_k(step);
+    if (left >= KT) {
+      read(0, 0);
 #pragma unroll
-      for (int i = 0; i < TM_; ++i)
+      for (int k = 0; k < KT; k += 2) {
+        if (k + 2 < KT) read((k / 2 + 1) & 1, k + 2);
+        multiply((k / 2) & 1);
+      }
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < left; k += 2) {
+        read(0, k);
+        multiply(0);
+      }
+    }
+    if (step % PIECES == PIECES - 1) {          // the round's segments are done
+      const int live = min(WARPS, (K - (step / PIECES) * WARPS * SEG + SEG - 1) / SEG);
 #pragma unroll
-        for (int j = 0; j < TN_; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+      for (int q = 0; q < WARPS; ++q) {         // the outputs whose sums warp q keeps
+        __syncthreads();
 #pragma unroll
-      for (int i = 0; i < TM_; ++i)
+        for (int e = 0; e < 16; ++e) parts[(warp * 16 + e) * 32 + lane] = halves(acc[2 * q + e / 8][e % 8]);
+        __syncthreads();
+        if (warp == q)
+          for (int w = 0; w < live; ++w)
 #pragma unroll
-        for (int j = 0; j < TN_; ++j) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+            for (int e = 0; e < 16; ++e) sum[e] += parts[(w * 16 + e) * 32 + lane];
+      }
 #pragma unroll
-      for (int i = 0; i < TM_; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < TN_; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0;
     }
   }
 #pragma unroll
-  for (int i = 0; i < TM_; ++i) {
-    const int m = m0 + tr + i * RG;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN_; ++j) {
-      const int n = n0 + tc + j * CG;
-      if (n >= N) continue;
-      const long long o = (long long)m * ldc + n;
-      if constexpr (ACCUM) C[o] = to_f32<TOut>(C[o]) + acc[i][j];
-      else C[o] = from_f32<TOut>(acc[i][j]);
-    }
+  for (int e = 0; e < 16; ++e) {
+    const int m = m0 + tr + (2 * warp + e / 8) * 4, n = n0 + tc + (e % 8) * 8;
+    if (m >= M || n >= N) continue;
+    const long long o = (long long)m * ldc + n;
+    if constexpr (ACCUM) C[o] = to_f32<TOut>(C[o]) + sum[e];
+    else C[o] = from_f32<TOut>(sum[e]);
   }
 }
 
 constexpr int ROWS_MAX_M = 16;
 
-template <int TPL, int KT, int STAGES, typename TOut, bool ACCUM>
-int launch_rows(const float* A, long long lda, const float* W, long long ldw, TOut* C, long long ldc, int M, int N, int K,
-                cudaStream_t stream) {
-  constexpr int smem = STAGES * (16 + 2 * TPL) * (KT + 4) * 4;
-  static_assert(smem <= 48 * 1024, "the ring fits without an opt-in");
-  hfee_launch(gemm_rows_kernel<TPL, KT, STAGES, TOut, ACCUM>, dim3((N + 15) / 16), dim3(32), smem, stream, A, lda, W, ldw, C, ldc,
+template <int TPL, int WARPS, typename TOut, bool ACCUM>
+int launch_rows_of(const float* A, long long lda, const float* W, long long ldw, TOut* C, long long ldc, int M, int N, int K,
+                   cudaStream_t stream) {
+  constexpr int smem = WARPS * (ROWS_STAGES * (16 + 2 * TPL) * (ROWS_KT + 4) + 2 * TPL * 32) * 4;
+  static const cudaError_t opted = cudaFuncSetAttribute(gemm_rows_kernel<TPL, WARPS, TOut, ACCUM>,
+                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (opted != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its rings");
+  hfee_launch(gemm_rows_kernel<TPL, WARPS, TOut, ACCUM>, dim3((N + 15) / 16), dim3(WARPS * 32), smem, stream, A, lda, W, ldw, C, ldc,
               M, N, K);
   return hfee_check_launch("gemm_simt rows");
 }
 
-template <int BM_, int BN_, int TM_, int TN_, typename TOut, bool ACCUM>
-int launch_tiles(const float* A, long long lda, const float* W, long long ldw, TOut* C, long long ldc, int M, int N, int K,
-                 cudaStream_t stream) {
-  constexpr int smem = 3 * (BM_ + BN_) * 36 * 4;
-  static const cudaError_t opted = cudaFuncSetAttribute(gemm_tiles_kernel<BM_, BN_, TM_, TN_, TOut, ACCUM>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (opted != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its tiles");
-  const int m_tiles = (M + BM_ - 1) / BM_;
-  const long long tiles = (long long)m_tiles * ((N + BN_ - 1) / BN_);
-  HFEE_REQUIRE(tiles <= 0x7fffffff, "gemm_simt: M=%d N=%d are too large", M, N);
-  hfee_launch(gemm_tiles_kernel<BM_, BN_, TM_, TN_, TOut, ACCUM>, dim3((unsigned)tiles), dim3((BM_ / TM_) * (BN_ / TN_)), smem, stream,
-              A, lda, W, ldw, C, ldc, M, N, K, m_tiles);
-  return hfee_check_launch("gemm_simt tiles");
+// As many warps as there are segments, up to eight.
+template <int TPL, typename TOut, bool ACCUM>
+int launch_rows(const float* A, long long lda, const float* W, long long ldw, TOut* C, long long ldc, int M, int N, int K,
+                cudaStream_t stream) {
+  if (K <= SEG) return launch_rows_of<TPL, 1, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  if (K <= 4 * SEG) return launch_rows_of<TPL, 4, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  return launch_rows_of<TPL, 8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
 }
 
 template <typename TOut, bool ACCUM>
 int launch_f32(const float* A, long long lda, const float* W, long long ldw, TOut* C, long long ldc, int M, int N, int K,
                cudaStream_t stream) {
   // Up to ROWS_MAX_M tokens the bytes of W bound the product; TPL tokens a lane cost TPL FFMA per weight.
-  if (M <= 2) return launch_rows<1, 64, 8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  if (M <= 4) return launch_rows<2, 64, 8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  if (M <= 8) return launch_rows<4, 64, 7, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  if (M <= ROWS_MAX_M) return launch_rows<8, 32, 8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  // The tile that needs the least time: rounds over the SMs x outputs x what an output costs with that tile (more reads of
-  // shared memory per FFMA in the smaller ones).
-  const int sms = hfee_sm_count() > 0 ? hfee_sm_count() : 1;
-  auto cost = [&](int bm, int bn, double each) {
-    const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-    return (double)((tiles + sms - 1) / sms) * bm * bn * each;
-  };
-  const double small = cost(32, 64, 1.25), middle = cost(64, 128, 1.08), large = cost(128, 128, 1.0);
-  if (small <= middle && small <= large) return launch_tiles<32, 64, 4, 4, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  if (middle <= large) return launch_tiles<64, 128, 8, 4, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  return launch_tiles<128, 128, 8, 8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  if (M <= 2) return launch_rows<1, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  if (M <= 4) return launch_rows<2, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  if (M <= 8) return launch_rows<4, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  if (M <= ROWS_MAX_M) return launch_rows<8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+  static const cudaError_t opted = cudaFuncSetAttribute(gemm_tiles_kernel<TOut, ACCUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILES_SMEM);
+  if (opted != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its tiles");
+  const int m_tiles = (M + TILE_M - 1) / TILE_M;
+  const long long tiles = (long long)m_tiles * ((N + TILE_N - 1) / TILE_N);
+  HFEE_REQUIRE(tiles <= 0x7fffffff, "gemm_simt: M=%d N=%d are too large", M, N);
+  hfee_launch_carved(100, gemm_tiles_kernel<TOut, ACCUM>, dim3((unsigned)tiles), dim3(TILE_WARPS * 32), TILES_SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K,
+              m_tiles);
+  return hfee_check_launch("gemm_simt tiles");
 }
 
 template <typename TIn>

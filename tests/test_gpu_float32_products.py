@@ -1,4 +1,4 @@
-"""The float32 product's kernels (a warp per 16 rows of the weights, three tile sizes, the general kernel) add in one order:
+"""The float32 product's kernels (16 rows of the weights a block, tiles, the general kernel) add in one order, segment by segment of 512:
 every output element is the same bits whichever of them runs."""
 import pytest
 import torch
@@ -20,9 +20,10 @@ def _shifted(t):
     return wide[:, 1:]
 
 
-# token counts around every change of kernel (2, 4, 8, 16) and of tile (32, 64, 128), widths around a warp's 16 rows and a
-# tile's 64 and 128, depths below, at and past a piece of 64 and of 32
-@pytest.mark.parametrize("n,k", [(1, 4), (16, 60), (17, 64), (130, 100), (2500, 36), (300, 2052), (20000, 8)])
+# token counts around every change of kernel (2, 4, 8, 16) and tile (32), widths around a warp's 16 rows and a
+# tile's 64, depths below, at and past a piece, a segment (512) and a round of segments (2,048, 4,096)
+@pytest.mark.parametrize("n,k", [(1, 4), (16, 60), (17, 64), (130, 100), (2500, 36), (300, 2052), (20000, 8), (40, 512), (40, 516),
+                                 (48, 8200)])
 def test_every_kernel_gives_the_same_bits(ops, n, k):
     g = torch.Generator().manual_seed(n + k)
     w = torch.randn(n, k, generator=g).cuda()
