@@ -343,24 +343,60 @@ moe_expert_kernel(const T* __restrict__ a, long long ld_a, int top, const T* __r
   }
 }
 
+// Bound by its bytes for a prompt and by one trip to memory for a decode step: a thread owns VEC neighbouring columns of a token, so
+// that a step of two tokens is four blocks of 256 threads (one block a token, a column at a time: 7.7 us in a decode step of
+// three tokens), and asks for everything of COMBINE_AHEAD experts before it adds, in their order.
+constexpr int COMBINE_AHEAD = 4;
+
+template <int VEC>
 __global__ void __launch_bounds__(THREADS)
 moe_combine_kernel(const float* __restrict__ pair_out, const float* __restrict__ weight, const int* __restrict__ place, int top,
                    float* __restrict__ y, int width, int accumulate,      // place: the row of each pair (null: the pair's index)
                    const float* __restrict__ extra, const float* __restrict__ extra_gate, long long ld_gate) {
   pdl_wait();
   pdl_launch_dependents();
-  const long long t = blockIdx.x;
-  // extra [n, width]: one more term per token (an expert every token uses), times sigmoid(extra_gate[t * ld_gate])
-  const float eg = extra != nullptr ? (extra_gate != nullptr ? 1.f / (1.f + expf(-extra_gate[t * ld_gate])) : 1.f) : 0.f;
-  for (int c = threadIdx.x; c < width; c += THREADS) {
-    float acc = accumulate ? y[t * width + c] : 0.f;
-    if (extra != nullptr) acc = fmaf(eg, extra[t * width + c], acc);
-    for (int k = 0; k < top; ++k) {
-      const long long row = place ? place[t * top + k] : t * top + k;
-      acc = fmaf(weight[t * top + k], pair_out[row * width + c], acc);
+  const long long t = blockIdx.y;
+  const int c = (blockIdx.x * THREADS + threadIdx.x) * VEC;
+  if (c >= width) return;
+  auto read = [](const float* p, float (&v)[VEC]) {
+    if constexpr (VEC == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+      v[0] = *p;
     }
-    y[t * width + c] = acc;
+  };
+  float acc[VEC], more[VEC], term[COMBINE_AHEAD][VEC], share[COMBINE_AHEAD];
+  auto request = [&](int k0) {
+#pragma unroll
+    for (int k = 0; k < COMBINE_AHEAD; ++k)
+      if (k0 + k < top) {
+        const long long pair = t * top + k0 + k;
+        share[k] = weight[pair];
+        read(pair_out + (place ? place[pair] : pair) * (long long)width + c, term[k]);
+      }
+  };
+  request(0);
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
+  if (accumulate) read(y + t * width + c, acc);
+  if (extra != nullptr) {
+    // extra [n, width]: one more term per token (an expert every token uses), times sigmoid(extra_gate[t * ld_gate])
+    read(extra + t * width + c, more);
+    const float eg = extra_gate != nullptr ? 1.f / (1.f + expf(-extra_gate[t * ld_gate])) : 1.f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) acc[i] = fmaf(eg, more[i], acc[i]);
   }
+  for (int k0 = 0; k0 < top; k0 += COMBINE_AHEAD) {
+    if (k0 > 0) request(k0);
+#pragma unroll
+    for (int k = 0; k < COMBINE_AHEAD; ++k)
+      if (k0 + k < top)
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) acc[i] = fmaf(share[k], term[k][i], acc[i]);
+  }
+  if constexpr (VEC == 4) *reinterpret_cast<float4*>(y + t * width + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  else y[t * width + c] = acc[0];
 }
 
 template <typename T>
@@ -453,8 +489,11 @@ HFEE_API int hfee_moe_combine_extra(const float* pair_out, const float* weight, 
   if (n == 0) return HFEE_OK;
   HFEE_REQUIRE(n > 0 && top > 0 && width > 0, "moe_combine: bad sizes");
   HFEE_REQUIRE(extra != nullptr || extra_gate == nullptr, "moe_combine: a gate without the term it gates");
-  hfee_launch(moe_combine_kernel, dim3(n), dim3(THREADS), 0, stream, pair_out, weight, place, top, y, width, accumulate, extra,
-              extra_gate, ld_gate);
+  HFEE_REQUIRE(n <= 65535, "moe_combine: %d tokens are too many", n);
+  const bool vec = width % 4 == 0 && ((uintptr_t)pair_out | (uintptr_t)y | (uintptr_t)extra) % 16 == 0;
+  const int per_block = THREADS * (vec ? 4 : 1);
+  hfee_launch(vec ? moe_combine_kernel<4> : moe_combine_kernel<1>, dim3((width + per_block - 1) / per_block, n), dim3(THREADS), 0, stream,
+              pair_out, weight, place, top, y, width, accumulate, extra, extra_gate, ld_gate);
   return hfee_check_launch("moe_combine");
 }
 

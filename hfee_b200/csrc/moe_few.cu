@@ -1,0 +1,198 @@
+// The experts' two products for a step of few (token, choice) pairs, in bfloat16 on mma.sync.
+//
+//   hfee_moe_few_gate_up   hidden[pair] = act(W_gate[e] x[token], W_up[e] x[token]) for every pair's expert e
+//   hfee_moe_few_down      pair_out[pair] = W_down[e] hidden[pair] (float32)
+//
+// Reference math of one expert: hostfog/hfee internal/ggml/ops.go:125-134 (the product), 160-165 (gate times up).
+//
+// Bound by the bytes of the chosen experts' weights, each read once.  The tiles of 128 rows that the large grouped product takes are
+// too few and too long for that: a step of three tokens (six experts of 2,048 x 2,048) ran 192 of them on 148 SMs, then 96, 28.6 +
+// 16.8 us with 5.5 more for the plan and the gathering of rows, where the bytes take 23.  Here a unit of work is 16 rows of one
+// expert's matrix.  The FEW_WARPS warps of a block take runs of 32 FEW_AHEAD k in turn, a lane 16 bytes of two rows at a time, which
+// are the A operands of two m16n8k16 products (k in the order the loads bring it, the same for both operands); up to eight pairs of
+// the expert are the columns of B.  Blocks stay and walk the units, and a lane asks for its next FEW_AHEAD pieces, of the next unit
+// if need be, before it multiplies the last ones: with a block for each unit, which starts cold, the same loads reached 3.2 TB/s.  The
+// warps' partial sums meet in shared memory in their order.  There is no plan: a warp lists the experts and the pairs that chose
+// them from the choices (one a lane, so at most 32).
+#include <type_traits>
+
+#include "mma_tiles.cuh"
+
+namespace {
+
+constexpr int FEW_WARPS = 4, FEW_AHEAD = 4, FEW_ROWS = 16, FEW_PAIRS = 32;
+
+__device__ __forceinline__ uint4 load_weights(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// x: rows of the pairs' inputs, row pair / share (share = top for tokens, 1 for rows by pair).  GATED: rows of w in runs of
+// [4 gate | 4 up], out bfloat16 [pairs, rows / 2]; else out float32 [pairs, rows], and the kernel in front is the gated one with the
+// same choices: it waited for whatever made them, so they (and the first weights) are read before the wait for it.
+template <bool GATED>
+__global__ void __launch_bounds__(FEW_WARPS * 32, 4)
+moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16* __restrict__ w, int rows, int K,
+               const int* __restrict__ choice, int pairs, void* __restrict__ out, long long ld_out, float limit, float alpha, float shift) {
+  __shared__ float part_s[2][FEW_WARPS][FEW_ROWS][8];
+  __shared__ int expert_s[FEW_PAIRS];
+  __shared__ unsigned members_s[FEW_PAIRS];
+  __shared__ int lists_s;
+  constexpr int RUN = 32 * FEW_AHEAD;             // k of a warp's batch
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if (GATED) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+  if (warp == 0) {
+    // the experts in the order of their first pair, each with at most eight of its pairs (one that has more comes again)
+    const int mine = lane < pairs ? choice[lane] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, mine);
+    unsigned leaders = __ballot_sync(0xffffffffu, mine >= 0 && __ffs(same) - 1 == lane);
+    int lists = 0;
+    while (leaders != 0) {
+      const int leader = __ffs(leaders) - 1;
+      leaders &= leaders - 1;
+      const int expert = __shfl_sync(0xffffffffu, mine, leader);
+      unsigned members = __shfl_sync(0xffffffffu, same, leader);
+      while (members != 0) {
+        unsigned rest = members;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) rest &= rest - 1;
+        if (lane == 0) { expert_s[lists] = expert; members_s[lists] = members ^ rest; }
+        ++lists;
+        members = rest;
+      }
+    }
+    if (lane == 0) lists_s = lists;
+  }
+  __syncthreads();
+  const int tiles = (rows + FEW_ROWS - 1) / FEW_ROWS, units = lists_s * tiles;
+  const int batches = (K + RUN * FEW_WARPS - 1) / (RUN * FEW_WARPS);
+
+  uint4 a0[2][FEW_AHEAD], a1[2][FEW_AHEAD], b[2][FEW_AHEAD];
+  auto load_a = [&](int unit, int batch, uint4 (&p)[FEW_AHEAD], uint4 (&q)[FEW_AHEAD]) {
+    const int row = (unit % tiles) * FEW_ROWS + g, k = (batch * FEW_WARPS + warp) * RUN + 8 * t;
+    const bf16* we = w + (long long)expert_s[unit / tiles] * rows * K + k;
+    const bf16* w0 = we + (long long)min(row, rows - 1) * K;
+    const bf16* w1 = we + (long long)min(row + 8, rows - 1) * K;
+#pragma unroll
+    for (int i = 0; i < FEW_AHEAD; ++i) {
+      const bool in = k + 32 * i < K;
+      p[i] = in ? load_weights(w0 + 32 * i) : make_uint4(0, 0, 0, 0);
+      q[i] = in ? load_weights(w1 + 32 * i) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  auto load_b = [&](int unit, int batch, uint4 (&r)[FEW_AHEAD]) {
+    unsigned from = members_s[unit / tiles];
+    for (int i = 0; i < g; ++i) from &= from - 1;
+    const int k = (batch * FEW_WARPS + warp) * RUN + 8 * t;                // column g of B has a pair if a member is left
+    const bf16* xr = x + (long long)(from != 0 ? (__ffs(from) - 1) / share : 0) * ld_x + k;
+#pragma unroll
+    for (int i = 0; i < FEW_AHEAD; ++i)
+      r[i] = from != 0 && k + 32 * i < K ? *reinterpret_cast<const uint4*>(xr + 32 * i) : make_uint4(0, 0, 0, 0);
+  };
+
+  int unit = blockIdx.x, batch = 0, half = 0;
+  if (unit < units) load_a(unit, 0, a0[0], a1[0]);
+  if (!GATED) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+  if (unit < units) load_b(unit, 0, b[0]);
+  float c[4] = {0.f, 0.f, 0.f, 0.f};
+  // one batch: asks for the one after it, multiplies, and after a unit's last puts the warps' sums together; false at the end
+  auto turn = [&](auto now) {
+    constexpr int NOW = decltype(now)::value;
+    if (unit >= units) return false;
+    const bool last = batch + 1 == batches;
+    const int next_unit = last ? unit + gridDim.x : unit, next_batch = last ? 0 : batch + 1;
+    if (next_unit < units) {
+      load_a(next_unit, next_batch, a0[NOW ^ 1], a1[NOW ^ 1]);
+      load_b(next_unit, next_batch, b[NOW ^ 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < FEW_AHEAD; ++i) {
+      const uint4 p = a0[NOW][i], q = a1[NOW][i], r = b[NOW][i];
+      const uint32_t first[4] = {p.x, q.x, p.y, q.y}, second[4] = {p.z, q.z, p.w, q.w};
+      mma_bf16(c, first, r.x, r.y);
+      mma_bf16(c, second, r.z, r.w);
+    }
+    if (last) {
+      float (*part)[FEW_ROWS][8] = part_s[half];   // two in turn: a warp is at most one unit ahead of the others
+      half ^= 1;
+      part[warp][g][2 * t] = c[0];
+      part[warp][g][2 * t + 1] = c[1];
+      part[warp][g + 8][2 * t] = c[2];
+      part[warp][g + 8][2 * t + 1] = c[3];
+      c[0] = c[1] = c[2] = c[3] = 0.f;
+      __syncthreads();
+      auto sum = [&](int r, int col) {
+        float v = part[0][r][col];
+#pragma unroll
+        for (int i = 1; i < FEW_WARPS; ++i) v += part[i][r][col];
+        return v;
+      };
+      const unsigned eight = members_s[unit / tiles];
+      const int row0 = (unit % tiles) * FEW_ROWS, count = __popc(eight);
+      constexpr int OUTS = GATED ? FEW_ROWS / 2 : FEW_ROWS;
+      const int r = threadIdx.x % OUTS;
+      for (int col = threadIdx.x / OUTS; col < count; col += FEW_WARPS * 32 / OUTS) {
+        unsigned rest = eight;
+        for (int i = 0; i < col; ++i) rest &= rest - 1;
+        const long long pair = __ffs(rest) - 1;
+        if constexpr (GATED) {
+          const int j = (r >> 2) * 8 + (r & 3);   // gate row j, up row j + 4
+          if (row0 + j + 4 < rows) {
+            const float gate = fminf(sum(j, col), limit), up = fminf(fmaxf(sum(j + 4, col), -limit), limit);
+            reinterpret_cast<bf16*>(out)[pair * ld_out + row0 / 2 + r] =
+                __float2bfloat16_rn(__fdividef(gate, 1.f + __expf(-alpha * gate)) * (up + shift));
+          }
+        } else if (row0 + r < rows) {
+          reinterpret_cast<float*>(out)[pair * ld_out + row0 + r] = sum(r, col);
+        }
+      }
+    }
+    unit = next_unit;
+    batch = next_batch;
+    return true;
+  };
+  while (turn(std::integral_constant<int, 0>{}) && turn(std::integral_constant<int, 1>{})) {}
+}
+
+unsigned few_blocks(int rows, int pairs) {
+  const long long units = (long long)((rows + FEW_ROWS - 1) / FEW_ROWS) * pairs, room = 4LL * (hfee_sm_count() > 0 ? hfee_sm_count() : 1);
+  return (unsigned)(units < room ? units : room);
+}
+
+int few_check(const char* name, const void* x, long long ld_x, const void* w, int rows, int K, int experts, int pairs) {
+  HFEE_REQUIRE(pairs > 0 && pairs <= FEW_PAIRS && experts > 0, "%s: %d pairs are outside 1..%d", name, pairs, FEW_PAIRS);
+  HFEE_REQUIRE(rows > 0 && K > 0 && K % 8 == 0 && ld_x % 8 == 0 && ld_x >= K && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0,
+               "%s: rows must be whole 16-byte pieces", name);
+  return HFEE_OK;
+}
+
+}  // namespace
+
+// x: [pairs / top, width] bfloat16; w: [experts, 2 * inner, width] with each expert's rows in runs of [4 gate | 4 up];
+// choice: [pairs], every one an expert; hidden: [pairs, inner].  The clamped gated activation of hfee_moe_gate_up.
+HFEE_API int hfee_moe_few_gate_up(const void* x, long long ld_x, int top, const void* w, int inner, int width, int experts, const int* choice,
+                                  int pairs, void* hidden, long long ld_hidden, float limit, float alpha, float shift, cudaStream_t stream) {
+  if (pairs == 0) return HFEE_OK;
+  const int rc = few_check("moe_few_gate_up", x, ld_x, w, 2 * inner, width, experts, pairs);
+  if (rc != HFEE_OK) return rc;
+  HFEE_REQUIRE(top > 0 && inner % 4 == 0 && ld_hidden >= inner && limit > 0.f, "moe_few_gate_up: bad sizes");
+  hfee_launch(moe_few_kernel<true>, dim3(few_blocks(2 * inner, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)x, ld_x, top, (const bf16*)w, 2 * inner, width, choice, pairs, hidden, ld_hidden, limit, alpha, shift);
+  return hfee_check_launch("moe_few_gate_up");
+}
+
+// hidden: [pairs, inner] bfloat16; w: [experts, width, inner]; pair_out: [pairs, width] float32.
+HFEE_API int hfee_moe_few_down(const void* hidden, long long ld_hidden, const void* w, int inner, int width, int experts, const int* choice,
+                               int pairs, float* pair_out, cudaStream_t stream) {
+  if (pairs == 0) return HFEE_OK;
+  const int rc = few_check("moe_few_down", hidden, ld_hidden, w, width, inner, experts, pairs);
+  if (rc != HFEE_OK) return rc;
+  hfee_launch(moe_few_kernel<false>, dim3(few_blocks(width, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)hidden, ld_hidden, 1, (const bf16*)w, width, inner, choice, pairs, pair_out, (long long)width, 0.f, 0.f, 0.f);
+  return hfee_check_launch("moe_few_down");
+}

@@ -94,6 +94,8 @@ _SIGNATURES = {
     "hfee_moe_gate_up": [_P, _L, _I, _P, _P, _L, _I, _I, _P, _P, _P, _P, _P, _L, _F, _F, _F, _I, _I, _P],
     "hfee_moe_down": [_P, _L, _I, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _P],
     "hfee_moe_combine": [_P, _P, _P, _I, _I, _P, _I, _I, _P],
+    "hfee_moe_few_gate_up": [_P, _L, _I, _P, _I, _I, _I, _P, _I, _P, _L, _F, _F, _F, _P],
+    "hfee_moe_few_down": [_P, _L, _P, _I, _I, _I, _P, _I, _P, _P],
     "hfee_moe_plan_tiles": [_P, _I, _I, _I, _P, _P, _P, _I, _P],
     "hfee_moe_gather_rows": [_P, _L, _I, _P, _P, _I, _P, _L, _I, _I, _P],
     "hfee_moe_route_chosen": [_P, _L, _P, _I, _I, _I, _F, _P, _P, _P],
@@ -1819,6 +1821,31 @@ def linear_clamped_glu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tens
         return
     linear(a, w_gate_up, scratch)
     clamped_glu(scratch, out, limit, alpha, granule, shift)
+
+
+# Steps of at most this many (token, choice) pairs take the experts' products that stream the chosen weights (a list of choices is one
+# word a lane of a warp); more take tiles of 128 rows on tcgen05.  16 experts of 2,048 x 2,048,
+# two a token, us against the tiles: 1 tokens 14.8 / 30.4, 4 tokens 36.0 / 49.9, 8 tokens 48.9 / 77.0, 16 tokens 64.6 / 83.2.
+MOE_FEW_PAIRS = 32
+
+
+def moe_experts_few(x: torch.Tensor, top: int, choice: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, limit: float,
+                    hidden: torch.Tensor, pair_out: torch.Tensor, alpha: float = CLAMPED_SWISH_ALPHA, shift: float = 1.0) -> None:
+    """:func:`moe_experts` for at most ``MOE_FEW_PAIRS`` pairs in bfloat16, without a plan: pair_out [pairs, width] float32 by pair.
+    ``w_gate_up`` [experts, 2 * inner, width] with each expert's rows in runs of [4 gate | 4 up] (:func:`interleave_gate_up`),
+    ``w_down`` [experts, width, inner], ``hidden`` [pairs, inner] bfloat16 scratch; sizes are multiples of 8."""
+    lib = library()
+    n, width = x.shape
+    experts, inner = w_gate_up.shape[0], w_gate_up.shape[1] // 2
+    pairs = n * top
+    _i32(choice, "choice")
+    assert choice.numel() == pairs and tuple(hidden.shape) == (pairs, inner) and tuple(pair_out.shape) == (pairs, width)
+    assert x.dtype == w_gate_up.dtype == w_down.dtype == hidden.dtype == torch.bfloat16 and pair_out.dtype == torch.float32
+    assert w_gate_up.is_contiguous() and w_down.is_contiguous() and pair_out.is_contiguous() and tuple(w_down.shape) == (experts, width, inner)
+    _check(lib.hfee_moe_few_gate_up(x.data_ptr(), _rows(x, "x"), top, w_gate_up.data_ptr(), inner, width, experts, choice.data_ptr(), pairs,
+                                    hidden.data_ptr(), _rows(hidden, "hidden"), float(limit), float(alpha), float(shift), _stream()), lib)
+    _check(lib.hfee_moe_few_down(hidden.data_ptr(), _rows(hidden, "hidden"), w_down.data_ptr(), inner, width, experts, choice.data_ptr(), pairs,
+                                 pair_out.data_ptr(), _stream()), lib)
 
 
 def moe_experts_grouped(x: torch.Tensor, top: int, choice: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, limit: float,

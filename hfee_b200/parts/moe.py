@@ -132,7 +132,13 @@ class RoutedExperts(Part):
             ops.moe_route(logits, top, self.router_scale, choice, weight)
         gate_col = logits[:, self.experts:self.experts + 1] if self.shared_gate else None
         place = None
-        if self.grouped:
+        if self.fused_act and n * top <= ops.MOE_FEW_PAIRS and xn.data_ptr() % 16 == 0 and xn.stride(0) % 8 == 0:
+            rows = self.tiles * ops.GROUPED_TILE_ROWS
+            hidden = rt.scratch("moe_hidden_rows", (rows, self.inner))[:n * top]
+            pair_out = rt.scratch("moe_rows_out", (rows, self.width), torch.float32)[:n * top]
+            ops.tag("experts")
+            ops.moe_experts_few(xn, top, choice, self.w_gate_up, self.w_down, self.limit, hidden, pair_out, self.alpha, self.shift)
+        elif self.grouped:
             rows = self.tiles * ops.GROUPED_TILE_ROWS
             place = rt.scratch("moe_place", (rt.max_tokens * top,), i32)
             row_pair = rt.scratch("moe_row_pair", (rows,), i32)
