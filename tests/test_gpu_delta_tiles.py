@@ -1,0 +1,67 @@
+"""The delta rule with one decay per head over portions of several tokens: tiles solved at once against the kernel that takes them one by
+one (no workspace) and against float64."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _step(portions):
+    cu = torch.tensor([0] + torch.tensor(portions).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots = torch.tensor([2 * i + 1 for i in range(len(portions))], dtype=torch.int32, device=DEV)
+    return types.SimpleNamespace(cu_tokens=cu, slots=slots, r=len(portions), n=sum(portions), max_new=max(portions))
+
+
+def _exact(q, k, v, b, a, a_log, dt_bias, s):
+    unit = lambda x: x / (x.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+    q, k = unit(q) * q.shape[-1] ** -0.5, unit(k)
+    beta, g = torch.sigmoid(b), torch.exp(-torch.exp(a_log) * torch.nn.functional.softplus(a + dt_bias))
+    out = []
+    for t in range(len(q)):
+        s = s * g[t][:, None, None]
+        u = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", s, k[t]))
+        s = s + k[t][:, :, None] * u[:, None, :]
+        out.append(torch.einsum("hdv,hd->hv", s, q[t]))
+    return torch.stack(out), s
+
+
+# portions around a tile of 16, single tokens beside longer ones; key sizes around 32 and 64 and not of whole 16 bytes; values
+# around a group of 16 columns and too long for a tile's solution; a before b and after it; offsets off 16 bytes
+@pytest.mark.parametrize("heads,groups,dim,vdim,portions", [(4, 2, 64, 64, [17, 1, 40]), (3, 1, 20, 17, [16, 15, 33]), (2, 2, 33, 8, [50]),
+                                                            (2, 1, 128, 40, [31, 2]), (1, 1, 8, 3000, [18])])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("a_first,shift,write", [(False, 0, True), (True, 3, False)])
+def test_tiles_match_one_by_one(heads, groups, dim, vdim, portions, dtype, a_first, shift, write):
+    from hfee_b200.kernels import ops
+    g = torch.Generator().manual_seed(dim + vdim)
+    rand = lambda *s: torch.randn(*s, generator=g)
+    step = _step(portions)
+    cols = 2 * groups * dim + heads * vdim
+    qkv = rand(step.n, shift + cols + 5).to(dtype).to(DEV)
+    ba = rand(step.n, 2 * heads + 3).to(dtype).to(DEV)
+    b_off, a_off = (heads + 2, 1) if a_first else (0, heads)
+    a_log, dt_bias = (rand(heads) - 1).to(DEV), rand(heads).to(DEV)
+    state = rand(2 * len(portions) + 1, heads, dim, vdim).to(DEV) * 0.3
+    ws = torch.empty(ops.channel_delta_workspace(step.r, step.n, heads, dim, vdim), device=DEV)
+    offs = (shift, shift + groups * dim, shift + 2 * groups * dim)
+    results = []
+    for workspace in (ws, None):
+        s, out = state.clone(), torch.full((step.n, heads * vdim), float("nan"), device=DEV)
+        ops.delta_rule(qkv, *offs, ba, b_off, a_off, a_log, dt_bias, s, step, out, heads, groups, dim, vdim, write, workspace)
+        ops.check_status()
+        results.append((out, s))
+    d = lambda t: t.double()
+    q, k = (d(qkv[:, o:o + groups * dim]).reshape(-1, groups, dim).repeat_interleave(heads // groups, 1) for o in offs[:2])
+    v = d(qkv[:, offs[2]:offs[2] + heads * vdim]).reshape(-1, heads, vdim)
+    b, a = d(ba[:, b_off:b_off + heads]), d(ba[:, a_off:a_off + heads])
+    for i, count in enumerate(portions):
+        at = slice(int(step.cu_tokens[i]), int(step.cu_tokens[i]) + count)
+        want, last = _exact(q[at], k[at], v[at], b[at], a[at], d(a_log), d(dt_bias), d(state[2 * i + 1]))
+        for out, s in results:                  # float32 sums of up to 128 products, carried over up to 50 tokens
+            assert (d(out[at]).reshape(want.shape) - want).norm() <= 1e-5 * want.norm()
+            assert (d(s[2 * i + 1]) - (last if write else d(state[2 * i + 1]))).norm() <= 1e-5 * last.norm()
+    for out, s in results:
+        assert torch.equal(s[::2], state[::2])
