@@ -466,6 +466,78 @@ namespace {
 constexpr int HG_SIGMOID = 0, HG_SILU = 1;
 constexpr int UA_RELU2 = 0;
 
+// The same where rows and heads are whole 16-byte pieces of x (8-byte pieces of a bfloat16 gate): a group of `lanes` lanes (a power of
+// two) has a (token, head), NI pieces of four a lane, all asked for before the first is used.  One element a lane and step, with the
+// gate asked for behind the sum, took 21 us in place for a prompt of 2,048 tokens and 32 heads of 64.
+template <typename T> struct alignas(4 * sizeof(T)) FourOf { T v[4]; };
+
+template <typename T, int NI>
+__global__ void __launch_bounds__(128)
+head_norm_gate_vec_kernel(const float* __restrict__ x, long long ld_x, const float* __restrict__ w, float eps,
+                          const T* __restrict__ gate, long long ld_g, T* __restrict__ out, long long ld_o, int n, int heads,
+                          int head_dim, int act, int w_head_stride, float out_scale, int lanes) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const unsigned task = (blockIdx.x * 128 + threadIdx.x) / (unsigned)lanes;
+  const int lane = threadIdx.x & (lanes - 1);
+  const bool live = task < (unsigned)n * (unsigned)heads;
+  const int i = live ? (int)(task / (unsigned)heads) : 0, h = live ? (int)(task - (unsigned)i * (unsigned)heads) : 0;
+  const float* xr = x + (long long)i * ld_x + (long long)h * head_dim;
+  const T* gr = gate + (long long)i * ld_g + (long long)h * head_dim;
+  float4 v[NI];
+  FourOf<T> g[NI];
+#pragma unroll
+  for (int j = 0; j < NI; ++j) {
+    const int d = (lane + lanes * j) * 4;
+    const bool in = live && d < head_dim;
+    v[j] = in ? *reinterpret_cast<const float4*>(xr + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (in) g[j] = *reinterpret_cast<const FourOf<T>*>(gr + d);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NI; ++j) {
+    ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+  }
+  for (int o = lanes >> 1; o >= 1; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (!live) return;
+  const float scale = out_scale / sqrtf(ss / (float)head_dim + eps);
+  const float* wh = w + (long long)h * w_head_stride;
+  T* orow = out + (long long)i * ld_o + (long long)h * head_dim;
+#pragma unroll
+  for (int j = 0; j < NI; ++j) {
+    const int d = (lane + lanes * j) * 4;
+    if (d >= head_dim) break;
+    const float xs[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+    FourOf<T> y;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float z = to_f32<T>(g[j].v[e]), s = sigmoid_f32(z);
+      y.v[e] = from_f32<T>(xs[e] * scale * wh[d + e] * (act == HG_SILU ? z * s : s));
+    }
+    *reinterpret_cast<FourOf<T>*>(orow + d) = y;
+  }
+}
+
+template <typename T>
+bool launch_head_norm_gate_vec(const float* x, long long ld_x, const float* w, float eps, const void* gate, long long ld_g, void* out,
+                               long long ld_o, int n, int heads, int head_dim, int act, int w_head_stride, float out_scale, cudaStream_t stream) {
+  if (head_dim % 4 != 0 || head_dim > 512 || ld_x % 4 != 0 || ld_g % 4 != 0 || ld_o % 4 != 0 || (uintptr_t)x % 16 != 0 ||
+      (uintptr_t)gate % (4 * sizeof(T)) != 0 || (uintptr_t)out % (4 * sizeof(T)) != 0)
+    return false;
+  int lanes = 1;
+  while (lanes < 32 && lanes * 4 < head_dim) lanes *= 2;
+  const long long threads = (long long)n * heads * lanes;
+  if (threads > (1ll << 31)) return false;
+  auto run = [&](auto kernel) {
+    hfee_launch(kernel, dim3((unsigned)((threads + 127) / 128)), dim3(128), 0, stream, x, ld_x, w, eps, (const T*)gate, ld_g, (T*)out, ld_o, n,
+                heads, head_dim, act, w_head_stride, out_scale, lanes);
+  };
+  if (head_dim <= 128) run(head_norm_gate_vec_kernel<T, 1>);
+  else if (head_dim <= 256) run(head_norm_gate_vec_kernel<T, 2>);
+  else run(head_norm_gate_vec_kernel<T, 4>);
+  return true;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 head_norm_gate_kernel(const float* __restrict__ x, long long ld_x, const float* __restrict__ w, float eps,
@@ -674,6 +746,10 @@ HFEE_API int hfee_head_norm_gate_scaled(const float* x, long long ld_x, const fl
   HFEE_REQUIRE(act == HG_SIGMOID || act == HG_SILU, "head_norm_gate: unknown gate activation %d", act);
   HFEE_REQUIRE((long long)n * heads < (1ll << 31), "head_norm_gate: too many (token, head) pairs for one launch");
   const unsigned blocks = (unsigned)(((long long)n * heads + 3) / 4);
+  if (dtype == HFEE_F32 ? launch_head_norm_gate_vec<float>(x, ld_x, w, eps, gate, ld_g, out, ld_o, n, heads, head_dim, act, w_head_stride, out_scale, stream)
+                        : dtype == HFEE_BF16 && launch_head_norm_gate_vec<__nv_bfloat16>(x, ld_x, w, eps, gate, ld_g, out, ld_o, n, heads, head_dim,
+                                                                                         act, w_head_stride, out_scale, stream))
+    return hfee_check_launch("head_norm_gate");
   if (dtype == HFEE_F32)
     hfee_launch(head_norm_gate_kernel<float>, dim3(blocks), dim3(128), 0, stream, x, ld_x, w, eps, (const float*)gate, ld_g, (float*)out, ld_o, n, heads, head_dim, act, w_head_stride, out_scale);
   else if (dtype == HFEE_BF16)
