@@ -92,9 +92,34 @@ __device__ __forceinline__ bool find_run(const int* __restrict__ cu_tokens, int 
   return false;
 }
 
+// Two float32 numbers side by side, multiplied and added as a pair.
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Bound by the issue of its multiply-adds (three per state element and token with an output) once nothing waits for memory: two rows
+// of a column are a pair for the packed instructions, and what the next stage needs is asked for while this one is walked.
 template <typename T, int MODE, int PASS>
-__global__ void __launch_bounds__(GR_LANES * (GR_MAX_DIM / GR_ROWS), 2)
+__global__ void __launch_bounds__(GR_LANES * (GR_MAX_DIM / GR_ROWS), PASS == PASS_WHOLE ? 1 : 2)
 gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, RecurrenceArgs p) {
+  constexpr int VALUES = 4;                           // values a thread asks for ahead: all of a stage's from four row groups on
   extern __shared__ __align__(16) float smem[];
   __shared__ float a_s[GR_STAGE], b_s[GR_STAGE], em_s[GR_STAGE];
   __shared__ float m_cur;
@@ -128,13 +153,18 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   const long long place = PASS == PASS_WHOLE ? (long long)slot * heads + head : (long long)blockIdx.y * heads + head;
   float* S_g = (PASS == PASS_WHOLE ? p.state : p.run_state) + (place * dim) * vdim;
   float* n_g = (PASS == PASS_WHOLE ? p.norm_state : p.run_norm) + place * dim;
-  float S[GR_NC][GR_ROWS];
+  uint64_t S[GR_NC][GR_ROWS / 2];                     // rows 2 i and 2 i + 1 of the thread's columns
 #pragma unroll
   for (int c = 0; c < GR_NC; ++c)
 #pragma unroll
-    for (int i = 0; i < GR_ROWS; ++i) {
-      const int row = g * GR_ROWS + i;
-      S[c][i] = (PASS != PASS_LOCAL && row < dim && col + c * GR_LANES < vdim) ? S_g[(long long)row * vdim + col + c * GR_LANES] : 0.f;
+    for (int i = 0; i < GR_ROWS / 2; ++i) {
+      float at[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int row = g * GR_ROWS + 2 * i + e;
+        at[e] = (PASS != PASS_LOCAL && row < dim && col + c * GR_LANES < vdim) ? S_g[(long long)row * vdim + col + c * GR_LANES] : 0.f;
+      }
+      S[c][i] = pair_of(at[0], at[1]);
     }
   float n_own = 0.f;                                  // n[g * GR_ROWS + j]
   float decay_own = 1.f;                              // PASS_LOCAL: product of the run's decays of that row
@@ -148,29 +178,70 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   const bool live_d = tid < dim;
   const int chan = (MODE == MODE_STEP ? head / p.qk_share : head) * dim + tid;
   const float z_bias = (MODE == MODE_CHANNEL_DECAY && live_d && !p.decays_given && p.bias != nullptr) ? p.bias[chan] : 0.f;
+  // what a thread brings for the next stage, asked for a stage ahead
+  T q_next[GR_STAGE], k_next[GR_STAGE], v_next[VALUES];
+  float z_next[MODE == MODE_CHANNEL_DECAY ? GR_STAGE : 1], gate_next[3];
+  auto fetch = [&](int t0) {
+    const int nt = min(GR_STAGE, count - t0);
+#pragma unroll
+    for (int t = 0; t < GR_STAGE; ++t)
+      if (t < nt && live_d) {
+        const long long at = (long long)(begin + t0 + t) * p.ld + chan;
+        if (PASS != PASS_LOCAL) q_next[t] = q[at];
+        k_next[t] = k[at];
+        if constexpr (MODE == MODE_CHANNEL_DECAY) z_next[t] = p.pre[(long long)(begin + t0 + t) * p.ld_pre + chan];
+      }
+#pragma unroll
+    for (int i = 0; i < VALUES; ++i) {
+      const int e = tid + i * threads, c = blockIdx.z * GR_COLS + e % GR_COLS;
+      if (e < nt * GR_COLS && c < vdim) v_next[i] = v[(long long)(begin + t0 + e / GR_COLS) * p.ld + (long long)head * vdim + c];
+    }
+    if constexpr (MODE != MODE_CHANNEL_DECAY && PASS != PASS_WHOLE) {
+      if (tid < nt) {                                 // the gates were computed for every token beforehand
+        const long long at = (long long)(begin + t0 + tid) * heads + head;
+        gate_next[0] = p.gates[at];
+        gate_next[1] = p.gates[p.gate_stride + at];
+        if constexpr (MODE == MODE_EXP_GATES) gate_next[2] = p.gates[2 * p.gate_stride + at];
+      }
+    }
+  };
+  constexpr bool AHEAD = PASS != PASS_WHOLE;          // the walk in one piece has a stage or two, and no registers left for this
+  if (AHEAD) fetch(0);
   for (int t0 = 0; t0 < count; t0 += GR_STAGE) {
     const int nt = min(GR_STAGE, count - t0);
     __syncthreads();                                  // the stage before is used up
+    if (!AHEAD) fetch(t0);
 #pragma unroll
     for (int t = 0; t < GR_STAGE; ++t) {
       if (t < nt) {
         const int e = t * dim_pad + tid;
-        const long long at = (long long)(begin + t0 + t) * p.ld + chan;
-        qs[e] = live_d ? to_f32<T>(q[at]) * p.q_scale : 0.f;
-        ks[e] = live_d ? to_f32<T>(k[at]) : 0.f;
+        if (PASS != PASS_LOCAL) qs[e] = live_d ? to_f32<T>(q_next[t]) * p.q_scale : 0.f;
+        ks[e] = live_d ? to_f32<T>(k_next[t]) : 0.f;
         if constexpr (MODE == MODE_CHANNEL_DECAY) {    // a decay, or the gate's pre-activation it comes from
           float a = 1.f;
           if (live_d) {
-            a = p.pre[(long long)(begin + t0 + t) * p.ld_pre + chan];
+            a = z_next[t];
             if (!p.decays_given) a = expf(log_sigmoid_f32(a + z_bias) * p.p0);
           }
           as[e] = a;
         }
       }
     }
-    for (int e = tid; e < nt * GR_COLS; e += threads) {
+#pragma unroll
+    for (int i = 0; i < VALUES; ++i) {
+      const int e = tid + i * threads, c = blockIdx.z * GR_COLS + e % GR_COLS;
+      if (e < nt * GR_COLS) vs[e] = c < vdim ? to_f32<T>(v_next[i]) : 0.f;
+    }
+    for (int e = tid + VALUES * threads; e < nt * GR_COLS; e += threads) {      // blocks of few warps bring more values than that
       const int t = e / GR_COLS, c = blockIdx.z * GR_COLS + e % GR_COLS;
       vs[e] = c < vdim ? to_f32<T>(v[(long long)(begin + t0 + t) * p.ld + (long long)head * vdim + c]) : 0.f;
+    }
+    if constexpr (MODE != MODE_CHANNEL_DECAY && PASS != PASS_WHOLE) {
+      if (tid < nt) {
+        a_s[tid] = gate_next[0];
+        b_s[tid] = gate_next[1];
+        if constexpr (MODE == MODE_EXP_GATES) em_s[tid] = gate_next[2];
+      }
     }
     if constexpr (MODE == MODE_STEP && PASS == PASS_WHOLE) {
       if (tid < nt) {
@@ -178,21 +249,6 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
                                       p.bias[head]);
         a_s[tid] = expf(-expf(p.a_log[head]) * dt);
         b_s[tid] = dt;
-      }
-    }
-    if constexpr (MODE == MODE_STEP && PASS != PASS_WHOLE) {
-      if (tid < nt) {
-        const long long at = (long long)(begin + t0 + tid) * heads + head;
-        a_s[tid] = p.gates[at];
-        b_s[tid] = p.gates[p.gate_stride + at];
-      }
-    }
-    if constexpr (MODE == MODE_EXP_GATES && PASS != PASS_WHOLE) {
-      if (tid < nt) {                                 // the gates were computed for every token beforehand
-        const long long at = (long long)(begin + t0 + tid) * heads + head;
-        a_s[tid] = p.gates[at];
-        b_s[tid] = p.gates[p.gate_stride + at];
-        em_s[tid] = p.gates[2 * p.gate_stride + at];
       }
     }
     if constexpr (MODE == MODE_EXP_GATES && PASS == PASS_WHOLE) {
@@ -215,40 +271,39 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
       }
     }
     __syncthreads();
+    if (AHEAD && t0 + GR_STAGE < count) fetch(t0 + GR_STAGE);
     for (int t = 0; t < nt; ++t) {
       const float vv = vs[t * GR_COLS + j], vw = vs[t * GR_COLS + GR_LANES + j];
-      const float4* k4 = reinterpret_cast<const float4*>(ks + t * dim_pad + g * GR_ROWS);
-      const float4* q4 = reinterpret_cast<const float4*>(qs + t * dim_pad + g * GR_ROWS);
-      float acc = 0.f, acd = 0.f;
+      const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(ks + t * dim_pad + g * GR_ROWS);
+      const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(qs + t * dim_pad + g * GR_ROWS);
+      uint64_t sum2[GR_NC] = {0, 0};
+      // a quarter of the rows' update and output, decays per pair
+      auto rows = [&](int i, uint64_t a0, uint64_t a1, const uint64_t (&value)[GR_NC]) {
+        const ulonglong2 kk = k4[i], qq = PASS != PASS_LOCAL ? q4[i] : kk;
+#pragma unroll
+        for (int c = 0; c < GR_NC; ++c) {
+          S[c][2 * i] = fma_pair(a0, S[c][2 * i], mul_pair(kk.x, value[c]));
+          S[c][2 * i + 1] = fma_pair(a1, S[c][2 * i + 1], mul_pair(kk.y, value[c]));
+          if constexpr (PASS != PASS_LOCAL) {
+            sum2[c] = fma_pair(S[c][2 * i], qq.x, sum2[c]);
+            sum2[c] = fma_pair(S[c][2 * i + 1], qq.y, sum2[c]);
+          }
+        }
+      };
       if constexpr (MODE == MODE_CHANNEL_DECAY) {
-        const float4* a4 = reinterpret_cast<const float4*>(as + t * dim_pad + g * GR_ROWS);
+        const ulonglong2* a4 = reinterpret_cast<const ulonglong2*>(as + t * dim_pad + g * GR_ROWS);
+        const uint64_t value[GR_NC] = {pair_of(vv, vv), pair_of(vw, vw)};
 #pragma unroll
         for (int i = 0; i < GR_ROWS / 4; ++i) {
-          const float4 kk = k4[i], qq = q4[i], aa = a4[i];
-          S[0][4 * i + 0] = fmaf(aa.x, S[0][4 * i + 0], kk.x * vv);  acc = fmaf(S[0][4 * i + 0], qq.x, acc);
-          S[0][4 * i + 1] = fmaf(aa.y, S[0][4 * i + 1], kk.y * vv);  acc = fmaf(S[0][4 * i + 1], qq.y, acc);
-          S[0][4 * i + 2] = fmaf(aa.z, S[0][4 * i + 2], kk.z * vv);  acc = fmaf(S[0][4 * i + 2], qq.z, acc);
-          S[0][4 * i + 3] = fmaf(aa.w, S[0][4 * i + 3], kk.w * vv);  acc = fmaf(S[0][4 * i + 3], qq.w, acc);
-          S[1][4 * i + 0] = fmaf(aa.x, S[1][4 * i + 0], kk.x * vw);  acd = fmaf(S[1][4 * i + 0], qq.x, acd);
-          S[1][4 * i + 1] = fmaf(aa.y, S[1][4 * i + 1], kk.y * vw);  acd = fmaf(S[1][4 * i + 1], qq.y, acd);
-          S[1][4 * i + 2] = fmaf(aa.z, S[1][4 * i + 2], kk.z * vw);  acd = fmaf(S[1][4 * i + 2], qq.z, acd);
-          S[1][4 * i + 3] = fmaf(aa.w, S[1][4 * i + 3], kk.w * vw);  acd = fmaf(S[1][4 * i + 3], qq.w, acd);
+          const ulonglong2 aa = a4[i];
+          rows(i, aa.x, aa.y, value);
         }
         if constexpr (PASS == PASS_LOCAL) decay_own *= as[t * dim_pad + own_row];
       } else {
         const float a = a_s[t], bv = b_s[t] * vv, bw = b_s[t] * vw;
+        const uint64_t value[GR_NC] = {pair_of(bv, bv), pair_of(bw, bw)}, a2 = pair_of(a, a);
 #pragma unroll
-        for (int i = 0; i < GR_ROWS / 4; ++i) {
-          const float4 kk = k4[i], qq = q4[i];
-          S[0][4 * i + 0] = fmaf(a, S[0][4 * i + 0], kk.x * bv);  acc = fmaf(S[0][4 * i + 0], qq.x, acc);
-          S[0][4 * i + 1] = fmaf(a, S[0][4 * i + 1], kk.y * bv);  acc = fmaf(S[0][4 * i + 1], qq.y, acc);
-          S[0][4 * i + 2] = fmaf(a, S[0][4 * i + 2], kk.z * bv);  acc = fmaf(S[0][4 * i + 2], qq.z, acc);
-          S[0][4 * i + 3] = fmaf(a, S[0][4 * i + 3], kk.w * bv);  acc = fmaf(S[0][4 * i + 3], qq.w, acc);
-          S[1][4 * i + 0] = fmaf(a, S[1][4 * i + 0], kk.x * bw);  acd = fmaf(S[1][4 * i + 0], qq.x, acd);
-          S[1][4 * i + 1] = fmaf(a, S[1][4 * i + 1], kk.y * bw);  acd = fmaf(S[1][4 * i + 1], qq.y, acd);
-          S[1][4 * i + 2] = fmaf(a, S[1][4 * i + 2], kk.z * bw);  acd = fmaf(S[1][4 * i + 2], qq.z, acd);
-          S[1][4 * i + 3] = fmaf(a, S[1][4 * i + 3], kk.w * bw);  acd = fmaf(S[1][4 * i + 3], qq.w, acd);
-        }
+        for (int i = 0; i < GR_ROWS / 4; ++i) rows(i, a2, a2, value);
         if constexpr (MODE == MODE_EXP_GATES) n_own = fmaf(a, n_own, b_s[t] * ks[t * dim_pad + own_row]);
         if constexpr (PASS == PASS_LOCAL) decay_own *= a;
         if constexpr (MODE == MODE_EXP_GATES && PASS != PASS_LOCAL) {
@@ -257,8 +312,11 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
         }
       }
       if constexpr (PASS != PASS_LOCAL) {
-        part[(t * groups + g) * GR_COLS + j] = acc;
-        part[(t * groups + g) * GR_COLS + GR_LANES + j] = acd;
+#pragma unroll
+        for (int c = 0; c < GR_NC; ++c) {
+          const float2 f = unpair(sum2[c]);
+          part[(t * groups + g) * GR_COLS + c * GR_LANES + j] = f.x + f.y;
+        }
       }
     }
     if constexpr (PASS == PASS_LOCAL) continue;       // a run's own sum: no outputs
@@ -281,9 +339,11 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 #pragma unroll
     for (int c = 0; c < GR_NC; ++c)
 #pragma unroll
-      for (int i = 0; i < GR_ROWS; ++i) {
-        const int row = g * GR_ROWS + i;
-        if (row < dim && col + c * GR_LANES < vdim) S_g[(long long)row * vdim + col + c * GR_LANES] = S[c][i];
+      for (int i = 0; i < GR_ROWS / 2; ++i) {
+        const int row = g * GR_ROWS + 2 * i;
+        const float2 f = unpair(S[c][i]);
+        if (row < dim && col + c * GR_LANES < vdim) S_g[(long long)row * vdim + col + c * GR_LANES] = f.x;
+        if (row + 1 < dim && col + c * GR_LANES < vdim) S_g[(long long)(row + 1) * vdim + col + c * GR_LANES] = f.y;
       }
     if (blockIdx.z == 0) {
       if constexpr (MODE == MODE_EXP_GATES) {
