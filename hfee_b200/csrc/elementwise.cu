@@ -182,25 +182,25 @@ rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, con
   }
 }
 
-// Many rows (a prompt portion), bfloat16 out: a warp per row and the whole row in registers, so a row
-// costs one memory round trip and no block-wide barrier, and a CTA of 8 warps keeps 8 rows in flight.
-// NV float4 per lane: rows of up to 128 * NV values.
-template <int NV>
+// Many rows (a prompt portion), bfloat16 out: TEAM warps per row and the whole row in registers, so a row costs one memory round
+// trip, and a CTA of 8 warps keeps 8 / TEAM rows in flight.  NV float4 per lane: rows of up to 128 * NV * TEAM values.
+template <int NV, int TEAM>
 __global__ void __launch_bounds__(256)
 rmsnorm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const int* __restrict__ rows,
                     __nv_bfloat16* __restrict__ out, int n, int width, float eps, int add_unit) {
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (r >= n) return;
-  const int src_row = rows ? rows[r] : r;                 // host-written, like the batch layout
+  __shared__ float sums[8];
+  const int warp = threadIdx.x >> 5, at = threadIdx.x % (32 * TEAM);      // place in the row's team
+  const int r = blockIdx.x * (8 / TEAM) + warp / TEAM;
+  const bool live = r < n;
+  const int src_row = live ? (rows ? rows[r] : r) : 0;                    // host-written, like the batch layout
   pdl_wait();
   pdl_launch_dependents();
   const float* xr = x + (long long)src_row * width;
   float4 xv[NV];
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
-    const int c = (lane + j * 32) * 4;
-    xv[j] = c < width ? *reinterpret_cast<const float4*>(xr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int c = (at + j * 32 * TEAM) * 4;
+    xv[j] = live && c < width ? *reinterpret_cast<const float4*>(xr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   float ss = 0.f;
 #pragma unroll
@@ -209,12 +209,20 @@ rmsnorm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, co
     ss = fmaf(xv[j].z, xv[j].z, ss); ss = fmaf(xv[j].w, xv[j].w, ss);
   }
   ss = warp_sum(ss);
+  if constexpr (TEAM > 1) {
+    if ((threadIdx.x & 31) == 0) sums[warp] = ss;
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < TEAM; ++i) ss += sums[warp / TEAM * TEAM + i];
+  }
+  if (!live) return;
   const float scale = 1.0f / sqrtf(ss / (float)width + eps);
   const float unit = add_unit ? 1.f : 0.f;
   __nv_bfloat16* dst = out + (long long)r * width;
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
-    const int c = (lane + j * 32) * 4;
+    const int c = (at + j * 32 * TEAM) * 4;
     if (c >= width) continue;
     const float4 g = __ldg(reinterpret_cast<const float4*>(w + c));
     __nv_bfloat162 lo = __floats2bfloat162_rn(xv[j].x * scale * (g.x + unit), xv[j].y * scale * (g.y + unit));
@@ -232,11 +240,15 @@ HFEE_API int hfee_rmsnorm(const float* x, const float* w, const int* rows, void*
     if (vector) hfee_launch(rmsnorm_vec_kernel<float, 256, 4>, dim3(n), dim3(256), 0, stream, x, w, rows, (float*)out, width, eps, add_unit);
     else hfee_launch(rmsnorm_kernel<float, 256>, dim3(n), dim3(256), 0, stream, x, w, rows, (float*)out, width, eps, add_unit);
   } else if (out_dtype == HFEE_BF16 && vector && n >= 256 && width <= 128 * 32) {
-    // enough rows to fill the GPU with a warp each
-    const dim3 grid((unsigned)((n + 7) / 8));
-    if (width <= 128 * 8) hfee_launch(rmsnorm_rows_kernel<8>, grid, dim3(256), 0, stream, x, w, rows, (__nv_bfloat16*)out, n, width, eps, add_unit);
-    else if (width <= 128 * 16) hfee_launch(rmsnorm_rows_kernel<16>, grid, dim3(256), 0, stream, x, w, rows, (__nv_bfloat16*)out, n, width, eps, add_unit);
-    else hfee_launch(rmsnorm_rows_kernel<32>, grid, dim3(256), 0, stream, x, w, rows, (__nv_bfloat16*)out, n, width, eps, add_unit);
+    auto run = [&](auto kernel, int team) {
+      const unsigned per = 8 / team;
+      hfee_launch(kernel, dim3(((unsigned)n + per - 1) / per), dim3(256), 0, stream, x, w, rows, (__nv_bfloat16*)out, n, width, eps, add_unit);
+    };
+    // A warp for a row of up to 2,048 values, four for more: 128 registers a lane for one row leave a CTA an SM and a second, nearly empty
+    // wave (2,048 rows of 4,096: 10.0 us with one warp a row, 7.1 with four; of 2,048: 3.8 with one, 4.4 with four).
+    if (width <= 128 * 8) run(rmsnorm_rows_kernel<8, 1>, 1);
+    else if (width <= 128 * 16) run(rmsnorm_rows_kernel<16, 1>, 1);
+    else run(rmsnorm_rows_kernel<8, 4>, 4);
   } else if (out_dtype == HFEE_BF16) {
     if (vector) hfee_launch(rmsnorm_vec_kernel<__nv_bfloat16, 256, 4>, dim3(n), dim3(256), 0, stream, x, w, rows, (__nv_bfloat16*)out, width, eps, add_unit);
     else hfee_launch(rmsnorm_kernel<__nv_bfloat16, 256>, dim3(n), dim3(256), 0, stream, x, w, rows, (__nv_bfloat16*)out, width, eps, add_unit);
