@@ -8,6 +8,7 @@ token, not only the last.
 """
 from __future__ import annotations
 
+import gc
 from typing import Any, List, Optional, Sequence
 
 import torch
@@ -153,8 +154,15 @@ class ModelRunner:
             graph = torch.cuda.CUDAGraph()
             before = ops.launch_count()
             torch.cuda.synchronize()
-            with torch.cuda.graph(graph):
-                out = self.model.forward(step, self.cache.views())
+            # a collector run in here could free another engine's graphs, which a capture does not survive
+            collecting = gc.isenabled()
+            gc.disable()
+            try:
+                with torch.cuda.graph(graph):
+                    out = self.model.forward(step, self.cache.views())
+            finally:
+                if collecting:
+                    gc.enable()
             while len(self._graphs) >= GRAPH_LIMIT:          # oldest first
                 self._graphs.pop(next(iter(self._graphs)))
             hit = self._graphs[key] = (graph, out, ops.launch_count() - before)
