@@ -19,8 +19,7 @@
 
 namespace {
 
-constexpr int ST_WARPS = 8;
-constexpr int ST_THREADS = ST_WARPS * 32;
+constexpr int ST_WARPS = 8, ST_WARPS_FEW = 16;       // a block's warps; where there are fewer tokens than SMs
 constexpr int ST_MAX_STREAMS = 64;
 
 struct StreamArgs {
@@ -62,12 +61,15 @@ template <> __device__ __forceinline__ void store_row<__nv_bfloat16, 4>(__nv_bfl
 }
 
 // S: number of streams, or 0 for any number (the streams are then read again for every output stream).
-template <typename T, int S, int VEC>
-__global__ void __launch_bounds__(ST_THREADS, S > 0 ? 3 : 2)
+// A decode step is the chain of one row's trips to memory: sixteen warps take a row of 2,048 in one go, and the weights that the
+// norm and the shift need at the end are brought into cache before the wait for the kernel in front.
+template <typename T, int S, int VEC, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == ST_WARPS ? (S > 0 ? 3 : 2) : 1)
 stream_step_kernel(StreamArgs p, T* __restrict__ h_out) {
+  constexpr int ST_THREADS = WARPS * 32;
   extern __shared__ __align__(16) float row_s[];       // [width]: u of the token in work; with a shift [width]: the row before
   __shared__ float coef_s[ST_MAX_STREAMS * 2 + (S > 0 ? S * S : ST_MAX_STREAMS * ST_MAX_STREAMS)];
-  __shared__ float red_s[2][ST_WARPS];
+  __shared__ float red_s[2][WARPS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int streams = S > 0 ? S : p.streams;
   float* in_s = coef_s;
@@ -83,9 +85,14 @@ stream_step_kernel(StreamArgs p, T* __restrict__ h_out) {
   float* prev_s = row_s + p.width;
   const int i0 = blockIdx.x * p.run, i1 = min(i0 + p.run, p.n);
   // warps share the groups out: a team of warps per group, or several groups per warp
-  const int teams = min(p.groups, ST_WARPS), per_team = ST_WARPS / teams;
+  const int teams = min(p.groups, WARPS), per_team = WARPS / teams;
   const int team = warp / per_team, in_team = warp - team * per_team;
   const int part = p.width / p.groups, vecs = part / VEC;
+  if constexpr (WARPS == ST_WARPS_FEW)
+    for (int c = tid * VEC; c < p.width; c += ST_THREADS * VEC) {
+      const float warm = p.norm_w[c] + (p.shift_w != nullptr ? p.shift_w[c] : 0.f);
+      asm volatile("" ::"f"(warm));
+    }
   __syncthreads();
   pdl_wait();
   pdl_launch_dependents();
@@ -217,16 +224,23 @@ stream_step_kernel(StreamArgs p, T* __restrict__ h_out) {
   }
 }
 
-template <typename T, int S, int VEC>
-int launch_stream_step(const StreamArgs& p, void* h_out, cudaStream_t stream) {
+template <typename T, int S, int VEC, int WARPS>
+int launch_stream_step_w(const StreamArgs& p, void* h_out, cudaStream_t stream) {
   const size_t smem = (size_t)p.width * sizeof(float) * (p.shift_w != nullptr ? 2 : 1);
   HFEE_REQUIRE(smem <= 160 * 1024, "stream_step: a row of %d columns does not fit shared memory", p.width);
   if (smem > 32 * 1024) {                              // the static part may take some 17 KB beside it
-    cudaError_t e = cudaFuncSetAttribute(stream_step_kernel<T, S, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(stream_step_kernel<T, S, VEC, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "stream_step: %s", cudaGetErrorString(e));
   }
-  hfee_launch(stream_step_kernel<T, S, VEC>, dim3((unsigned)((p.n + p.run - 1) / p.run)), dim3(ST_THREADS), smem, stream, p, (T*)h_out);
+  hfee_launch(stream_step_kernel<T, S, VEC, WARPS>, dim3((unsigned)((p.n + p.run - 1) / p.run)), dim3(WARPS * 32), smem, stream, p, (T*)h_out);
   return hfee_check_launch("stream_step");
+}
+
+template <typename T, int S, int VEC>
+int launch_stream_step(const StreamArgs& p, void* h_out, cudaStream_t stream) {
+  if constexpr (S > 0)      // a row each for fewer blocks than SMs, and work for sixteen warps in it
+    if (p.n <= hfee_sm_count() && p.width > ST_WARPS * 32 * VEC) return launch_stream_step_w<T, S, VEC, ST_WARPS_FEW>(p, h_out, stream);
+  return launch_stream_step_w<T, S, VEC, ST_WARPS>(p, h_out, stream);
 }
 
 template <typename T>
