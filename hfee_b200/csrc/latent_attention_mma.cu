@@ -83,8 +83,6 @@ latent_attention_kernel(LatentParams p) {
   const int begin = p.cu_tokens[req], count = p.cu_tokens[req + 1] - begin;     // host-written batch layout
   const int split = blockIdx.x % p.splits;
   const int t0 = blockIdx.x / p.splits * p.tokens_per_tile;
-  pdl_wait();
-  pdl_launch_dependents();
   if (t0 >= count) return;
   const int tokens = min(p.tokens_per_tile, count - t0);
   const int slot = p.slots[req], before = p.context_before[req];
@@ -107,15 +105,7 @@ latent_attention_kernel(LatentParams p) {
     m_s[tid] = -INFINITY;
     l_s[tid] = 0.f;
   }
-  // queries of the tile
   const int pieces = dk >> 3;
-  for (int e = tid; e < ROWS * pieces; e += THREADS) {
-    const int r = e / pieces, c = (e - r * pieces) * 8;
-    const int t = r / p.rows_per_token, h = head0 + r % p.rows_per_token;
-    const bool valid = t < tokens && h < p.heads;
-    const bf16* src = p.q + (long long)(begin + t0 + (valid ? t : 0)) * p.ld_q + (long long)(valid ? h : 0) * dk + c;
-    la_cp_async16(Qs + r * ldk + c, src, valid);
-  }
   auto load_block = [&](int block_start, int buf) {
     bf16* dst = Ks + (long long)buf * LA_BN * ldk;
     for (int e = tid; e < LA_BN * pieces; e += THREADS) {
@@ -128,7 +118,21 @@ latent_attention_kernel(LatentParams p) {
     }
   };
   const int first_block = (lo / LA_BN) * LA_BN;
-  load_block(first_block, 0);
+  // a block of positions that earlier steps wrote is requested before the wait for the kernel in front (and the batch layout and
+  // the block table come from the host)
+  const bool early = first_block + LA_BN <= before && lo <= p_last;
+  if (early) load_block(first_block, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  // queries of the tile
+  for (int e = tid; e < ROWS * pieces; e += THREADS) {
+    const int r = e / pieces, c = (e - r * pieces) * 8;
+    const int t = r / p.rows_per_token, h = head0 + r % p.rows_per_token;
+    const bool valid = t < tokens && h < p.heads;
+    const bf16* src = p.q + (long long)(begin + t0 + (valid ? t : 0)) * p.ld_q + (long long)(valid ? h : 0) * dk + c;
+    la_cp_async16(Qs + r * ldk + c, src, valid);
+  }
+  if (!early) load_block(first_block, 0);
   la_commit();
 
   float o[NG][2][2][4];          // [group][column tile of 8][row tile of 16][fragment]
@@ -307,16 +311,25 @@ latent_attention_kernel(LatentParams p) {
 
 // A block per (token, head), a thread per pair of value columns: the shares' outputs against the largest of their maxima
 // (and the sink's).
-constexpr int LC_THREADS = 128;
+constexpr int LC_THREADS = 128, LC_SHARES = 32;
 __global__ void __launch_bounds__(LC_THREADS)
 latent_combine_kernel(const float* __restrict__ partial, int splits, int n_tokens, int heads, int dv, const float* __restrict__ sink,
                       bf16* __restrict__ out, long long ld_o) {
-  __shared__ float w_s[32];
+  __shared__ float w_s[LC_SHARES];
   pdl_wait();
   pdl_launch_dependents();
   const int h = blockIdx.x, t = blockIdx.y, lane = threadIdx.x & 31;
   const long long stride = (long long)n_tokens * heads * (dv + 2);
   const float* mine = partial + ((long long)t * heads + h) * (dv + 2);
+  // every share's numbers of the first columns are asked for together, and before the weights are known: the second trip to memory
+  // behind the first one's sums was half of the kernel in a decode step of one token
+  float2 v[LC_SHARES];
+  auto request = [&](int d) {
+#pragma unroll
+    for (int s = 0; s < LC_SHARES; ++s)
+      if (s < splits && d < dv) v[s] = *reinterpret_cast<const float2*>(mine + s * stride + d);
+  };
+  request(2 * threadIdx.x);
   if (threadIdx.x < 32) {                                      // lane s: share s (at most 32 of them)
     float m = -INFINITY, l = 0.f;
     if (lane < splits) {
@@ -332,13 +345,14 @@ latent_combine_kernel(const float* __restrict__ partial, int splits, int n_token
   __syncthreads();
   bf16* dst = out + (long long)t * ld_o + (long long)h * dv;
   for (int d = 2 * threadIdx.x; d < dv; d += 2 * LC_THREADS) {
+    if (d > 2 * LC_THREADS - 1) request(d);
     float a = 0.f, b = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < splits; ++s) {
-      const float2 v = *reinterpret_cast<const float2*>(mine + s * stride + d);
-      a = fmaf(w_s[s], v.x, a);
-      b = fmaf(w_s[s], v.y, b);
-    }
+#pragma unroll
+    for (int s = 0; s < LC_SHARES; ++s)
+      if (s < splits) {
+        a = fmaf(w_s[s], v[s].x, a);
+        b = fmaf(w_s[s], v[s].y, b);
+      }
     *reinterpret_cast<__nv_bfloat162*>(dst + d) = __floats2bfloat162_rn(a, b);
   }
 }
