@@ -15,11 +15,11 @@
 // projection buffer (type T); the gates' pre-activations z, x_i, x_f are float32, and so are the decays, their
 // logarithms and exponentials, the states, every product and o.
 //
-// hfee_gated_recurrence walks a request's tokens one after the other.  A thread keeps GR_ROWS rows
-// of two state columns in registers (a staged q, k or decay is read from shared memory once for both); a warp covers
-// GR_COLS = 64 columns of those rows, a block all rows (blockDim.y row groups whose partial outputs meet in shared
-// memory in a fixed order) of 64 columns; blockIdx = (head, request, column tile).
-// Lane j of row group g also keeps n[g * 32 + j].  Tokens are staged GR_STAGE at a time; the scalar recurrence of
+// hfee_gated_recurrence walks a request's tokens one after the other.  A thread keeps ROWS = 32 rows
+// of NC = 2 state columns in registers (a staged q, k or decay is read from shared memory once for all of them); a warp covers
+// 32 NC columns of those rows, a block all rows (blockDim.y row groups whose partial outputs meet in shared
+// memory in a fixed order) of as many columns; blockIdx = (head, request, column tile).
+// Lane j of row group g also keeps n[g * ROWS + j].  Tokens are staged GR_STAGE at a time; the scalar recurrence of
 // the running maximum is walked by one thread per stage.  The order of the sums does not depend on how a prompt was
 // cut, and a state is what the tokens before left, so neither does a position's output.
 //
@@ -33,10 +33,8 @@
 
 namespace {
 
-constexpr int GR_ROWS = 32;
 constexpr int GR_LANES = 32;         // threads of a row group: one warp
-constexpr int GR_NC = 2;             // state columns per thread (lane j: columns j and j + 32 of the block's 64)
-constexpr int GR_COLS = GR_LANES * GR_NC;
+constexpr int GR_COLS = 64;          // state columns of a block, at least
 constexpr int GR_STAGE = 8;
 constexpr int GR_MAX_DIM = 256;
 constexpr int GC_T = 64;             // tokens of a run of the chunked path
@@ -114,11 +112,15 @@ __device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
   return r;
 }
 
-// Bound by the issue of its multiply-adds (three per state element and token with an output) once nothing waits for memory: two rows
-// of a column are a pair for the packed instructions, and what the next stage needs is asked for while this one is walked.
-template <typename T, int MODE, int PASS>
-__global__ void __launch_bounds__(GR_LANES * (GR_MAX_DIM / GR_ROWS), PASS == PASS_WHOLE ? 1 : 2)
+// Bound by the reads of q, k and decays from shared memory (a row's three numbers for every NC elements of the state) and the issue of
+// its multiply-adds: two rows of a column are a pair for the packed instructions, what the next stage needs is asked for while
+// this one is walked, and the runs of the chunked path take 16 rows of four columns a thread in place of 32 of two where the
+// values fill 128 columns, which halves the reads (the four passes of a prompt of 2,048 tokens, 8 heads of 128 x 256 and 64 x 256: 404 ->
+// 351 us in place).
+template <typename T, int MODE, int PASS, int ROWS, int NC>
+__global__ void __launch_bounds__(GR_LANES * (GR_MAX_DIM / ROWS), PASS == PASS_WHOLE || ROWS < 32 ? 1 : 2)
 gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, RecurrenceArgs p) {
+  constexpr int COLS = GR_LANES * NC, SHARE = GR_LANES / ROWS, TOKENS = GR_STAGE / SHARE;      // threads a channel; tokens of a stage each brings
   constexpr int VALUES = 4;                           // values a thread asks for ahead: all of a stage's from four row groups on
   extern __shared__ __align__(16) float smem[];
   __shared__ float a_s[GR_STAGE], b_s[GR_STAGE], em_s[GR_STAGE];
@@ -128,16 +130,16 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   if constexpr (PASS != PASS_WHOLE) {
     if (!find_run(p.cu_tokens, p.requests, blockIdx.y, &req, &run)) return;
   }
-  const int groups = blockDim.y, dim_pad = groups * GR_ROWS;
+  const int groups = blockDim.y, dim_pad = groups * ROWS;
   const int j = threadIdx.x, g = threadIdx.y;
-  const int col = blockIdx.z * GR_COLS + j;            // and col + 32
+  const int col = blockIdx.z * COLS + j;            // and col + 32 c
   const int tid = g * GR_LANES + j, threads = GR_LANES * groups;
   const int heads = p.heads, dim = p.dim, vdim = p.vdim;
   float* qs = smem;                                   // [GR_STAGE][dim_pad]
   float* ks = qs + GR_STAGE * dim_pad;                // [GR_STAGE][dim_pad]
-  float* vs = ks + GR_STAGE * dim_pad;                // [GR_STAGE][GR_COLS]
-  float* part = vs + GR_STAGE * GR_COLS;              // [GR_STAGE][groups][GR_COLS]
-  float* part_n = part + GR_STAGE * groups * GR_COLS; // [GR_STAGE][groups]
+  float* vs = ks + GR_STAGE * dim_pad;                // [GR_STAGE][COLS]
+  float* part = vs + GR_STAGE * COLS;              // [GR_STAGE][groups][COLS]
+  float* part_n = part + GR_STAGE * groups * COLS; // [GR_STAGE][groups]
   float* as = part_n + GR_STAGE * groups;             // [GR_STAGE][dim_pad]   (channel decay)
   int begin = p.cu_tokens[req], count = p.cu_tokens[req + 1] - begin;
   if constexpr (PASS != PASS_WHOLE) {
@@ -153,48 +155,51 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   const long long place = PASS == PASS_WHOLE ? (long long)slot * heads + head : (long long)blockIdx.y * heads + head;
   float* S_g = (PASS == PASS_WHOLE ? p.state : p.run_state) + (place * dim) * vdim;
   float* n_g = (PASS == PASS_WHOLE ? p.norm_state : p.run_norm) + place * dim;
-  uint64_t S[GR_NC][GR_ROWS / 2];                     // rows 2 i and 2 i + 1 of the thread's columns
+  uint64_t S[NC][ROWS / 2];                     // rows 2 i and 2 i + 1 of the thread's columns
 #pragma unroll
-  for (int c = 0; c < GR_NC; ++c)
+  for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int i = 0; i < GR_ROWS / 2; ++i) {
+    for (int i = 0; i < ROWS / 2; ++i) {
       float at[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int row = g * GR_ROWS + 2 * i + e;
+        const int row = g * ROWS + 2 * i + e;
         at[e] = (PASS != PASS_LOCAL && row < dim && col + c * GR_LANES < vdim) ? S_g[(long long)row * vdim + col + c * GR_LANES] : 0.f;
       }
       S[c][i] = pair_of(at[0], at[1]);
     }
-  float n_own = 0.f;                                  // n[g * GR_ROWS + j]
+  float n_own = 0.f;                                  // n[g * ROWS + j] (lanes below ROWS)
   float decay_own = 1.f;                              // PASS_LOCAL: product of the run's decays of that row
-  const int own_row = g * GR_ROWS + j;
+  const int own_row = g * ROWS + (j < ROWS ? j : 0);
   if constexpr (MODE == MODE_EXP_GATES) {
-    if (PASS != PASS_LOCAL && own_row < dim) n_own = n_g[own_row];
+    if (PASS != PASS_LOCAL && j < ROWS && own_row < dim) n_own = n_g[own_row];
     if (PASS == PASS_WHOLE && tid == 0) m_cur = p.max_state[(long long)slot * heads + head];
   }
-  // A block has as many threads as a staged token has (padded) key channels: thread `tid` brings channel `tid` of every
+  // A block has SHARE threads for each (padded) key channel of a staged token: a thread brings its channel of every SHARE-th
   // token of a stage, and its share of the stage's values.
-  const bool live_d = tid < dim;
-  const int chan = (MODE == MODE_STEP ? head / p.qk_share : head) * dim + tid;
+  const int ch = SHARE == 1 ? tid : tid % dim_pad, first_t = SHARE == 1 ? 0 : tid / dim_pad;
+  const bool live_d = ch < dim, has_own = j < ROWS && own_row < dim;
+  const int chan = (MODE == MODE_STEP ? head / p.qk_share : head) * dim + ch;
   const float z_bias = (MODE == MODE_CHANNEL_DECAY && live_d && !p.decays_given && p.bias != nullptr) ? p.bias[chan] : 0.f;
   // what a thread brings for the next stage, asked for a stage ahead
-  T q_next[GR_STAGE], k_next[GR_STAGE], v_next[VALUES];
-  float z_next[MODE == MODE_CHANNEL_DECAY ? GR_STAGE : 1], gate_next[3];
+  T q_next[TOKENS], k_next[TOKENS], v_next[VALUES];
+  float z_next[MODE == MODE_CHANNEL_DECAY ? TOKENS : 1], gate_next[3];
   auto fetch = [&](int t0) {
     const int nt = min(GR_STAGE, count - t0);
 #pragma unroll
-    for (int t = 0; t < GR_STAGE; ++t)
+    for (int u = 0; u < TOKENS; ++u) {
+      const int t = first_t + SHARE * u;
       if (t < nt && live_d) {
         const long long at = (long long)(begin + t0 + t) * p.ld + chan;
-        if (PASS != PASS_LOCAL) q_next[t] = q[at];
-        k_next[t] = k[at];
-        if constexpr (MODE == MODE_CHANNEL_DECAY) z_next[t] = p.pre[(long long)(begin + t0 + t) * p.ld_pre + chan];
+        if (PASS != PASS_LOCAL) q_next[u] = q[at];
+        k_next[u] = k[at];
+        if constexpr (MODE == MODE_CHANNEL_DECAY) z_next[u] = p.pre[(long long)(begin + t0 + t) * p.ld_pre + chan];
       }
+    }
 #pragma unroll
     for (int i = 0; i < VALUES; ++i) {
-      const int e = tid + i * threads, c = blockIdx.z * GR_COLS + e % GR_COLS;
-      if (e < nt * GR_COLS && c < vdim) v_next[i] = v[(long long)(begin + t0 + e / GR_COLS) * p.ld + (long long)head * vdim + c];
+      const int e = tid + i * threads, c = blockIdx.z * COLS + e % COLS;
+      if (e < nt * COLS && c < vdim) v_next[i] = v[(long long)(begin + t0 + e / COLS) * p.ld + (long long)head * vdim + c];
     }
     if constexpr (MODE != MODE_CHANNEL_DECAY && PASS != PASS_WHOLE) {
       if (tid < nt) {                                 // the gates were computed for every token beforehand
@@ -212,15 +217,16 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     __syncthreads();                                  // the stage before is used up
     if (!AHEAD) fetch(t0);
 #pragma unroll
-    for (int t = 0; t < GR_STAGE; ++t) {
+    for (int u = 0; u < TOKENS; ++u) {
+      const int t = first_t + SHARE * u;
       if (t < nt) {
-        const int e = t * dim_pad + tid;
-        if (PASS != PASS_LOCAL) qs[e] = live_d ? to_f32<T>(q_next[t]) * p.q_scale : 0.f;
-        ks[e] = live_d ? to_f32<T>(k_next[t]) : 0.f;
+        const int e = t * dim_pad + ch;
+        if (PASS != PASS_LOCAL) qs[e] = live_d ? to_f32<T>(q_next[u]) * p.q_scale : 0.f;
+        ks[e] = live_d ? to_f32<T>(k_next[u]) : 0.f;
         if constexpr (MODE == MODE_CHANNEL_DECAY) {    // a decay, or the gate's pre-activation it comes from
           float a = 1.f;
           if (live_d) {
-            a = z_next[t];
+            a = z_next[u];
             if (!p.decays_given) a = expf(log_sigmoid_f32(a + z_bias) * p.p0);
           }
           as[e] = a;
@@ -229,11 +235,11 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     }
 #pragma unroll
     for (int i = 0; i < VALUES; ++i) {
-      const int e = tid + i * threads, c = blockIdx.z * GR_COLS + e % GR_COLS;
-      if (e < nt * GR_COLS) vs[e] = c < vdim ? to_f32<T>(v_next[i]) : 0.f;
+      const int e = tid + i * threads, c = blockIdx.z * COLS + e % COLS;
+      if (e < nt * COLS) vs[e] = c < vdim ? to_f32<T>(v_next[i]) : 0.f;
     }
-    for (int e = tid + VALUES * threads; e < nt * GR_COLS; e += threads) {      // blocks of few warps bring more values than that
-      const int t = e / GR_COLS, c = blockIdx.z * GR_COLS + e % GR_COLS;
+    for (int e = tid + VALUES * threads; e < nt * COLS; e += threads) {      // blocks of few warps bring more values than that
+      const int t = e / COLS, c = blockIdx.z * COLS + e % COLS;
       vs[e] = c < vdim ? to_f32<T>(v[(long long)(begin + t0 + t) * p.ld + (long long)head * vdim + c]) : 0.f;
     }
     if constexpr (MODE != MODE_CHANNEL_DECAY && PASS != PASS_WHOLE) {
@@ -273,17 +279,19 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     __syncthreads();
     if (AHEAD && t0 + GR_STAGE < count) fetch(t0 + GR_STAGE);
     for (int t = 0; t < nt; ++t) {
-      const float vv = vs[t * GR_COLS + j], vw = vs[t * GR_COLS + GR_LANES + j];
-      const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(ks + t * dim_pad + g * GR_ROWS);
-      const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(qs + t * dim_pad + g * GR_ROWS);
-      uint64_t sum2[GR_NC] = {0, 0};
+      float value[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) value[c] = vs[t * COLS + c * GR_LANES + j];
+      const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(ks + t * dim_pad + g * ROWS);
+      const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(qs + t * dim_pad + g * ROWS);
+      uint64_t sum2[NC] = {};
       // a quarter of the rows' update and output, decays per pair
-      auto rows = [&](int i, uint64_t a0, uint64_t a1, const uint64_t (&value)[GR_NC]) {
+      auto rows = [&](int i, uint64_t a0, uint64_t a1, const uint64_t (&pairs)[NC]) {
         const ulonglong2 kk = k4[i], qq = PASS != PASS_LOCAL ? q4[i] : kk;
 #pragma unroll
-        for (int c = 0; c < GR_NC; ++c) {
-          S[c][2 * i] = fma_pair(a0, S[c][2 * i], mul_pair(kk.x, value[c]));
-          S[c][2 * i + 1] = fma_pair(a1, S[c][2 * i + 1], mul_pair(kk.y, value[c]));
+        for (int c = 0; c < NC; ++c) {
+          S[c][2 * i] = fma_pair(a0, S[c][2 * i], mul_pair(kk.x, pairs[c]));
+          S[c][2 * i + 1] = fma_pair(a1, S[c][2 * i + 1], mul_pair(kk.y, pairs[c]));
           if constexpr (PASS != PASS_LOCAL) {
             sum2[c] = fma_pair(S[c][2 * i], qq.x, sum2[c]);
             sum2[c] = fma_pair(S[c][2 * i + 1], qq.y, sum2[c]);
@@ -291,67 +299,72 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
         }
       };
       if constexpr (MODE == MODE_CHANNEL_DECAY) {
-        const ulonglong2* a4 = reinterpret_cast<const ulonglong2*>(as + t * dim_pad + g * GR_ROWS);
-        const uint64_t value[GR_NC] = {pair_of(vv, vv), pair_of(vw, vw)};
+        const ulonglong2* a4 = reinterpret_cast<const ulonglong2*>(as + t * dim_pad + g * ROWS);
+        uint64_t pairs[NC];
 #pragma unroll
-        for (int i = 0; i < GR_ROWS / 4; ++i) {
+        for (int c = 0; c < NC; ++c) pairs[c] = pair_of(value[c], value[c]);
+#pragma unroll
+        for (int i = 0; i < ROWS / 4; ++i) {
           const ulonglong2 aa = a4[i];
-          rows(i, aa.x, aa.y, value);
+          rows(i, aa.x, aa.y, pairs);
         }
         if constexpr (PASS == PASS_LOCAL) decay_own *= as[t * dim_pad + own_row];
       } else {
-        const float a = a_s[t], bv = b_s[t] * vv, bw = b_s[t] * vw;
-        const uint64_t value[GR_NC] = {pair_of(bv, bv), pair_of(bw, bw)}, a2 = pair_of(a, a);
+        const float a = a_s[t], b = b_s[t];
+        const uint64_t a2 = pair_of(a, a);
+        uint64_t pairs[NC];
 #pragma unroll
-        for (int i = 0; i < GR_ROWS / 4; ++i) rows(i, a2, a2, value);
+        for (int c = 0; c < NC; ++c) pairs[c] = pair_of(b * value[c], b * value[c]);
+#pragma unroll
+        for (int i = 0; i < ROWS / 4; ++i) rows(i, a2, a2, pairs);
         if constexpr (MODE == MODE_EXP_GATES) n_own = fmaf(a, n_own, b_s[t] * ks[t * dim_pad + own_row]);
         if constexpr (PASS == PASS_LOCAL) decay_own *= a;
         if constexpr (MODE == MODE_EXP_GATES && PASS != PASS_LOCAL) {
-          const float nq = warp_sum(n_own * qs[t * dim_pad + own_row]);
+          const float nq = warp_sum(j < ROWS ? n_own * qs[t * dim_pad + own_row] : 0.f);
           if (j == 0) part_n[t * groups + g] = nq;
         }
       }
       if constexpr (PASS != PASS_LOCAL) {
 #pragma unroll
-        for (int c = 0; c < GR_NC; ++c) {
+        for (int c = 0; c < NC; ++c) {
           const float2 f = unpair(sum2[c]);
-          part[(t * groups + g) * GR_COLS + c * GR_LANES + j] = f.x + f.y;
+          part[(t * groups + g) * COLS + c * GR_LANES + j] = f.x + f.y;
         }
       }
     }
     if constexpr (PASS == PASS_LOCAL) continue;       // a run's own sum: no outputs
     __syncthreads();
-    for (int e = tid; e < nt * GR_COLS; e += threads) {
-      const int t = e / GR_COLS, jj = e % GR_COLS, c = blockIdx.z * GR_COLS + jj;
+    for (int e = tid; e < nt * COLS; e += threads) {
+      const int t = e / COLS, jj = e % COLS, c = blockIdx.z * COLS + jj;
       float sum = 0.f;
-      for (int gg = 0; gg < groups; ++gg) sum += part[(t * groups + gg) * GR_COLS + jj];
+      for (int gg = 0; gg < groups; ++gg) sum += part[(t * groups + gg) * COLS + jj];
       if constexpr (MODE == MODE_EXP_GATES) {
         float nq = 0.f;
         for (int gg = 0; gg < groups; ++gg) nq += part_n[t * groups + gg];
         sum /= fmaxf(fabsf(nq), em_s[t]) + 1e-6f;
       }
-      if constexpr (MODE == MODE_STEP) sum = fmaf(p.d_skip[head], vs[t * GR_COLS + jj], sum);
+      if constexpr (MODE == MODE_STEP) sum = fmaf(p.d_skip[head], vs[t * COLS + jj], sum);
       if (c < vdim) p.out[(long long)(begin + t0 + t) * p.ld_o + (long long)head * vdim + c] = sum;
     }
   }
   if constexpr (PASS == PASS_OUT) return;
   if (PASS == PASS_LOCAL || p.write_state) {
 #pragma unroll
-    for (int c = 0; c < GR_NC; ++c)
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
-      for (int i = 0; i < GR_ROWS / 2; ++i) {
-        const int row = g * GR_ROWS + 2 * i;
+      for (int i = 0; i < ROWS / 2; ++i) {
+        const int row = g * ROWS + 2 * i;
         const float2 f = unpair(S[c][i]);
         if (row < dim && col + c * GR_LANES < vdim) S_g[(long long)row * vdim + col + c * GR_LANES] = f.x;
         if (row + 1 < dim && col + c * GR_LANES < vdim) S_g[(long long)(row + 1) * vdim + col + c * GR_LANES] = f.y;
       }
     if (blockIdx.z == 0) {
       if constexpr (MODE == MODE_EXP_GATES) {
-        if (own_row < dim) n_g[own_row] = n_own;
+        if (has_own) n_g[own_row] = n_own;
         if (PASS == PASS_WHOLE && tid == 0) p.max_state[(long long)slot * heads + head] = m_cur;
       }
       if constexpr (PASS == PASS_LOCAL) {
-        if (own_row < dim) p.run_decay[place * dim + own_row] = decay_own;
+        if (has_own) p.run_decay[place * dim + own_row] = decay_own;
       }
     }
   }
@@ -498,21 +511,33 @@ recurrence_carry_kernel(RecurrenceArgs p, int with_norm) {
   }
 }
 
+template <typename T, int PASS, int ROWS, int NC>
+int launch_recurrence_tiles(int mode, const void* q, const void* k, const void* v, const RecurrenceArgs& p, int grid_y, cudaStream_t stream) {
+  constexpr int COLS = GR_LANES * NC;
+  const int groups = (p.dim + ROWS - 1) / ROWS, dim_pad = groups * ROWS;
+  const dim3 grid(p.heads, grid_y, (p.vdim + COLS - 1) / COLS), block(GR_LANES, groups);
+  size_t floats = (size_t)GR_STAGE * (2 * dim_pad + COLS + groups * COLS + groups);
+  if (mode == MODE_CHANNEL_DECAY) floats += (size_t)GR_STAGE * dim_pad;
+  const size_t smem = floats * sizeof(float);
+  auto run = [&](auto kernel) {
+    if (smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gated_recurrence: %s", cudaGetErrorString(e));
+    }
+    hfee_launch(kernel, grid, block, smem, stream, (const T*)q, (const T*)k, (const T*)v, p);
+    return hfee_check_launch("gated_recurrence");
+  };
+  if (mode == MODE_CHANNEL_DECAY) return run(gated_recurrence_kernel<T, MODE_CHANNEL_DECAY, PASS, ROWS, NC>);
+  if (mode == MODE_STEP) return run(gated_recurrence_kernel<T, MODE_STEP, PASS, ROWS, NC>);
+  return run(gated_recurrence_kernel<T, MODE_EXP_GATES, PASS, ROWS, NC>);
+}
+
 template <typename T, int PASS>
 int launch_recurrence(int mode, const void* q, const void* k, const void* v, const RecurrenceArgs& p, int grid_y,
                       cudaStream_t stream) {
-  const int groups = (p.dim + GR_ROWS - 1) / GR_ROWS, dim_pad = groups * GR_ROWS;
-  const dim3 grid(p.heads, grid_y, (p.vdim + GR_COLS - 1) / GR_COLS), block(GR_LANES, groups);
-  size_t floats = (size_t)GR_STAGE * (2 * dim_pad + GR_COLS + groups * GR_COLS + groups);
-  if (mode == MODE_CHANNEL_DECAY) floats += (size_t)GR_STAGE * dim_pad;
-  const size_t smem = floats * sizeof(float);
-  if (mode == MODE_CHANNEL_DECAY)
-    hfee_launch(gated_recurrence_kernel<T, MODE_CHANNEL_DECAY, PASS>, grid, block, smem, stream, (const T*)q, (const T*)k, (const T*)v, p);
-  else if (mode == MODE_STEP)
-    hfee_launch(gated_recurrence_kernel<T, MODE_STEP, PASS>, grid, block, smem, stream, (const T*)q, (const T*)k, (const T*)v, p);
-  else
-    hfee_launch(gated_recurrence_kernel<T, MODE_EXP_GATES, PASS>, grid, block, smem, stream, (const T*)q, (const T*)k, (const T*)v, p);
-  return hfee_check_launch("gated_recurrence");
+  if constexpr (PASS != PASS_WHOLE)
+    if (p.vdim > GR_COLS) return launch_recurrence_tiles<T, PASS, 16, 4>(mode, q, k, v, p, grid_y, stream);
+  return launch_recurrence_tiles<T, PASS, 32, 2>(mode, q, k, v, p, grid_y, stream);
 }
 
 template <typename T>
