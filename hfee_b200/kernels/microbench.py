@@ -361,7 +361,8 @@ def _distance_attention(args) -> dict:
 
 def _moe_experts(args) -> dict:
     """The routed experts of ``--tokens`` tokens (``--experts`` of inner size ``--inner``, ``--top`` a token, width ``--k``):
-    plan, gather, both grouped products and the activation between them, and the weighted sum."""
+    plan, gather, both grouped products and the activation between them, and the weighted sum (for few pairs without ``--unfused``
+    the two products that stream the chosen weights)."""
     n, w, f, e, top = args.tokens, args.k, args.inner, args.experts, args.top
     x = torch.randn(n, w, device=DEV).to(torch.bfloat16)
     w_gu = (torch.randn(e, 2 * f, w, device=DEV) * w ** -0.5).to(torch.bfloat16)      # rows in runs of [4 gate | 4 up]
@@ -379,12 +380,18 @@ def _moe_experts(args) -> dict:
     rows_out = torch.empty(rows, w, dtype=torch.float32, device=DEV)
     y = torch.zeros(n, w, dtype=torch.float32, device=DEV)
 
+    few = n * top <= ops.MOE_FEW_PAIRS and not args.unfused
+
     def fn(i):
+        if few:
+            ops.moe_experts_few(x, top, choice, w_gu, w_d, 7.0, hidden[:n * top], rows_out[:n * top])
+            ops.moe_combine(rows_out, weight, y, False)
+            return
         ops.moe_experts_grouped(x, top, choice, w_gu, w_d, 7.0, place, row_pair, tile_group, rows_in, gate_up, hidden, rows_out)
         ops.moe_combine(rows_out, weight, y, False, place)
     sec = _time(fn, args.warmup, args.iters)
     flops = 2.0 * n * top * 3 * f * w
-    return {"kernel": "moe_experts_grouped", "tokens": n, "width": w, "inner": f, "experts": e, "top": top, "tiles": tiles,
+    return {"kernel": "moe_experts_few" if few else "moe_experts_grouped", "tokens": n, "width": w, "inner": f, "experts": e, "top": top, "tiles": tiles,
             "us": round(sec * 1e6, 2), "tflops": round(flops / sec / 1e12, 1)}
 
 
