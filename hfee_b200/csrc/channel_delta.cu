@@ -65,34 +65,6 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
   return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
 }
 
-// Two float32 numbers side by side, multiplied and added as a pair.
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpair(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-
 // ---------------------------------------------------------------------------------------------------------------
 // One token per request.  A thread keeps RPT rows of VEC neighbouring columns in registers; 32 / VEC threads side by
 // side make a row of CD_COLS columns.
@@ -270,20 +242,6 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
       if constexpr (!HEAD) reinterpret_cast<float4*>(g_s)[e] = g;
     }
   } else {
-  if constexpr (HEAD) {
-    // an exponential of the log-decays' sum over j + 1 .. t each (j = -1: G_t), the missing ones of t < j unused
-    for (int e = tid; e < CD_TILE * (CD_TILE + 1); e += CD_THREADS) {
-      const int t = e / (CD_TILE + 1), j = e - t * (CD_TILE + 1) - 1;
-      float sum = 0.f;
-#pragma unroll
-      for (int i = 0; i < CD_TILE; ++i) {
-        const float raw = raw_s[i];
-        if (i > j && i <= t) sum += raw;
-      }
-      if (j < 0) upto_s[t] = expf(sum);
-      else ratio_s[t][j] = expf(sum);
-    }
-  }
     for (int e = tid; e < CD_TILE * DP; e += CD_THREADS) {
       const int t = e / DP, d = e - t * DP;
       float kv = 0.f, qv = 0.f, g = 1.f;
@@ -312,6 +270,20 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
   }
   if (tid < CD_TILE) beta_s[tid] = tid < tt ? 1.f / (1.f + expf(-b_own)) : 0.f;
   __syncthreads();
+  if constexpr (HEAD) {
+    // an exponential of the log-decays' sum over j + 1 .. t each (j = -1: G_t), the missing ones of t < j unused
+    for (int e = tid; e < CD_TILE * (CD_TILE + 1); e += CD_THREADS) {
+      const int t = e / (CD_TILE + 1), j = e - t * (CD_TILE + 1) - 1;
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < CD_TILE; ++i) {
+        const float raw = raw_s[i];
+        if (i > j && i <= t) sum += raw;
+      }
+      if (j < 0) upto_s[t] = expf(sum);
+      else ratio_s[t][j] = expf(sum);
+    }
+  }
   const float q_unit = 1.0f / sqrtf((float)dim);
 #pragma unroll
   for (int half = 0; half < 2; ++half) {       // eight lanes per vector: 16 keys, then 16 queries
@@ -333,10 +305,6 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
   {
     // the tables: eight lanes per row j, each with its share of the channels of G_t / G_j * k_j as t runs on from j
     const int j = tid >> 3, sl = tid & 7;
-      if constexpr (HEAD) {
-        a *= ratio_s[t][j];
-        c *= ratio_s[t][j];
-      }
     const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(k_s);
     const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(q_s);
     const ulonglong2* g4 = reinterpret_cast<const ulonglong2*>(g_s);
@@ -363,8 +331,11 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
 #pragma unroll
       for (int o = 4; o >= 1; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
-      if constexpr (HEAD) after = pair_of(upto_s[CD_TILE - 1], upto_s[CD_TILE - 1]);
         c += __shfl_xor_sync(0xffffffffu, c, o);
+      }
+      if constexpr (HEAD) {
+        a *= ratio_s[t][j];
+        c *= ratio_s[t][j];
       }
       if (sl == 0) {
         A_s[t][j] = t > j ? make_float2(-a, -a) : make_float2(0.f, 0.f);
@@ -392,6 +363,7 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
         *reinterpret_cast<uint64_t*>(wh + (2 * CD_TILE + t) * DP + c) = mul_pair(after, k);
         if constexpr (!HEAD) after = mul_pair(after, *reinterpret_cast<const uint64_t*>(g_s + t * DP + c));
       }
+      if constexpr (HEAD) after = pair_of(upto_s[CD_TILE - 1], upto_s[CD_TILE - 1]);
       *reinterpret_cast<uint64_t*>(wh + 3 * CD_TILE * DP + c) = after;
       continue;
     }
@@ -612,7 +584,7 @@ int launch_token_r(const void* qkv, const void* b, const float* z, const float* 
   return hfee_check_launch("channel_delta_token");
 }
 
-template <typename T, bool HEAD = false>
+template <typename T>
 int launch_token(const void* qkv, const void* b, const float* z, const float* a_log, const float* dt_bias, float* state,
                  const int* cu_tokens, const int* slots, float* out, const ChannelDeltaArgs& p, int requests, cudaStream_t stream) {
 #define HFEE_CD(V, R) return launch_token_r<T, V, R>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, stream)
@@ -652,7 +624,7 @@ int launch_tiles_n(const void* qkv, const void* b, const float* z, const float* 
   return hfee_check_launch("channel_delta_walk");
 }
 
-template <typename T>
+template <typename T, bool HEAD = false>
 int launch_tiles(const void* qkv, const void* b, const float* z, const float* a_log, const float* dt_bias, float* state,
                  const int* cu_tokens, const int* slots, float* out, const ChannelDeltaArgs& p, int requests, int max_new,
                  float* ws_head, float* ws_uo, int* status, cudaStream_t stream) {
