@@ -33,9 +33,6 @@ constexpr int THREADS = 256;
 constexpr int PLAN_THREADS = 1024;
 constexpr int MAX_EXPERTS = 1024;
 
-// The plans take a number that is no expert's for the nearest one's, so that nothing behind them reads or writes out of range.
-__device__ __forceinline__ int expert_of(int choice, int experts) { return min(max(choice, 0), experts - 1); }
-
 __global__ void moe_route_kernel(const float* __restrict__ logits, int experts, int top, float scale, int* __restrict__ choice,
                                  float* __restrict__ weight, int n) {
   extern __shared__ float score_s[];       // [warps][experts]
@@ -68,7 +65,6 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int experts, 
       const int oa = __shfl_xor_sync(0xffffffffu, at, o);
       if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
     }
-    if (at >= experts) { at = 0; best = NAN; }               // no score is left that is a number: an expert that exists, a weight that shows it
     if (lane == 0) {
       choice[(long long)t * top + k] = at;
       weight[(long long)t * top + k] = best / sum * scale;
@@ -126,7 +122,6 @@ __global__ void moe_route_grouped_kernel(const float* __restrict__ logits, int l
       const int oa = __shfl_xor_sync(0xffffffffu, at, o);
       if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
     }
-    if (at >= experts) { at = 0; best = NAN; }               // as above
     sum += best;
     if (lane == 0) {
       choice[(long long)t * top + k] = at;
@@ -189,7 +184,7 @@ moe_plan_kernel(const int* __restrict__ choice, int pairs, int experts, int* __r
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[expert_of(choice[i], experts)], 1);
+  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[choice[i]], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int off = 0, tile = 0;
@@ -211,7 +206,7 @@ moe_plan_kernel(const int* __restrict__ choice, int pairs, int experts, int* __r
     }
   for (int j = first_tile[experts] + threadIdx.x; j < max_tiles; j += PLAN_THREADS) tile_expert[j] = -1;
   for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) {
-    const int e = expert_of(choice[i], experts);
+    const int e = choice[i];
     sorted[off_s[e] + atomicAdd(&cursor[e], 1)] = i;
   }
 }
@@ -226,7 +221,7 @@ moe_plan_tiles_kernel(const int* __restrict__ choice, int pairs, int experts, in
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[expert_of(choice[i], experts)], 1);
+  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[choice[i]], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int tile = 0;
@@ -244,7 +239,7 @@ moe_plan_tiles_kernel(const int* __restrict__ choice, int pairs, int experts, in
   for (long long r = threadIdx.x; r < (long long)used * tile_rows; r += PLAN_THREADS) row_pair[r] = -1;
   __syncthreads();
   for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) {
-    const int e = expert_of(choice[i], experts);
+    const int e = choice[i];
     const int row = first_tile[e] * tile_rows + atomicAdd(&cursor[e], 1);
     place_of_pair[i] = row;
     row_pair[row] = i;
@@ -360,8 +355,8 @@ moe_combine_kernel(const float* __restrict__ pair_out, const float* __restrict__
                    const float* __restrict__ extra, const float* __restrict__ extra_gate, long long ld_gate) {
   pdl_wait();
   pdl_launch_dependents();
-  const long long t = blockIdx.x;              // any number of tokens fits the grid's first axis only
-  const int c = (blockIdx.y * THREADS + threadIdx.x) * VEC;
+  const long long t = blockIdx.y;
+  const int c = (blockIdx.x * THREADS + threadIdx.x) * VEC;
   if (c >= width) return;
   auto read = [](const float* p, float (&v)[VEC]) {
     if constexpr (VEC == 4) {
@@ -494,9 +489,10 @@ HFEE_API int hfee_moe_combine_extra(const float* pair_out, const float* weight, 
   if (n == 0) return HFEE_OK;
   HFEE_REQUIRE(n > 0 && top > 0 && width > 0, "moe_combine: bad sizes");
   HFEE_REQUIRE(extra != nullptr || extra_gate == nullptr, "moe_combine: a gate without the term it gates");
+  HFEE_REQUIRE(n <= 65535, "moe_combine: %d tokens are too many", n);
   const bool vec = width % 4 == 0 && ((uintptr_t)pair_out | (uintptr_t)y | (uintptr_t)extra) % 16 == 0;
   const int per_block = THREADS * (vec ? 4 : 1);
-  hfee_launch(vec ? moe_combine_kernel<4> : moe_combine_kernel<1>, dim3(n, (width + per_block - 1) / per_block), dim3(THREADS), 0, stream,
+  hfee_launch(vec ? moe_combine_kernel<4> : moe_combine_kernel<1>, dim3((width + per_block - 1) / per_block, n), dim3(THREADS), 0, stream,
               pair_out, weight, place, top, y, width, accumulate, extra, extra_gate, ld_gate);
   return hfee_check_launch("moe_combine");
 }

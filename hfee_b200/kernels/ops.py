@@ -37,7 +37,7 @@ _SIGNATURES = {
     "hfee_gemm_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _L, _P, _P],
     "hfee_gemm_tcgen05_stream_k": [_I, _I, _I, _I, _L],
     "hfee_gemm_tcgen05_pair": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
-    "hfee_gemm_tcgen05_rope": [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "hfee_gemm_tcgen05_rope": [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "hfee_gemm_tcgen05_rope_supports": [_I, _I],
     "hfee_gemm_skinny": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "hfee_gemm_skinny_splits": [_I, _I, _I, _L],
@@ -125,7 +125,7 @@ _SIGNATURES = {
     "hfee_moe_route_grouped": [_P, _L, _I, _I, _I, _I, _I, _F, _P, _P, _P],
     "hfee_conv_act_launches": [_I, _I, _I],
     "hfee_delta_rule": [_P, _L, _I, _I, _I, _P, _L, _I, _I, _I, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _P, _L, _P, _P],
-    "hfee_delta_rule_launches": [_I, _I, _I, _I, _I, _I, _L],
+    "hfee_delta_rule_launches": [_I, _I, _I, _I],
     "hfee_head_norm_gate": [_P, _L, _P, _F, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
     "hfee_unary_act": [_P, _L, _P, _L, _I, _I, _I, _I, _P],
     "hfee_head_gate": [_P, _L, _P, _L, _I, _I, _I, _I, _P],
@@ -156,8 +156,6 @@ def library() -> ctypes.CDLL:
     lib.hfee_attention_tc_supports.restype = _I
     lib.hfee_linear_attention_chunked_workspace.restype = _L
     lib.hfee_linear_attention_chunked_workspace.argtypes = [_I, _I, _I, _I, _I]
-    lib.hfee_delta_rule_workspace.restype = _L
-    lib.hfee_delta_rule_workspace.argtypes = [_I, _I, _I, _I, _I]
     lib.hfee_channel_delta_workspace.restype = _L
     lib.hfee_channel_delta_workspace.argtypes = [_I, _I, _I, _I, _I]
     lib.hfee_gated_recurrence_workspace.restype = _L
@@ -399,14 +397,11 @@ def linear_rope_cache(a: torch.Tensor, w: torch.Tensor, cs: Optional[torch.Tenso
     if k_pool is not None:
         assert k_pool.dtype == v_pool.dtype == torch.bfloat16 and k_pool.is_contiguous() and v_pool.is_contiguous()
         assert tuple(k_pool.shape[1:]) == (kv_heads, page_size, head_dim)
-    # tiles of whole heads; the benchmark model's q/k/v product at 2,048 tokens: 128 pair tiles of 256 x 192 (three 64-dim heads) are two
-    # rounds, as are 96 of 256 x 256 (prompt pass 3.69 against 3.76 ms)
-    pairs, block_n = tile_choice(n, want, sm_count(), USE_PAIRS, True, k, narrow=head_dim == 64)
     _check(lib.hfee_gemm_tcgen05_rope(a.data_ptr(), _rows(a, "a"), w.data_ptr(), _rows(w, "w"), n, want, k, _ptr(cs),
                                       positions.data_ptr(), slot_of_token.data_ptr(), q_out.data_ptr(),
                                       _rows(q_out, "q_out"), _ptr(k_pool), _ptr(v_pool), block_table.data_ptr(),
                                       block_table.shape[1], page_size, heads, kv_heads, head_dim, int(interleaved),
-                                      block_n, int(pairs), _status().data_ptr(), _stream()), lib)
+                                      _status().data_ptr(), _stream()), lib)
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor, granule: Optional[int] = None) -> None:
@@ -509,8 +504,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
     assert w.shape[1] == k and a.dtype == w.dtype == torch.bfloat16
     assert tuple(out.shape) == (m, n // 2 if epilogue in EPI_GATED else n)
     if block_n is None:
-        split = USE_STREAM_K if stream_k is None else stream_k          # a caller that asks for the split by K gets a kind that has it
-        pairs, block_n = tile_choice(m, n, sm_count(), USE_PAIRS and stream_k is not True, epilogue == EPI_STORE, k, split)
+        pairs, block_n = tile_choice(m, n, sm_count(), USE_PAIRS, epilogue == EPI_STORE)
         if pairs:
             gemm_tcgen05_pair(a, w, out, epilogue, block_n)
             return
@@ -524,46 +518,28 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
 
 
 USE_PAIRS = True
-# Times of the tcgen05 products' kinds of tile (pairs of CTAs?, columns): a fixed part per round of tiles (one on every SM or pair of
-# SMs) and a part per 1,024 of K, us, beside LAUNCH once: a persistent kernel pays its start and last epilogue once.  Fitted to 3,600
-# measured products (65 to 2,048 rows, 192 to 128,256 columns, K = 256 to 14,336, plain, accumulating and gated), mean error 6 %.
-TILE_TIMES = {(False, 128): (1.1, 4.48), (False, 192): (1.3, 5.29), (False, 256): (1.6, 5.73), (True, 192): (1.7, 3.74),
-              (True, 256): (2.4, 4.85)}
-LAUNCH, HAND_OVER, HAND_OVER_PIECE = 3.0, 3.0, 0.5       # the last two for 128 columns: partial tiles of a product split by K
-
-
-def split_pieces(tiles: int, k: int, sms: int) -> int:
-    """CTAs that share the K blocks of every tile (the rule of the launch: ``plan_stream_k`` in gemm_tcgen05.cu)."""
-    blocks = -(-k // 64)
-    if tiles * 2 > sms or blocks < 64:
-        return 1
-    pieces = min(sms // tiles, 4)
-    while pieces > 1 and blocks // pieces < 8:
-        pieces -= 1
-    return pieces
+# What a round of tiles takes, one on every SM (or pair of SMs), against a round of single-CTA tiles of 128 x 256.  Measured
+# with one round of each (us at K = 2,048 / 8,192 / 14,336): 128 x 128 13.5 / 40 / 64, 128 x 256 17.6 / 56 / 92, pairs of CTAs on
+# 256 x 256 16.4 / 47 / 72; tiles of 192 columns take 0.8 of those of 256 plus their fixed part.
+ROUND_128, ROUND_192, ROUND_256, ROUND_PAIR_192, ROUND_PAIR_256 = 0.72, 0.86, 1.0, 0.70, 0.85
 
 
 @functools.lru_cache(maxsize=4096)
-def tile_choice(m: int, n: int, sms: int, pairs: bool, store: bool, k: int = 2048, split: bool = False, narrow: bool = True):
-    """(pairs of CTAs?, columns of a tile) of the tcgen05 product of m rows and n columns: the kind that TILE_TIMES say takes least.
-    A kind that leaves its last round nearly empty gives way to one that does not (564 rows x 4,096 columns x K = 14,336: 160 tiles of
-    128 x 128 are two rounds on 148 SMs, 190 us, 48 pair tiles one, 70 us; 1,100 x 4,096 x 4,096: 80 pair tiles are two rounds of
-    74, 44 us, 144 single tiles one, 31 us), and tiles so few that their K is split (``split``) are weighed with their hand-over (256 x 768 x
-    8,192: 12 tiles of 128 x 128 in four pieces each 20 us, 4 pair tiles of 192 columns 32 us).  Over the 1,041 shapes measured the choice takes
-    0.3 % longer than the best kind of each, 12 % at worst; by rounds alone 3 and 65 %.  Pairs need more than 128 rows; tiles of 192
-    columns are taken where they divide the columns (``narrow``; by pairs only in plain stores)."""
-    best = None
-    for (two, columns), (fixed, per_k) in TILE_TIMES.items():
-        if two and not (pairs and m > 128 and sms > 1 and (columns == 256 or store)) or columns == 192 and (n % 192 or not narrow):
-            continue
-        tiles = -(-m // (256 if two else 128)) * -(-n // columns)
-        pieces = split_pieces(tiles, k, sms) if split and not two else 1
-        time = LAUNCH + -(-tiles // (sms // 2 if two else sms)) * (fixed + per_k * k / 1024 / pieces)
-        if pieces > 1:
-            time += (HAND_OVER + HAND_OVER_PIECE * pieces) * columns / 128
-        if best is None or time < best[0]:
-            best = time, (two, columns)
-    return best[1]
+def tile_choice(m: int, n: int, sms: int, pairs: bool, store: bool):
+    """(pairs of CTAs?, columns of a tile) of the tcgen05 product of m rows and n columns: the kind whose rounds of tiles take
+    least, so a kind that leaves its last round nearly empty gives way to one that does not.  564 rows x 4,096 columns x K = 14,336:
+    160 tiles of 128 x 128 are two rounds on 148 SMs (190 us), 48 pair tiles one (70 us); 1,100 x 4,096 x 4,096: 80 pair tiles are
+    two rounds of 74 (44 us), 144 single tiles one (31 us).  Pairs need more than 128 rows; tiles of 192 columns are taken where
+    they divide the columns (by pairs only in plain stores)."""
+    rounds = lambda rows, cols, units: -(-(-(-m // rows) * -(-n // cols)) // units)
+    kinds = [(rounds(128, 256, sms) * ROUND_256, False, 256), (rounds(128, 128, sms) * ROUND_128, False, 128)]
+    if n % 192 == 0:
+        kinds.append((rounds(128, 192, sms) * ROUND_192, False, 192))
+    if pairs and m > 128 and sms > 1:
+        kinds.append((rounds(256, 256, sms // 2) * ROUND_PAIR_256, True, 256))
+        if n % 192 == 0 and store:
+            kinds.append((rounds(256, 192, sms // 2) * ROUND_PAIR_192, True, 192))
+    return min(kinds)[1:]
 
 
 def gemm_tcgen05_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE, block_n: int = 256) -> None:
@@ -1378,7 +1354,7 @@ def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, ba: torch.
     vectors per head first (q also times dim^-1/2), beta = sigmoid(b) and g = exp(-exp(a_log) softplus(a + dt_bias)).
     ``qkv`` rows hold the queries and keys of ``qk_heads`` heads and the values of ``heads`` heads at the given
     column offsets, ``ba`` rows one b and one a per head.  ``out`` is float32 [n, heads * vdim].  With ``workspace``
-    (float32, see :func:`delta_rule_workspace`) a step that has a portion of several tokens runs as two kernels: what
+    (float32, see :func:`channel_delta_workspace`) a step that has a portion of several tokens runs as two kernels: what
     does not depend on the state for all tiles of 16 tokens at once, then the walk over each request's tiles."""
     lib = library()
     n = qkv.shape[0]
@@ -1393,16 +1369,7 @@ def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, ba: torch.
                                step.cu_tokens.data_ptr(), step.slots.data_ptr(), out.data_ptr(), _rows(out, "out"), step.r,
                                heads, qk_heads, dim, vdim, int(write_state), step.n, step.max_new, _ptr(workspace),
                                workspace.numel() if workspace is not None else 0, _status().data_ptr(), _stream()), lib)
-    count_launches(lib.hfee_delta_rule_launches(step.max_new, step.r, step.n, heads, dim, vdim,
-                                                workspace.numel() if workspace is not None else 0) - 1)
-
-
-def delta_rule_workspace(requests: int, tokens: int, heads: int, qk_heads: int, dim: int, vdim: Optional[int] = None) -> int:
-    """Floats of workspace the two-kernel delta rule takes for steps of at most ``tokens`` tokens in ``requests`` requests, with
-    values of ``vdim`` numbers (None: as many as the keys); 0 for values too long for it (the one-kernel form runs).  Every tile of
-    16 tokens and every request's last one needs, per head, three matrices [16, dim] and two [16, vdim]: 102 MB for 2,048 tokens of 24
-    requests with 32 heads of 64, 203 MB with heads of 128."""
-    return int(library().hfee_delta_rule_workspace(requests, tokens, heads, dim, dim if vdim is None else vdim))
+    count_launches(lib.hfee_delta_rule_launches(step.max_new, dim, vdim, int(workspace is not None)) - 1)
 
 
 def channel_delta(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, b: torch.Tensor, z: torch.Tensor, a_log: torch.Tensor,
@@ -2299,10 +2266,9 @@ for _name in ("rmsnorm_add_norm", "latent_attention", "linear_act", "attention_s
               "head_norm_gate", "unary_act", "head_gate", "attention_simt_masked", "short_conv", "linear_attention", "rmsnorm_add", "norm_gate", "gated_act", "scale_", "cast_rows", "sigmoid_attention",
               "qk_norm_rope_cache", "embed", "rmsnorm", "rope_table", "rope_cache_write", "swiglu", "linear", "linear_normed", "linear_swiglu", "linear_rope_cache",
               "linear_swiglu_normed", "paged_attention", "paged_attention_rope", "sample", "argmax", "sample_chain",
-              "mingru", "selective_scan", "distance_attention", "moe_route", "moe_plan", "moe_experts", "moe_experts_grouped", "moe_experts_few", "moe_combine",
+              "mingru", "selective_scan", "distance_attention", "moe_route", "moe_plan", "moe_experts", "moe_experts_grouped", "moe_combine",
               "clamped_glu", "linear_clamped_glu", "depth_average", "scaled_add_norm", "scaled_add", "add_sinusoid", "softcap_",
               "channel_delta", "stream_step", "latent_attend_prepare", "softmax_attention", "attention_prepare", "gated_recurrence",
-              "add_bias", "layernorm", "embed_bigram",
               "head_norm_gate_scaled", "moe_route_grouped", "moe_route_chosen", "head_scan", "gate_parts_norm", "embed_norm"):
     globals()[_name] = _measurable(globals()[_name])
 del _name
