@@ -121,9 +121,10 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
       if constexpr (SIGMOID) {
         p = key <= end ? 1.f / (1.f + expf(-(s * h_scale + h_bias))) : 0.f;
       } else {
-        float m_new = fmaxf(m, warp_max(s));
-        p = key <= end ? expf(s - m_new) : 0.f;
-        float alpha = expf(m - m_new);          // exp(-inf) = 0 on the first block
+        // a part may have seen no finite score yet (its block can be one key): its weights are 0, not exp(inf - inf)
+        const float m_new = fmaxf(m, warp_max(s)), m_use = m_new == -INFINITY ? 0.f : m_new;
+        p = key <= end ? expf(s - m_use) : 0.f;
+        const float alpha = expf(m - m_use);    // exp(-inf) = 0 on the first block
         l = l * alpha + warp_sum(p);
 #pragma unroll
         for (int j = 0; j < DPL; ++j) o[j] *= alpha;
@@ -148,6 +149,7 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
   if (warp != 0) return;
   m = m_s[0];
   for (int w = 1; w < parts; ++w) m = fmaxf(m, m_s[w]);
+  if (m == -INFINITY) m = 0.f;
   l = 0.f;
 #pragma unroll
   for (int j = 0; j < DPL; ++j) o[j] = 0.f;
