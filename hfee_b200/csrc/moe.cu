@@ -33,6 +33,9 @@ constexpr int THREADS = 256;
 constexpr int PLAN_THREADS = 1024;
 constexpr int MAX_EXPERTS = 1024;
 
+// The plans take a number that is no expert's for the nearest one's, so that nothing behind them reads or writes out of range.
+__device__ __forceinline__ int expert_of(int choice, int experts) { return min(max(choice, 0), experts - 1); }
+
 __global__ void moe_route_kernel(const float* __restrict__ logits, int experts, int top, float scale, int* __restrict__ choice,
                                  float* __restrict__ weight, int n) {
   extern __shared__ float score_s[];       // [warps][experts]
@@ -65,6 +68,7 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int experts, 
       const int oa = __shfl_xor_sync(0xffffffffu, at, o);
       if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
     }
+    if (at >= experts) { at = 0; best = NAN; }               // no score is left that is a number: an expert that exists, a weight that shows it
     if (lane == 0) {
       choice[(long long)t * top + k] = at;
       weight[(long long)t * top + k] = best / sum * scale;
@@ -122,6 +126,7 @@ __global__ void moe_route_grouped_kernel(const float* __restrict__ logits, int l
       const int oa = __shfl_xor_sync(0xffffffffu, at, o);
       if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
     }
+    if (at >= experts) { at = 0; best = NAN; }               // as above
     sum += best;
     if (lane == 0) {
       choice[(long long)t * top + k] = at;
@@ -184,7 +189,7 @@ moe_plan_kernel(const int* __restrict__ choice, int pairs, int experts, int* __r
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[choice[i]], 1);
+  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[expert_of(choice[i], experts)], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int off = 0, tile = 0;
@@ -206,7 +211,7 @@ moe_plan_kernel(const int* __restrict__ choice, int pairs, int experts, int* __r
     }
   for (int j = first_tile[experts] + threadIdx.x; j < max_tiles; j += PLAN_THREADS) tile_expert[j] = -1;
   for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) {
-    const int e = choice[i];
+    const int e = expert_of(choice[i], experts);
     sorted[off_s[e] + atomicAdd(&cursor[e], 1)] = i;
   }
 }
@@ -221,7 +226,7 @@ moe_plan_tiles_kernel(const int* __restrict__ choice, int pairs, int experts, in
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[choice[i]], 1);
+  for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) atomicAdd(&count[expert_of(choice[i], experts)], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int tile = 0;
@@ -239,7 +244,7 @@ moe_plan_tiles_kernel(const int* __restrict__ choice, int pairs, int experts, in
   for (long long r = threadIdx.x; r < (long long)used * tile_rows; r += PLAN_THREADS) row_pair[r] = -1;
   __syncthreads();
   for (int i = threadIdx.x; i < pairs; i += PLAN_THREADS) {
-    const int e = choice[i];
+    const int e = expert_of(choice[i], experts);
     const int row = first_tile[e] * tile_rows + atomicAdd(&cursor[e], 1);
     place_of_pair[i] = row;
     row_pair[row] = i;

@@ -34,7 +34,7 @@ __device__ __forceinline__ uint4 load_weights(const bf16* p) {
 template <bool GATED>
 __global__ void __launch_bounds__(FEW_WARPS * 32, 4)
 moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16* __restrict__ w, int rows, int K,
-               const int* __restrict__ choice, int pairs, void* __restrict__ out, long long ld_out, float limit, float alpha, float shift) {
+               int experts, const int* __restrict__ choice, int pairs, void* __restrict__ out, long long ld_out, float limit, float alpha, float shift) {
   __shared__ float part_s[2][FEW_WARPS][FEW_ROWS][8];
   __shared__ int expert_s[FEW_PAIRS];
   __shared__ unsigned members_s[FEW_PAIRS];
@@ -47,7 +47,8 @@ moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16
   }
   if (warp == 0) {
     // the experts in the order of their first pair, each with at most eight of its pairs (one that has more comes again)
-    const int mine = lane < pairs ? choice[lane] : -1;
+    // (a number that is no expert's counts as the nearest one's: nothing is read past the last matrix)
+    const int mine = lane < pairs ? min(max(choice[lane], 0), experts - 1) : -1;
     const unsigned same = __match_any_sync(0xffffffffu, mine);
     unsigned leaders = __ballot_sync(0xffffffffu, mine >= 0 && __ffs(same) - 1 == lane);
     int lists = 0;
@@ -183,16 +184,17 @@ HFEE_API int hfee_moe_few_gate_up(const void* x, long long ld_x, int top, const 
   const int rc = few_check("moe_few_gate_up", x, ld_x, w, 2 * inner, width, experts, pairs);
   if (rc != HFEE_OK) return rc;
   HFEE_REQUIRE(top > 0 && inner % 4 == 0 && ld_hidden >= inner && limit > 0.f, "moe_few_gate_up: bad sizes");
-  hfee_launch(moe_few_kernel<true>, dim3(few_blocks(2 * inner, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)x, ld_x, top, (const bf16*)w, 2 * inner, width, choice, pairs, hidden, ld_hidden, limit, alpha, shift);
+  hfee_launch(moe_few_kernel<true>, dim3(few_blocks(2 * inner, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)x, ld_x, top, (const bf16*)w, 2 * inner, width, experts, choice, pairs, hidden, ld_hidden, limit, alpha, shift);
   return hfee_check_launch("moe_few_gate_up");
 }
 
-// hidden: [pairs, inner] bfloat16; w: [experts, width, inner]; pair_out: [pairs, width] float32.
+// hidden: [pairs, inner] bfloat16; w: [experts, width, inner]; pair_out: [pairs, width] float32.  To be launched right behind
+// hfee_moe_few_gate_up with the same choices, which it reads before it waits for that kernel.
 HFEE_API int hfee_moe_few_down(const void* hidden, long long ld_hidden, const void* w, int inner, int width, int experts, const int* choice,
                                int pairs, float* pair_out, cudaStream_t stream) {
   if (pairs == 0) return HFEE_OK;
   const int rc = few_check("moe_few_down", hidden, ld_hidden, w, width, inner, experts, pairs);
   if (rc != HFEE_OK) return rc;
-  hfee_launch(moe_few_kernel<false>, dim3(few_blocks(width, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)hidden, ld_hidden, 1, (const bf16*)w, width, inner, choice, pairs, pair_out, (long long)width, 0.f, 0.f, 0.f);
+  hfee_launch(moe_few_kernel<false>, dim3(few_blocks(width, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)hidden, ld_hidden, 1, (const bf16*)w, width, inner, experts, choice, pairs, pair_out, (long long)width, 0.f, 0.f, 0.f);
   return hfee_check_launch("moe_few_down");
 }
