@@ -360,8 +360,8 @@ moe_combine_kernel(const float* __restrict__ pair_out, const float* __restrict__
                    const float* __restrict__ extra, const float* __restrict__ extra_gate, long long ld_gate) {
   pdl_wait();
   pdl_launch_dependents();
-  const long long t = blockIdx.y;
-  const int c = (blockIdx.x * THREADS + threadIdx.x) * VEC;
+  const long long t = blockIdx.x;              // any number of tokens fits the grid's first axis only
+  const int c = (blockIdx.y * THREADS + threadIdx.x) * VEC;
   if (c >= width) return;
   auto read = [](const float* p, float (&v)[VEC]) {
     if constexpr (VEC == 4) {
@@ -494,10 +494,9 @@ HFEE_API int hfee_moe_combine_extra(const float* pair_out, const float* weight, 
   if (n == 0) return HFEE_OK;
   HFEE_REQUIRE(n > 0 && top > 0 && width > 0, "moe_combine: bad sizes");
   HFEE_REQUIRE(extra != nullptr || extra_gate == nullptr, "moe_combine: a gate without the term it gates");
-  HFEE_REQUIRE(n <= 65535, "moe_combine: %d tokens are too many", n);
   const bool vec = width % 4 == 0 && ((uintptr_t)pair_out | (uintptr_t)y | (uintptr_t)extra) % 16 == 0;
   const int per_block = THREADS * (vec ? 4 : 1);
-  hfee_launch(vec ? moe_combine_kernel<4> : moe_combine_kernel<1>, dim3((width + per_block - 1) / per_block, n), dim3(THREADS), 0, stream,
+  hfee_launch(vec ? moe_combine_kernel<4> : moe_combine_kernel<1>, dim3(n, (width + per_block - 1) / per_block), dim3(THREADS), 0, stream,
               pair_out, weight, place, top, y, width, accumulate, extra, extra_gate, ld_gate);
   return hfee_check_launch("moe_combine");
 }

@@ -39,7 +39,7 @@ def test_few_pairs(n, top, experts, width, inner, limit, alpha, shift):
     assert bool((out[-1] == 7.0).all())
 
 
-@pytest.mark.parametrize("n,top,width", [(1, 1, 4), (3, 2, 2048), (2, 6, 1030), (5, 9, 12), (300, 2, 1028)])
+@pytest.mark.parametrize("n,top,width", [(1, 1, 4), (3, 2, 2048), (2, 6, 1030), (5, 9, 12), (300, 2, 1028), (70000, 1, 8), (66000, 2, 5)])
 @pytest.mark.parametrize("accumulate,extra,placed", [(False, False, False), (True, True, True), (True, False, True), (False, True, False)])
 def test_weighted_sum(n, top, width, accumulate, extra, placed):
     from hfee_b200.kernels import ops
