@@ -2266,9 +2266,10 @@ for _name in ("rmsnorm_add_norm", "latent_attention", "linear_act", "attention_s
               "head_norm_gate", "unary_act", "head_gate", "attention_simt_masked", "short_conv", "linear_attention", "rmsnorm_add", "norm_gate", "gated_act", "scale_", "cast_rows", "sigmoid_attention",
               "qk_norm_rope_cache", "embed", "rmsnorm", "rope_table", "rope_cache_write", "swiglu", "linear", "linear_normed", "linear_swiglu", "linear_rope_cache",
               "linear_swiglu_normed", "paged_attention", "paged_attention_rope", "sample", "argmax", "sample_chain",
-              "mingru", "selective_scan", "distance_attention", "moe_route", "moe_plan", "moe_experts", "moe_experts_grouped", "moe_combine",
+              "mingru", "selective_scan", "distance_attention", "moe_route", "moe_plan", "moe_experts", "moe_experts_grouped", "moe_experts_few", "moe_combine",
               "clamped_glu", "linear_clamped_glu", "depth_average", "scaled_add_norm", "scaled_add", "add_sinusoid", "softcap_",
               "channel_delta", "stream_step", "latent_attend_prepare", "softmax_attention", "attention_prepare", "gated_recurrence",
+              "add_bias", "layernorm", "embed_bigram",
               "head_norm_gate_scaled", "moe_route_grouped", "moe_route_chosen", "head_scan", "gate_parts_norm", "embed_norm"):
     globals()[_name] = _measurable(globals()[_name])
 del _name

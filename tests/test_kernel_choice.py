@@ -34,3 +34,19 @@ def test_key_splits_fill_the_gpu_about_once(sms):
     few = [ops.attention_splits(r, 8, 1 << 16, sms) for r in range(1, ops.FEW_PAIRS // 8 + 1)]
     many = [ops.attention_splits(r, 8, 1 << 16, sms) for r in range(ops.FEW_PAIRS // 8 + 1, 80)]
     assert all(a >= b for a, b in zip(few, few[1:])) and all(a >= b for a, b in zip(many, many[1:]))
+
+
+def test_every_launch_of_a_part_can_be_left_out():
+    """What a part or the sampler calls and that launches a kernel itself goes through the switch that ``bench.py --breakdown``
+    measures classes with; else a class left out would still run it."""
+    import ast
+    import inspect
+    import pathlib
+    package = pathlib.Path(ops.__file__).parent.parent
+    called = {node.func.attr for path in [*package.glob("parts/*.py"), *package.glob("sampling/*.py")]
+              for node in ast.walk(ast.parse(path.read_text()))
+              if isinstance(node, ast.Call) and isinstance(node.func, ast.Attribute)
+              and isinstance(node.func.value, ast.Name) and node.func.value.id == "ops"}
+    launching = [name for name in called if "_check(lib." in inspect.getsource(inspect.unwrap(getattr(ops, name)))]
+    assert len(launching) > 40 and "moe_experts_few" in launching
+    assert [name for name in launching if not hasattr(getattr(ops, name), "__wrapped__")] == []
