@@ -476,14 +476,23 @@ int hfee_delta_tiles(const void* qkv, long long ld_qkv, int q_off, int k_off, in
                      long long ld_out, int requests, int heads, int qk_heads, int dim, int vdim, int write_state, int n_tokens, int max_new,
                      float* workspace, long long workspace_floats, int* status, cudaStream_t stream);
 
-// Launches hfee_delta_rule makes for a step.
-HFEE_API int hfee_delta_rule_launches(int max_new, int dim, int vdim, int has_workspace) {
-  return has_workspace && max_new > 1 && hfee_delta_tiles_fit(dim, vdim) ? 2 : 1;
+HFEE_API long long hfee_channel_delta_workspace(int requests, int n_tokens, int heads, int dim, int vdim);
+
+// Floats of workspace with which a step that has a portion of several tokens runs on the kernels of channel_delta.cu; 0: its values are
+// too long for those.
+HFEE_API long long hfee_delta_rule_workspace(int requests, int n_tokens, int heads, int dim, int vdim) {
+  return hfee_delta_tiles_fit(dim, vdim) ? hfee_channel_delta_workspace(requests, n_tokens, heads, dim, vdim) : 0;
 }
 
-// With a workspace (hfee_channel_delta_workspace floats) and a portion of more than one token in the step (max_new > 1), the step
-// runs on the kernels of channel_delta.cu; without one, for single tokens and for values too long for those, as one kernel.
-// `status` (device int) is set to 1 if a kernel gave up a wait.
+// Launches hfee_delta_rule makes for a step.
+HFEE_API int hfee_delta_rule_launches(int max_new, int requests, int n_tokens, int heads, int dim, int vdim, long long workspace_floats) {
+  const long long need = hfee_delta_rule_workspace(requests, n_tokens, heads, dim, vdim);
+  return max_new > 1 && need > 0 && workspace_floats >= need ? 2 : 1;
+}
+
+// With a workspace (hfee_delta_rule_workspace floats) and a portion of more than one token in the step (max_new > 1), the step
+// runs on the kernels of channel_delta.cu; without one, for single tokens, for values too long for those, and with a workspace that
+// is large enough for values of the keys' length but not for these, as one kernel.  `status` (device int) is set to 1 if a kernel gave up a wait.
 // qkv rows: head g's query at q_off + g * dim, its key at k_off + g * dim (g < qk_heads; head h of `heads` uses
 // g = h / (heads / qk_heads)), head h's value at v_off + h * vdim.  ba rows: b_off + h and a_off + h.
 // state: [slots, heads, dim, vdim] float32.  out: float32 [n, heads * vdim].
@@ -500,7 +509,10 @@ HFEE_API int hfee_delta_rule(const void* qkv, long long ld_qkv, int q_off, int k
                   (uintptr_t)qkv % 16 == 0;
   DeltaArgs p{ld_qkv, ld_ba, ld_out, q_off, k_off, v_off, b_off, a_off, heads, qk_heads, dim, vdim, write_state, vec};
   HFEE_REQUIRE(dtype == HFEE_F32 || dtype == HFEE_BF16, "delta_rule: unknown dtype %d", dtype);
-  if (hfee_delta_rule_launches(max_new, dim, vdim, workspace != nullptr) == 2)
+  if (workspace != nullptr && max_new > 1 && hfee_delta_tiles_fit(dim, vdim))
+    HFEE_REQUIRE(workspace_floats >= hfee_channel_delta_workspace(requests, n_tokens, heads, dim, vdim < dim ? vdim : dim),
+                 "delta_rule: the workspace is too small");
+  if (hfee_delta_rule_launches(max_new, requests, n_tokens, heads, dim, vdim, workspace != nullptr ? workspace_floats : 0) == 2)
     return hfee_delta_tiles(qkv, ld_qkv, q_off, k_off, v_off, (const char*)ba + (long long)b_off * (dtype == HFEE_F32 ? 4 : 2), ld_ba,
                             a_off - b_off, dtype, a_log, dt_bias, state, cu_tokens, slots, out, ld_out, requests, heads, qk_heads, dim, vdim,
                             write_state, n_tokens, max_new, workspace, workspace_floats, status, stream);

@@ -125,7 +125,7 @@ _SIGNATURES = {
     "hfee_moe_route_grouped": [_P, _L, _I, _I, _I, _I, _I, _F, _P, _P, _P],
     "hfee_conv_act_launches": [_I, _I, _I],
     "hfee_delta_rule": [_P, _L, _I, _I, _I, _P, _L, _I, _I, _I, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _P, _L, _P, _P],
-    "hfee_delta_rule_launches": [_I, _I, _I, _I],
+    "hfee_delta_rule_launches": [_I, _I, _I, _I, _I, _I, _L],
     "hfee_head_norm_gate": [_P, _L, _P, _F, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
     "hfee_unary_act": [_P, _L, _P, _L, _I, _I, _I, _I, _P],
     "hfee_head_gate": [_P, _L, _P, _L, _I, _I, _I, _I, _P],
@@ -156,6 +156,8 @@ def library() -> ctypes.CDLL:
     lib.hfee_attention_tc_supports.restype = _I
     lib.hfee_linear_attention_chunked_workspace.restype = _L
     lib.hfee_linear_attention_chunked_workspace.argtypes = [_I, _I, _I, _I, _I]
+    lib.hfee_delta_rule_workspace.restype = _L
+    lib.hfee_delta_rule_workspace.argtypes = [_I, _I, _I, _I, _I]
     lib.hfee_channel_delta_workspace.restype = _L
     lib.hfee_channel_delta_workspace.argtypes = [_I, _I, _I, _I, _I]
     lib.hfee_gated_recurrence_workspace.restype = _L
@@ -1354,7 +1356,7 @@ def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, ba: torch.
     vectors per head first (q also times dim^-1/2), beta = sigmoid(b) and g = exp(-exp(a_log) softplus(a + dt_bias)).
     ``qkv`` rows hold the queries and keys of ``qk_heads`` heads and the values of ``heads`` heads at the given
     column offsets, ``ba`` rows one b and one a per head.  ``out`` is float32 [n, heads * vdim].  With ``workspace``
-    (float32, see :func:`channel_delta_workspace`) a step that has a portion of several tokens runs as two kernels: what
+    (float32, see :func:`delta_rule_workspace`) a step that has a portion of several tokens runs as two kernels: what
     does not depend on the state for all tiles of 16 tokens at once, then the walk over each request's tiles."""
     lib = library()
     n = qkv.shape[0]
@@ -1369,7 +1371,16 @@ def delta_rule(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, ba: torch.
                                step.cu_tokens.data_ptr(), step.slots.data_ptr(), out.data_ptr(), _rows(out, "out"), step.r,
                                heads, qk_heads, dim, vdim, int(write_state), step.n, step.max_new, _ptr(workspace),
                                workspace.numel() if workspace is not None else 0, _status().data_ptr(), _stream()), lib)
-    count_launches(lib.hfee_delta_rule_launches(step.max_new, dim, vdim, int(workspace is not None)) - 1)
+    count_launches(lib.hfee_delta_rule_launches(step.max_new, step.r, step.n, heads, dim, vdim,
+                                                workspace.numel() if workspace is not None else 0) - 1)
+
+
+def delta_rule_workspace(requests: int, tokens: int, heads: int, qk_heads: int, dim: int, vdim: Optional[int] = None) -> int:
+    """Floats of workspace the two-kernel delta rule takes for steps of at most ``tokens`` tokens in ``requests`` requests, with
+    values of ``vdim`` numbers (None: as many as the keys); 0 for values too long for it (the one-kernel form runs).  Every tile of
+    16 tokens and every request's last one needs, per head, three matrices [16, dim] and two [16, vdim]: 102 MB for 2,048 tokens of 24
+    requests with 32 heads of 64, 203 MB with heads of 128."""
+    return int(library().hfee_delta_rule_workspace(requests, tokens, heads, dim, dim if vdim is None else vdim))
 
 
 def channel_delta(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int, b: torch.Tensor, z: torch.Tensor, a_log: torch.Tensor,

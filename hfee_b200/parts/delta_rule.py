@@ -87,8 +87,8 @@ class GatedDeltaRule(Mixer):
         workspace = None
         if step.max_new > 1:
             # the state-independent part of every tile of 16 tokens; sized once for the engine's limits
-            workspace = rt.scratch("delta_tiles", (ops.channel_delta_workspace(
-                rt.max_requests, rt.max_tokens, self.heads, self.key_dim, self.value_dim),), torch.float32)
+            floats = ops.delta_rule_workspace(rt.max_requests, rt.max_tokens, self.heads, self.qk_heads, self.key_dim, self.value_dim)
+            workspace = rt.scratch("delta_tiles", (floats,), torch.float32) if floats else None
         ops.delta_rule(qkv, 0, self.qk_cols, 2 * self.qk_cols, proj, self.b_at, self.a_at, self.a_log, self.dt_bias,
                        cache.states["recurrent"], step, o, self.heads, self.qk_heads, self.key_dim, self.value_dim,
                        writes_cache, workspace)

@@ -31,7 +31,7 @@ def _exact(q, k, v, b, a, a_log, dt_bias, s):
 # portions around a tile of 16, single tokens beside longer ones; key sizes around 32 and 64 and not of whole 16 bytes; values
 # around a group of 16 columns and too long for a tile's solution; a before b and after it; offsets off 16 bytes
 @pytest.mark.parametrize("heads,groups,dim,vdim,portions", [(4, 2, 64, 64, [17, 1, 40]), (3, 1, 20, 17, [16, 15, 33]), (2, 2, 33, 8, [50]),
-                                                            (2, 1, 128, 40, [31, 2]), (1, 1, 8, 3000, [18])])
+                                                            (2, 1, 128, 40, [31, 2]), (1, 1, 8, 3000, [18]), (1, 1, 8, 3200, [18])])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("a_first,shift,write", [(False, 0, True), (True, 3, False)])
 def test_tiles_match_one_by_one(heads, groups, dim, vdim, portions, dtype, a_first, shift, write):
@@ -65,3 +65,37 @@ def test_tiles_match_one_by_one(heads, groups, dim, vdim, portions, dtype, a_fir
             assert (d(s[2 * i + 1]) - (last if write else d(state[2 * i + 1]))).norm() <= 1e-5 * last.norm()
     for out, s in results:
         assert torch.equal(s[::2], state[::2])
+
+
+def test_workspaces_of_every_size(monkeypatch):
+    """A workspace of the size asked for takes the tiles; one for values of the keys' length runs longer values as one kernel; values
+    too long for the tiles want none; less is refused."""
+    from hfee_b200.kernels import ops
+    heads, groups, dim, portions = 2, 1, 32, [20, 3]
+    step = _step(portions)
+    launches = []
+    real = ops.count_launches
+    monkeypatch.setattr(ops, "count_launches", lambda k: (launches.append(k), real(k)))
+
+    def run(vdim, floats):
+        g = torch.Generator().manual_seed(vdim)
+        rand = lambda *s: torch.randn(*s, generator=g).to(DEV)
+        qkv, ba, state = rand(step.n, 2 * groups * dim + heads * vdim), rand(step.n, 2 * heads), rand(4, heads, dim, vdim)
+        out = torch.empty(step.n, heads * vdim, device=DEV)
+        ws = torch.empty(floats, device=DEV) if floats else None
+        launches.clear()
+        ops.delta_rule(qkv, 0, groups * dim, 2 * groups * dim, ba, 0, heads, rand(heads), rand(heads), state, step, out, heads, groups, dim,
+                       vdim, True, ws)
+        ops.check_status()
+        return out, state, sum(launches)
+    size = lambda *v: ops.delta_rule_workspace(step.r, step.n, heads, groups, dim, *v)
+    assert size() == size(dim) < size(100) and size(5000) == 0
+    for vdim, floats, kernels in ((dim, size(), 2), (8, size(8), 2), (8, size(), 2), (100, size(100), 2), (100, size(), 1), (5000, size(), 1)):
+        got, want = run(vdim, floats), run(vdim, 0)
+        assert got[2] - want[2] == kernels - 1
+        for a, b in zip(got[:2], want[:2]):
+            assert torch.equal(a, b) if kernels == 1 else (a - b).norm() <= 2e-5 * b.norm()
+    for vdim, floats in ((dim, size() - 1), (8, size(8) - 1), (100, size() - 1)):
+        with pytest.raises(ops.KernelLibraryError):
+            run(vdim, floats)
+
