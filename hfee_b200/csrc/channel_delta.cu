@@ -24,9 +24,11 @@
 // for all tiles at once, and `channel_delta_walk` goes through a request's tiles with three small products per tile.
 // The ratios G_t / G_j are running products of decays from j on (never a quotient of two products, which could be 0 / 0),
 // so strong decays underflow to zero and nothing overflows.  With one decay per head (the plain delta rule of delta_rule.cu) the
-// same kernels run with that decay in every channel: 2,048 tokens, 32 heads on 8, sizes 64, in 190 us where a walk without solved
-// tiles (16 substitution steps of a warp between the products with the state) took 345.  The result depends on how a prompt was cut only through the
-// order of float32 sums.
+// same kernels run, and every ratio is the exponential of a running sum of log-decays from j on: one rounding of an exponential where a
+// product of 16 decays near one has sixteen that lean one way (256 tokens, sizes 256, error of the state against 64 bits: 2.4e-7 by sums,
+// 1.6e-6 by products, 2.7e-7 token by token).  2,048 tokens, 32 heads on 8, sizes 64: 186 us where a walk without solved tiles (16
+// substitution steps of a warp between the products with the state) took 345.  The result depends on how a prompt was cut only through
+// the order of float32 sums.
 //
 // A tile's part of the workspace (its place: (first token of the tile) / 16 + request, different for any two tiles of a
 // step), per head, rows of DP = dim rounded up to 32 floats:  W [16] | P [16] | Khat [16] (= G_last / G_j * k_j) | G_last,
@@ -46,7 +48,7 @@ struct ChannelDeltaArgs {
   int heads, qk_heads, dim, vdim;
   int write_state;
   int vec;                     // rows of q, k, z and dt_bias can be fetched four channels at a time
-  int per_head, a_off;         // per_head: one decay per head, from b's row at a_off + h and dt_bias[h], in place of z
+  int a_off;                   // with one decay per head: its place in b's rows beside the head's b
 };
 
 __device__ __forceinline__ float softplus_cd(float z) { return z > 20.f ? z : log1pf(expf(z)); }
@@ -213,8 +215,9 @@ __host__ __device__ inline long long cd_head_floats(int dim) { return (3ll * CD_
 __host__ __device__ inline int cd_col_tiles(int vdim) { return (vdim + CW_COLS - 1) / CW_COLS; }
 constexpr int CD_UO = 2 * CD_TILE * CW_COLS;
 
-// NI: float4 per lane of a row (a row of DP = 32 * NI floats shared by 8 lanes)
-template <typename T, int NI>
+// NI: float4 per lane of a row (a row of DP = 32 * NI floats shared by 8 lanes).  HEAD: one decay per head, from b's row at a_off + h and
+// dt_bias[h], in place of z.
+template <typename T, int NI, bool HEAD>
 __global__ void __launch_bounds__(CD_THREADS, NI <= 4 ? 6 : 3)
 channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b, const float* __restrict__ z,
                              const float* __restrict__ a_log, const float* __restrict__ dt_bias,
@@ -224,7 +227,8 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
   extern __shared__ __align__(128) float smem[];
   float* k_s = smem;                         // [16][DP]
   float* q_s = k_s + CD_TILE * DP;
-  float* g_s = q_s + CD_TILE * DP;
+  float* g_s = q_s + CD_TILE * DP;           // decays per channel; HEAD: none
+  __shared__ float raw_s[CD_TILE], upto_s[CD_TILE], ratio_s[HEAD ? CD_TILE : 1][CD_TILE];      // HEAD: log-decays; G_t; G_t / G_j
   __shared__ __align__(16) float2 A_s[CD_TILE][CD_TILE], B_s[CD_TILE][CD_TILE];      // -A and B, every number twice: operands of pairs
   __shared__ float beta_s[CD_TILE];
   const int req = blockIdx.z, h = blockIdx.y, tile0 = blockIdx.x * CD_TILE;
@@ -240,11 +244,11 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
   // work of the last part: pairs of columns of the triangular system (key channels, then values), then pairs of key
   // channels once more
   const int value_cols = cd_col_tiles(vdim) * CW_COLS, items = DP + value_cols / 2;
-  float* v_s = g_s + CD_TILE * DP;           // [16][value_cols]
+  float* v_s = g_s + (HEAD ? 0 : CD_TILE * DP);      // [16][value_cols]
   const float b_own = tid < tt ? to_f32<T>(b[(tok0 + tid) * p.ld_b + h]) : 0.f;
   const float rate = expf(a_log[h]);
   // a missing token is the identity: no write, no decay
-  auto head_decay = [&](int t) { return expf(-rate * softplus_cd(to_f32<T>(b[(tok0 + t) * p.ld_b + p.a_off + h]) + dt_bias[h])); };
+  if (HEAD && tid < CD_TILE) raw_s[tid] = tid < tt ? -rate * softplus_cd(to_f32<T>(b[(tok0 + tid) * p.ld_b + p.a_off + h]) + dt_bias[h]) : 0.f;
   if (p.vec) {
 #pragma unroll
     for (int n = 0; n < NI; ++n) {
@@ -254,10 +258,7 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
         const T* row = qkv + (tok0 + t) * p.ld_qkv + (long long)kh * dim + d;
         kv = load4<T>(row + p.k_off);
         qv = load4<T>(row + p.q_off);
-        if (p.per_head) {
-          const float one = head_decay(t);
-          g = make_float4(one, one, one, one);
-        } else {
+        if constexpr (!HEAD) {
           const float4 zz = *reinterpret_cast<const float4*>(z + (tok0 + t) * p.ld_z + (long long)h * dim + d);
           const float4 bb = *reinterpret_cast<const float4*>(dt_bias + (long long)h * dim + d);
           g = make_float4(channel_decay<T>(rate, zz.x + bb.x), channel_decay<T>(rate, zz.y + bb.y), channel_decay<T>(rate, zz.z + bb.z),
@@ -266,7 +267,7 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
       }
       reinterpret_cast<float4*>(k_s)[e] = kv;
       reinterpret_cast<float4*>(q_s)[e] = qv;
-      reinterpret_cast<float4*>(g_s)[e] = g;
+      if constexpr (!HEAD) reinterpret_cast<float4*>(g_s)[e] = g;
     }
   } else {
     for (int e = tid; e < CD_TILE * DP; e += CD_THREADS) {
@@ -276,11 +277,11 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
         const T* row = qkv + (tok0 + t) * p.ld_qkv + (long long)kh * dim + d;
         kv = to_f32<T>(row[p.k_off]);
         qv = to_f32<T>(row[p.q_off]);
-        g = p.per_head ? head_decay(t) : channel_decay<T>(rate, z[(tok0 + t) * p.ld_z + (long long)h * dim + d] + dt_bias[(long long)h * dim + d]);
+        if constexpr (!HEAD) g = channel_decay<T>(rate, z[(tok0 + t) * p.ld_z + (long long)h * dim + d] + dt_bias[(long long)h * dim + d]);
       }
       k_s[e] = kv;
       q_s[e] = qv;
-      g_s[e] = g;
+      if constexpr (!HEAD) g_s[e] = g;
     }
   }
   if (p.vec && vdim % 4 == 0) {
@@ -297,6 +298,20 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
   }
   if (tid < CD_TILE) beta_s[tid] = tid < tt ? 1.f / (1.f + expf(-b_own)) : 0.f;
   __syncthreads();
+  if constexpr (HEAD) {
+    // an exponential of the log-decays' sum over j + 1 .. t each (j = -1: G_t), the missing ones of t < j unused
+    for (int e = tid; e < CD_TILE * (CD_TILE + 1); e += CD_THREADS) {
+      const int t = e / (CD_TILE + 1), j = e - t * (CD_TILE + 1) - 1;
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < CD_TILE; ++i) {
+        const float raw = raw_s[i];
+        if (i > j && i <= t) sum += raw;
+      }
+      if (j < 0) upto_s[t] = expf(sum);
+      else ratio_s[t][j] = expf(sum);
+    }
+  }
   const float q_unit = 1.0f / sqrtf((float)dim);
 #pragma unroll
   for (int half = 0; half < 2; ++half) {       // eight lanes per vector: 16 keys, then 16 queries
@@ -331,7 +346,7 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
       for (int i = 0; i < NI; ++i) {
         const int at = t * (DP / 4) + sl + 8 * i;
         const ulonglong2 kk = k4[at], qq = q4[at];
-        if (t > j) {
+        if (!HEAD && t > j) {
           const ulonglong2 g = g4[at];
           w[i].x = mul_pair(w[i].x, g.x);
           w[i].y = mul_pair(w[i].y, g.y);
@@ -345,6 +360,10 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
       for (int o = 4; o >= 1; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
         c += __shfl_xor_sync(0xffffffffu, c, o);
+      }
+      if constexpr (HEAD) {
+        a *= ratio_s[t][j];
+        c *= ratio_s[t][j];
       }
       if (sl == 0) {
         A_s[t][j] = t > j ? make_float2(-a, -a) : make_float2(0.f, 0.f);
@@ -367,10 +386,12 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
       uint64_t after = pair_of(1.f, 1.f);
 #pragma unroll
       for (int t = CD_TILE - 1; t >= 0; --t) {
-        const uint64_t k = *reinterpret_cast<const uint64_t*>(k_s + t * DP + c), g = *reinterpret_cast<const uint64_t*>(g_s + t * DP + c);
+        const uint64_t k = *reinterpret_cast<const uint64_t*>(k_s + t * DP + c);
+        if constexpr (HEAD) after = pair_of(ratio_s[CD_TILE - 1][t], ratio_s[CD_TILE - 1][t]);
         *reinterpret_cast<uint64_t*>(wh + (2 * CD_TILE + t) * DP + c) = mul_pair(after, k);
-        after = mul_pair(after, g);
+        if constexpr (!HEAD) after = mul_pair(after, *reinterpret_cast<const uint64_t*>(g_s + t * DP + c));
       }
+      if constexpr (HEAD) after = pair_of(upto_s[CD_TILE - 1], upto_s[CD_TILE - 1]);
       *reinterpret_cast<uint64_t*>(wh + 3 * CD_TILE * DP + c) = after;
       continue;
     }
@@ -385,7 +406,8 @@ channel_delta_prepare_kernel(const T* __restrict__ qkv, const T* __restrict__ b,
       asm volatile("" ::: "memory");           // or all the tokens' loads would be moved up here and overflow the registers
       uint64_t r, second;
       if (key) {
-        run = mul_pair(run, *reinterpret_cast<const uint64_t*>(g_s + t * DP + c));
+        if constexpr (HEAD) run = pair_of(upto_s[t], upto_s[t]);
+        else run = mul_pair(run, *reinterpret_cast<const uint64_t*>(g_s + t * DP + c));
         r = mul_pair(run, *reinterpret_cast<const uint64_t*>(k_s + t * DP + c));
         second = mul_pair(run, *reinterpret_cast<const uint64_t*>(q_s + t * DP + c));
       } else {
@@ -605,23 +627,23 @@ int launch_token(const void* qkv, const void* b, const float* z, const float* a_
 #undef HFEE_CD
 }
 
-template <typename T, int NI>
+template <typename T, int NI, bool HEAD>
 int launch_tiles_n(const void* qkv, const void* b, const float* z, const float* a_log, const float* dt_bias, float* state,
                    const int* cu_tokens, const int* slots, float* out, const ChannelDeltaArgs& p, int requests, int max_new,
                    float* ws_head, float* ws_uo, int* status, cudaStream_t stream) {
   constexpr int C = NI <= 4 ? 4 : 2;                          // columns per warp of the walk: what its registers hold
-  const size_t prep = (size_t)CD_TILE * (3 * 32 * NI + cd_col_tiles(p.vdim) * CW_COLS) * sizeof(float);
+  const size_t prep = (size_t)CD_TILE * ((HEAD ? 2 : 3) * 32 * NI + cd_col_tiles(p.vdim) * CW_COLS) * sizeof(float);
   HFEE_REQUIRE(prep <= 200 * 1024, "channel_delta: values of %d numbers per head do not fit shared memory", p.vdim);
   const size_t walk = (size_t)CW_STAGES * ((3 * CD_TILE + 1) * 32 * NI + CD_UO) * sizeof(float);
   if (prep > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(channel_delta_prepare_kernel<T, NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
+    cudaError_t e = cudaFuncSetAttribute(channel_delta_prepare_kernel<T, NI, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
     if (e != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "channel_delta_prepare: %s", cudaGetErrorString(e));
   }
   if (walk > 40 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(channel_delta_walk_kernel<NI, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk);
     if (e != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "channel_delta_walk: %s", cudaGetErrorString(e));
   }
-  hfee_launch(channel_delta_prepare_kernel<T, NI>, dim3((unsigned)((max_new + CD_TILE - 1) / CD_TILE), (unsigned)p.heads, (unsigned)requests),
+  hfee_launch(channel_delta_prepare_kernel<T, NI, HEAD>, dim3((unsigned)((max_new + CD_TILE - 1) / CD_TILE), (unsigned)p.heads, (unsigned)requests),
               dim3(CD_THREADS), prep, stream, (const T*)qkv, (const T*)b, z, a_log, dt_bias, cu_tokens, ws_head, ws_uo, p);
   const int rc = hfee_check_launch("channel_delta_prepare");
   if (rc != HFEE_OK) return rc;
@@ -630,14 +652,14 @@ int launch_tiles_n(const void* qkv, const void* b, const float* z, const float* 
   return hfee_check_launch("channel_delta_walk");
 }
 
-template <typename T>
+template <typename T, bool HEAD = false>
 int launch_tiles(const void* qkv, const void* b, const float* z, const float* a_log, const float* dt_bias, float* state,
                  const int* cu_tokens, const int* slots, float* out, const ChannelDeltaArgs& p, int requests, int max_new,
                  float* ws_head, float* ws_uo, int* status, cudaStream_t stream) {
-#define HFEE_CT(N) case N: return launch_tiles_n<T, N>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, ws_head, ws_uo, status, stream)
+#define HFEE_CT(N) case N: return launch_tiles_n<T, N, HEAD>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, ws_head, ws_uo, status, stream)
   switch (cd_pad(p.dim) / 32) {
     HFEE_CT(1); HFEE_CT(2); HFEE_CT(3); HFEE_CT(4); HFEE_CT(5); HFEE_CT(6); HFEE_CT(7);
-    default: return launch_tiles_n<T, 8>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, ws_head, ws_uo, status, stream);
+    default: return launch_tiles_n<T, 8, HEAD>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, ws_head, ws_uo, status, stream);
   }
 #undef HFEE_CT
 }
@@ -667,7 +689,7 @@ HFEE_API int hfee_channel_delta(const void* qkv, long long ld_qkv, int q_off, in
   HFEE_REQUIRE(dtype == HFEE_F32 || dtype == HFEE_BF16, "channel_delta: unknown dtype %d", dtype);
   const int vec = dim % 4 == 0 && ld_qkv % 4 == 0 && ld_z % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
                   (uintptr_t)qkv % (dtype == HFEE_F32 ? 16 : 8) == 0 && (uintptr_t)z % 16 == 0 && (uintptr_t)dt_bias % 16 == 0;
-  const ChannelDeltaArgs p{ld_qkv, ld_b, ld_z, ld_out, q_off, k_off, v_off, heads, qk_heads, dim, vdim, write_state, vec, 0, 0};
+  const ChannelDeltaArgs p{ld_qkv, ld_b, ld_z, ld_out, q_off, k_off, v_off, heads, qk_heads, dim, vdim, write_state, vec, 0};
   if (max_new == 1) {
     if (dtype == HFEE_F32) return launch_token<float>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, stream);
     return launch_token<__nv_bfloat16>(qkv, b, z, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, stream);
@@ -684,7 +706,7 @@ HFEE_API int hfee_channel_delta(const void* qkv, long long ld_qkv, int q_off, in
 // Values this long still fit the shared memory of a tile's solution.
 int hfee_delta_tiles_fit(int dim, int vdim) {
   return dim > 0 && dim <= CD_MAX_DIM && vdim > 0 &&
-         (long long)CD_TILE * (3 * cd_pad(dim) + (long long)cd_col_tiles(vdim) * CW_COLS) * (long long)sizeof(float) <= 200 * 1024;
+         (long long)CD_TILE * (2 * cd_pad(dim) + (long long)cd_col_tiles(vdim) * CW_COLS) * (long long)sizeof(float) <= 200 * 1024;
 }
 
 // The delta rule with one decay per head over portions of several tokens, for hfee_delta_rule, which has checked the arguments:
@@ -698,9 +720,9 @@ int hfee_delta_tiles(const void* qkv, long long ld_qkv, int q_off, int k_off, in
                status != nullptr, "delta_rule: the workspace is too small or not 16-byte aligned");
   const int vec = dim % 4 == 0 && ld_qkv % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
                   (uintptr_t)qkv % (dtype == HFEE_F32 ? 16 : 8) == 0;
-  const ChannelDeltaArgs p{ld_qkv, ld_b, 0, ld_out, q_off, k_off, v_off, heads, qk_heads, dim, vdim, write_state, vec, 1, a_off};
+  const ChannelDeltaArgs p{ld_qkv, ld_b, 0, ld_out, q_off, k_off, v_off, heads, qk_heads, dim, vdim, write_state, vec, a_off};
   float* ws_uo = workspace + cd_places(requests, n_tokens) * heads * cd_head_floats(dim);
   if (dtype == HFEE_F32)
-    return launch_tiles<float>(qkv, b, nullptr, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, workspace, ws_uo, status, stream);
-  return launch_tiles<__nv_bfloat16>(qkv, b, nullptr, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, workspace, ws_uo, status, stream);
+    return launch_tiles<float, true>(qkv, b, nullptr, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, workspace, ws_uo, status, stream);
+  return launch_tiles<__nv_bfloat16, true>(qkv, b, nullptr, a_log, dt_bias, state, cu_tokens, slots, out, p, requests, max_new, workspace, ws_uo, status, stream);
 }

@@ -99,3 +99,46 @@ def test_workspaces_of_every_size(monkeypatch):
         with pytest.raises(ops.KernelLibraryError):
             run(vdim, floats)
 
+
+# many tiles, small and large keys, sizes that do not fill their rows
+@pytest.mark.parametrize("dim,vdim,tokens", [(64, 64, 256), (256, 64, 200), (20, 17, 300)])
+def test_decays_are_as_exact_as_one_by_one(dim, vdim, tokens):
+    """Against 64 bits the tiles are no further off than the token-by-token kernel (whose error is 2 to 3e-7 here)."""
+    from hfee_b200.kernels import ops
+    heads, groups = 4, 2
+    g = torch.Generator().manual_seed(dim)
+    rand = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    step = _step([tokens])
+    qkv, ba, state = rand(tokens, 2 * groups * dim + heads * vdim), rand(tokens, 2 * heads), rand(2, heads, dim, vdim) * 0.1
+    a_log, dt_bias = torch.linspace(-4, 1, heads, device=DEV), torch.linspace(-3, 1, heads, device=DEV)
+    d = lambda t: t.double()
+    q, k = (d(qkv[:, o:o + groups * dim]).reshape(-1, groups, dim).repeat_interleave(heads // groups, 1) for o in (0, groups * dim))
+    want = _exact(q, k, d(qkv[:, 2 * groups * dim:]).reshape(-1, heads, vdim), d(ba[:, :heads]), d(ba[:, heads:]), d(a_log), d(dt_bias),
+                  d(state[1]))
+    errors = []
+    for workspace in (torch.empty(ops.delta_rule_workspace(1, tokens, heads, groups, dim, vdim), device=DEV), None):
+        s, out = state.clone(), torch.empty(tokens, heads * vdim, device=DEV)
+        ops.delta_rule(qkv, 0, groups * dim, 2 * groups * dim, ba, 0, heads, a_log, dt_bias, s, step, out, heads, groups, dim, vdim, True, workspace)
+        ops.check_status()
+        errors.append([float((d(got) - ref).norm() / ref.norm()) for got, ref in ((out.reshape(want[0].shape), want[0]), (s[1], want[1]))])
+    assert max(errors[0]) <= 4e-7 and all(a <= 1.2 * b for a, b in zip(*errors)), errors
+
+
+def test_decays_to_nothing():
+    from hfee_b200.kernels import ops
+    heads, dim, tokens = 2, 32, 40
+    g = torch.Generator().manual_seed(1)
+    rand = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    step = _step([tokens])
+    qkv, ba, state = rand(tokens, 4 * dim + heads * dim), rand(tokens, 2 * heads), rand(2, heads, dim, dim)
+    ba[3::7, heads:] = 80.0                                    # exp(-exp(88) * 80): the logarithm itself is minus infinity in 32 bits
+    a_log, dt_bias = torch.tensor([0.5, 88.0], device=DEV), torch.zeros(heads, device=DEV)
+    s, out = state.clone(), torch.empty(tokens, heads * dim, device=DEV)
+    ops.delta_rule(qkv, 0, 2 * dim, 4 * dim, ba, 0, heads, a_log, dt_bias, s, step, out, heads, 2, dim, dim, True,
+                   torch.empty(ops.delta_rule_workspace(1, tokens, heads, 2, dim), device=DEV))
+    ops.check_status()
+    d = lambda t: t.double()
+    q, k, v = (d(qkv[:, o:o + 2 * dim]).reshape(tokens, 2, dim) for o in (0, 2 * dim, 4 * dim))
+    want, last = _exact(q, k, v, d(ba[:, :heads]), d(ba[:, heads:]), d(a_log), d(dt_bias), d(state[1]))
+    for got, ref in ((out.reshape(want.shape), want), (s[1], last)):
+        assert (d(got) - ref).norm() <= 1e-6 * ref.norm()
