@@ -62,7 +62,8 @@ template <> __device__ __forceinline__ void store_row<__nv_bfloat16, 4>(__nv_bfl
 
 // S: number of streams, or 0 for any number (the streams are then read again for every output stream).
 // A decode step is the chain of one row's trips to memory: sixteen warps take a row of 2,048 in one go, and the weights that the
-// norm and the shift need at the end are brought into cache before the wait for the kernel in front.
+// norm and the shift need at the end are brought into cache before the wait for the kernel in front.  Both forms add a row's squares
+// in one order, the eight warps': a token's row does not depend on how many tokens the step has.
 template <typename T, int S, int VEC, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == ST_WARPS ? (S > 0 ? 3 : 2) : 1)
 stream_step_kernel(StreamArgs p, T* __restrict__ h_out) {
@@ -88,6 +89,7 @@ stream_step_kernel(StreamArgs p, T* __restrict__ h_out) {
   const int teams = min(p.groups, WARPS), per_team = WARPS / teams;
   const int team = warp / per_team, in_team = warp - team * per_team;
   const int part = p.width / p.groups, vecs = part / VEC;
+  const int shares = WARPS == ST_WARPS ? per_team : ST_WARPS / min(p.groups, ST_WARPS);      // warps of a team in the form with eight
   if constexpr (WARPS == ST_WARPS_FEW)
     for (int c = tid * VEC; c < p.width; c += ST_THREADS * VEC) {
       const float warm = p.norm_w[c] + (p.shift_w != nullptr ? p.shift_w[c] : 0.f);
@@ -163,16 +165,27 @@ stream_step_kernel(StreamArgs p, T* __restrict__ h_out) {
             for (int e = 0; e < VEC; ++e) u.v[e] = fmaf(in_s[t], a.v[e], u.v[e]);
           }
         }
-        u.store(u_s + c);                              // read back by the same thread only
+        u.store(u_s + c);                              // read back by the same thread, and above sixteen warps' sum by another
 #pragma unroll
         for (int e = 0; e < VEC; ++e) ss = fmaf(u.v[e], u.v[e], ss);
+      }
+      if (WARPS == ST_WARPS_FEW && per_team > 1) {     // the squares again, in the order of the form with eight warps
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(per_team * 32) : "memory");
+        ss = 0.f;
+        if (in_team < shares)
+          for (int j = in_team * 32 + lane; j < vecs; j += shares * 32) {
+            Pack<VEC> u;
+            u.load(u_s + g * part + j * VEC);
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) ss = fmaf(u.v[e], u.v[e], ss);
+          }
       }
       ss = warp_sum(ss);
       if (per_team > 1) {                              // then every team has exactly one group
         if (lane == 0) red_s[turn][warp] = ss;
         asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(per_team * 32) : "memory");
         ss = 0.f;
-        for (int w = 0; w < per_team; ++w) ss += red_s[turn][team * per_team + w];
+        for (int w = 0; w < shares; ++w) ss += red_s[turn][team * per_team + w];
       }
       const float scale = 1.0f / sqrtf(ss / (float)part + p.eps);
       for (int j = in_team * 32 + lane; j < vecs; j += per_team * 32) {
@@ -238,8 +251,11 @@ int launch_stream_step_w(const StreamArgs& p, void* h_out, cudaStream_t stream) 
 
 template <typename T, int S, int VEC>
 int launch_stream_step(const StreamArgs& p, void* h_out, cudaStream_t stream) {
-  if constexpr (S > 0)      // a row each for fewer blocks than SMs, and work for sixteen warps in it
-    if (p.n <= hfee_sm_count() && p.width > ST_WARPS * 32 * VEC) return launch_stream_step_w<T, S, VEC, ST_WARPS_FEW>(p, h_out, stream);
+  // a row each for fewer blocks than SMs (half as many with a shift, whose blocks then have a second row to read: 96 tokens of 2,048, 5.5 us
+  // against 5.1 with eight warps; 64 tokens 4.8 / 5.3), and work for sixteen warps in it
+  if constexpr (S > 0)
+    if ((long long)p.n * (p.shift_w != nullptr ? 2 : 1) <= hfee_sm_count() && p.width > ST_WARPS * 32 * VEC)
+      return launch_stream_step_w<T, S, VEC, ST_WARPS_FEW>(p, h_out, stream);
   return launch_stream_step_w<T, S, VEC, ST_WARPS>(p, h_out, stream);
 }
 
