@@ -8,7 +8,7 @@ token, not only the last.
 """
 from __future__ import annotations
 
-import gc
+import weakref
 from typing import Any, List, Optional, Sequence
 
 import torch
@@ -18,6 +18,7 @@ from ..config import EngineConfig, resolve_model_dir
 from ..parts import DecoderModel, Runtime
 from ..weights import Checkpoint
 from .batch import Step, StepBuffers, StepEntry
+from .graphs import capturing, retire
 
 _DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 # A decode step is a chain of short kernels, and an SM changes its split between shared memory and L1
@@ -61,6 +62,7 @@ class ModelRunner:
         # decode-only steps are captured in a CUDA graph per batch size: first sight runs
         # eagerly (and makes every scratch buffer), second sight captures, later ones replay
         self._graphs = {}
+        weakref.finalize(self, retire, self._graphs).atexit = False
         self._graph_seen = set()
         self.graph_replays = 0
 
@@ -154,17 +156,10 @@ class ModelRunner:
             graph = torch.cuda.CUDAGraph()
             before = ops.launch_count()
             torch.cuda.synchronize()
-            # a collector run in here could free another engine's graphs, which a capture does not survive
-            collecting = gc.isenabled()
-            gc.disable()
-            try:
-                with torch.cuda.graph(graph):
-                    out = self.model.forward(step, self.cache.views())
-            finally:
-                if collecting:
-                    gc.enable()
+            with capturing(), torch.cuda.graph(graph):
+                out = self.model.forward(step, self.cache.views())
             while len(self._graphs) >= GRAPH_LIMIT:          # oldest first
-                self._graphs.pop(next(iter(self._graphs)))
+                retire(self._graphs, next(iter(self._graphs)))
             hit = self._graphs[key] = (graph, out, ops.launch_count() - before)
         graph, out, kernels = hit
         graph.replay()
