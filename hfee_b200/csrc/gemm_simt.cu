@@ -13,6 +13,7 @@
 // Three kernels.  float32 operands whose rows start on 16-byte boundaries take `gemm_rows_kernel` (at most
 // ROWS_MAX_M tokens) or `gemm_tiles_kernel` (more); bfloat16 operands and other alignments take `gemm_simt_kernel`.
 // Reference: out[t*Rows+r] = Dot(W[r,:], x[t,:]), hostfog/hfee internal/ggml/ops.go:54-70.
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -334,13 +335,27 @@ gemm_tiles_kernel(const float* __restrict__ A, long long lda, const float* __res
 
 constexpr int ROWS_MAX_M = 16;
 
+// Which devices have been asked for a kernel's shared memory: the consent is each device's own.
+struct OptIn {
+  std::atomic<unsigned long long> asked{0};
+  template <typename Kernel>
+  bool room(Kernel kernel, int bytes) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    const unsigned long long bit = device < 64 ? 1ull << device : 0;
+    if (asked.load(std::memory_order_relaxed) & bit) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    asked.fetch_or(bit, std::memory_order_relaxed);
+    return true;
+  }
+};
+
 template <int TPL, int WARPS, typename TOut, bool ACCUM>
 int launch_rows_of(const float* A, long long lda, const float* W, long long ldw, TOut* C, long long ldc, int M, int N, int K,
                    cudaStream_t stream) {
   constexpr int smem = WARPS * (ROWS_STAGES * (16 + 2 * TPL) * (ROWS_KT + 4) + 2 * TPL * 32) * 4;
-  static const cudaError_t opted = cudaFuncSetAttribute(gemm_rows_kernel<TPL, WARPS, TOut, ACCUM>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (opted != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its rings");
+  static OptIn opted;
+  if (!opted.room(gemm_rows_kernel<TPL, WARPS, TOut, ACCUM>, smem)) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its rings");
   hfee_launch(gemm_rows_kernel<TPL, WARPS, TOut, ACCUM>, dim3((N + 15) / 16), dim3(WARPS * 32), smem, stream, A, lda, W, ldw, C, ldc,
               M, N, K);
   return hfee_check_launch("gemm_simt rows");
@@ -363,8 +378,8 @@ int launch_f32(const float* A, long long lda, const float* W, long long ldw, TOu
   if (M <= 4) return launch_rows<2, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
   if (M <= 8) return launch_rows<4, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
   if (M <= ROWS_MAX_M) return launch_rows<8, TOut, ACCUM>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-  static const cudaError_t opted = cudaFuncSetAttribute(gemm_tiles_kernel<TOut, ACCUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILES_SMEM);
-  if (opted != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its tiles");
+  static OptIn opted;
+  if (!opted.room(gemm_tiles_kernel<TOut, ACCUM>, TILES_SMEM)) return hfee_fail(HFEE_ERR_CUDA, "gemm_simt: no shared memory for its tiles");
   const int m_tiles = (M + TILE_M - 1) / TILE_M;
   const long long tiles = (long long)m_tiles * ((N + TILE_N - 1) / TILE_N);
   HFEE_REQUIRE(tiles <= 0x7fffffff, "gemm_simt: M=%d N=%d are too large", M, N);

@@ -43,3 +43,17 @@ def test_every_kernel_gives_the_same_bits(ops, n, k):
         narrow = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
         ops.gemm_simt(a, w, narrow)
         assert torch.equal(narrow, plain.bfloat16()), m
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_every_device_gives_the_kernels_their_shared_memory(ops):
+    """The consent to more than 48 KB of shared memory is each device's own."""
+    for m, k in ((2, 2048), (40, 2048)):
+        a, w = torch.randn(m, k), torch.randn(64, k)
+        got = []
+        for device in ("cuda:0", "cuda:1"):
+            with torch.cuda.device(device):
+                out = torch.empty(m, 64, device=device)
+                ops.gemm_simt(a.to(device), w.to(device), out)
+                got.append(out.cpu())
+        assert torch.equal(*got)
