@@ -11,7 +11,8 @@
 // 29 TFLOP/s).
 //
 // Three kernels.  float32 operands whose rows start on 16-byte boundaries take `gemm_rows_kernel` (at most
-// ROWS_MAX_M tokens) or `gemm_tiles_kernel` (more); bfloat16 operands and other alignments take `gemm_simt_kernel`.
+// ROWS_MAX_M tokens) or `gemm_tiles_kernel` (more) unless their sums are short; bfloat16 operands, other alignments and short sums
+// (`short_sums`) take `gemm_simt_kernel`.
 // Reference: out[t*Rows+r] = Dot(W[r,:], x[t,:]), hostfog/hfee internal/ggml/ops.go:54-70.
 #include <atomic>
 #include <type_traits>
@@ -21,6 +22,7 @@
 namespace {
 
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, THREADS = 256;
+constexpr unsigned EARLY_BLOCKS = 128;      // grids of no more than these let the kernel behind in at once
 constexpr int SEG = 512;        // k of a segment; a multiple of every kernel's piece of K
 
 template <typename T>
@@ -28,13 +30,17 @@ __device__ __forceinline__ float load_guarded(const T* p, long long ld, int r, i
   return (r < rows && c < cols) ? to_f32<T>(p[(long long)r * ld + c]) : 0.f;
 }
 
-// TOut: float or bf16.  ACCUM (float out only): out += product (the residual add).
-template <typename TIn, typename TOut, bool ACCUM>
-__global__ void __launch_bounds__(THREADS)
+// TOut: float or bf16.  ACCUM (float out only): out += product (the residual add).  ONE: K is one segment, without the segments' sums
+// (2,048 x 8,192 x 512 732 us with them, 676 without).  Three blocks an SM: with registers for two 700 x 2,048 x 512 in bfloat16 takes 102 us in
+// place of 77, with four 99.
+template <typename TIn, typename TOut, bool ACCUM, bool ONE>
+__global__ void __launch_bounds__(THREADS, 3)
 gemm_simt_kernel(const TIn* __restrict__ A, long long lda, const TIn* __restrict__ W, long long ldw,
                  TOut* __restrict__ C, long long ldc, int M, int N, int K) {
   pdl_wait();
-  pdl_launch_dependents();
+  // blocks of a kernel behind that are let in while this one has one or two an SM settle unevenly: 2,048 x 512 x 512 79 us in a row of such
+  const bool early = gridDim.x * gridDim.y <= EARLY_BLOCKS;
+  if (early) pdl_launch_dependents();
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[BK][BN + 4];
   int tid = threadIdx.x;
@@ -45,15 +51,31 @@ gemm_simt_kernel(const TIn* __restrict__ A, long long lda, const TIn* __restrict
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = sum[i][j] = 0.f;
+  auto add = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) { sum[i][j] += acc[0][i][j] + acc[1][i][j]; acc[0][i][j] = acc[1][i][j] = 0.f; }
+  };
 
-  // each thread stages 4 consecutive k of one row of A and one row of W
+  // each thread stages 4 consecutive k of one row of A and one row of W, asked for while the piece before is multiplied
   int lr = tid / (BK / 4), lk = (tid % (BK / 4)) * 4;   // 64 rows x 4 groups
+  float next_a[4], next_w[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      next_a[j] = load_guarded(A, lda, m0 + lr, k0 + lk + j, M, K);
+      next_w[j] = load_guarded(W, ldw, n0 + lr, k0 + lk + j, N, K);
+    }
+  };
+  fetch(0);
   for (int k0 = 0; k0 < K; k0 += BK) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      As[lk + j][lr] = load_guarded(A, lda, m0 + lr, k0 + lk + j, M, K);
-      Ws[lk + j][lr] = load_guarded(W, ldw, n0 + lr, k0 + lk + j, N, K);
+      As[lk + j][lr] = next_a[j];
+      Ws[lk + j][lr] = next_w[j];
     }
+    if (k0 + BK < K) fetch(k0 + BK);
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
@@ -68,12 +90,10 @@ gemm_simt_kernel(const TIn* __restrict__ A, long long lda, const TIn* __restrict
         for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
     }
     __syncthreads();
-    if ((k0 + BK) % SEG == 0 || k0 + BK >= K)
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) { sum[i][j] += acc[0][i][j] + acc[1][i][j]; acc[0][i][j] = acc[1][i][j] = 0.f; }
+    if (!ONE && (k0 + BK) % SEG == 0 && k0 + BK < K) add();
   }
+  add();
+  if (!early) pdl_launch_dependents();
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     int r = m0 + tr * TM + i;
@@ -214,6 +234,8 @@ gemm_rows_kernel(const float* __restrict__ A, long long lda, const float* __rest
 // the running sums of its quarter.  The next pair of k is read while one is multiplied, and two CTAs share an SM, for which the
 // launch asks for all of its shared memory: with the step's carve-out one CTA fits, and its four warps stop at 25 TFLOP/s.
 // The four products of a 1B layer at 285 tokens: 954 us, with tiles of 32 x 64 and 4 x 4 a thread 1,220.  8 x 16 a thread spills.
+// Rows and columns that are not there are not read (whatever lies in their place gives outputs that nobody stores): read again from the
+// last row, all tiles' copies met in one line (33 tokens, N = 8,192, K = 1,024: 75 us, 64 tokens 62).
 // A thread's rows lie 4 and its columns 8 apart, rows of a piece KT + 4 floats: no bank is hit
 // twice.  M tiles run fastest over the grid, so that a W tile is read from L2 by its row tiles.
 constexpr int TILE_M = 32, TILE_N = 64, TILE_KT = 16, TILE_STAGES = 3, TILE_WARPS = 4;
@@ -239,14 +261,16 @@ gemm_tiles_kernel(const float* __restrict__ A, long long lda, const float* __res
     const int k = first_k(step) + lk;
     if (k < K)
 #pragma unroll
-      for (int i = 0; i < TILE_N / 8; ++i) cp_async16(dst + i * 8 * LD, W + (long long)min(n0 + lr + i * 8, N - 1) * ldw + k);
+      for (int i = 0; i < TILE_N / 8; ++i)
+        if (n0 + lr + i * 8 < N) cp_async16(dst + i * 8 * LD, W + (long long)(n0 + lr + i * 8) * ldw + k);
   };
   auto load_a = [&](int step) {
     float* dst = ring + (step % STAGES) * STAGE + lr * LD + lk;
     const int k = first_k(step) + lk;
     if (k < K)
 #pragma unroll
-      for (int i = 0; i < TILE_M / 8; ++i) cp_async16(dst + i * 8 * LD, A + (long long)min(m0 + lr + i * 8, M - 1) * lda + k);
+      for (int i = 0; i < TILE_M / 8; ++i)
+        if (m0 + lr + i * 8 < M) cp_async16(dst + i * 8 * LD, A + (long long)(m0 + lr + i * 8) * lda + k);
   };
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) load_w(s);
@@ -388,30 +412,45 @@ int launch_f32(const float* A, long long lda, const float* W, long long ldw, TOu
   return hfee_check_launch("gemm_simt tiles");
 }
 
+// Products whose sums are too short for the two kernels above, which the general one takes (its blocks are 64 x 64; the order of the sums
+// is the same).  us, the kernel above / the general one.  A decode step's ring of copies: 8 tokens, N = 512: K = 32 4.9 / 2.8, 64 5.1 / 4.4,
+// 96 5.3 / 5.9.  The tiles give each of their four warps whole segments, so up to K = 512 three have nothing to do and up to 1,024 two: 2,048
+// tokens, N = 2,048: K = 32 54 / 15, 256 145 / 89, 512 248 / 172, 640 259 / 234, 768 268 / 312, 1,024 325 / 375.  Where all tiles fit the chip
+// side by side they take what one segment takes: 285 tokens, N = 512: K = 512 35 / 30, 640 35 / 42; and up to K = 512 they win only where
+// the general kernel's blocks do not fit: 285 tokens, N = 2,048: K = 128 14.0 / 13.7, 256 21.5 / 25.6, 512 36 / 49.
+bool short_sums(int M, int N, int K) {
+  if (M <= ROWS_MAX_M) return K <= 64;
+  if (K >= 3 * SEG / 2 || (M + BM - 1) / BM > 65535) return false;      // (rows of blocks a grid can have)
+  const long long sms = hfee_sm_count();
+  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
+  const long long blocks = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  return tiles > 2 * sms || K < SEG / 2 || (K <= SEG && blocks <= sms);
+}
+
 template <typename TIn>
 int launch(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
            int accumulate, int M, int N, int K, cudaStream_t stream) {
   if constexpr (sizeof(TIn) == 4) {
-    const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+    const bool aligned = !short_sums(M, N, K) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
     if (aligned && out_dtype == HFEE_F32)
       return accumulate ? launch_f32<float, true>((const float*)A, lda, (const float*)W, ldw, (float*)C, ldc, M, N, K, stream)
                         : launch_f32<float, false>((const float*)A, lda, (const float*)W, ldw, (float*)C, ldc, M, N, K, stream);
     if (aligned && out_dtype == HFEE_BF16 && !accumulate)
       return launch_f32<__nv_bfloat16, false>((const float*)A, lda, (const float*)W, ldw, (__nv_bfloat16*)C, ldc, M, N, K, stream);
   }
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+  auto run = [&](auto kernel, auto* out) {
+    hfee_launch(kernel, grid, dim3(THREADS), 0, stream, (const TIn*)A, lda, (const TIn*)W, ldw, out, ldc, M, N, K);
+    return hfee_check_launch("gemm_simt");
+  };
+  const bool one = K <= SEG;
   if (out_dtype == HFEE_F32) {
-    if (accumulate)
-      hfee_launch(gemm_simt_kernel<TIn, float, true>, dim3(grid), dim3(THREADS), 0, stream, (const TIn*)A, lda, (const TIn*)W, ldw, (float*)C, ldc, M, N, K);
-    else
-      hfee_launch(gemm_simt_kernel<TIn, float, false>, dim3(grid), dim3(THREADS), 0, stream, (const TIn*)A, lda, (const TIn*)W, ldw, (float*)C, ldc, M, N, K);
-  } else if (out_dtype == HFEE_BF16) {
-    if (accumulate) return hfee_fail(HFEE_ERR_ARG, "gemm_simt: accumulate needs a float32 output");
-    hfee_launch(gemm_simt_kernel<TIn, __nv_bfloat16, false>, dim3(grid), dim3(THREADS), 0, stream, (const TIn*)A, lda, (const TIn*)W, ldw, (__nv_bfloat16*)C, ldc, M, N, K);
-  } else {
-    return hfee_fail(HFEE_ERR_ARG, "gemm_simt: unknown output dtype %d", out_dtype);
+    if (accumulate) return run(one ? gemm_simt_kernel<TIn, float, true, true> : gemm_simt_kernel<TIn, float, true, false>, (float*)C);
+    return run(one ? gemm_simt_kernel<TIn, float, false, true> : gemm_simt_kernel<TIn, float, false, false>, (float*)C);
   }
-  return hfee_check_launch("gemm_simt");
+  if (out_dtype != HFEE_BF16) return hfee_fail(HFEE_ERR_ARG, "gemm_simt: unknown output dtype %d", out_dtype);
+  if (accumulate) return hfee_fail(HFEE_ERR_ARG, "gemm_simt: accumulate needs a float32 output");
+  return run(one ? gemm_simt_kernel<TIn, __nv_bfloat16, false, true> : gemm_simt_kernel<TIn, __nv_bfloat16, false, false>, (__nv_bfloat16*)C);
 }
 
 }  // namespace

@@ -45,6 +45,21 @@ def test_every_kernel_gives_the_same_bits(ops, n, k):
         assert torch.equal(narrow, plain.bfloat16()), m
 
 
+# depths on both sides of every change between the general kernel and the others, remainders of a piece and of a segment; token counts and
+# widths whose tiles fit the chip once, twice and more, and whose 64 x 64 blocks do and do not
+@pytest.mark.parametrize("k", [8, 64, 68, 252, 256, 512, 516, 764, 768, 1020, 1028, 1536])
+@pytest.mark.parametrize("m,n", [(3, 70), (16, 1000), (17, 8200), (33, 8192), (285, 2048), (64, 130), (300, 5000)])
+def test_short_sums_give_the_same_bits(ops, m, n, k):
+    g = torch.Generator().manual_seed(m + n + k)
+    a, w = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    plain, out = torch.empty(m, n, device="cuda"), torch.full((m, n + 2), 7.0, device="cuda")
+    ops.gemm_simt(_shifted(a), _shifted(w), plain)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert ((plain.double() - ref).abs() <= (k + 1) * 2.0 ** -24 * size).all()
+    ops.gemm_simt(a, w, out[:, :n])
+    assert torch.equal(out[:, :n], plain) and (out[:, n:] == 7.0).all()
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_every_device_gives_the_kernels_their_shared_memory(ops):
     """The consent to more than 48 KB of shared memory is each device's own."""
