@@ -28,16 +28,19 @@ constexpr int MAX_HD = 640;      // key size
 constexpr int MAX_VD = 512;      // value size
 constexpr int GATE_NONE = 0, GATE_ELEMENT = 1, GATE_PER_HEAD = 2;
 
-// Bound by the latency of its loads: a block of 32 keys is one trip for the keys (a lane's key is read 16 bytes at a time where
-// VEC says that keys start on 16-byte boundaries) and the values of VALUES_AHEAD keys at a time, the first of them requested with
-// the keys.  A decode step has few (token, head) pairs, so the parts of one pair run side by side in eight warps (two
-// tokens behind prompts of 150: 15 us a layer, with one warp a pair 52); the many pairs of a prompt portion have two warps each,
-// since most of eight would have nothing to do.  DPL, the value dimensions a lane owns, is the smallest that covers
-// the value size.
-constexpr int VALUES_AHEAD = 8;
+// Bound by the latency of its loads: a block of 32 keys is one trip for the keys (a lane's key is read 16 bytes at a time, and its
+// share of a value four numbers at a time, where VEC says that rows start on 16-byte boundaries) and the values of AHEAD keys at a time,
+// the first of them requested with the keys; values are read without a condition (a key or column that is not there reads one that is,
+// and is not used), since a branch around each load ends the overlap.  A decode step has few (token, head) pairs, so the parts of one
+// pair run side by side in eight warps (two tokens behind prompts of 150: 7.6 us a layer, with one warp a pair 52); the many pairs of a
+// prompt portion have two warps each, since most of eight would have nothing to do.  DPL, the value dimensions a lane owns, is the
+// smallest that covers the value size; the more it owns, the fewer keys it takes ahead, or the registers leave too few warps an SM:
+// 285 tokens, 8 heads of 256 on 2: 136 us (float32), 90 us (bfloat16); eight ahead, keys one number at a time and conditional
+// values took 308 and 579, one key at a time in one warp a pair 526 and 503.
+template <int N, typename T> struct alignas(N * sizeof(T)) PieceOf { T v[N]; };
 
 template <typename T, bool SIGMOID, int DPL, bool VEC, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 2 ? 32 / DPL : DPL == 2 ? 4 : 1)
 attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k_pool,
                       const T* __restrict__ v_pool, PagedCache cache, PagedCache vcache, int vd,
                       const int* __restrict__ positions,
@@ -46,6 +49,8 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
                       const float* __restrict__ head_bias, const T* __restrict__ gate, long long ld_gate,
                       int gate_mode, const float* __restrict__ dist_r1, const float* __restrict__ dist_r2, float out_scale,
                       const float* __restrict__ sink, int keep_first, float softcap) {
+  constexpr int AHEAD = DPL <= 4 ? 8 : 32 / DPL;
+  constexpr int VW = VEC ? (DPL < 4 ? DPL : 4) : 1, KW = 16 / (int)sizeof(T);      // numbers of a piece of a value, of a key
   pdl_wait();
   pdl_launch_dependents();
   __shared__ __align__(16) float q_s[MAX_HD];
@@ -84,15 +89,17 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
       const int count = min(32, end + 1 - base);
       const int key = base + lane;
       const long long k_at = key <= end ? paged_offset(cache, slot, key, kvh) : 0, v_at = key <= end ? paged_offset(vcache, slot, key, kvh) : 0;
-      float v[VALUES_AHEAD][DPL];
+      float v[AHEAD][DPL];
       auto request = [&](int t0) {
 #pragma unroll
-        for (int t = 0; t < VALUES_AHEAD; ++t) {
+        for (int t = 0; t < AHEAD; ++t) {
           const T* vr = v_pool + __shfl_sync(0xffffffffu, v_at, min(t0 + t, count - 1));
 #pragma unroll
-          for (int j = 0; j < DPL; ++j) {
-            const int d = lane + 32 * j;
-            v[t][j] = t0 + t < count && d < vd ? to_f32<T>(vr[d]) : 0.f;
+          for (int j = 0; j < DPL / VW; ++j) {
+            const int d = (lane + 32 * j) * VW;
+            const PieceOf<VW, T> x = *reinterpret_cast<const PieceOf<VW, T>*>(vr + (d < vd ? d : 0));
+#pragma unroll
+            for (int e = 0; e < VW; ++e) v[t][j * VW + e] = to_f32<T>(x.v[e]);
           }
         }
       };
@@ -102,13 +109,11 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
         const T* kr = k_pool + k_at;
         float acc = 0.f;
         if constexpr (VEC) {
-#pragma unroll 8
-          for (int d = 0; d < hd; d += 4) {
-            const float4 kv = *(const float4*)(kr + d), qv = *(const float4*)(q_s + d);
-            acc = fmaf(qv.x, kv.x, acc);
-            acc = fmaf(qv.y, kv.y, acc);
-            acc = fmaf(qv.z, kv.z, acc);
-            acc = fmaf(qv.w, kv.w, acc);
+#pragma unroll 4
+          for (int d = 0; d < hd; d += KW) {
+            const PieceOf<KW, T> x = *reinterpret_cast<const PieceOf<KW, T>*>(kr + d);
+#pragma unroll
+            for (int e = 0; e < KW; ++e) acc = fmaf(q_s[d + e], to_f32<T>(x.v[e]), acc);
           }
         } else {
           for (int d = 0; d < hd; ++d) acc = fmaf(q_s[d], to_f32<T>(kr[d]), acc);
@@ -130,10 +135,10 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
         for (int j = 0; j < DPL; ++j) o[j] *= alpha;
         m = m_new;
       }
-      for (int t0 = 0; t0 < count; t0 += VALUES_AHEAD) {
+      for (int t0 = 0; t0 < count; t0 += AHEAD) {
         if (t0 > 0) request(t0);
 #pragma unroll
-        for (int t = 0; t < VALUES_AHEAD; ++t) {
+        for (int t = 0; t < AHEAD; ++t) {
           if (t0 + t >= count) break;
           const float pt = __shfl_sync(0xffffffffu, p, t0 + t);
 #pragma unroll
@@ -165,7 +170,7 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
   if (gate_mode == GATE_PER_HEAD) inv *= 1.f / (1.f + expf(-to_f32<T>(gate[(long long)i * ld_gate + h])));
 #pragma unroll
   for (int j = 0; j < DPL; ++j) {
-    int d = lane + 32 * j;
+    const int d = (lane + 32 * (j / VW)) * VW + j % VW;
     if (d < vd) {
       float v = o[j] * inv;
       if (grow != nullptr) v *= 1.f / (1.f + expf(-to_f32<T>(grow[d])));
@@ -196,13 +201,12 @@ void launch_one(const void* q, int ld_q, const void* k_pool, const void* v_pool,
 template <typename T, bool SIGMOID, typename... Args>
 void launch_weights(const void* q, int ld_q, const void* k_pool, const void* v_pool, const PagedCache& c, const PagedCache& vc, int vd,
                     Args... args) {
-  const bool vec = sizeof(T) == 4 && c.head_dim % 4 == 0 && (uintptr_t)k_pool % 16 == 0;
+  // whole 16-byte pieces of keys, whole pieces of four values (rows follow one another in a page, so pools and sizes decide)
+  const bool vec = c.head_dim % (16 / (int)sizeof(T)) == 0 && vd % 4 == 0 && ((uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0;
   auto with = [&](auto dpl) {
     constexpr int DPL = decltype(dpl)::value;
-    if constexpr (sizeof(T) == 4) {
-      if (vec) return launch_one<T, SIGMOID, DPL, true>(q, ld_q, k_pool, v_pool, c, vc, vd, args...);
-    }
-    launch_one<T, SIGMOID, DPL, false>(q, ld_q, k_pool, v_pool, c, vc, vd, args...);
+    if (vec) launch_one<T, SIGMOID, DPL, true>(q, ld_q, k_pool, v_pool, c, vc, vd, args...);
+    else launch_one<T, SIGMOID, DPL, false>(q, ld_q, k_pool, v_pool, c, vc, vd, args...);
   };
   if (vd <= 64) with(std::integral_constant<int, 2>{});
   else if (vd <= 128) with(std::integral_constant<int, 4>{});
