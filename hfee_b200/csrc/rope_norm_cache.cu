@@ -20,6 +20,8 @@
 //                               dimensions of every query and key head, pairing dimension i with i + rope_dim/2 or
 //                               2i with 2i + 1; queries to a buffer, keys and values to their cache pages.  Key and
 //                               value sizes are independent.  One block per token, the row in shared memory.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace {
@@ -281,9 +283,10 @@ attention_prepare_kernel(const T* __restrict__ src, long long ld_src, int q_off,
 
 // attention_prepare for rows that 16-byte accesses can read: a work item is one 16-byte piece of a query, key or value head (with
 // half-split pairing, the piece in the first half of the rotated dimensions and its partner).  ROW: with biases or norms; a norm
-// is over all of a token's query or key columns, so every block that holds some of them reads them all first (4 KB, from L2 for
-// all but one).  The kernel above takes one element at a time through shared memory: 22 us a prompt of 2,048 tokens with norms and
-// biases, 8.5 us a decode step of two.
+// is over all of a token's query or key columns, so every block of a token reads them all first, whatever it stores (from L2 for all
+// but one; queries that overwrite the projection they come from take the kernel above, which reads a token in one block).  The kernel
+// above takes one element at a time through shared memory: 22 us a prompt of 2,048 tokens with norms and biases, 8.5 us a decode step
+// of two.
 template <typename T, int VEC>
 struct alignas(16) PreparePiece { T v[VEC]; };
 
@@ -434,10 +437,16 @@ bool launch_attention_prepare_vec(const void* src, long long ld_src, int n, int 
   for (const void* p : {src, (const void*)q_out, (const void*)k_pool, (const void*)v_pool, (const void*)first_values, (const void*)pr.bq,
                         (const void*)pr.bk, (const void*)pr.bv, (const void*)pr.wq, (const void*)pr.wk})
     if ((uintptr_t)p % 16 != 0) return false;
+  const bool rows = pr.bq != nullptr || pr.bk != nullptr || pr.bv != nullptr || pr.wq != nullptr || pr.wk != nullptr;
+  // Several blocks read a token's columns for a norm: not while one of them stores queries over some.
+  int end = q_off + heads * key_dim;
+  if (k_pool != nullptr) end = std::max({end, k_off + kc.kv_heads * key_dim, v_off + kc.kv_heads * vc.head_dim});
+  const char *from = (const char*)src, *from_end = from + ((long long)(n - 1) * ld_src + end) * (long long)sizeof(T);
+  const char *to = (const char*)q_out, *to_end = to + ((long long)(n - 1) * ld_q + heads * key_dim) * (long long)sizeof(T);
+  if (rows && from < to_end && to < from_end) return false;
   const int items = heads * (key_dim / VEC) + (k_pool != nullptr ? kc.kv_heads * (key_dim + vc.head_dim) / VEC : 0);
   // few tokens: one piece per thread; many: a few pieces each
   const int blocks = (items + AP_THREADS - 1) / AP_THREADS;
-  const bool rows = pr.bq != nullptr || pr.bk != nullptr || pr.bv != nullptr || pr.wq != nullptr || pr.wk != nullptr;
   const dim3 grid((unsigned)n, (unsigned)(n >= 512 ? (blocks + 3) / 4 : blocks));
   hfee_launch(rows ? attention_prepare_vec_kernel<T, VEC, true> : attention_prepare_vec_kernel<T, VEC, false>, grid, dim3(AP_THREADS), 0, stream,
               (const T*)src, ld_src, q_off, k_off, v_off, pr, cs, rope_dim, interleaved, positions, slot_of_token, (T*)q_out, ld_q, (T*)k_pool, kc,
