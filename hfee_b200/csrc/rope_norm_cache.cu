@@ -445,9 +445,12 @@ bool launch_attention_prepare_vec(const void* src, long long ld_src, int n, int 
   const char *to = (const char*)q_out, *to_end = to + ((long long)(n - 1) * ld_q + heads * key_dim) * (long long)sizeof(T);
   if (rows && from < to_end && to < from_end) return false;
   const int items = heads * (key_dim / VEC) + (k_pool != nullptr ? kc.kv_heads * (key_dim + vc.head_dim) / VEC : 0);
-  // few tokens: one piece per thread; many: a few pieces each
-  const int blocks = (items + AP_THREADS - 1) / AP_THREADS;
-  const dim3 grid((unsigned)n, (unsigned)(n >= 512 ? (blocks + 3) / 4 : blocks));
+  // few tokens: one piece per thread; many: a few pieces each, and with norms, which every block of a token reads its columns for, as
+  // few blocks a token as still give every SM about four (285 tokens, 64 heads of 128 on 8, float32: 23 us with all of the pieces' blocks)
+  const int blocks = (items + AP_THREADS - 1) / AP_THREADS, least = (blocks + 3) / 4;
+  int per_token = n >= 512 ? least : blocks;
+  if (pr.wq != nullptr || pr.wk != nullptr) per_token = std::max(least, std::min(blocks, 4 * hfee_sm_count() / n));
+  const dim3 grid((unsigned)n, (unsigned)per_token);
   hfee_launch(rows ? attention_prepare_vec_kernel<T, VEC, true> : attention_prepare_vec_kernel<T, VEC, false>, grid, dim3(AP_THREADS), 0, stream,
               (const T*)src, ld_src, q_off, k_off, v_off, pr, cs, rope_dim, interleaved, positions, slot_of_token, (T*)q_out, ld_q, (T*)k_pool, kc,
               (T*)v_pool, vc, heads, key_dim, (T*)first_values, ld_first, mix_mode, share);
