@@ -115,7 +115,8 @@ __device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
 // Bound by the reads of q, k and decays from shared memory (a row's three numbers for every NC elements of the state) and the issue of
 // its multiply-adds: two rows of a column are a pair for the packed instructions, what the next stage needs is asked for while
 // this one is walked, and the runs of the chunked path take 16 rows of four columns a thread in place of 32 of two where the
-// values fill 128 columns, which halves the reads (the four passes of a prompt of 2,048 tokens, 8 heads of 128 x 256 and 64 x 256: 404 ->
+// values are more than 64 columns and the keys more than 16 rows (with 16 a block would be one warp, with 1,024 values a stage to
+// bring: 200 tokens, 4 heads of 16 x 128, 192 us against 153), which halves the reads (the four passes of a prompt of 2,048 tokens, 8 heads of 128 x 256 and 64 x 256: 404 ->
 // 351 us in place).
 template <typename T, int MODE, int PASS, int ROWS, int NC>
 __global__ void __launch_bounds__(GR_LANES * (GR_MAX_DIM / ROWS), PASS == PASS_WHOLE || ROWS < 32 ? 1 : 2)
@@ -285,7 +286,7 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
       const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(ks + t * dim_pad + g * ROWS);
       const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(qs + t * dim_pad + g * ROWS);
       uint64_t sum2[NC] = {};
-      // a quarter of the rows' update and output, decays per pair
+      // update and output of four rows, decays per pair
       auto rows = [&](int i, uint64_t a0, uint64_t a1, const uint64_t (&pairs)[NC]) {
         const ulonglong2 kk = k4[i], qq = PASS != PASS_LOCAL ? q4[i] : kk;
 #pragma unroll
@@ -536,7 +537,7 @@ template <typename T, int PASS>
 int launch_recurrence(int mode, const void* q, const void* k, const void* v, const RecurrenceArgs& p, int grid_y,
                       cudaStream_t stream) {
   if constexpr (PASS != PASS_WHOLE)
-    if (p.vdim > GR_COLS) return launch_recurrence_tiles<T, PASS, 16, 4>(mode, q, k, v, p, grid_y, stream);
+    if (p.vdim > GR_COLS && p.dim > 16) return launch_recurrence_tiles<T, PASS, 16, 4>(mode, q, k, v, p, grid_y, stream);
   return launch_recurrence_tiles<T, PASS, 32, 2>(mode, q, k, v, p, grid_y, stream);
 }
 
