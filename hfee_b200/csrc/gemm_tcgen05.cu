@@ -577,12 +577,13 @@ HFEE_API int hfee_gemm_tcgen05_rope_supports(int head_dim, int rope_dim) {
 // A [M, K] tokens, W [N, K] with N = (heads + 2 kv_heads) * head_dim rows [q heads | k heads | v heads],
 // or N = heads * head_dim and null pools for a run that reads another run's cache.  cs [M, head_dim/2]
 // (cos, sin) pairs or null; queries go to q_out [M, ld_q], keys and values to the pages of
-// (slot_of_token, positions).
+// (slot_of_token, positions).  Tiles of block_n columns (192: three heads of 64), by pairs of CTAs (192 or 256) or single ones: tile_choice
+// in ops.py.
 HFEE_API int hfee_gemm_tcgen05_rope(const void* A, long long lda, const void* W, long long ldw, int M, int N, int K,
                                     const float* cs, const int* positions, const int* slot_of_token, void* q_out,
                                     long long ld_q, void* k_pool, void* v_pool, const int* block_table, int max_pages,
-                                    int page_size, int heads, int kv_heads, int head_dim, int interleaved, int* status,
-                                    cudaStream_t stream) {
+                                    int page_size, int heads, int kv_heads, int head_dim, int interleaved, int block_n, int pairs,
+                                    int* status, cudaStream_t stream) {
   if (M == 0 || N == 0) return HFEE_OK;
   HFEE_REQUIRE(hfee_gemm_tcgen05_rope_supports(head_dim, head_dim), "gemm_tcgen05_rope: head_dim %d is not 64 or 128", head_dim);
   HFEE_REQUIRE(M > 0 && K > 0 && K % 8 == 0, "gemm_tcgen05_rope: K=%d must be a positive multiple of 8", K);
@@ -600,31 +601,15 @@ HFEE_API int hfee_gemm_tcgen05_rope(const void* A, long long lda, const void* W,
   HFEE_REQUIRE(make_paged_cache(&rope.cache, block_table, max_pages, page_size, kv_heads, head_dim),
                "gemm_tcgen05_rope: page_size %d must be a power of two", page_size);
   rope.heads = heads; rope.kv_heads = kv_heads; rope.head_dim = head_dim; rope.interleaved = interleaved;
-  // Tiles of whole heads, of the kind whose rounds take least: percent of a round of 128 x 256 tiles, as in ops.py (tile_choice);
-  // 192 columns are three 64-dim heads.  The benchmark model's q/k/v product at 2,048 tokens: 128 pair tiles of 256 x 192 are two
-  // rounds, as are 96 of 256 x 256 (prompt pass 3.69 against 3.76 ms).
-  const int sms = hfee_sm_count();
-  if (sms < 2) return hfee_fail(HFEE_ERR_CUDA, "gemm_tcgen05_rope: cannot ask the device for its number of SMs");
-  auto cost = [&](int rows, int cols, int units, int percent) {
-    const long long tiles = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols);
-    return (tiles + units - 1) / units * percent;
-  };
-  int bn = 256, pairs = 0;
-  long long best = cost(BM, 256, sms, 100);
-  auto consider = [&](long long c, int block, int two) { if (c < best) { best = c; bn = block; pairs = two; } };
-  consider(cost(BM, 128, sms, 72), 128, 0);
-  if (head_dim == 64 && N % 192 == 0) consider(cost(BM, 192, sms, 86), 192, 0);
-  if (M > BM) {
-    consider(cost(2 * BM, 256, sms / 2, 85), 256, 1);
-    if (head_dim == 64 && N % 192 == 0) consider(cost(2 * BM, 192, sms / 2, 70), 192, 1);
-  }
-  if (pairs) return hfee_gemm_pair_rope(A, lda, W, ldw, M, N, K, rope, bn, status, stream);
+  HFEE_REQUIRE(block_n == 256 || (block_n == 192 && head_dim == 64 && N % 192 == 0) || (block_n == 128 && !pairs),
+               "gemm_tcgen05_rope: tiles of %d columns (pairs: %d) do not hold whole heads of %d", block_n, pairs, head_dim);
+  if (pairs) return hfee_gemm_pair_rope(A, lda, W, ldw, M, N, K, rope, block_n, status, stream);
   CUtensorMap ma, mw;
   int rc = make_map(&ma, A, M, K, lda, BM);
   if (rc != HFEE_OK) return rc;
-  rc = make_map(&mw, W, N, K, ldw, bn);
+  rc = make_map(&mw, W, N, K, ldw, block_n);
   if (rc != HFEE_OK) return rc;
-  if (bn == 256) return launch<256, EPI_ROPE, __nv_bfloat16>(ma, mw, nullptr, 0, M, N, K, status, nullptr, 0, nullptr, stream, rope);
-  if (bn == 192) return launch<192, EPI_ROPE, __nv_bfloat16>(ma, mw, nullptr, 0, M, N, K, status, nullptr, 0, nullptr, stream, rope);
+  if (block_n == 256) return launch<256, EPI_ROPE, __nv_bfloat16>(ma, mw, nullptr, 0, M, N, K, status, nullptr, 0, nullptr, stream, rope);
+  if (block_n == 192) return launch<192, EPI_ROPE, __nv_bfloat16>(ma, mw, nullptr, 0, M, N, K, status, nullptr, 0, nullptr, stream, rope);
   return launch<128, EPI_ROPE, __nv_bfloat16>(ma, mw, nullptr, 0, M, N, K, status, nullptr, 0, nullptr, stream, rope);
 }

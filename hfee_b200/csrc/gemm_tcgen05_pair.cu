@@ -436,8 +436,8 @@ HFEE_API int hfee_gemm_tcgen05_pair_clamped(const void* A, long long lda, const 
 }
 
 // The q/k/v product with rotation and cache write in its epilogue (hfee_gemm_tcgen05_rope) on pairs of
-// CTAs; called by that entry point, which has checked the arguments, for shapes with at least two
-// rounds of 256 x 256 tiles, or with tiles of 256 x 192 (block_n = 192, heads of 64 dims).
+// CTAs; called by that entry point, which has checked the arguments, with tiles of 256 x 256 or of 256 x 192
+// (block_n = 192, heads of 64 dims).
 int hfee_gemm_pair_rope(const void* A, long long lda, const void* W, long long ldw, int M, int N, int K,
                         const tc::RopeEpi& rope, int block_n, int* status, cudaStream_t stream) {
   CUtensorMap ma, mw;

@@ -37,7 +37,7 @@ _SIGNATURES = {
     "hfee_gemm_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _L, _P, _P],
     "hfee_gemm_tcgen05_stream_k": [_I, _I, _I, _I, _L],
     "hfee_gemm_tcgen05_pair": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
-    "hfee_gemm_tcgen05_rope": [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+    "hfee_gemm_tcgen05_rope": [_P, _L, _P, _L, _I, _I, _I, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "hfee_gemm_tcgen05_rope_supports": [_I, _I],
     "hfee_gemm_skinny": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "hfee_gemm_skinny_splits": [_I, _I, _I, _L],
@@ -399,11 +399,14 @@ def linear_rope_cache(a: torch.Tensor, w: torch.Tensor, cs: Optional[torch.Tenso
     if k_pool is not None:
         assert k_pool.dtype == v_pool.dtype == torch.bfloat16 and k_pool.is_contiguous() and v_pool.is_contiguous()
         assert tuple(k_pool.shape[1:]) == (kv_heads, page_size, head_dim)
+    # tiles of whole heads; the benchmark model's q/k/v product at 2,048 tokens: 128 pair tiles of 256 x 192 (three 64-dim heads) are two
+    # rounds, as are 96 of 256 x 256 (prompt pass 3.69 against 3.76 ms)
+    pairs, block_n = tile_choice(n, want, sm_count(), USE_PAIRS, True, k, narrow=head_dim == 64)
     _check(lib.hfee_gemm_tcgen05_rope(a.data_ptr(), _rows(a, "a"), w.data_ptr(), _rows(w, "w"), n, want, k, _ptr(cs),
                                       positions.data_ptr(), slot_of_token.data_ptr(), q_out.data_ptr(),
                                       _rows(q_out, "q_out"), _ptr(k_pool), _ptr(v_pool), block_table.data_ptr(),
                                       block_table.shape[1], page_size, heads, kv_heads, head_dim, int(interleaved),
-                                      _status().data_ptr(), _stream()), lib)
+                                      block_n, int(pairs), _status().data_ptr(), _stream()), lib)
 
 
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor, granule: Optional[int] = None) -> None:
@@ -506,7 +509,8 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
     assert w.shape[1] == k and a.dtype == w.dtype == torch.bfloat16
     assert tuple(out.shape) == (m, n // 2 if epilogue in EPI_GATED else n)
     if block_n is None:
-        pairs, block_n = tile_choice(m, n, sm_count(), USE_PAIRS, epilogue == EPI_STORE)
+        split = USE_STREAM_K if stream_k is None else stream_k          # a caller that asks for the split by K gets a kind that has it
+        pairs, block_n = tile_choice(m, n, sm_count(), USE_PAIRS and stream_k is not True, epilogue == EPI_STORE, k, split)
         if pairs:
             gemm_tcgen05_pair(a, w, out, epilogue, block_n)
             return
@@ -520,28 +524,46 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
 
 
 USE_PAIRS = True
-# What a round of tiles takes, one on every SM (or pair of SMs), against a round of single-CTA tiles of 128 x 256.  Measured
-# with one round of each (us at K = 2,048 / 8,192 / 14,336): 128 x 128 13.5 / 40 / 64, 128 x 256 17.6 / 56 / 92, pairs of CTAs on
-# 256 x 256 16.4 / 47 / 72; tiles of 192 columns take 0.8 of those of 256 plus their fixed part.
-ROUND_128, ROUND_192, ROUND_256, ROUND_PAIR_192, ROUND_PAIR_256 = 0.72, 0.86, 1.0, 0.70, 0.85
+# Times of the tcgen05 products' kinds of tile (pairs of CTAs?, columns): a fixed part per round of tiles (one on every SM or pair of
+# SMs) and a part per 1,024 of K, us, beside LAUNCH once: a persistent kernel pays its start and last epilogue once.  Fitted to 3,600
+# measured products (65 to 2,048 rows, 192 to 128,256 columns, K = 256 to 14,336, plain, accumulating and gated), mean error 6 %.
+TILE_TIMES = {(False, 128): (1.1, 4.48), (False, 192): (1.3, 5.29), (False, 256): (1.6, 5.73), (True, 192): (1.7, 3.74),
+              (True, 256): (2.4, 4.85)}
+LAUNCH, HAND_OVER, HAND_OVER_PIECE = 3.0, 3.0, 0.5       # the last two for 128 columns: partial tiles of a product split by K
+
+
+def split_pieces(tiles: int, k: int, sms: int) -> int:
+    """CTAs that share the K blocks of every tile (the rule of the launch: ``plan_stream_k`` in gemm_tcgen05.cu)."""
+    blocks = -(-k // 64)
+    if tiles * 2 > sms or blocks < 64:
+        return 1
+    pieces = min(sms // tiles, 4)
+    while pieces > 1 and blocks // pieces < 8:
+        pieces -= 1
+    return pieces
 
 
 @functools.lru_cache(maxsize=4096)
-def tile_choice(m: int, n: int, sms: int, pairs: bool, store: bool):
-    """(pairs of CTAs?, columns of a tile) of the tcgen05 product of m rows and n columns: the kind whose rounds of tiles take
-    least, so a kind that leaves its last round nearly empty gives way to one that does not.  564 rows x 4,096 columns x K = 14,336:
-    160 tiles of 128 x 128 are two rounds on 148 SMs (190 us), 48 pair tiles one (70 us); 1,100 x 4,096 x 4,096: 80 pair tiles are
-    two rounds of 74 (44 us), 144 single tiles one (31 us).  Pairs need more than 128 rows; tiles of 192 columns are taken where
-    they divide the columns (by pairs only in plain stores)."""
-    rounds = lambda rows, cols, units: -(-(-(-m // rows) * -(-n // cols)) // units)
-    kinds = [(rounds(128, 256, sms) * ROUND_256, False, 256), (rounds(128, 128, sms) * ROUND_128, False, 128)]
-    if n % 192 == 0:
-        kinds.append((rounds(128, 192, sms) * ROUND_192, False, 192))
-    if pairs and m > 128 and sms > 1:
-        kinds.append((rounds(256, 256, sms // 2) * ROUND_PAIR_256, True, 256))
-        if n % 192 == 0 and store:
-            kinds.append((rounds(256, 192, sms // 2) * ROUND_PAIR_192, True, 192))
-    return min(kinds)[1:]
+def tile_choice(m: int, n: int, sms: int, pairs: bool, store: bool, k: int = 2048, split: bool = False, narrow: bool = True):
+    """(pairs of CTAs?, columns of a tile) of the tcgen05 product of m rows and n columns: the kind that TILE_TIMES say takes least.
+    A kind that leaves its last round nearly empty gives way to one that does not (564 rows x 4,096 columns x K = 14,336: 160 tiles of
+    128 x 128 are two rounds on 148 SMs, 190 us, 48 pair tiles one, 70 us; 1,100 x 4,096 x 4,096: 80 pair tiles are two rounds of
+    74, 44 us, 144 single tiles one, 31 us), and tiles so few that their K is split (``split``) are weighed with their hand-over (256 x 768 x
+    8,192: 12 tiles of 128 x 128 in four pieces each 20 us, 4 pair tiles of 192 columns 32 us).  Over the 1,041 shapes measured the choice takes
+    0.3 % longer than the best kind of each, 12 % at worst; by rounds alone 3 and 65 %.  Pairs need more than 128 rows; tiles of 192
+    columns are taken where they divide the columns (``narrow``; by pairs only in plain stores)."""
+    best = None
+    for (two, columns), (fixed, per_k) in TILE_TIMES.items():
+        if two and not (pairs and m > 128 and sms > 1 and (columns == 256 or store)) or columns == 192 and (n % 192 or not narrow):
+            continue
+        tiles = -(-m // (256 if two else 128)) * -(-n // columns)
+        pieces = split_pieces(tiles, k, sms) if split and not two else 1
+        time = LAUNCH + -(-tiles // (sms // 2 if two else sms)) * (fixed + per_k * k / 1024 / pieces)
+        if pieces > 1:
+            time += (HAND_OVER + HAND_OVER_PIECE * pieces) * columns / 128
+        if best is None or time < best[0]:
+            best = time, (two, columns)
+    return best[1]
 
 
 def gemm_tcgen05_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = EPI_STORE, block_n: int = 256) -> None:
