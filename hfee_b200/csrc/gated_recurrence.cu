@@ -90,28 +90,6 @@ __device__ __forceinline__ bool find_run(const int* __restrict__ cu_tokens, int 
   return false;
 }
 
-// Two float32 numbers side by side, multiplied and added as a pair.
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpair(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // Bound by the reads of q, k and decays from shared memory (a row's three numbers for every NC elements of the state) and the issue of
 // its multiply-adds: two rows of a column are a pair for the packed instructions, what the next stage needs is asked for while
 // this one is walked, and the runs of the chunked path take 16 rows of four columns a thread in place of 32 of two where the
