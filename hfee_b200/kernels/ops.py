@@ -756,7 +756,7 @@ def linear_gated_normed(inp, w_gate_up: torch.Tensor, out: torch.Tensor, granule
 def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor,
                    page_size: int, positions: torch.Tensor, slot_of_token: torch.Tensor, out: torch.Tensor,
                    heads: int, kv_heads: int, head_dim: int, scale: float, window: int = 0) -> None:
-    """Causal GQA over the paged cache, one warp per (token, head), float32 math."""
+    """Causal GQA over the paged cache, a block per (token, head), float32 math."""
     lib = library()
     _i32(positions, "positions"); _i32(slot_of_token, "slot_of_token"); _i32(block_table, "block_table")
     n = q.shape[0]
