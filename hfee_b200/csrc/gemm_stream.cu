@@ -12,8 +12,11 @@
 // Three kernels share the operand trick: this K-split one, a warp-per-tile one for many weight
 // rows, and, for at most 8 tokens, one that keeps the tokens in registers (see further down).
 //
-// Epilogues: store (bf16 or f32), accumulate into a float32 output (the residual
-// add), or SwiGLU over rows interleaved as [4 gate rows | 4 up rows] per group of 8.
+// Epilogues: store (bf16 or f32), the square of relu, accumulate into a float32 output (the residual
+// add), or a gated activation over rows interleaved as [4 gate rows | 4 up rows] per group of 8.
+// An activation in a kernel of its own between two products of a few microseconds each costs a
+// decode step a whole dependent launch (its wait, one round trip to memory, its end), whatever it computes:
+// 1.4 us the square of relu and 3.4 us the clamped gate, at one and two tokens of 8,192.
 // Reference: out[t*Rows+r] = Dot(W[r,:], x[t,:]), hostfog/hfee internal/ggml/ops.go:54-70
 // ("each row is read once for all n inputs").
 #include "common.cuh"
@@ -22,7 +25,24 @@ namespace {
 
 constexpr int LOADS_IN_FLIGHT = 4;   // 16-byte weight loads per lane in one batch; two batches are in flight
 
-enum Epilogue { EPI_STORE = 0, EPI_ACCUM = 1, EPI_SWIGLU = 2, EPI_GEGLU = 4, EPI_REGLU = 7 };
+enum Epilogue { EPI_STORE = 0, EPI_ACCUM = 1, EPI_SWIGLU = 2, EPI_GEGLU = 4, EPI_RELU2 = 5, EPI_CLAMPED = 6, EPI_REGLU = 7 };
+
+constexpr __host__ __device__ bool is_gated(int epi) { return epi == EPI_SWIGLU || epi == EPI_GEGLU || epi == EPI_REGLU || epi == EPI_CLAMPED; }
+
+// The clamped gated activation: g sigmoid(alpha g) (u + shift), g = min(gate, limit), u = clamp(up, -limit, limit).
+struct GluArgs { float limit, alpha, shift; };
+
+template <int EPI> __device__ __forceinline__ float gated_out(float gate, float up, const GluArgs& glu) {
+  if constexpr (EPI == EPI_CLAMPED) {
+    const float g = fminf(gate, glu.limit), u = fminf(fmaxf(up, -glu.limit), glu.limit);
+    return g / (1.f + expf(-glu.alpha * g)) * (u + glu.shift);
+  }
+  return gate_value<EPI>(gate) * up;
+}
+template <int EPI> __device__ __forceinline__ float stored_out(float v) {
+  if constexpr (EPI == EPI_RELU2) { v = fmaxf(v, 0.f); return v * v; }
+  return v;
+}
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
@@ -66,7 +86,7 @@ struct NormArgs {
 template <int MT, int NT, int NW, int EPI, typename TOut>
 __global__ void __launch_bounds__(NW * 32, 2048 / (NW * 32) >= 4 ? 2 : 1)
 gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __nv_bfloat16* __restrict__ W,
-                   long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K) {
+                   long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K, GluArgs glu) {
   constexpr int ROWS = 8 * NT;
   constexpr int UNROLL = LOADS_IN_FLIGHT / NT;     // k32-steps per batch of loads
   constexpr int STRIDE = NW * UNROLL;              // k32-steps all warps cover per batch
@@ -153,7 +173,7 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __n
         for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.f;
       }
     __syncthreads();
-    if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_REGLU) {
+    if constexpr (is_gated(EPI)) {
       // rows of a group of 8: [gate x4 | up x4] -> 4 outputs at columns (n0/2 + group*4 ..)
       constexpr int OUTS = ROWS / 2;
       for (int idx = threadIdx.x; idx < MT * 16 * OUTS; idx += NW * 32) {
@@ -164,7 +184,7 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __n
         float gate = 0.f, up = 0.f;
 #pragma unroll
         for (int w = 0; w < NW; ++w) { gate += red[w][t][gr]; up += red[w][t][gr + 4]; }
-        C[(long long)t * ldc + col] = from_f32<TOut>(gate_value<EPI>(gate) * up);
+        C[(long long)t * ldc + col] = from_f32<TOut>(gated_out<EPI>(gate, up, glu));
       }
     } else {
       for (int idx = threadIdx.x; idx < MT * 16 * ROWS; idx += NW * 32) {
@@ -175,7 +195,7 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __n
         for (int w = 0; w < NW; ++w) v += red[w][t][r];
         long long o = (long long)t * ldc + n0 + r;
         if constexpr (EPI == EPI_ACCUM) C[o] = to_f32<TOut>(C[o]) + v;
-        else C[o] = from_f32<TOut>(v);
+        else C[o] = from_f32<TOut>(stored_out<EPI>(v));
       }
     }
     __syncthreads();
@@ -214,7 +234,7 @@ constexpr int ROWS_UNROLL = 8;                   // 16-byte weight loads per lan
 template <int MT, int EPI, typename TOut>
 __global__ void __launch_bounds__(ROWS_WARPS * 32, 2)
 gemm_stream_rows_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __nv_bfloat16* __restrict__ W,
-                        long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K) {
+                        long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K, GluArgs glu) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, c = lane & 3;
   const int warps = (int)gridDim.x * ROWS_WARPS;
@@ -272,7 +292,7 @@ gemm_stream_rows_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
     const int n0 = (first + tile_no * warps) * 8;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
-      if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_REGLU) {
+      if constexpr (is_gated(EPI)) {
         // rows 0-3 gate, 4-7 up: lanes c = 0,1 hold gate, c = 2,3 the matching up values
         float u0 = __shfl_xor_sync(0xffffffffu, acc[mt][0], 2), u1 = __shfl_xor_sync(0xffffffffu, acc[mt][1], 2);
         float u2 = __shfl_xor_sync(0xffffffffu, acc[mt][2], 2), u3 = __shfl_xor_sync(0xffffffffu, acc[mt][3], 2);
@@ -288,7 +308,7 @@ gemm_stream_rows_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
             for (int e = 0; e < 2; ++e) {
               if (col + e >= N / 2) continue;
               float gate = gv[2 * h + e], up = uv[2 * h + e];
-              C[(long long)t * ldc + col + e] = from_f32<TOut>(gate_value<EPI>(gate) * up);
+              C[(long long)t * ldc + col + e] = from_f32<TOut>(gated_out<EPI>(gate, up, glu));
             }
           }
         }
@@ -304,7 +324,7 @@ gemm_stream_rows_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
             const long long o = (long long)t * ldc + col;
             const float v = acc[mt][2 * h + e];
             if constexpr (EPI == EPI_ACCUM) C[o] = to_f32<TOut>(C[o]) + v;
-            else C[o] = from_f32<TOut>(v);
+            else C[o] = from_f32<TOut>(stored_out<EPI>(v));
           }
         }
       }
@@ -356,7 +376,7 @@ constexpr int SL_TOKEN_PITCH = SL_GROUP * 8 + 8;         // floats per token row
 template <int EPI, bool NORM, typename TOut>
 __global__ void __launch_bounds__(SL_WARPS * 32, 2)
 gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __nv_bfloat16* __restrict__ W,
-                          long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K, NormArgs norm) {
+                          long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K, GluArgs glu, NormArgs norm) {
   __shared__ __align__(16) float red[2][SL_WARPS][8][SL_TOKEN_PITCH];
   __shared__ __align__(16) float norm_w[NORM ? SL_PASS : 4];       // NORM: the scales of this pass, staged before the wait
   __shared__ float sq_part[SL_WARPS][8];
@@ -464,7 +484,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
     const int gs = group_size(grp);
     const int t0 = t_begin + grp * SL_GROUP;
     const float (*part)[8][SL_TOKEN_PITCH] = red[grp & 1];
-    if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_REGLU) {
+    if constexpr (is_gated(EPI)) {
       // rows of a tile: [gate x4 | up x4] -> 4 outputs at columns tile*4 ..
       const int t = threadIdx.x >> 5, o = threadIdx.x & 31;
       const int tile = o >> 2, i = o & 3;
@@ -473,7 +493,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
         float gate = 0.f, up = 0.f;
 #pragma unroll
         for (int w = 0; w < SL_WARPS; ++w) { gate += part[w][t][tile * 8 + i]; up += part[w][t][tile * 8 + 4 + i]; }
-        C[(long long)t * ldc + col] = from_f32<TOut>(gate_value<EPI>(gate) * up);
+        C[(long long)t * ldc + col] = from_f32<TOut>(gated_out<EPI>(gate, up, glu));
       }
     } else {
 #pragma unroll
@@ -486,7 +506,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
           for (int w = 0; w < SL_WARPS; ++w) v += part[w][t][o];
           const long long at = (long long)t * ldc + col;
           if constexpr (EPI == EPI_ACCUM) C[at] = to_f32<TOut>(C[at]) + v;
-          else C[at] = from_f32<TOut>(v);
+          else C[at] = from_f32<TOut>(stored_out<EPI>(v));
         }
       }
     }
@@ -539,7 +559,7 @@ constexpr int WD_DEPTH = 4;
 template <int EPI, typename TOut>
 __global__ void __launch_bounds__(WD_WARPS * 32, 1)
 gemm_stream_wide_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __nv_bfloat16* __restrict__ W,
-                        long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K) {
+                        long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K, GluArgs glu) {
   extern __shared__ __align__(16) float red_raw[];       // [WD_WARPS][16][SL_TOKEN_PITCH]
   float (*red)[16][SL_TOKEN_PITCH] = reinterpret_cast<float (*)[16][SL_TOKEN_PITCH]>(red_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -579,7 +599,7 @@ gemm_stream_wide_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
   auto finish_group = [&](int grp) {
     const int gs = group_size(grp);
     const int t0 = t_begin + grp * SL_GROUP;
-    if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_REGLU) {
+    if constexpr (is_gated(EPI)) {
       const int t = threadIdx.x >> 5, o = threadIdx.x & 31;             // 16 tokens x 32 outputs = 512 threads
       const int tile = o >> 2, i = o & 3;
       const long long col = (long long)(t0 + tile) * 4 + i;
@@ -587,7 +607,7 @@ gemm_stream_wide_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
         float gate = 0.f, up = 0.f;
 #pragma unroll
         for (int w = 0; w < WD_WARPS; ++w) { gate += red[w][t][tile * 8 + i]; up += red[w][t][tile * 8 + 4 + i]; }
-        C[(long long)t * ldc + col] = from_f32<TOut>(gate_value<EPI>(gate) * up);
+        C[(long long)t * ldc + col] = from_f32<TOut>(gated_out<EPI>(gate, up, glu));
       }
     } else {
 #pragma unroll
@@ -600,7 +620,7 @@ gemm_stream_wide_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
           for (int w = 0; w < WD_WARPS; ++w) v += red[w][t][o];
           const long long at = (long long)t * ldc + col;
           if constexpr (EPI == EPI_ACCUM) C[at] = to_f32<TOut>(C[at]) + v;
-          else C[at] = from_f32<TOut>(v);
+          else C[at] = from_f32<TOut>(stored_out<EPI>(v));
         }
       }
     }
@@ -633,8 +653,30 @@ gemm_stream_wide_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
   }
 }
 
+// HFEE_GO(EPI, T) for the epilogue and output type of a call.
+#define HFEE_BY_EPILOGUE()                                                                                                    \
+  do {                                                                                                                        \
+    const bool bf = out_dtype == HFEE_BF16;                                                                                   \
+    switch (epilogue) {                                                                                                       \
+      case EPI_ACCUM:                                                                                                         \
+        if (bf) return hfee_fail(HFEE_ERR_ARG, "gemm_stream: accumulate needs a float32 output");                             \
+        HFEE_GO(EPI_ACCUM, float);                                                                                            \
+        break;                                                                                                                \
+      case EPI_SWIGLU: if (bf) HFEE_GO(EPI_SWIGLU, __nv_bfloat16); else HFEE_GO(EPI_SWIGLU, float); break;                    \
+      case EPI_GEGLU: if (bf) HFEE_GO(EPI_GEGLU, __nv_bfloat16); else HFEE_GO(EPI_GEGLU, float); break;                       \
+      case EPI_REGLU: if (bf) HFEE_GO(EPI_REGLU, __nv_bfloat16); else HFEE_GO(EPI_REGLU, float); break;                       \
+      case EPI_RELU2:                                                                                                         \
+      case EPI_CLAMPED:                                                                                                       \
+        if (!bf) return hfee_fail(HFEE_ERR_ARG, "gemm_stream: epilogue %d needs a bfloat16 output", epilogue);                \
+        if (epilogue == EPI_RELU2) HFEE_GO(EPI_RELU2, __nv_bfloat16);                                                         \
+        else HFEE_GO(EPI_CLAMPED, __nv_bfloat16);                                                                             \
+        break;                                                                                                                \
+      default: if (bf) HFEE_GO(EPI_STORE, __nv_bfloat16); else HFEE_GO(EPI_STORE, float);                                     \
+    }                                                                                                                         \
+  } while (0)
+
 int launch_wide(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
-                int epilogue, int M, int N, int K, cudaStream_t stream) {
+                int epilogue, int M, int N, int K, const GluArgs& glu, cudaStream_t stream) {
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   const int sms = hfee_sm_count();
@@ -650,53 +692,31 @@ int launch_wide(const void* A, long long lda, const void* W, long long ldw, void
       if (e != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_stream: cannot get shared memory: %s", cudaGetErrorString(e)); \
       configured = true;                                                                                                  \
     }                                                                                                                     \
-    hfee_launch(gemm_stream_wide_kernel<EPI, T>, dim3(grid), dim3(WD_WARPS * 32), RED_BYTES, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K); \
+    hfee_launch(gemm_stream_wide_kernel<EPI, T>, dim3(grid), dim3(WD_WARPS * 32), RED_BYTES, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K, glu); \
   } while (0)
-  if (epilogue == EPI_ACCUM) {
-    if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_stream: accumulate needs a float32 output");
-    HFEE_GO(EPI_ACCUM, float);
-  } else if (epilogue == EPI_SWIGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_SWIGLU, __nv_bfloat16); else HFEE_GO(EPI_SWIGLU, float);
-  } else if (epilogue == EPI_GEGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_GEGLU, __nv_bfloat16); else HFEE_GO(EPI_GEGLU, float);
-  } else if (epilogue == EPI_REGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_REGLU, __nv_bfloat16); else HFEE_GO(EPI_REGLU, float);
-  } else {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_STORE, __nv_bfloat16); else HFEE_GO(EPI_STORE, float);
-  }
+  HFEE_BY_EPILOGUE();
 #undef HFEE_GO
   return hfee_check_launch("gemm_stream_wide");
 }
 
 template <bool NORM>
 int launch_slices(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
-                  int epilogue, int M, int N, int K, const NormArgs& norm, cudaStream_t stream) {
+                  int epilogue, int M, int N, int K, const GluArgs& glu, const NormArgs& norm, cudaStream_t stream) {
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   const int resident = 2 * hfee_sm_count();
   if (resident <= 0) return hfee_fail(HFEE_ERR_CUDA, "gemm_stream: cannot ask the device for its number of SMs");
   const int n_tiles = (N + 7) / 8;
   unsigned grid = (unsigned)(n_tiles < resident ? n_tiles : resident);
-#define HFEE_GO(EPI, T) hfee_launch(gemm_stream_slices_kernel<EPI, NORM, T>, dim3(grid), dim3(SL_WARPS * 32), 0, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K, norm)
-  if (epilogue == EPI_ACCUM) {
-    if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_stream: accumulate needs a float32 output");
-    HFEE_GO(EPI_ACCUM, float);
-  } else if (epilogue == EPI_SWIGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_SWIGLU, __nv_bfloat16); else HFEE_GO(EPI_SWIGLU, float);
-  } else if (epilogue == EPI_GEGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_GEGLU, __nv_bfloat16); else HFEE_GO(EPI_GEGLU, float);
-  } else if (epilogue == EPI_REGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_REGLU, __nv_bfloat16); else HFEE_GO(EPI_REGLU, float);
-  } else {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_STORE, __nv_bfloat16); else HFEE_GO(EPI_STORE, float);
-  }
+#define HFEE_GO(EPI, T) hfee_launch(gemm_stream_slices_kernel<EPI, NORM, T>, dim3(grid), dim3(SL_WARPS * 32), 0, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K, glu, norm)
+  HFEE_BY_EPILOGUE();
 #undef HFEE_GO
   return hfee_check_launch("gemm_stream_slices");
 }
 
 template <int MT, int NT, int NW>
 int launch(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
-           int epilogue, int M, int N, int K, cudaStream_t stream) {
+           int epilogue, int M, int N, int K, const GluArgs& glu, cudaStream_t stream) {
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   static int resident = 0;                       // CTAs of this instantiation the whole GPU holds at once
@@ -708,19 +728,8 @@ int launch(const void* A, long long lda, const void* W, long long ldw, void* C, 
   }
   int n_tiles = (N + 8 * NT - 1) / (8 * NT);
   unsigned grid = (unsigned)(n_tiles < resident ? n_tiles : resident);
-#define HFEE_GO(EPI, T) hfee_launch(gemm_stream_kernel<MT, NT, NW, EPI, T>, dim3(grid), dim3(NW * 32), 0, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K)
-  if (epilogue == EPI_ACCUM) {
-    if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_stream: accumulate needs a float32 output");
-    HFEE_GO(EPI_ACCUM, float);
-  } else if (epilogue == EPI_SWIGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_SWIGLU, __nv_bfloat16); else HFEE_GO(EPI_SWIGLU, float);
-  } else if (epilogue == EPI_GEGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_GEGLU, __nv_bfloat16); else HFEE_GO(EPI_GEGLU, float);
-  } else if (epilogue == EPI_REGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_REGLU, __nv_bfloat16); else HFEE_GO(EPI_REGLU, float);
-  } else {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_STORE, __nv_bfloat16); else HFEE_GO(EPI_STORE, float);
-  }
+#define HFEE_GO(EPI, T) hfee_launch(gemm_stream_kernel<MT, NT, NW, EPI, T>, dim3(grid), dim3(NW * 32), 0, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K, glu)
+  HFEE_BY_EPILOGUE();
 #undef HFEE_GO
   return hfee_check_launch("gemm_stream");
 }
@@ -730,7 +739,7 @@ int launch(const void* A, long long lda, const void* W, long long ldw, void* C, 
 namespace {
 template <int MT>
 int launch_rows(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
-                int epilogue, int M, int N, int K, cudaStream_t stream) {
+                int epilogue, int M, int N, int K, const GluArgs& glu, cudaStream_t stream) {
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   int n_tiles = (N + 7) / 8;
@@ -738,19 +747,8 @@ int launch_rows(const void* A, long long lda, const void* W, long long ldw, void
   const int resident = 2 * hfee_sm_count();              // two CTAs of this kernel share an SM
   if (resident <= 0) return hfee_fail(HFEE_ERR_CUDA, "gemm_stream: cannot ask the device for its number of SMs");
   unsigned grid = (unsigned)(ctas < resident ? ctas : resident);
-#define HFEE_GO(EPI, T) hfee_launch(gemm_stream_rows_kernel<MT, EPI, T>, dim3(grid), dim3(ROWS_WARPS * 32), 0, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K)
-  if (epilogue == EPI_ACCUM) {
-    if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_stream: accumulate needs a float32 output");
-    HFEE_GO(EPI_ACCUM, float);
-  } else if (epilogue == EPI_SWIGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_SWIGLU, __nv_bfloat16); else HFEE_GO(EPI_SWIGLU, float);
-  } else if (epilogue == EPI_GEGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_GEGLU, __nv_bfloat16); else HFEE_GO(EPI_GEGLU, float);
-  } else if (epilogue == EPI_REGLU) {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_REGLU, __nv_bfloat16); else HFEE_GO(EPI_REGLU, float);
-  } else {
-    if (out_dtype == HFEE_BF16) HFEE_GO(EPI_STORE, __nv_bfloat16); else HFEE_GO(EPI_STORE, float);
-  }
+#define HFEE_GO(EPI, T) hfee_launch(gemm_stream_rows_kernel<MT, EPI, T>, dim3(grid), dim3(ROWS_WARPS * 32), 0, stream, a, lda, w, ldw, (T*)C, ldc, M, N, K, glu)
+  HFEE_BY_EPILOGUE();
 #undef HFEE_GO
   return hfee_check_launch("gemm_stream_rows");
 }
@@ -759,10 +757,10 @@ int launch_rows(const void* A, long long lda, const void* W, long long ldw, void
 constexpr int ROWS_MIN_TILES = 1536;
 
 int by_tokens(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
-              int epilogue, int M, int N, int K, cudaStream_t stream) {
-  if (M <= 16) return launch<1, 1, 16>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
-  if (M <= 32) return launch<2, 2, 8>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
-  return launch<4, 4, 4>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
+              int epilogue, int M, int N, int K, const GluArgs& glu, cudaStream_t stream) {
+  if (M <= 16) return launch<1, 1, 16>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
+  if (M <= 32) return launch<2, 2, 8>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
+  return launch<4, 4, 4>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
 }
 
 int check_common(const void* W, long long ldw, long long ldc, int epilogue, int M, int N, int K) {
@@ -770,29 +768,45 @@ int check_common(const void* W, long long ldw, long long ldc, int epilogue, int 
   HFEE_REQUIRE(N > 0 && K > 0 && K % 8 == 0, "gemm_stream: K=%d must be a positive multiple of 8", K);
   HFEE_REQUIRE(ldw % 8 == 0 && ldw >= K, "gemm_stream: the weights' leading dimension %lld must be a multiple of 8 and at least K", ldw);
   HFEE_REQUIRE((uintptr_t)W % 16 == 0, "gemm_stream: weights must be 16-byte aligned");
-  HFEE_REQUIRE((epilogue >= 0 && epilogue <= 2) || epilogue == EPI_GEGLU || epilogue == EPI_REGLU, "gemm_stream: unknown epilogue %d", epilogue);
-  HFEE_REQUIRE((epilogue != EPI_SWIGLU && epilogue != EPI_GEGLU && epilogue != EPI_REGLU) || N % 8 == 0, "gemm_stream: SwiGLU needs N %% 8 == 0, got %d", N);
-  HFEE_REQUIRE(ldc >= ((epilogue == EPI_SWIGLU || epilogue == EPI_GEGLU || epilogue == EPI_REGLU) ? N / 2 : N), "gemm_stream: ldc=%lld is too small", ldc);
+  HFEE_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_ACCUM || epilogue == EPI_RELU2 || is_gated(epilogue), "gemm_stream: unknown epilogue %d", epilogue);
+  HFEE_REQUIRE(!is_gated(epilogue) || N % 8 == 0, "gemm_stream: a gated epilogue needs N %% 8 == 0, got %d", N);
+  HFEE_REQUIRE(ldc >= (is_gated(epilogue) ? N / 2 : N), "gemm_stream: ldc=%lld is too small", ldc);
   return HFEE_OK;
 }
 }  // namespace
 
-// epilogue: 0 store, 1 accumulate into float32 C, 2 SwiGLU and 4 the same with a tanh-GELU gate (C is [M, N/2]; N % 8 == 0).
-HFEE_API int hfee_gemm_stream(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
-                              int out_dtype, int epilogue, int M, int N, int K, cudaStream_t stream) {
+namespace {
+int stream_any(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype, int epilogue,
+               int M, int N, int K, const GluArgs& glu, cudaStream_t stream) {
   if (M == 0 || N == 0) return HFEE_OK;
   int rc = check_common(W, ldw, ldc, epilogue, M, N, K);
   if (rc != HFEE_OK) return rc;
   HFEE_REQUIRE(lda % 8 == 0 && lda >= K && (uintptr_t)A % 16 == 0,
                "gemm_stream: the tokens' leading dimension %lld must be a multiple of 8, at least K, and 16-byte aligned", lda);
   NormArgs none{nullptr, 0, nullptr, nullptr, 0.f, 0};
-  if (M <= 8) return launch_slices<false>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, none, stream);
-  if (M <= 16 && K <= WD_WARPS * WD_SLICE) return launch_wide(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
+  if (M <= 8) return launch_slices<false>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, none, stream);
+  if (M <= 16 && K <= WD_WARPS * WD_SLICE) return launch_wide(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
   if ((N + 7) / 8 >= ROWS_MIN_TILES && M <= 32) {
-    if (M <= 16) return launch_rows<1>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
-    return launch_rows<2>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
+    if (M <= 16) return launch_rows<1>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
+    return launch_rows<2>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
   }
-  return by_tokens(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, stream);
+  return by_tokens(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
+}
+}  // namespace
+
+// epilogue: 0 store, 1 accumulate into float32 C, 2 SwiGLU, 4 and 7 the same with a tanh-GELU or relu gate (C is [M, N/2];
+// N % 8 == 0), 5 the square of relu (C bfloat16).
+HFEE_API int hfee_gemm_stream(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
+                              int out_dtype, int epilogue, int M, int N, int K, cudaStream_t stream) {
+  HFEE_REQUIRE(epilogue != EPI_CLAMPED, "gemm_stream: the clamped activation has an entry point of its own");
+  return stream_any(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, GluArgs{0.f, 0.f, 0.f}, stream);
+}
+
+// The product with the clamped gated activation behind it: C [M, N/2] bfloat16.
+HFEE_API int hfee_gemm_stream_clamped(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
+                                      int M, int N, int K, float limit, float alpha, float shift, cudaStream_t stream) {
+  HFEE_REQUIRE(limit > 0.f, "gemm_stream_clamped: the limit must be positive");
+  return stream_any(A, lda, W, ldw, C, ldc, HFEE_BF16, EPI_CLAMPED, M, N, K, GluArgs{limit, alpha, shift}, stream);
 }
 
 // The same with the RMS norm of float32 rows X fused in front: tokens = bf16(norm(X[rows])).  For at
@@ -807,6 +821,7 @@ HFEE_API int hfee_gemm_stream_norm(const float* X, long long ldx, const int* row
   HFEE_REQUIRE(M <= 8 && K <= SL_PASS, "gemm_stream_norm: the fused norm takes at most 8 tokens and K <= %d (got M=%d, K=%d)", SL_PASS, M, K);
   HFEE_REQUIRE(ldx % 4 == 0 && ldx >= K && (uintptr_t)X % 16 == 0 && (uintptr_t)norm_weight % 16 == 0,
                "gemm_stream_norm: float32 rows need a leading dimension %% 4 == 0 and 16-byte alignment");
+  HFEE_REQUIRE(epilogue != EPI_CLAMPED, "gemm_stream_norm: the clamped activation takes normed rows");
   NormArgs norm{X, ldx, rows, norm_weight, eps, add_unit};
-  return launch_slices<true>(nullptr, 0, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, norm, stream);
+  return launch_slices<true>(nullptr, 0, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, GluArgs{0.f, 0.f, 0.f}, norm, stream);
 }

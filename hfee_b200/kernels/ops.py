@@ -33,6 +33,7 @@ _SIGNATURES = {
     "hfee_rope_cache_write": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "hfee_swiglu": [_P, _I, _P, _I, _I, _I, _I, _I, _P],
     "hfee_gemm_stream": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
+    "hfee_gemm_stream_clamped": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _F, _F, _F, _P],
     "hfee_gemm_stream_norm": [_P, _L, _P, _P, _F, _I, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
     "hfee_gemm_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _L, _P, _P],
     "hfee_gemm_tcgen05_stream_k": [_I, _I, _I, _I, _L],
@@ -432,7 +433,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: b
 
 STREAM_MAX_TOKENS = 64
 USE_TCGEN05 = True
-EPI_STORE, EPI_ACCUM, EPI_SWIGLU, EPI_GEGLU, EPI_RELU2, EPI_REGLU = 0, 1, 2, 4, 5, 7      # 5 (tcgen05 kernels only): store relu(x)^2
+EPI_STORE, EPI_ACCUM, EPI_SWIGLU, EPI_GEGLU, EPI_RELU2, EPI_REGLU = 0, 1, 2, 4, 5, 7      # 5: store relu(x)^2
 EPI_GATED = (EPI_SWIGLU, EPI_GEGLU, EPI_REGLU)         # out = act(gate) * up over rows of w interleaved as [4 gate | 4 up]
 
 
@@ -1253,8 +1254,11 @@ def latent_mma_supports(heads: int, cached_dim: int, value_dim: int) -> bool:
 
 
 def linear_act(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, activation: str) -> None:
-    """out = act(a @ w.T) for an activation of :data:`UNARY_ACTIVATIONS`: in the product's epilogue where the
+    """out = act(a @ w.T) for an activation of :data:`UNARY_ACTIVATIONS`: in the product's epilogue where the streaming or the
     large-tile tcgen05 kernels take the shape, else by a pass of its own over the result."""
+    if activation == "relu2" and a.shape[0] <= STREAM_BEST_TOKENS and _streamable(a, w) and out.dtype == torch.bfloat16:
+        gemm_stream(a, w, out, EPI_RELU2)
+        return
     if (activation == "relu2" and USE_TCGEN05 and not _streamable(a, w) and _tensor_core_ok(a, w)
             and out.dtype == torch.bfloat16):
         gemm_tcgen05(a, w, out, EPI_RELU2)
@@ -1834,10 +1838,17 @@ CLAMPED_PAIR_MIN_TOKENS = 65
 def linear_clamped_glu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, granule: int, scratch: torch.Tensor,
                        limit: float, alpha: float = 1.702, shift: float = 1.0) -> None:
     """out = :func:`clamped_glu` of ``a @ w_gate_up^T`` (rows of ``w_gate_up`` in runs of ``granule`` gate and ``granule`` up
-    rows): in the epilogue of the paired tcgen05 product for prompt portions in bfloat16, else through ``scratch``
-    [m, 2 * inner]."""
+    rows): in bfloat16 in the epilogue of the streaming product for few tokens and of the paired tcgen05 product for prompt
+    portions, else through ``scratch`` [m, 2 * inner]."""
     m, k = a.shape
     n = w_gate_up.shape[0]
+    if granule == SWIGLU_GRANULE and n % 8 == 0 and m <= STREAM_BEST_TOKENS and _streamable(a, w_gate_up) and out.dtype == torch.bfloat16:
+        lib = library()
+        assert w_gate_up.shape[1] == k and tuple(out.shape) == (m, n // 2)
+        _check(lib.hfee_gemm_stream_clamped(a.data_ptr(), _rows(a, "gemm a"), w_gate_up.data_ptr(), _rows(w_gate_up, "gemm w"),
+                                            out.data_ptr(), _rows(out, "gemm out"), m, n, k, float(limit), float(alpha),
+                                            float(shift), _stream()), lib)
+        return
     if (granule == SWIGLU_GRANULE and n % 8 == 0 and m >= CLAMPED_PAIR_MIN_TOKENS and USE_TCGEN05 and USE_PAIRS
             and _tensor_core_ok(a, w_gate_up) and out.dtype == torch.bfloat16):
         lib = library()

@@ -1,0 +1,46 @@
+"""Activations in the epilogue of the streaming products of few tokens: the square of relu and the clamped gated activation."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rand(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(torch.bfloat16).to(DEV)
+
+
+# every kernel of the choice by tokens (8, 16, and past 16), one pass over K and several, rows that end inside a tile and a group of
+# tiles, enough tiles for the kernel with a warp per tile
+SHAPES = [(1, 8, 8), (1, 2048, 2048), (3, 24, 200), (8, 4104, 2056), (9, 40, 2048), (16, 136, 512), (12, 72, 2056), (16, 12296, 64)]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_square_of_relu(m, n, k):
+    from hfee_b200.kernels import ops
+    a, w = _rand((m, k + 8), 1)[:, :k], _rand((n, k), 2, 0.1)
+    out = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device=DEV)
+    before = ops.launch_count()
+    ops.linear_act(a, w, out[:m], "relu2")
+    assert ops.launch_count() == before + 1
+    want = torch.relu(a.double() @ w.double().t()) ** 2
+    assert (out[:m].double() - want).norm() <= 4e-3 * want.norm() + 1e-9       # rounded to bfloat16: 2^-9 an element
+    assert bool((out[m] == 7.0).all())
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+@pytest.mark.parametrize("limit,alpha,shift", [(1.5, 1.702, 1.0), (float("inf"), 1.0, 0.0)])
+def test_clamped_gate(m, n, k, limit, alpha, shift):
+    from hfee_b200.kernels import ops
+    a = _rand((m, k + 8), 3)[:, :k]
+    gate, up = _rand((n // 2, k), 4, 0.1), _rand((n // 2, k), 5, 0.1)
+    out = torch.full((m + 1, n // 2), 7.0, dtype=torch.bfloat16, device=DEV)
+    scratch = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    before = ops.launch_count()
+    ops.linear_clamped_glu(a, ops.interleave_gate_up(gate, up), out[:m], ops.SWIGLU_GRANULE, scratch, limit, alpha, shift)
+    assert ops.launch_count() == before + 1
+    g, u = a.double() @ gate.double().t(), a.double() @ up.double().t()
+    g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+    want = g * torch.sigmoid(alpha * g) * (u + shift)
+    assert (out[:m].double() - want).norm() <= 4e-3 * want.norm() + 1e-9       # rounded to bfloat16: 2^-9 an element
+    assert bool((out[m] == 7.0).all())
