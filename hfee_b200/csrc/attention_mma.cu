@@ -8,8 +8,10 @@
 // to absolute multiples of 64; a block's rows are fetched page by page with
 // cp.async (double buffered), rows outside the tile's key range are zero-filled so
 // that stale page content never reaches an MMA.  With num_splits > 1 the key blocks
-// of a tile are divided among CTAs which write unnormalised partial results; the
-// combine kernel merges them in split order.
+// of a tile are divided among CTAs.  Where all of a launch's CTAs fit the chip at one per SM,
+// those of a tile are a cluster: they leave their unnormalised partial results in their
+// shared memory and each merges a share of the outputs from all of them, in split order.
+// Otherwise they write them to memory, and the combine kernel merges them the same way.
 // Reference: hostfog/hfee internal/llm/forward.go:146-178, internal/ggml/ops.go:136-150.
 #include "common.cuh"
 
@@ -20,6 +22,7 @@
 namespace {
 
 constexpr int BLOCK_N = 64;
+constexpr int MAX_CLUSTER = 8;
 
 struct AttnParams {
   const __nv_bfloat16* q; int ld_q;
@@ -34,6 +37,7 @@ struct AttnParams {
   int window;                  // 0: all keys
   int tokens_per_tile;         // query tokens per tile = rows / group
   int num_splits;
+  int in_cluster;              // the splits of a tile are one cluster
   float* part_o;               // [(token*heads + head)*num_splits + split][HD]
   float* part_ml;              // [...][2] = (max in log2 units, sum)
   // Fused rotary + cache write (decode steps with one new token per request): q is unused;
@@ -137,6 +141,22 @@ __device__ __forceinline__ float fast_reciprocal(float x) {
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
+}
+
+// Shared memory of another block of the cluster: the address of `p` there, and loads from it.
+__device__ __forceinline__ uint32_t peer_address(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float2 ld_peer2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // KSPLIT = false: each warp owns 16 query rows and visits all 64 keys of a block (prefill).
@@ -506,6 +526,9 @@ attention_mma_kernel(AttnParams p) {
     float* mo = reinterpret_cast<float*>(k_s);                 // [NWARPS][16][HD]
     float* mm = mo + NWARPS * 16 * HD;                         // [NWARPS][16] max
     float* ml = mm + NWARPS * 16;                              // [NWARPS][16] sum
+    float* fo = ml + NWARPS * 16;                              // [16][HD] this split's merged outputs, and
+    float* fm = fo + 16 * HD;                                  // [16][2] its (max, sum): for the other CTAs of the cluster
+    static_assert((NWARPS * 16 * (HD + 2) + 16 * (HD + 2)) * 4 <= 2 * STAGES * BLOCK_N * PITCH * 2, "they lie in the stages");
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       int row = g + 8 * h;
@@ -539,11 +562,49 @@ attention_mma_kernel(AttnParams p) {
         if constexpr (DIST) inv *= p.out_scale;
         __nv_bfloat16* dst = p.out + (long long)(tok0 + t) * p.ld_o + (long long)head * vdim;
         if (d < vdim) *reinterpret_cast<__nv_bfloat162*>(dst + d) = __floats2bfloat162_rn(o0 * inv, o1 * inv);
+      } else if (p.in_cluster) {
+        *reinterpret_cast<float2*>(fo + row * HD + d) = make_float2(o0, o1);
+        if (d == 0) *reinterpret_cast<float2*>(fm + row * 2) = make_float2(m, l);
       } else {
         long long pi = ((long long)(tok0 + t) * p.heads + head) * p.num_splits + split;
         *reinterpret_cast<float2*>(p.part_o + pi * HD + d) = make_float2(o0, o1);
         if (d == 0) { p.part_ml[pi * 2] = m; p.part_ml[pi * 2 + 1] = l; }
       }
+    }
+    if (p.in_cluster) {
+      // Every split's results are in its CTA's shared memory; split s is rank s.  This CTA merges an equal share of the (row, pair
+      // of dims); all splits' values are asked for before the first is used.
+      constexpr int MAX = MAX_CLUSTER;
+      cluster_sync();
+      const int pairs = rows_used * (HD / 2), share = (pairs + p.num_splits - 1) / p.num_splits;
+      const int end = min(pairs, (split + 1) * share);
+      for (int idx = split * share + tid; idx < end; idx += THREADS) {
+        const int row = idx / (HD / 2), d = (idx % (HD / 2)) * 2;
+        float2 o[MAX], s_ml[MAX];
+#pragma unroll
+        for (int s = 0; s < MAX; ++s) {
+          o[s] = s < p.num_splits ? ld_peer2(peer_address(fo + row * HD + d, s)) : make_float2(0.f, 0.f);
+          s_ml[s] = s < p.num_splits ? ld_peer2(peer_address(fm + row * 2, s)) : make_float2(-INFINITY, 0.f);
+        }
+        float m = -INFINITY, l = 0.f, o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int s = 0; s < MAX; ++s) m = fmaxf(m, s_ml[s].x);
+#pragma unroll
+        for (int s = 0; s < MAX; ++s) {
+          const float sc = s_ml[s].x == -INFINITY ? 0.f : exp2f(s_ml[s].x - m);
+          l += sc * s_ml[s].y;
+          o0 += sc * o[s].x;
+          o1 += sc * o[s].y;
+        }
+        const int t = t_first + row / p.group, head = kvh * p.group + row % p.group;
+        if constexpr (DIST)
+          if (p.sink != nullptr && m != -INFINITY) l += exp2f(p.sink[head] * 1.4426950408889634f - m);
+        float inv = l > 0.f ? 1.f / l : 0.f;
+        if constexpr (DIST) inv *= p.out_scale;
+        __nv_bfloat16* dst = p.out + (long long)(tok0 + t) * p.ld_o + (long long)head * vdim;
+        if (d < vdim) *reinterpret_cast<__nv_bfloat162*>(dst + d) = __floats2bfloat162_rn(o0 * inv, o1 * inv);
+      }
+      cluster_sync();                // no CTA of the cluster ends while another reads its shared memory
     }
   } else {
 #pragma unroll
@@ -648,7 +709,8 @@ int launch(const AttnParams& p, int q_tiles, int kv_heads, int requests, cudaStr
     configured = true;
   }
   dim3 grid((unsigned)kv_heads, (unsigned)(q_tiles * p.num_splits), (unsigned)requests);
-  hfee_launch(attention_mma_kernel<HD, NWARPS, KSPLIT, STAGES, DIST>, dim3(grid), dim3(NWARPS * 32), smem, stream, p);
+  hfee_launch_with(hfee_carveout(), p.in_cluster ? dim3(1, (unsigned)p.num_splits, 1) : dim3(0, 0, 0),
+                   attention_mma_kernel<HD, NWARPS, KSPLIT, STAGES, DIST>, grid, dim3(NWARPS * 32), smem, stream, p);
   return hfee_check_launch("attention_mma");
 }
 
@@ -668,6 +730,12 @@ int dispatch_mode(const AttnParams& p, bool ksplit, int q_tiles, int kv_heads, i
 // Scratch floats needed for `num_splits` > 1: n_tokens * heads * num_splits * (head_dim + 2).
 HFEE_API long long hfee_attention_mma_scratch_floats(int n_tokens, int heads, int head_dim, int num_splits) {
   return num_splits > 1 ? (long long)n_tokens * heads * num_splits * (head_dim + 2) : 0;
+}
+
+// 1 when that many splits of each of `pairs` (request, kv head) pairs are clusters, which merge their results themselves: no scratch is
+// used and no combine kernel launched.  Clusters that have to wait for room cost more than the combine kernel.
+HFEE_API int hfee_attention_mma_in_cluster(int num_splits, int pairs) {
+  return (num_splits == 2 || num_splits == 4 || num_splits == MAX_CLUSTER) && (long long)num_splits * pairs <= hfee_sm_count();
 }
 
 // max_new: most new tokens of any request in the batch.  num_splits > 1 needs max_new * group <= rows
@@ -706,7 +774,7 @@ int attention_mma_impl(const void* q, int ld_q, const void* k_pool, const void* 
   HFEE_REQUIRE((long long)q_tiles * num_splits <= 65535, "attention_mma: %d new tokens of one request exceed one grid", max_new);
   HFEE_REQUIRE(num_splits == 1 || (ld_o % 4 == 0 && (uintptr_t)out % 8 == 0 && (uintptr_t)scratch % 16 == 0),
                "attention_mma: with split keys the output needs 8-byte alignment (ld %% 4 == 0) and the scratch 16-byte alignment");
-  HFEE_REQUIRE(num_splits == 1 || (q_tiles == 1 && scratch != nullptr),
+  HFEE_REQUIRE(num_splits == 1 || (q_tiles == 1 && (scratch != nullptr || (ksplit && hfee_attention_mma_in_cluster(num_splits, requests * kv_heads)))),
                "attention_mma: splitting the keys needs one query tile per request and scratch memory");
   AttnParams p;
   p.q = (const __nv_bfloat16*)q; p.ld_q = ld_q;
@@ -724,6 +792,7 @@ int attention_mma_impl(const void* q, int ld_q, const void* k_pool, const void* 
   p.heads = heads; p.group = group;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.window = window; p.tokens_per_tile = tokens_per_tile; p.num_splits = num_splits;
+  p.in_cluster = ksplit && hfee_attention_mma_in_cluster(num_splits, requests * kv_heads);
   p.part_o = scratch;
   p.part_ml = scratch ? scratch + (long long)n_tokens * heads * num_splits * head_dim : nullptr;
   p.rope_qkv = nullptr; p.ld_qkv = 0; p.rope_cs = nullptr; p.rope_dim = 0; p.rope_interleaved = 0;
@@ -756,7 +825,7 @@ int attention_mma_impl(const void* q, int ld_q, const void* k_pool, const void* 
 #undef HFEE_CASE
     default: return hfee_fail(HFEE_ERR_ARG, "attention_mma: head_dim %d", head_dim);
   }
-  if (rc != HFEE_OK || num_splits == 1) return rc;
+  if (rc != HFEE_OK || num_splits == 1 || p.in_cluster) return rc;
   int pairs = n_tokens * heads;
   hfee_launch(attention_combine_kernel, dim3((unsigned)((pairs + COMBINE_WARPS - 1) / COMBINE_WARPS)),
               dim3(COMBINE_WARPS * 32), 0, stream, p.part_o, p.part_ml, p.out, ld_o, heads, dist ? dist->value_dim : head_dim,
@@ -766,7 +835,7 @@ int attention_mma_impl(const void* q, int ld_q, const void* k_pool, const void* 
 }  // namespace
 
 // q [n_tokens, ld_q], out [n_tokens, ld_o]: bfloat16; pools [num_pages, kv_heads, page_size, head_dim].
-// num_splits > 1 (only when max_new * group <= 16) needs `scratch` of
+// num_splits > 1 (only when max_new * group <= 16), unless in clusters, needs `scratch` of
 // n_tokens * heads * num_splits * (head_dim + 2) floats and launches the combine kernel too.
 HFEE_API int hfee_attention_mma(const void* q, int ld_q, const void* k_pool, const void* v_pool,
                                 const int* block_table, int max_pages, int page_size, const int* cu_tokens,

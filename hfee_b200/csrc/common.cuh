@@ -46,15 +46,16 @@ int hfee_pdl_enabled();
 int hfee_carveout();
 
 // carve: the split between shared memory and L1 to ask for (percent), below 0 for the driver's choice.
+// cluster: blocks of a cluster, 0 for none (at most 8 in all, which every such GPU takes).
 template <typename... KArgs, typename... Args>
-cudaError_t hfee_launch_carved(int carve, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                               Args&&... args) {
+cudaError_t hfee_launch_with(int carve, dim3 cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = hfee_pdl_enabled();
   cfg.attrs = attr;
@@ -64,7 +65,17 @@ cudaError_t hfee_launch_carved(int carve, void (*kernel)(KArgs...), dim3 grid, d
     attr[1].val.sharedMemCarveout = (unsigned int)carve;
     cfg.numAttrs = 2;
   }
+  if (cluster.x > 0) {
+    cudaLaunchAttribute& at = attr[cfg.numAttrs++];
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cluster.x; at.val.clusterDim.y = cluster.y; at.val.clusterDim.z = cluster.z;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t hfee_launch_carved(int carve, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               Args&&... args) {
+  return hfee_launch_with(carve, dim3(0, 0, 0), kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 template <typename... KArgs, typename... Args>
 cudaError_t hfee_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

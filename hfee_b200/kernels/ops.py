@@ -783,14 +783,31 @@ def attention_splits(requests: int, kv_heads: int, max_context: int, sms: Option
     two CTAs per SM: those grids take the kernel variant with four key blocks in flight per CTA, of
     which the step's shared-memory carve-out holds one per SM (decode step of the benchmark model at
     batch 2 / 3 / 4 / 5 / 6: 0.742 / 0.777 / 0.786 / 0.802 / 0.817 ms against 0.755 / 0.798 / 0.809 /
-    0.812 / 0.823 with four per SM; at batch 8: 0.857 against 0.838)."""
+    0.812 / 0.823 with four per SM; at batch 8: 0.857 against 0.838).
+
+    One or two requests take clusters of eight instead, which need no combine kernel (decode step of one request at 1,024 keys 684 us
+    against 706 with 32 splits and the combine kernel, at 3,900 keys 736 against 725; of two requests at 2,048 keys 710 against 720;
+    clusters of 16 at 1,024 / 3,900: 690 / 710, and at 80 keys no faster than the combine kernel, which eights beat by 12 us).  More clusters than the chip holds at once wait for room among the kernels around them: eight
+    requests at 2,048 keys 848 us against 833, 64 requests 1,565 against 1,532."""
     pairs = max(1, requests * kv_heads)
     per_sm = 2 if pairs <= FEW_PAIRS else 4
-    want = max(4, per_sm * (sms or sm_count()) // pairs)
-    return max(1, min(MAX_SPLITS, want, max_context // 128))
+    sms = sms or sm_count()
+    want = max(1, min(MAX_SPLITS, max(4, per_sm * sms // pairs), max_context // 128))
+    if max_context <= CLUSTER_MAX_CONTEXT:
+        for size in (8, 4, 2):
+            if size <= want and (size == 8 or 2 * size > want) and splits_in_cluster(size, pairs, sms):
+                return size
+    return want
 
 
 FEW_PAIRS = 48
+CLUSTER_MAX_CONTEXT = 4096      # from here on few pairs take more splits than a cluster has
+
+
+def splits_in_cluster(splits: int, pairs: int, sms: Optional[int] = None) -> bool:
+    """True where the splits of each of ``pairs`` (request, kv head) pairs are one cluster of CTAs, which merges its results itself (the
+    launch's rule); others need the combine kernel."""
+    return splits in (2, 4, 8) and splits * pairs <= (sms or sm_count())
 
 
 def attention_mma(q, k_pool, v_pool, block_table, page_size, cu_tokens, slots, context_before, out, n_tokens,
@@ -811,7 +828,7 @@ def attention_mma(q, k_pool, v_pool, block_table, page_size, cu_tokens, slots, c
                                   slots.data_ptr(), context_before.data_ptr(), out.data_ptr(),
                                   _rows(out, "attention out"), n_tokens, requests, max_new, heads, kv_heads,
                                   head_dim, float(scale), int(window or 0), num_splits, _ptr(scratch), _stream()), lib)
-    if num_splits > 1:
+    if num_splits > 1 and not splits_in_cluster(num_splits, requests * kv_heads):
         count_launches(1)
 
 
@@ -912,7 +929,7 @@ def paged_attention_rope(qkv, cs, rope_dim, interleaved, write_cache, k_pool, v_
                                        step.context_before.data_ptr(), out.data_ptr(), _rows(out, "attention out"),
                                        step.n, step.r, heads, kv_heads, head_dim, float(scale), int(window or 0), splits,
                                        _ptr(scratch) if splits > 1 else None, _stream()), lib)
-    if splits > 1:
+    if splits > 1 and not splits_in_cluster(splits, step.r * kv_heads):
         count_launches(1)
 
 
@@ -1140,7 +1157,7 @@ def distance_attention(q, k_pool, v_pool, block_table, page_size, step, out, hea
                                            step.r, step.max_new, heads, kv_heads, head_dim, value_dim, float(scale), r1.data_ptr(),
                                            r2.data_ptr(), float(out_scale), int(window or 0), splits,
                                            _ptr(scratch) if splits > 1 else None, _stream()), lib)
-    if splits > 1:
+    if splits > 1 and not splits_in_cluster(splits, step.r * kv_heads):
         count_launches(1)
 
 
@@ -2084,7 +2101,7 @@ def softmax_attention(q, k_pool, v_pool, block_table, page_size, step, out, head
                                           step.r, step.max_new, heads, kv_heads, head_dim, value_dim, float(scale), None, None,
                                           _ptr(sink), float(out_scale), int(window or 0), int(keep_first), cap, splits,
                                           _ptr(scratch) if splits > 1 else None, _stream()), lib)
-    if splits > 1:
+    if splits > 1 and not splits_in_cluster(splits, step.r * kv_heads):
         count_launches(1)
 
 

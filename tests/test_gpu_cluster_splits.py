@@ -1,0 +1,76 @@
+"""Split-key attention of decode steps: splits that are one cluster merge their results themselves, like the combine kernel does."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+class _Step:
+    def __init__(self, before, page, max_pages):
+        r = len(before)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        self.n = self.r = r
+        self.max_new, self.max_context = 1, max(before) + 1
+        self.cu_tokens, self.slots, self.context_before = i32(list(range(r + 1))), i32(list(range(r))), i32(before)
+        self.positions, self.slot_of_token = i32(before), i32(list(range(r)))
+        need = [-(-(b + 1) // page) for b in before]
+        table = np.zeros((r, max_pages), dtype=np.int32)
+        order = np.random.default_rng(0).permutation(sum(need))
+        at = 0
+        for i, k in enumerate(need):
+            table[i, :k] = order[at:at + k]
+            at += k
+        self.table, self.pages = i32(table.tolist()), sum(need)
+
+
+def _rand(shape, seed):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).to(DEV)
+
+
+# contexts of one key up to several blocks a split: most splits find no keys at the short ones, and the last block is ragged
+@pytest.mark.parametrize("dim,heads,kv_heads", [(64, 32, 8), (128, 8, 8), (16, 16, 1), (256, 6, 3)])
+@pytest.mark.parametrize("splits", [2, 4, 8])
+@pytest.mark.parametrize("window", [0, 100])
+def test_cluster_against_the_combine_kernel(dim, heads, kv_heads, splits, window):
+    from hfee_b200.kernels import ops
+    page = 64
+    contexts = [0, 1, 63, 64, 127, 700, 1535, 2049]
+    contexts = contexts[-max(1, min(8, ops.sm_count() // (splits * kv_heads))):]       # more CTAs than SMs go through memory
+    step = _Step(contexts, page, 40)
+    k, v = _rand((step.pages, kv_heads, page, dim), 1), _rand((step.pages, kv_heads, page, dim), 2)
+    q = _rand((step.n, heads * dim), 3)
+    outs = []
+    for s in (splits, 3):                                  # three splits go through memory and the combine kernel
+        assert ops.splits_in_cluster(s, step.r * kv_heads) == (s != 3)
+        out = torch.full((step.n + 1, heads * dim), 7.0, dtype=torch.bfloat16, device=DEV)
+        scratch = torch.full((step.n * heads * s * (dim + 2),), float("nan"), device=DEV)
+        ops.attention_mma(q, k, v, step.table, page, step.cu_tokens, step.slots, step.context_before, out[:step.n], step.n, step.r, 1,
+                          heads, kv_heads, dim, dim ** -0.5, window, s, scratch)
+        assert bool((out[step.n] == 7.0).all()) and (s == 3 or bool(torch.isnan(scratch).all()))
+        outs.append(out[:step.n].double())
+    for i in range(step.n):
+        before = int(step.context_before[i])
+        lo = max(0, before + 1 - window) if window else 0
+        rows = torch.arange(lo, before + 1, device=DEV)
+        at = step.table[i, rows // page].long() * page + rows % page
+        group = heads // kv_heads
+        for h in range(heads):
+            ks = k.transpose(1, 2).reshape(-1, kv_heads, dim)[at, h // group].double()
+            vs = v.transpose(1, 2).reshape(-1, kv_heads, dim)[at, h // group].double()
+            p = torch.softmax(ks @ q[i, h * dim:(h + 1) * dim].double() * dim ** -0.5, 0)
+            want = p @ vs
+            # weights rounded to bfloat16 (2^-9 each, averaged over the keys), the output once more
+            for out in outs:
+                assert (out[i, h * dim:(h + 1) * dim] - want).norm() <= 6e-3 * want.norm() + 1e-3
+    assert (outs[0] - outs[1]).norm() <= 4e-3 * outs[1].norm()       # both round their output to bfloat16
+
+
+def test_rule_takes_clusters_where_they_fit_the_chip_and_more_splits_behind_a_context():
+    from hfee_b200.kernels import ops
+    for requests in (1, 2):
+        for context in (256, 512, 1024, 4096):
+            assert ops.splits_in_cluster(ops.attention_splits(requests, 8, context, 148), requests * 8, 148)
+    assert ops.attention_splits(3, 8, 4096, 148) == 12 and ops.attention_splits(8, 8, 4096, 148) == 9
+    assert ops.attention_splits(1, 8, 1 << 16, 148) == ops.MAX_SPLITS
