@@ -40,7 +40,10 @@ template <int EPI> __device__ __forceinline__ float gated_out(float gate, float 
   return gate_value<EPI>(gate) * up;
 }
 template <int EPI> __device__ __forceinline__ float stored_out(float v) {
-  if constexpr (EPI == EPI_RELU2) { v = fmaxf(v, 0.f); return v * v; }
+  if constexpr (EPI == EPI_RELU2) {       // of the product as it is stored: what a kernel of its own would read
+    v = fmaxf(__bfloat162float(__float2bfloat16_rn(v)), 0.f);
+    return v * v;
+  }
   return v;
 }
 

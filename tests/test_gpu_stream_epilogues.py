@@ -24,7 +24,11 @@ def test_square_of_relu(m, n, k):
     ops.linear_act(a, w, out[:m], "relu2")
     assert ops.launch_count() == before + 1
     want = torch.relu(a.double() @ w.double().t()) ** 2
-    assert (out[:m].double() - want).norm() <= 4e-3 * want.norm() + 1e-9       # rounded to bfloat16: 2^-9 an element
+    assert (out[:m].double() - want).norm() <= 8e-3 * want.norm() + 1e-9       # the product and its square rounded to bfloat16: 2^-9 each, the first twice
+    plain = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_stream(a, w, plain)
+    ops.unary_act(plain, plain, "relu2")
+    assert bool((out[:m] == plain).all())                                      # bit for bit what two kernels give
     assert bool((out[m] == 7.0).all())
 
 
