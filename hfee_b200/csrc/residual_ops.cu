@@ -83,6 +83,8 @@ __device__ __forceinline__ float block_sum(float v, float* shared) {
   return total;
 }
 
+template <typename T> struct alignas(4 * sizeof(T)) FourOf { T v[4]; };
+
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
 scaled_add_norm_kernel(const float* __restrict__ y, float m, float* __restrict__ residual, const float* __restrict__ w,
@@ -102,6 +104,61 @@ scaled_add_norm_kernel(const float* __restrict__ y, float m, float* __restrict__
   const float inv = 1.f / sqrtf(block_sum(sq, partial) / (float)width + eps);
   T* o = out + (long long)blockIdx.x * ld_out;
   for (int c = threadIdx.x; c < width; c += ROW_THREADS) o[c] = from_f32<T>(rr[c] * inv * w[c]);   // the thread's own writes
+}
+
+// The same for widths that are multiples of 4 and at most ROW_THREADS * 4 * NCH, rows on 16 bytes: both rows are asked for at once in
+// 16-byte pieces and stay in registers, the weights come before the wait.
+template <typename T, int NCH>
+__global__ void __launch_bounds__(ROW_THREADS)
+scaled_add_norm_vec_kernel(const float* __restrict__ y, float m, float* __restrict__ residual, const float* __restrict__ w,
+                           float eps, T* __restrict__ out, long long ld_out, int width) {
+  __shared__ float partial[ROW_THREADS / 32];
+  float4 wv[NCH], v[NCH], r[NCH];
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int j = 0; j < NCH; ++j) {
+    const int c = (threadIdx.x + j * ROW_THREADS) * 4;
+    wv[j] = out != nullptr && c < width ? __ldg(reinterpret_cast<const float4*>(w + c)) : none;
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  const float* yr = y + (long long)blockIdx.x * width;
+  float* rr = residual + (long long)blockIdx.x * width;
+#pragma unroll
+  for (int j = 0; j < NCH; ++j) {
+    const int c = (threadIdx.x + j * ROW_THREADS) * 4;
+    v[j] = c < width ? *reinterpret_cast<const float4*>(yr + c) : none;
+    r[j] = c < width ? *reinterpret_cast<const float4*>(rr + c) : none;
+  }
+  float sq = 0.f;
+#pragma unroll
+  for (int j = 0; j < NCH; ++j) {
+    const int c = (threadIdx.x + j * ROW_THREADS) * 4;
+    r[j] = make_float4(fmaf(m, v[j].x, r[j].x), fmaf(m, v[j].y, r[j].y), fmaf(m, v[j].z, r[j].z), fmaf(m, v[j].w, r[j].w));
+    if (c < width) *reinterpret_cast<float4*>(rr + c) = r[j];
+    sq = fmaf(r[j].x, r[j].x, fmaf(r[j].y, r[j].y, fmaf(r[j].z, r[j].z, fmaf(r[j].w, r[j].w, sq))));
+  }
+  if (out == nullptr) return;            // the sum alone (the same for every thread of the launch)
+  const float inv = 1.f / sqrtf(block_sum(sq, partial) / (float)width + eps);
+  T* o = out + (long long)blockIdx.x * ld_out;
+#pragma unroll
+  for (int j = 0; j < NCH; ++j) {
+    const int c = (threadIdx.x + j * ROW_THREADS) * 4;
+    if (c >= width) continue;
+    FourOf<T> p{{from_f32<T>(r[j].x * inv * wv[j].x), from_f32<T>(r[j].y * inv * wv[j].y), from_f32<T>(r[j].z * inv * wv[j].z),
+                 from_f32<T>(r[j].w * inv * wv[j].w)}};
+    *reinterpret_cast<FourOf<T>*>(o + c) = p;
+  }
+}
+
+template <typename T>
+void launch_scaled_add_norm(const float* y, float m, float* residual, const float* w, float eps, T* out, long long ld_out, int n, int width,
+                            cudaStream_t stream) {
+  const bool pieces = width % 4 == 0 && width <= ROW_THREADS * 16 && (uintptr_t)y % 16 == 0 && (uintptr_t)residual % 16 == 0 &&
+                      (out == nullptr || ((uintptr_t)w % 16 == 0 && (uintptr_t)out % (4 * sizeof(T)) == 0 && ld_out % 4 == 0));
+  auto kernel = !pieces ? scaled_add_norm_kernel<T> : width <= ROW_THREADS * 4 ? scaled_add_norm_vec_kernel<T, 1>
+                : width <= ROW_THREADS * 8 ? scaled_add_norm_vec_kernel<T, 2> : scaled_add_norm_vec_kernel<T, 4>;
+  hfee_launch(kernel, dim3((unsigned)n), dim3(ROW_THREADS), 0, stream, y, m, residual, w, eps, out, ld_out, width);
 }
 
 constexpr int MAX_DEPTH = 256;
@@ -163,10 +220,9 @@ HFEE_API int hfee_scaled_add_norm(const float* y, float m, float* residual, cons
   if (n == 0) return HFEE_OK;
   HFEE_REQUIRE(n > 0 && width > 0 && (out == nullptr || (ld_out >= width && w != nullptr)), "scaled_add_norm: bad sizes");
   if (dtype == HFEE_F32)
-    hfee_launch(scaled_add_norm_kernel<float>, dim3(n), dim3(ROW_THREADS), 0, stream, y, m, residual, w, eps, (float*)out, ld_out, width);
+    launch_scaled_add_norm<float>(y, m, residual, w, eps, (float*)out, ld_out, n, width, stream);
   else if (dtype == HFEE_BF16)
-    hfee_launch(scaled_add_norm_kernel<__nv_bfloat16>, dim3(n), dim3(ROW_THREADS), 0, stream, y, m, residual, w, eps,
-                (__nv_bfloat16*)out, ld_out, width);
+    launch_scaled_add_norm<__nv_bfloat16>(y, m, residual, w, eps, (__nv_bfloat16*)out, ld_out, n, width, stream);
   else
     return hfee_fail(HFEE_ERR_ARG, "scaled_add_norm: unknown dtype %d", dtype);
   return hfee_check_launch("scaled_add_norm");

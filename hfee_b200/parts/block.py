@@ -152,9 +152,18 @@ class ScaledPreNormBlock(Block):
     """``y = x + m * mixer(norm(x)); r = y + m * feed_forward(norm(y))`` with one multiplier ``m`` on every
     sublayer's output (spec ``residual_scale``), and an optional ``merge`` part that turns the layer's result r into
     what the next layer reads.  ``ffn`` with ``ffn_norm`` is optional.  The scaled sum and the next norm leave in one
-    kernel; the last sum is the merge's, when there is one."""
+    kernel, behind the last sublayer too where the next layer is of this kind (``entry`` and ``then``, as in
+    :class:`PreNormBlock`); the last sum is the merge's, when there is one."""
     needs = ("mixer", "mixer_norm")
     graph_safe = True
+
+    @property
+    def takes_entry(self) -> bool:
+        params = getattr(self.mixer_norm, "fused_params", None)
+        return self.merge is None and params is not None and not params()[2]
+
+    def entry(self, residual: torch.Tensor, step: Any) -> LazyNormed:
+        return LazyNormed(self.mixer_norm, residual, self.rt.scratch("block_normed", (self.rt.max_tokens, self.width))[:step.n])
 
     def __init__(self, spec, tensors, rt, parts):
         super().__init__(spec, tensors, rt, parts)
@@ -165,13 +174,16 @@ class ScaledPreNormBlock(Block):
         self.merge = parts.get("merge")
         self.width, self.scale = int(spec.width), float(spec.residual_scale)
 
-    def forward(self, residual: torch.Tensor, step: Any, cache: Any, writes_cache: bool) -> None:
+    def forward(self, residual: torch.Tensor, step: Any, cache: Any, writes_cache: bool, entry=None, then=None) -> None:
         rt, n = self.rt, step.n
         xn = rt.scratch("block_normed", (rt.max_tokens, self.width))[:n]
         y = rt.scratch("block_sublayer_out", (rt.max_tokens, self.width), torch.float32)[:n]
         if self.merge is not None:
             self.merge.begin(residual, step)
-        self.mixer_norm.forward(residual, xn)
+        if entry is not None:
+            entry.tensor()
+        else:
+            self.mixer_norm.forward(residual, xn)
         OutputNormBlock._run(self.mixer, y, xn, step, cache, writes_cache)
         if self.feed_forward is not None:
             ops.tag("norm")
@@ -179,8 +191,13 @@ class ScaledPreNormBlock(Block):
             OutputNormBlock._run(self.feed_forward, y, xn, step)
         if self.merge is not None:
             self.merge.forward(residual, y, self.scale, step)
+            return
+        ops.tag("norm")
+        params = then.fused_params() if then is not None and then.rows is None else None
+        if params is not None and not params[2] and then.buffer.shape == residual.shape:
+            ops.scaled_add_norm(y, self.scale, residual, params[0], params[1], then.buffer)
+            then.in_buffer()
         else:
-            ops.tag("norm")
             ops.scaled_add(y, self.scale, residual)
 
 
