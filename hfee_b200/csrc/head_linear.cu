@@ -6,7 +6,9 @@
 //
 // bfloat16 with 16-byte aligned head slices runs on the tensor cores (mma.sync.m16n8k16, float32 accumulation): a block
 // takes 64 tokens x 64 output columns of one head, stages 64 columns of k of both operands in shared memory at a
-// time, and each of its four warps owns 32 x 32 of the tile.  Everything else runs on the CUDA cores with float32
+// time, and each of its four warps owns 32 x 32 of the tile.  At most HF_TOKENS tokens (a decode step) take
+// `head_linear_few_kernel`, whose inputs may also be the shares of a latent attention with split keys
+// (hfee_head_linear_parts).  Everything else runs on the CUDA cores with float32
 // accumulation over k in order: a block takes HL_TOKENS tokens of one head, keeps their inputs in shared memory,
 // and every thread owns output columns for all of those tokens.
 #include "mma_tiles.cuh"
@@ -142,6 +144,118 @@ head_linear_mma_kernel(const bf16* __restrict__ in, long long ld_in, int in_off,
   }
 }
 
+// A few tokens: the product is one trip to memory for the weights (1 MB) and one for the inputs, so the weights are in registers before
+// the wait for the kernel in front; the tile kernel above fetches both 64 columns of k at a time behind it, a trip each.  A warp has
+// four rows of W, `lanes` lanes (8, 16 or 32) on each with CH pieces of 16 bytes; the inputs lie in shared memory in float32.
+// With `partial` the input of (token, head) is put together here from the `splits` shares of its split keys, each an unnormalised
+// output of n_in numbers, a maximum (log2 units) and a sum ([splits][n][heads][n_in + 2]), as latent_combine_kernel does it.
+// One token, 32 heads, in place: 64 x 256 matrices (queries) 3.5 -> 2.5 us, 256 x 64 behind 9 shares 2.6 + 5.0 -> 4.7 us for both kernels.
+constexpr int HF_TOKENS = 8, HF_PART_TOKENS = 2, HF_ROWS = 16, HF_THREADS = 128, HF_SHARES = 32;
+
+struct FewInput {
+  const bf16* in; long long ld; int off, stride;
+  const float* partial; int splits, heads; const float* sink;
+};
+
+template <int CH, bool PARTS>
+__global__ void __launch_bounds__(HF_THREADS)
+head_linear_few_kernel(FewInput x, const bf16* __restrict__ w, bf16* __restrict__ out, long long ld_out, int out_off, int out_stride, int n,
+                       int n_in, int n_out, const bf16* __restrict__ gate, long long ld_gate, int lanes) {
+  constexpr int MAX_N = PARTS ? HF_PART_TOKENS : HF_TOKENS;
+  __shared__ __align__(16) float in_s[MAX_N * 256 * CH];                                       // [n][n_in]
+  __shared__ float share_s[PARTS ? HF_PART_TOKENS * HF_SHARES : 1];
+  const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int at = lane % lanes, rows_at_once = 32 / lanes, trips = lanes / 8;
+  const int row0 = blockIdx.x * HF_ROWS + warp * 4 + lane / lanes;
+  const bf16* wh = w + (long long)h * n_out * n_in;
+  uint4 wv[4][CH];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int r = row0 + i * rows_at_once, k = (at + c * 32) * 8;
+      wv[i][c] = i < trips && r < n_out && k < n_in ? __ldg(reinterpret_cast<const uint4*>(wh + (long long)r * n_in + k)) : make_uint4(0, 0, 0, 0);
+    }
+  pdl_wait();
+  pdl_launch_dependents();
+  float gv = 1.f;                              // of token `at`, whose results this lane stores
+  if (gate != nullptr && at < n) gv = 1.f / (1.f + expf(-__bfloat162float(gate[(long long)at * ld_gate + h])));
+  if constexpr (PARTS) {
+    const long long stride = (long long)n * x.heads * (n_in + 2);
+    if (warp < n) {                            // lane s: share s
+      const float* mine = x.partial + ((long long)warp * x.heads + h) * (n_in + 2);
+      float m = -INFINITY, l = 0.f;
+      if (lane < x.splits) { m = mine[lane * stride + n_in]; l = mine[lane * stride + n_in + 1]; }
+      const float s2 = x.sink != nullptr ? x.sink[h] * 1.4426950408889634f : -INFINITY;
+      const float top = fmaxf(warp_max(m), s2);
+      const float e = m == -INFINITY ? 0.f : exp2f(m - top);
+      const float total = warp_sum(e * l) + (x.sink != nullptr ? exp2f(s2 - top) : 0.f);
+      share_s[warp * HF_SHARES + lane] = total > 0.f ? e / total : 0.f;
+    }
+    for (int base = 0; base < n * n_in; base += 2 * HF_THREADS) {
+      const int e = base + 2 * threadIdx.x, t = e / n_in, k = e - t * n_in;
+      const bool ok = e < n * n_in;
+      const float* mine = x.partial + ((long long)(ok ? t : 0) * x.heads + h) * (n_in + 2) + (ok ? k : 0);
+      float2 v[HF_SHARES];
+#pragma unroll
+      for (int s = 0; s < HF_SHARES; ++s) v[s] = s < x.splits ? *reinterpret_cast<const float2*>(mine + s * stride) : make_float2(0.f, 0.f);
+      if (base == 0) __syncthreads();          // asked for before the shares' weights are known
+      float a = 0.f, b = 0.f;
+#pragma unroll
+      for (int s = 0; s < HF_SHARES; ++s)
+        if (s < x.splits && ok) { a = fmaf(share_s[t * HF_SHARES + s], v[s].x, a); b = fmaf(share_s[t * HF_SHARES + s], v[s].y, b); }
+      if (ok) *reinterpret_cast<float2*>(in_s + e) = make_float2(a, b);
+    }
+  } else {
+    for (int e = threadIdx.x; e < n * (n_in / 8); e += HF_THREADS) {
+      const int t = e / (n_in / 8), k = (e - t * (n_in / 8)) * 8;
+      const uint4 v = *reinterpret_cast<const uint4*>(x.in + (long long)t * x.ld + x.off + (long long)h * x.stride + k);
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float2*>(in_s + t * n_in + k + 2 * i) = make_float2(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xffff0000u));
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (i >= trips) break;
+    const int r = row0 + i * rows_at_once;
+    float mine = 0.f;
+#pragma unroll
+    for (int t = 0; t < MAX_N; ++t) {
+      if (t >= n) break;
+      float acc = 0.f;
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        const int k = (at + c * 32) * 8;
+        if (k < n_in) {
+          const uint4 q = wv[i][c];
+          const float4 x0 = *reinterpret_cast<const float4*>(in_s + t * n_in + k), x1 = *reinterpret_cast<const float4*>(in_s + t * n_in + k + 4);
+          acc = fmaf(__uint_as_float(q.x << 16), x0.x, acc); acc = fmaf(__uint_as_float(q.x & 0xffff0000u), x0.y, acc);
+          acc = fmaf(__uint_as_float(q.y << 16), x0.z, acc); acc = fmaf(__uint_as_float(q.y & 0xffff0000u), x0.w, acc);
+          acc = fmaf(__uint_as_float(q.z << 16), x1.x, acc); acc = fmaf(__uint_as_float(q.z & 0xffff0000u), x1.y, acc);
+          acc = fmaf(__uint_as_float(q.w << 16), x1.z, acc); acc = fmaf(__uint_as_float(q.w & 0xffff0000u), x1.w, acc);
+        }
+      }
+      for (int o = lanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (at == t) mine = acc;
+    }
+    if (at < n && r < n_out) out[(long long)at * ld_out + out_off + (long long)h * out_stride + r] = __float2bfloat16_rn(mine * gv);
+  }
+}
+
+template <bool PARTS>
+int launch_head_linear_few(const FewInput& x, const void* w, void* out, long long ld_out, int out_off, int out_stride, int n, int heads,
+                           int n_in, int n_out, const void* gate, long long ld_gate, cudaStream_t stream) {
+  int lanes = 8;
+  while (lanes < 32 && lanes * 8 < n_in) lanes *= 2;
+  auto kernel = n_in <= 256 ? head_linear_few_kernel<1, PARTS> : head_linear_few_kernel<2, PARTS>;
+  hfee_launch(kernel, dim3((unsigned)((n_out + HF_ROWS - 1) / HF_ROWS), (unsigned)heads), dim3(HF_THREADS), 0, stream, x, (const bf16*)w,
+              (bf16*)out, ld_out, out_off, out_stride, n, n_in, n_out, (const bf16*)gate, ld_gate, lanes);
+  return hfee_check_launch("head_linear_few");
+}
+
 bool head_linear_mma_takes(const void* in, long long ld_in, int in_off, int in_stride, const void* w, int n_in) {
   return n_in % 8 == 0 && ld_in % 8 == 0 && in_off % 8 == 0 && in_stride % 8 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)w % 16 == 0;
 }
@@ -170,6 +284,9 @@ HFEE_API int hfee_head_linear(const void* in, long long ld_in, int in_off, int i
   HFEE_REQUIRE(heads > 0 && n_in > 0 && n_out > 0 && n_in <= 2048, "head_linear: bad sizes (n_in at most 2048)");
   if (dtype == HFEE_F32)
     return launch_head_linear<float>(in, ld_in, in_off, in_stride, w, out, ld_out, out_off, out_stride, n, heads, n_in, n_out, gate, ld_gate, stream);
+  if (dtype == HFEE_BF16 && n <= HF_TOKENS && n_in <= 512 && heads <= 65535 && head_linear_mma_takes(in, ld_in, in_off, in_stride, w, n_in))
+    return launch_head_linear_few<false>(FewInput{(const bf16*)in, ld_in, in_off, in_stride, nullptr, 0, heads, nullptr}, w, out, ld_out, out_off,
+                                         out_stride, n, heads, n_in, n_out, gate, ld_gate, stream);
   if (dtype == HFEE_BF16 && head_linear_mma_takes(in, ld_in, in_off, in_stride, w, n_in)) {
     // rows of the output that start on 16 bytes and hold whole 16-byte pieces leave through shared memory
     const int wide = n_out % 8 == 0 && ld_out % 8 == 0 && out_off % 8 == 0 && out_stride % 8 == 0 && (uintptr_t)out % 16 == 0;
@@ -181,4 +298,18 @@ HFEE_API int hfee_head_linear(const void* in, long long ld_in, int in_off, int i
   if (dtype == HFEE_BF16)
     return launch_head_linear<__nv_bfloat16>(in, ld_in, in_off, in_stride, w, out, ld_out, out_off, out_stride, n, heads, n_in, n_out, gate, ld_gate, stream);
   return hfee_fail(HFEE_ERR_ARG, "head_linear: unknown dtype %d", dtype);
+}
+
+// The same in bfloat16 for at most 2 tokens whose inputs are shares of a latent attention with split keys: partial
+// [splits][n][heads][n_in + 2] float32 (see hfee_latent_attention_mma without an output), sink: per head or null.
+HFEE_API int hfee_head_linear_parts(const float* partial, int splits, const float* sink, const void* w, void* out, long long ld_out,
+                                    int out_off, int out_stride, int n, int heads, int n_in, int n_out, const void* gate, long long ld_gate,
+                                    cudaStream_t stream) {
+  if (n == 0) return HFEE_OK;
+  HFEE_REQUIRE(n > 0 && n <= HF_PART_TOKENS && heads > 0 && heads <= 65535 && n_in > 0 && n_in % 8 == 0 && n_in <= 512 && n_out > 0,
+               "head_linear_parts: takes at most %d tokens and n_in a multiple of 8 up to 512 (got %d, %d)", HF_PART_TOKENS, n, n_in);
+  HFEE_REQUIRE(splits >= 1 && splits <= HF_SHARES && partial != nullptr && (uintptr_t)partial % 8 == 0 && (uintptr_t)w % 16 == 0,
+               "head_linear_parts: %d shares, or operands off their boundaries", splits);
+  return launch_head_linear_few<true>(FewInput{nullptr, 0, 0, 0, partial, splits, heads, sink}, w, out, ld_out, out_off, out_stride, n, heads,
+                                      n_in, n_out, gate, ld_gate, stream);
 }

@@ -381,7 +381,8 @@ HFEE_API int hfee_latent_attention_mma_supports(int heads, int dk, int dv) {
   return heads > 0 && dk > 0 && dk % 16 == 0 && dv > 0 && dv % 16 == 0 && dv <= dk && dv <= 512 && latent_smem(dk, LA_ROWS) <= 227 * 1024;
 }
 
-// splits > 1 (at most 32): that many CTAs share a tile's keys through `partial`, [splits][n_tokens][heads][dv + 2] floats.
+// splits > 1 (at most 32): that many CTAs share a tile's keys through `partial`, [splits][n_tokens][heads][dv + 2] floats; without
+// an output (null) the shares stay there, for hfee_head_linear_parts.
 HFEE_API int hfee_latent_attention_mma(const void* q, long long ld_q, const void* pool, const int* block_table, int max_pages,
                                        int page_size, const int* cu_tokens, const int* slots, const int* context_before,
                                        void* out, long long ld_o, int requests, int max_new, int heads, int dk, int dv,
@@ -391,6 +392,7 @@ HFEE_API int hfee_latent_attention_mma(const void* q, long long ld_q, const void
   HFEE_REQUIRE(hfee_latent_attention_mma_supports(heads, dk, dv), "latent_attention_mma: sizes %d heads, %d key, %d value dimensions are not taken", heads, dk, dv);
   HFEE_REQUIRE(page_size > 0 && (page_size & (page_size - 1)) == 0, "page_size %d must be a power of two", page_size);
   HFEE_REQUIRE(ld_q % 8 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)pool % 16 == 0, "latent_attention_mma: queries and cache must be 16-byte aligned");
+  HFEE_REQUIRE(out != nullptr || splits > 1, "latent_attention_mma: no output, and no shares of split keys to leave");
   HFEE_REQUIRE(ld_o % 2 == 0 && (uintptr_t)out % 4 == 0, "latent_attention_mma: the output's rows must start on 4 bytes");
   HFEE_REQUIRE(requests <= 65535 && window >= 0, "latent_attention_mma: bad batch or window");
   HFEE_REQUIRE(splits >= 1 && splits <= 32 && (splits == 1 || (partial != nullptr && (uintptr_t)partial % 8 == 0 && n_tokens > 0)),
@@ -428,7 +430,7 @@ HFEE_API int hfee_latent_attention_mma(const void* q, long long ld_q, const void
     else if (per_warp <= 4) rc = launch_latent<4, 1>(p, grid, stream);
     else rc = launch_latent<8, 1>(p, grid, stream);
   }
-  if (rc != HFEE_OK || splits == 1) return rc;
+  if (rc != HFEE_OK || splits == 1 || out == nullptr) return rc;
   hfee_launch(latent_combine_kernel, dim3((unsigned)heads, (unsigned)n_tokens), dim3(LC_THREADS), 0, stream, partial, splits,
               n_tokens, heads, dv, sink, (bf16*)out, ld_o);
   return hfee_check_launch("latent_combine");

@@ -77,6 +77,7 @@ _SIGNATURES = {
     "hfee_channel_delta": [_P, _L, _I, _I, _I, _P, _L, _P, _L, _I, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "hfee_latent_attention_mma_supports": [_I, _I, _I],
     "hfee_head_linear": [_P, _L, _I, _I, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P, _L, _I, _P],
+    "hfee_head_linear_parts": [_P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P, _L, _P],
     "hfee_conv_act": [_P, _L, _I, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
     "hfee_attention_simt_distance": [_P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P, _L, _I,
                                      _P, _P, _F, _I, _P],
@@ -1179,12 +1180,14 @@ def softmax_attention_on_tensor_cores(q: torch.Tensor, out: torch.Tensor, heads:
 
 def latent_attention(q: torch.Tensor, k_pool: torch.Tensor, block_table: torch.Tensor, page_size: int, step,
                      out: torch.Tensor, heads: int, cached_dim: int, value_dim: int, scale: float, window: int = 0,
-                     sink: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None) -> None:
+                     sink: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None, leave_parts: bool = False) -> int:
     """Softmax attention of ``heads`` query heads over ONE cached vector per token (``k_pool`` [pages, 1, page_size,
     cached_dim]) whose leading ``value_dim`` dimensions are also the values: ``out`` [n, heads * value_dim].
     ``sink`` (float32 per head): the denominator also holds exp(sink[h]).  ``scratch`` (float32) lets a step of single
     tokens split its keys among CTAs.  bfloat16 runs on the tensor cores where the sizes allow it (portions of LATENT_TC_MIN_ROWS
-    (token, head) rows and more on tcgen05, shorter ones and decode steps on ``mma.sync`` tiles), everything else on the CUDA cores in float32."""
+    (token, head) rows and more on tcgen05, shorter ones and decode steps on ``mma.sync`` tiles), everything else on the CUDA cores in float32.
+    ``leave_parts``: where the keys are split, ``out`` stays as it is and the shares are left in ``scratch`` for
+    :func:`head_linear_parts`; returns their number, or 0 where ``out`` is written."""
     assert sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == heads)
     if (USE_LATENT_TC and q.dtype == torch.bfloat16 and step.max_new * heads >= LATENT_TC_MIN_ROWS and scale > 0
             and latent_tc_supports(heads, cached_dim, value_dim, page_size) and _rows(q, "q") % 8 == 0 and q.data_ptr() % 16 == 0
@@ -1201,7 +1204,7 @@ def latent_attention(q: torch.Tensor, k_pool: torch.Tensor, block_table: torch.T
                                             step.context_before.data_ptr(), out.data_ptr(), _rows(out, "out"), step.n, step.r,
                                             step.max_new, heads, cached_dim, value_dim, float(scale), int(window or 0), _ptr(sink),
                                             _status().data_ptr(), _stream()), lib)
-        return
+        return 0
     if (USE_LATENT_MMA and q.dtype == torch.bfloat16 and latent_mma_supports(heads, cached_dim, value_dim)
             and _rows(q, "q") % 8 == 0 and q.data_ptr() % 16 == 0 and _rows(out, "out") % 2 == 0 and out.data_ptr() % 4 == 0):
         lib = library()
@@ -1217,18 +1220,21 @@ def latent_attention(q: torch.Tensor, k_pool: torch.Tensor, block_table: torch.T
             splits = getattr(step, "attention_splits", None) or latent_splits(
                 step.r, heads, getattr(step, "planning_context", step.max_context), int(window or 0))
             splits = max(1, min(splits, scratch.numel() // max(1, step.n * heads * (value_dim + 2))))
+        leave_parts = leave_parts and splits > 1
         _check(lib.hfee_latent_attention_mma(q.data_ptr(), _rows(q, "q"), k_pool.data_ptr(), block_table.data_ptr(),
                                              block_table.shape[1], page_size, step.cu_tokens.data_ptr(), step.slots.data_ptr(),
-                                             step.context_before.data_ptr(), out.data_ptr(), _rows(out, "out"), step.r,
-                                             step.max_new, heads, cached_dim, value_dim, float(scale), int(window or 0),
+                                             step.context_before.data_ptr(), None if leave_parts else out.data_ptr(), _rows(out, "out"),
+                                             step.r, step.max_new, heads, cached_dim, value_dim, float(scale), int(window or 0),
                                              _ptr(sink), splits, _ptr(scratch) if splits > 1 else None, step.n, _stream()), lib)
+        if leave_parts:
+            return splits
         if splits > 1:
             count_launches(1)
-        return
+        return 0
     if sink is None:
         attention_simt_general(q, k_pool, None, block_table, page_size, step.positions, step.slot_of_token, out, heads, 1,
                                cached_dim, value_dim, scale, window)
-        return
+        return 0
     lib = library()
     _i32(step.positions, "positions"); _i32(step.slot_of_token, "slot_of_token"); _i32(block_table, "block_table")
     n = q.shape[0]
@@ -1239,6 +1245,7 @@ def latent_attention(q: torch.Tensor, k_pool: torch.Tensor, block_table: torch.T
                                         out.data_ptr(), _rows(out, "out"), n, heads, 1, cached_dim, value_dim, 1, float(scale),
                                         int(window or 0), 0, WEIGHTS_SOFTMAX, None, None, None, 0, GATE_NONE, None, None, 1.0,
                                         sink.data_ptr(), _dt(q), _stream()), lib)
+    return 0
 
 
 def latent_splits(requests: int, heads: int, max_context: int, window: int) -> int:
@@ -1370,6 +1377,27 @@ def head_linear(x: torch.Tensor, in_off: int, in_stride: int, w: torch.Tensor, o
     _check(lib.hfee_head_linear(x.data_ptr(), _rows(x, "x"), in_off, in_stride, w.data_ptr(), out.data_ptr(), _rows(out, "out"),
                                 out_off, out_stride, n, heads, n_in, n_out, _ptr(gate),
                                 _rows(gate, "gate") if gate is not None else 0, _dt(x), _stream()), lib)
+
+
+HEAD_LINEAR_PARTS_TOKENS = 2      # each token's shares are a trip to memory of their own
+
+
+def head_linear_takes_parts(tokens: int, w: torch.Tensor) -> bool:
+    return w.dtype == torch.bfloat16 and tokens <= HEAD_LINEAR_PARTS_TOKENS and w.shape[2] % 8 == 0 and w.shape[2] <= 512 and w.data_ptr() % 16 == 0
+
+
+def head_linear_parts(partial: torch.Tensor, splits: int, sink: Optional[torch.Tensor], w: torch.Tensor, out: torch.Tensor, out_off: int,
+                      out_stride: int, gate: Optional[torch.Tensor] = None) -> None:
+    """:func:`head_linear` of the latent outputs whose ``splits`` shares :func:`latent_attention` left in ``partial``."""
+    lib = library()
+    heads, n_out, n_in = w.shape
+    n = out.shape[0]
+    assert w.is_contiguous() and w.dtype == out.dtype == torch.bfloat16 and partial.dtype == torch.float32
+    assert partial.numel() >= splits * n * heads * (n_in + 2) and out_off + (heads - 1) * out_stride + n_out <= out.shape[1]
+    assert gate is None or (gate.dtype == w.dtype and gate.shape == (n, heads))
+    _check(lib.hfee_head_linear_parts(partial.data_ptr(), splits, _ptr(sink), w.data_ptr(), out.data_ptr(), _rows(out, "out"), out_off,
+                                      out_stride, n, heads, n_in, n_out, _ptr(gate), _rows(gate, "gate") if gate is not None else 0,
+                                      _stream()), lib)
 
 
 def conv_act(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor, step, out: torch.Tensor, activation: str = "silu",
@@ -2323,7 +2351,7 @@ def argmax(logits: torch.Tensor, out: torch.Tensor, scratch: torch.Tensor, slots
 
 
 # the entry points the parts and the sampler launch through can be left out by class (see tag())
-for _name in ("rmsnorm_add_norm", "latent_attention", "linear_act", "attention_simt_general", "rope_norm_cache", "latent_norm_rope_cache", "head_linear", "conv_act", "delta_rule",
+for _name in ("rmsnorm_add_norm", "latent_attention", "linear_act", "attention_simt_general", "rope_norm_cache", "latent_norm_rope_cache", "head_linear", "head_linear_parts", "conv_act", "delta_rule",
               "head_norm_gate", "unary_act", "head_gate", "attention_simt_masked", "short_conv", "linear_attention", "rmsnorm_add", "norm_gate", "gated_act", "scale_", "cast_rows", "sigmoid_attention",
               "qk_norm_rope_cache", "embed", "rmsnorm", "rope_table", "rope_cache_write", "swiglu", "linear", "linear_normed", "linear_swiglu", "linear_rope_cache",
               "linear_swiglu_normed", "paged_attention", "paged_attention_rope", "sample", "argmax", "sample_chain",

@@ -125,12 +125,15 @@ class LatentAttention(Mixer):
         scratch = None
         if rt.dtype == torch.bfloat16:
             scratch = rt.scratch("lattn_partial", (max(2 * rt.max_requests, 160) * h * (rank + 2),), torch.float32)
-        ops.latent_attention(qf, cache.k, cache.block_table, cache.page_size, step, ol, h, self.cached_dim, rank,
-                             self.scale, int(self.window or 0), self.sink, scratch)
+        parts = ops.latent_attention(qf, cache.k, cache.block_table, cache.page_size, step, ol, h, self.cached_dim, rank,
+                                     self.scale, int(self.window or 0), self.sink, scratch, ops.head_linear_takes_parts(n, self.w_uv))
         att = rt.scratch("lattn_out", (rt.max_tokens, pad8(h * v)))[:n, :h * v]
         gate = proj[:, self.g_at:self.g_at + h] if self.g_at is not None else None
         ops.tag("expand")
-        ops.head_linear(ol, 0, rank, self.w_uv, att, 0, v, gate)
+        if parts:            # the product puts the shares of the split keys together itself
+            ops.head_linear_parts(scratch, parts, self.sink, self.w_uv, att, 0, v, gate)
+        else:
+            ops.head_linear(ol, 0, rank, self.w_uv, att, 0, v, gate)
         ops.tag("o")
         ops.linear(att, self.w_o, out, accumulate=accumulate)
 

@@ -1,0 +1,59 @@
+"""One matrix per head for a few tokens, from rows and from the shares of a latent attention with split keys."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rand(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
+
+
+# a row of one 16-byte piece up to two for every lane; rows of W that end inside a block of 16 and inside a warp's four; n_in that is
+# no power of two; one token more than the few-token kernel takes
+SHAPES = [(1, 32, 64, 256), (1, 32, 256, 64), (8, 3, 8, 5), (2, 5, 96, 72), (5, 4, 264, 33), (8, 2, 512, 16), (9, 4, 256, 64), (3, 1, 520, 24)]
+
+
+@pytest.mark.parametrize("n,heads,n_in,n_out", SHAPES)
+@pytest.mark.parametrize("gated", [False, True])
+def test_rows(n, heads, n_in, n_out, gated):
+    from hfee_b200.kernels import ops
+    step = -(-n_in // 8) * 8 + 8                              # heads with a gap between them
+    x = _rand((n, 16 + heads * step), 1).to(torch.bfloat16)
+    w = _rand((heads, n_out, n_in), 2, 0.1).to(torch.bfloat16)
+    gate = _rand((n, heads), 3).to(torch.bfloat16) if gated else None
+    out = torch.full((n + 1, 3 + heads * (n_out + 2)), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.head_linear(x, 16, step, w, out[:n], 3, n_out + 2, gate)
+    xs = torch.stack([x[:, 16 + h * step:16 + h * step + n_in] for h in range(heads)], 1).double()
+    want = torch.einsum("nhk,hok->nho", xs, w.double())
+    if gated:
+        want = want * torch.sigmoid(gate.double())[:, :, None]
+    cells = out[:n, 3:].reshape(n, heads, n_out + 2).double()
+    assert (cells[:, :, :n_out] - want).norm() <= 4e-3 * want.norm()            # rounded to bfloat16: 2^-9 an element
+    assert bool((cells[:, :, n_out:] == 7.0).all()) and bool((out[n] == 7.0).all()) and bool((out[:, :3] == 7.0).all())
+
+
+@pytest.mark.parametrize("n,heads,n_in,n_out", [(1, 32, 256, 64), (2, 5, 96, 40), (1, 3, 8, 5), (2, 2, 512, 33), (1, 4, 264, 16)])
+@pytest.mark.parametrize("splits", [1, 2, 7, 32])
+@pytest.mark.parametrize("sink", [False, True])
+def test_shares(n, heads, n_in, n_out, splits, sink):
+    from hfee_b200.kernels import ops
+    w = _rand((heads, n_out, n_in), 4, 0.1).to(torch.bfloat16)
+    assert ops.head_linear_takes_parts(n, w)
+    partial = torch.empty(splits, n, heads, n_in + 2, device=DEV)
+    partial[..., :n_in] = _rand((splits, n, heads, n_in), 5)
+    partial[..., n_in] = _rand((splits, n, heads), 6, 3.0)                       # maxima in log2 units
+    partial[..., n_in + 1] = _rand((splits, n, heads), 7).abs() + 0.1
+    if splits > 2:                                                               # shares without keys
+        partial[splits - 1, ..., :n_in], partial[splits - 1, ..., n_in], partial[splits - 1, ..., n_in + 1] = 0.0, -float("inf"), 0.0
+    sinks = _rand((heads,), 8) if sink else None
+    gate = _rand((n, heads), 9).to(torch.bfloat16)
+    out = torch.full((n, heads * n_out), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.head_linear_parts(partial, splits, sinks, w, out, 0, n_out, gate)
+    p = partial.double()
+    e = torch.exp2(p[..., n_in])
+    total = (e * p[..., n_in + 1]).sum(0) + (torch.exp(sinks.double())[None] if sink else 0)
+    x = (e[..., None] * p[..., :n_in]).sum(0) / total[..., None]
+    want = torch.einsum("nhk,hok->nho", x, w.double()) * torch.sigmoid(gate.double())[:, :, None]
+    assert (out.reshape(n, heads, n_out).double() - want).norm() <= 4e-3 * want.norm()
