@@ -105,32 +105,53 @@ latent_attention_kernel(LatentParams p) {
     m_s[tid] = -INFINITY;
     l_s[tid] = 0.f;
   }
-  const int pieces = dk >> 3;
+  // A thread's pieces of 16 bytes lie THREADS apart, counted row by row: the steps from one to the next are divided once.  (With two
+  // divisions and a look into the block table for every piece, a block's requests alone took as long as its products.)
+  const int pieces = dk >> 3, row_step = THREADS / pieces, piece_step = THREADS - row_step * pieces;
+  const int r_first = tid / pieces, c_first = tid - r_first * pieces;
   auto load_block = [&](int block_start, int buf) {
     bf16* dst = Ks + (long long)buf * LA_BN * ldk;
+    const bool one_page = p.page_mask + 1 >= LA_BN;            // then the block lies inside a page (both are powers of two)
+    const bf16* page = p.pool;
+    if (one_page && block_start <= p_last)
+      page += (long long)table[block_start >> p.page_shift] * page_stride + (long long)(block_start & p.page_mask) * dk;
+    int r = r_first, c = c_first;
+#pragma unroll 4
     for (int e = tid; e < LA_BN * pieces; e += THREADS) {
-      const int r = e / pieces, c = (e - r * pieces) * 8;
       const int kp = block_start + r;
       const bool valid = kp >= lo && kp <= p_last;
       const bf16* src = p.pool;
-      if (valid) src += (long long)table[kp >> p.page_shift] * page_stride + (long long)(kp & p.page_mask) * dk + c;
-      la_cp_async16(dst + r * ldk + c, src, valid);
+      if (valid)
+        src = one_page ? page + r * dk + c * 8
+                       : src + (long long)table[kp >> p.page_shift] * page_stride + (long long)(kp & p.page_mask) * dk + c * 8;
+      la_cp_async16(dst + r * ldk + c * 8, src, valid);
+      r += row_step;
+      c += piece_step;
+      if (c >= pieces) { c -= pieces; ++r; }
     }
   };
   const int first_block = (lo / LA_BN) * LA_BN;
-  // a block of positions that earlier steps wrote is requested before the wait for the kernel in front (and the batch layout and
-  // the block table come from the host)
+  // Blocks of positions that earlier steps wrote are requested before the wait for the kernel in front (and the batch layout and
+  // the block table come from the host): as many as there are buffers, of which a share of split keys often has no more.
   const bool early = first_block + LA_BN <= before && lo <= p_last;
+  const bool early_next = early && first_block + 2 * LA_BN <= before && first_block + LA_BN <= p_last;
   if (early) load_block(first_block, 0);
+  if (early_next) load_block(first_block + LA_BN, 1);
   pdl_wait();
   pdl_launch_dependents();
   // queries of the tile
-  for (int e = tid; e < ROWS * pieces; e += THREADS) {
-    const int r = e / pieces, c = (e - r * pieces) * 8;
-    const int t = r / p.rows_per_token, h = head0 + r % p.rows_per_token;
-    const bool valid = t < tokens && h < p.heads;
-    const bf16* src = p.q + (long long)(begin + t0 + (valid ? t : 0)) * p.ld_q + (long long)(valid ? h : 0) * dk + c;
-    la_cp_async16(Qs + r * ldk + c, src, valid);
+  {
+    int r = r_first, c = c_first;
+#pragma unroll 4
+    for (int e = tid; e < ROWS * pieces; e += THREADS) {
+      const int t = p.rows_per_token == ROWS ? 0 : r / p.rows_per_token, h = head0 + r - t * p.rows_per_token;
+      const bool valid = t < tokens && h < p.heads;
+      const bf16* src = p.q + (long long)(begin + t0 + (valid ? t : 0)) * p.ld_q + (long long)(valid ? h : 0) * dk + c * 8;
+      la_cp_async16(Qs + r * ldk + c * 8, src, valid);
+      r += row_step;
+      c += piece_step;
+      if (c >= pieces) { c -= pieces; ++r; }
+    }
   }
   if (!early) load_block(first_block, 0);
   la_commit();
@@ -151,7 +172,7 @@ latent_attention_kernel(LatentParams p) {
   for (int block_start = first_block; block_start <= p_last; block_start += LA_BN, buf ^= 1) {
     la_wait_all();
     __syncthreads();
-    if (block_start + LA_BN <= p_last) load_block(block_start + LA_BN, buf ^ 1);
+    if (block_start + LA_BN <= p_last && !(early_next && block_start == first_block)) load_block(block_start + LA_BN, buf ^ 1);
     la_commit();
     const bf16* Kb = Ks + (long long)buf * LA_BN * ldk;
 
