@@ -3,6 +3,10 @@
 //   hfee_moe_few_gate_up   hidden[pair] = act(W_gate[e] x[token], W_up[e] x[token]) for every pair's expert e
 //   hfee_moe_few_down      pair_out[pair] = W_down[e] hidden[pair] (float32)
 //
+// Both also take the products of a shared expert that every token passes: two launches in place of four, and its weights, which
+// depend on no choice, are the first that a block asks for, before the wait for the choices.  Three tokens, two of 16 experts of
+// 2,048 x 2,048 and a shared one of 4,096: 19.0 + 10.5 + 7.9 + 5.1 us in place, together 22.9 + 16.1.
+//
 // Reference math of one expert: hostfog/hfee internal/ggml/ops.go:125-134 (the product), 160-165 (gate times up).
 //
 // Bound by the bytes of the chosen experts' weights, each read once.  The tiles of 128 rows that the large grouped product takes are
@@ -28,19 +32,80 @@ __device__ __forceinline__ uint4 load_weights(const bf16* p) {
   return v;
 }
 
-// x: rows of the pairs' inputs, row pair / share (share = top for tokens, 1 for rows by pair).  GATED: rows of w in runs of
-// [4 gate | 4 up], out bfloat16 [pairs, rows / 2]; else out float32 [pairs, rows], and the kernel in front is the gated one with the
-// same choices: it waited for whatever made them, so they (and the first weights) are read before the wait for it.
+// One matrix of a kind: the inputs' rows, the weights, the results' rows.
+struct FewSide {
+  const bf16* x; long long ld_x;
+  const bf16* w; int rows, K;
+  void* out; long long ld_out;
+  float limit;
+};
+
+// routed.x: rows of the pairs' inputs, row pair / share (share = top for tokens, 1 for rows by pair); its w is one matrix after another.
+// shared: the expert that every one of `tokens` tokens passes, or w null: its units come first, whose weights do not wait for the choices.
+// GATED: rows of w in runs of [4 gate | 4 up], out bfloat16 [pairs, rows / 2]; else out float32 [pairs, rows], and the kernel in front is
+// the gated one with the same choices: it waited for whatever made them, so they (and the first weights) are read before the wait for it.
 template <bool GATED>
 __global__ void __launch_bounds__(FEW_WARPS * 32, 4)
-moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16* __restrict__ w, int rows, int K,
-               int experts, const int* __restrict__ choice, int pairs, void* __restrict__ out, long long ld_out, float limit, float alpha, float shift) {
+moe_few_kernel(FewSide routed, int share, int experts, const int* __restrict__ choice, int pairs, FewSide shared, int tokens, float alpha,
+               float shift) {
   __shared__ float part_s[2][FEW_WARPS][FEW_ROWS][8];
   __shared__ int expert_s[FEW_PAIRS];
   __shared__ unsigned members_s[FEW_PAIRS];
   __shared__ int lists_s;
   constexpr int RUN = 32 * FEW_AHEAD;             // k of a warp's batch
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int shared_tiles = shared.w != nullptr ? (shared.rows + FEW_ROWS - 1) / FEW_ROWS : 0;
+  const int shared_units = shared_tiles * ((tokens + 7) / 8);
+  const int tiles = (routed.rows + FEW_ROWS - 1) / FEW_ROWS;
+  // a unit's matrix, rows and pairs (bits of the choices; of the tokens for the shared expert)
+  struct Unit { bool common; int row0; const bf16* w; unsigned members; };
+  auto find = [&](int unit) {
+    Unit u;
+    u.common = unit < shared_units;
+    if (u.common) {
+      const int list = unit / shared_tiles, left = min(8, tokens - 8 * list);
+      u.row0 = (unit - list * shared_tiles) * FEW_ROWS;
+      u.w = shared.w;
+      u.members = ((1u << left) - 1u) << (8 * list);
+    } else {
+      const int list = (unit - shared_units) / tiles;
+      u.row0 = (unit - shared_units - list * tiles) * FEW_ROWS;
+      u.w = routed.w + (long long)expert_s[list] * routed.rows * routed.K;
+      u.members = members_s[list];
+    }
+    return u;
+  };
+
+  uint4 a0[2][FEW_AHEAD], a1[2][FEW_AHEAD], b[2][FEW_AHEAD];
+  auto load_a = [&](const Unit& u, int batch, uint4 (&p)[FEW_AHEAD], uint4 (&q)[FEW_AHEAD]) {
+    const int rows = u.common ? shared.rows : routed.rows, K = u.common ? shared.K : routed.K;
+    const int row = u.row0 + g, k = (batch * FEW_WARPS + warp) * RUN + 8 * t;
+    const bf16* w0 = u.w + (long long)min(row, rows - 1) * K + k;
+    const bf16* w1 = u.w + (long long)min(row + 8, rows - 1) * K + k;
+#pragma unroll
+    for (int i = 0; i < FEW_AHEAD; ++i) {
+      const bool in = k + 32 * i < K;
+      p[i] = in ? load_weights(w0 + 32 * i) : make_uint4(0, 0, 0, 0);
+      q[i] = in ? load_weights(w1 + 32 * i) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  auto load_b = [&](const Unit& u, int batch, uint4 (&r)[FEW_AHEAD]) {
+    unsigned from = u.members;
+    for (int i = 0; i < g; ++i) from &= from - 1;
+    const int K = u.common ? shared.K : routed.K, k = (batch * FEW_WARPS + warp) * RUN + 8 * t;      // column g of B has a pair if a member is left
+    const int row = from != 0 ? (u.common ? __ffs(from) - 1 : (__ffs(from) - 1) / share) : 0;
+    const bf16* xr = (u.common ? shared.x : routed.x) + row * (u.common ? shared.ld_x : routed.ld_x) + k;
+#pragma unroll
+    for (int i = 0; i < FEW_AHEAD; ++i)
+      r[i] = from != 0 && k + 32 * i < K ? *reinterpret_cast<const uint4*>(xr + 32 * i) : make_uint4(0, 0, 0, 0);
+  };
+
+  int unit = blockIdx.x, batch = 0, half = 0;
+  Unit now_at = {};
+  if (unit < shared_units) {
+    now_at = find(unit);
+    load_a(now_at, 0, a0[0], a1[0]);
+  }
   if (GATED) {
     pdl_wait();
     pdl_launch_dependents();
@@ -69,49 +134,30 @@ moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16
     if (lane == 0) lists_s = lists;
   }
   __syncthreads();
-  const int tiles = (rows + FEW_ROWS - 1) / FEW_ROWS, units = lists_s * tiles;
-  const int batches = (K + RUN * FEW_WARPS - 1) / (RUN * FEW_WARPS);
+  const int units = shared_units + lists_s * tiles;
+  auto batches_of = [&](const Unit& u) { return ((u.common ? shared.K : routed.K) + RUN * FEW_WARPS - 1) / (RUN * FEW_WARPS); };
 
-  uint4 a0[2][FEW_AHEAD], a1[2][FEW_AHEAD], b[2][FEW_AHEAD];
-  auto load_a = [&](int unit, int batch, uint4 (&p)[FEW_AHEAD], uint4 (&q)[FEW_AHEAD]) {
-    const int row = (unit % tiles) * FEW_ROWS + g, k = (batch * FEW_WARPS + warp) * RUN + 8 * t;
-    const bf16* we = w + (long long)expert_s[unit / tiles] * rows * K + k;
-    const bf16* w0 = we + (long long)min(row, rows - 1) * K;
-    const bf16* w1 = we + (long long)min(row + 8, rows - 1) * K;
-#pragma unroll
-    for (int i = 0; i < FEW_AHEAD; ++i) {
-      const bool in = k + 32 * i < K;
-      p[i] = in ? load_weights(w0 + 32 * i) : make_uint4(0, 0, 0, 0);
-      q[i] = in ? load_weights(w1 + 32 * i) : make_uint4(0, 0, 0, 0);
-    }
-  };
-  auto load_b = [&](int unit, int batch, uint4 (&r)[FEW_AHEAD]) {
-    unsigned from = members_s[unit / tiles];
-    for (int i = 0; i < g; ++i) from &= from - 1;
-    const int k = (batch * FEW_WARPS + warp) * RUN + 8 * t;                // column g of B has a pair if a member is left
-    const bf16* xr = x + (long long)(from != 0 ? (__ffs(from) - 1) / share : 0) * ld_x + k;
-#pragma unroll
-    for (int i = 0; i < FEW_AHEAD; ++i)
-      r[i] = from != 0 && k + 32 * i < K ? *reinterpret_cast<const uint4*>(xr + 32 * i) : make_uint4(0, 0, 0, 0);
-  };
-
-  int unit = blockIdx.x, batch = 0, half = 0;
-  if (unit < units) load_a(unit, 0, a0[0], a1[0]);
+  if (unit >= shared_units && unit < units) {
+    now_at = find(unit);
+    load_a(now_at, 0, a0[0], a1[0]);
+  }
   if (!GATED) {
     pdl_wait();
     pdl_launch_dependents();
   }
-  if (unit < units) load_b(unit, 0, b[0]);
+  if (unit < units) load_b(now_at, 0, b[0]);
   float c[4] = {0.f, 0.f, 0.f, 0.f};
   // one batch: asks for the one after it, multiplies, and after a unit's last puts the warps' sums together; false at the end
   auto turn = [&](auto now) {
     constexpr int NOW = decltype(now)::value;
     if (unit >= units) return false;
-    const bool last = batch + 1 == batches;
+    const bool last = batch + 1 == batches_of(now_at);
     const int next_unit = last ? unit + gridDim.x : unit, next_batch = last ? 0 : batch + 1;
+    Unit next_at = now_at;
     if (next_unit < units) {
-      load_a(next_unit, next_batch, a0[NOW ^ 1], a1[NOW ^ 1]);
-      load_b(next_unit, next_batch, b[NOW ^ 1]);
+      if (last) next_at = find(next_unit);
+      load_a(next_at, next_batch, a0[NOW ^ 1], a1[NOW ^ 1]);
+      load_b(next_at, next_batch, b[NOW ^ 1]);
     }
 #pragma unroll
     for (int i = 0; i < FEW_AHEAD; ++i) {
@@ -135,8 +181,11 @@ moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16
         for (int i = 1; i < FEW_WARPS; ++i) v += part[i][r][col];
         return v;
       };
-      const unsigned eight = members_s[unit / tiles];
-      const int row0 = (unit % tiles) * FEW_ROWS, count = __popc(eight);
+      const unsigned eight = now_at.members;
+      const int row0 = now_at.row0, count = __popc(eight);
+      const int rows = now_at.common ? shared.rows : routed.rows;
+      void* out = now_at.common ? shared.out : routed.out;
+      const long long ld_out = now_at.common ? shared.ld_out : routed.ld_out;
       constexpr int OUTS = GATED ? FEW_ROWS / 2 : FEW_ROWS;
       const int r = threadIdx.x % OUTS;
       for (int col = threadIdx.x / OUTS; col < count; col += FEW_WARPS * 32 / OUTS) {
@@ -146,6 +195,7 @@ moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16
         if constexpr (GATED) {
           const int j = (r >> 2) * 8 + (r & 3);   // gate row j, up row j + 4
           if (row0 + j + 4 < rows) {
+            const float limit = now_at.common ? shared.limit : routed.limit;
             const float gate = fminf(sum(j, col), limit), up = fminf(fmaxf(sum(j + 4, col), -limit), limit);
             reinterpret_cast<bf16*>(out)[pair * ld_out + row0 / 2 + r] =
                 __float2bfloat16_rn(__fdividef(gate, 1.f + __expf(-alpha * gate)) * (up + shift));
@@ -157,19 +207,22 @@ moe_few_kernel(const bf16* __restrict__ x, long long ld_x, int share, const bf16
     }
     unit = next_unit;
     batch = next_batch;
+    now_at = next_at;
     return true;
   };
   while (turn(std::integral_constant<int, 0>{}) && turn(std::integral_constant<int, 1>{})) {}
 }
 
-unsigned few_blocks(int rows, int pairs) {
-  const long long units = (long long)((rows + FEW_ROWS - 1) / FEW_ROWS) * pairs, room = 4LL * (hfee_sm_count() > 0 ? hfee_sm_count() : 1);
+unsigned few_blocks(const FewSide& routed, int pairs, const FewSide& shared, int tokens) {
+  long long units = (long long)((routed.rows + FEW_ROWS - 1) / FEW_ROWS) * pairs;
+  if (shared.w != nullptr) units += (long long)((shared.rows + FEW_ROWS - 1) / FEW_ROWS) * ((tokens + 7) / 8);
+  const long long room = 4LL * (hfee_sm_count() > 0 ? hfee_sm_count() : 1);
   return (unsigned)(units < room ? units : room);
 }
 
-int few_check(const char* name, const void* x, long long ld_x, const void* w, int rows, int K, int experts, int pairs) {
+int few_check(const char* name, const FewSide& s, int experts, int pairs) {
   HFEE_REQUIRE(pairs > 0 && pairs <= FEW_PAIRS && experts > 0, "%s: %d pairs are outside 1..%d", name, pairs, FEW_PAIRS);
-  HFEE_REQUIRE(rows > 0 && K > 0 && K % 8 == 0 && ld_x % 8 == 0 && ld_x >= K && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0,
+  HFEE_REQUIRE(s.rows > 0 && s.K > 0 && s.K % 8 == 0 && s.ld_x % 8 == 0 && s.ld_x >= s.K && (uintptr_t)s.x % 16 == 0 && (uintptr_t)s.w % 16 == 0,
                "%s: rows must be whole 16-byte pieces", name);
   return HFEE_OK;
 }
@@ -178,23 +231,38 @@ int few_check(const char* name, const void* x, long long ld_x, const void* w, in
 
 // x: [pairs / top, width] bfloat16; w: [experts, 2 * inner, width] with each expert's rows in runs of [4 gate | 4 up];
 // choice: [pairs], every one an expert; hidden: [pairs, inner].  The clamped gated activation of hfee_moe_gate_up.
+// shared_w (or null): the same of one more expert that all pairs / top tokens pass, [2 * shared_inner, width], into shared_hidden.
 HFEE_API int hfee_moe_few_gate_up(const void* x, long long ld_x, int top, const void* w, int inner, int width, int experts, const int* choice,
-                                  int pairs, void* hidden, long long ld_hidden, float limit, float alpha, float shift, cudaStream_t stream) {
+                                  int pairs, void* hidden, long long ld_hidden, float limit, float alpha, float shift, const void* shared_w,
+                                  int shared_inner, void* shared_hidden, long long ld_shared, float shared_limit, cudaStream_t stream) {
   if (pairs == 0) return HFEE_OK;
-  const int rc = few_check("moe_few_gate_up", x, ld_x, w, 2 * inner, width, experts, pairs);
+  const FewSide routed{(const bf16*)x, ld_x, (const bf16*)w, 2 * inner, width, hidden, ld_hidden, limit};
+  const FewSide shared{(const bf16*)x, ld_x, (const bf16*)shared_w, 2 * shared_inner, width, shared_hidden, ld_shared, shared_limit};
+  int rc = few_check("moe_few_gate_up", routed, experts, pairs);
+  if (rc == HFEE_OK && shared_w != nullptr) rc = few_check("moe_few_gate_up", shared, experts, pairs);
   if (rc != HFEE_OK) return rc;
-  HFEE_REQUIRE(top > 0 && inner % 4 == 0 && ld_hidden >= inner && limit > 0.f, "moe_few_gate_up: bad sizes");
-  hfee_launch(moe_few_kernel<true>, dim3(few_blocks(2 * inner, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)x, ld_x, top, (const bf16*)w, 2 * inner, width, experts, choice, pairs, hidden, ld_hidden, limit, alpha, shift);
+  HFEE_REQUIRE(top > 0 && pairs % top == 0 && inner % 4 == 0 && ld_hidden >= inner && limit > 0.f, "moe_few_gate_up: bad sizes");
+  HFEE_REQUIRE(shared_w == nullptr || (shared_inner % 4 == 0 && ld_shared >= shared_inner && shared_limit > 0.f && shared_hidden != nullptr),
+               "moe_few_gate_up: bad sizes of the shared expert");
+  hfee_launch(moe_few_kernel<true>, dim3(few_blocks(routed, pairs, shared, pairs / top)), dim3(FEW_WARPS * 32), 0, stream, routed, top, experts,
+              choice, pairs, shared, pairs / top, alpha, shift);
   return hfee_check_launch("moe_few_gate_up");
 }
 
 // hidden: [pairs, inner] bfloat16; w: [experts, width, inner]; pair_out: [pairs, width] float32.  To be launched right behind
-// hfee_moe_few_gate_up with the same choices, which it reads before it waits for that kernel.
+// hfee_moe_few_gate_up with the same choices, which it reads before it waits for that kernel.  shared_w (or null): [width, shared_inner],
+// of shared_hidden [tokens, shared_inner] into shared_out [tokens, width] float32.
 HFEE_API int hfee_moe_few_down(const void* hidden, long long ld_hidden, const void* w, int inner, int width, int experts, const int* choice,
-                               int pairs, float* pair_out, cudaStream_t stream) {
+                               int pairs, float* pair_out, const void* shared_hidden, long long ld_shared, const void* shared_w,
+                               int shared_inner, int tokens, float* shared_out, cudaStream_t stream) {
   if (pairs == 0) return HFEE_OK;
-  const int rc = few_check("moe_few_down", hidden, ld_hidden, w, width, inner, experts, pairs);
+  const FewSide routed{(const bf16*)hidden, ld_hidden, (const bf16*)w, width, inner, pair_out, (long long)width, 0.f};
+  const FewSide shared{(const bf16*)shared_hidden, ld_shared, (const bf16*)shared_w, width, shared_inner, shared_out, (long long)width, 0.f};
+  int rc = few_check("moe_few_down", routed, experts, pairs);
+  if (rc == HFEE_OK && shared_w != nullptr) rc = few_check("moe_few_down", shared, experts, pairs);
   if (rc != HFEE_OK) return rc;
-  hfee_launch(moe_few_kernel<false>, dim3(few_blocks(width, pairs)), dim3(FEW_WARPS * 32), 0, stream, (const bf16*)hidden, ld_hidden, 1, (const bf16*)w, width, inner, experts, choice, pairs, pair_out, (long long)width, 0.f, 0.f, 0.f);
+  HFEE_REQUIRE(shared_w == nullptr || (tokens > 0 && tokens <= FEW_PAIRS && shared_out != nullptr), "moe_few_down: bad sizes of the shared expert");
+  hfee_launch(moe_few_kernel<false>, dim3(few_blocks(routed, pairs, shared, tokens)), dim3(FEW_WARPS * 32), 0, stream, routed, 1, experts, choice,
+              pairs, shared, tokens, 0.f, 0.f);
   return hfee_check_launch("moe_few_down");
 }

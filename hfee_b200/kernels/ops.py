@@ -96,8 +96,8 @@ _SIGNATURES = {
     "hfee_moe_gate_up": [_P, _L, _I, _P, _P, _L, _I, _I, _P, _P, _P, _P, _P, _L, _F, _F, _F, _I, _I, _P],
     "hfee_moe_down": [_P, _L, _I, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _P],
     "hfee_moe_combine": [_P, _P, _P, _I, _I, _P, _I, _I, _P],
-    "hfee_moe_few_gate_up": [_P, _L, _I, _P, _I, _I, _I, _P, _I, _P, _L, _F, _F, _F, _P],
-    "hfee_moe_few_down": [_P, _L, _P, _I, _I, _I, _P, _I, _P, _P],
+    "hfee_moe_few_gate_up": [_P, _L, _I, _P, _I, _I, _I, _P, _I, _P, _L, _F, _F, _F, _P, _I, _P, _L, _F, _P],
+    "hfee_moe_few_down": [_P, _L, _P, _I, _I, _I, _P, _I, _P, _P, _L, _P, _I, _I, _P, _P],
     "hfee_moe_plan_tiles": [_P, _I, _I, _I, _P, _P, _P, _I, _P],
     "hfee_moe_gather_rows": [_P, _L, _I, _P, _P, _I, _P, _L, _I, _I, _P],
     "hfee_moe_route_chosen": [_P, _L, _P, _I, _I, _I, _F, _P, _P, _P],
@@ -1913,8 +1913,10 @@ MOE_FEW_PAIRS = 32
 
 
 def moe_experts_few(x: torch.Tensor, top: int, choice: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, limit: float,
-                    hidden: torch.Tensor, pair_out: torch.Tensor, alpha: float = CLAMPED_SWISH_ALPHA, shift: float = 1.0) -> None:
+                    hidden: torch.Tensor, pair_out: torch.Tensor, alpha: float = CLAMPED_SWISH_ALPHA, shift: float = 1.0, shared=None) -> None:
     """:func:`moe_experts` for at most ``MOE_FEW_PAIRS`` pairs in bfloat16, without a plan: pair_out [pairs, width] float32 by pair.
+    ``shared`` = (w_gate_up [2 * s, width] in runs of [4 gate | 4 up], w_down [width, s], limit, hidden [n, s] bfloat16 scratch, out
+    [n, width] float32): one more expert that every token passes, in the same launches.
     ``w_gate_up`` [experts, 2 * inner, width] with each expert's rows in runs of [4 gate | 4 up] (:func:`interleave_gate_up`),
     ``w_down`` [experts, width, inner], ``hidden`` [pairs, inner] bfloat16 scratch; sizes are multiples of 8."""
     lib = library()
@@ -1925,10 +1927,19 @@ def moe_experts_few(x: torch.Tensor, top: int, choice: torch.Tensor, w_gate_up: 
     assert choice.numel() == pairs and tuple(hidden.shape) == (pairs, inner) and tuple(pair_out.shape) == (pairs, width)
     assert x.dtype == w_gate_up.dtype == w_down.dtype == hidden.dtype == torch.bfloat16 and pair_out.dtype == torch.float32
     assert w_gate_up.is_contiguous() and w_down.is_contiguous() and pair_out.is_contiguous() and tuple(w_down.shape) == (experts, width, inner)
+    w_in = w_out = s_hidden = s_out = None
+    s, s_limit, ld_s = 0, 1.0, 0
+    if shared is not None:
+        w_in, w_out, s_limit, s_hidden, s_out = shared
+        s, ld_s = w_out.shape[1], _rows(s_hidden, "shared hidden")
+        assert tuple(w_in.shape) == (2 * s, width) and tuple(w_out.shape) == (width, s) and tuple(s_hidden.shape) == (n, s)
+        assert tuple(s_out.shape) == (n, width) and s_out.is_contiguous() and s_out.dtype == torch.float32
+        assert w_in.dtype == w_out.dtype == s_hidden.dtype == torch.bfloat16 and w_in.is_contiguous() and w_out.is_contiguous()
     _check(lib.hfee_moe_few_gate_up(x.data_ptr(), _rows(x, "x"), top, w_gate_up.data_ptr(), inner, width, experts, choice.data_ptr(), pairs,
-                                    hidden.data_ptr(), _rows(hidden, "hidden"), float(limit), float(alpha), float(shift), _stream()), lib)
+                                    hidden.data_ptr(), _rows(hidden, "hidden"), float(limit), float(alpha), float(shift), _ptr(w_in), s,
+                                    _ptr(s_hidden), ld_s, float(s_limit), _stream()), lib)
     _check(lib.hfee_moe_few_down(hidden.data_ptr(), _rows(hidden, "hidden"), w_down.data_ptr(), inner, width, experts, choice.data_ptr(), pairs,
-                                 pair_out.data_ptr(), _stream()), lib)
+                                 pair_out.data_ptr(), _ptr(s_hidden), ld_s, _ptr(w_out), s, n, _ptr(s_out), _stream()), lib)
 
 
 def moe_experts_grouped(x: torch.Tensor, top: int, choice: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, limit: float,

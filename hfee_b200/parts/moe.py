@@ -131,13 +131,22 @@ class RoutedExperts(Part):
         else:
             ops.moe_route(logits, top, self.router_scale, choice, weight)
         gate_col = logits[:, self.experts:self.experts + 1] if self.shared_gate else None
-        place = None
+        place = extra = None
+        few_shared = False
         if self.fused_act and n * top <= ops.MOE_FEW_PAIRS and xn.data_ptr() % 16 == 0 and xn.stride(0) % 8 == 0:
             rows = self.tiles * ops.GROUPED_TILE_ROWS
             hidden = rt.scratch("moe_hidden_rows", (rows, self.inner))[:n * top]
             pair_out = rt.scratch("moe_rows_out", (rows, self.width), torch.float32)[:n * top]
+            shared = None
+            if self.shared_inner is not None and self.shared_granule == ops.SWIGLU_GRANULE and self.shared_inner % 8 == 0:
+                # the shared expert in the same launches; it joins the routed ones in the weighted sum
+                s = self.shared_inner
+                few_shared = True
+                extra = rt.scratch("moe_shared_out", (rt.max_tokens, self.width), torch.float32)[:n]
+                h = rt.scratch("ffn_hidden", (rt.max_tokens, pad8(s)))[:n, :s]
+                shared = (self.w_shared_in, self.w_shared_down, self.shared_limit, h, extra)
             ops.tag("experts")
-            ops.moe_experts_few(xn, top, choice, self.w_gate_up, self.w_down, self.limit, hidden, pair_out, self.alpha, self.shift)
+            ops.moe_experts_few(xn, top, choice, self.w_gate_up, self.w_down, self.limit, hidden, pair_out, self.alpha, self.shift, shared)
         elif self.grouped:
             rows = self.tiles * ops.GROUPED_TILE_ROWS
             place = rt.scratch("moe_place", (rt.max_tokens * top,), i32)
@@ -161,8 +170,7 @@ class RoutedExperts(Part):
             ops.tag("experts")
             ops.moe_experts(xn, top, self.w_gate, self.w_up, self.w_down, self.limit, offsets, order, tile_expert, tile_row,
                             hidden, pair_out, self.alpha, self.shift)
-        extra = None
-        if self.shared_inner is not None:
+        if self.shared_inner is not None and not few_shared:
             s = self.shared_inner
             gu = rt.scratch("ffn_gate_up", (rt.max_tokens, pad8(2 * s)))[:n, :2 * s]
             h = rt.scratch("ffn_hidden", (rt.max_tokens, pad8(s)))[:n, :s]

@@ -1,0 +1,49 @@
+"""The shared expert in the launches of the routed experts of few (token, choice) pairs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rand(shape, seed, scale=1.0, dtype=torch.bfloat16):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(dtype).to(DEV)
+
+
+def _act(gate, up, limit, alpha, shift):
+    a, b = gate.clamp(max=limit), up.clamp(-limit, limit)
+    return a * torch.sigmoid(alpha * a) * (b + shift)
+
+
+# one token up to four lists of eight; a shared expert smaller and larger than the routed ones (fewer and more batches of k), rows that
+# end inside a tile of 16, and sizes at which the shared expert's units are more than the chip holds at once
+@pytest.mark.parametrize("n,top,experts,width,inner,shared", [(1, 1, 1, 8, 8, 8), (1, 2, 16, 2048, 2048, 4096), (3, 2, 16, 72, 24, 264),
+                                                              (32, 1, 2, 40, 264, 8), (9, 3, 4, 1032, 96, 24), (16, 2, 5, 520, 56, 9008)])
+@pytest.mark.parametrize("limit,shared_limit,alpha,shift", [(7.0, 2.0, 1.702, 1.0), (float("inf"), float("inf"), 1.0, 0.0)])
+def test_shared_expert(n, top, experts, width, inner, shared, limit, shared_limit, alpha, shift):
+    from hfee_b200.kernels import ops
+    x = _rand((n, width + 8), 1)[:, :width]
+    gate, up, down = _rand((experts, inner, width), 2, 0.1), _rand((experts, inner, width), 3, 0.1), _rand((experts, width, inner), 4, 0.1)
+    s_gate, s_up, s_down = _rand((shared, width), 5, 0.1), _rand((shared, width), 6, 0.1), _rand((width, shared), 7, 0.1)
+    g = torch.Generator().manual_seed(n + experts)
+    choice = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(n)]).to(torch.int32).to(DEV)
+    hidden = torch.full((n * top, inner), float("nan"), dtype=torch.bfloat16, device=DEV)
+    out = torch.full((n * top + 1, width), 7.0, dtype=torch.float32, device=DEV)
+    s_hidden = torch.full((n + 1, shared + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    s_out = torch.full((n + 1, width), 7.0, dtype=torch.float32, device=DEV)
+    ops.moe_experts_few(x, top, choice, ops.interleave_gate_up(gate, up), down, limit, hidden, out[:-1], alpha, shift,
+                        (ops.interleave_gate_up(s_gate, s_up), s_down, shared_limit, s_hidden[:n, :shared], s_out[:n]))
+    for t in range(n):
+        for k in range(top):
+            e = int(choice[t, k])
+            want = _act(gate[e].double() @ x[t].double(), up[e].double() @ x[t].double(), limit, alpha, shift)
+            got = hidden[t * top + k].double()
+            assert (got - want).norm() <= 4e-3 * want.norm()                              # rounded to bfloat16: 2^-9 an element
+            y = down[e].double() @ got
+            assert (out[t * top + k].double() - y).norm() <= 1e-5 * y.norm() + 1e-6       # float32 sums
+    want = _act(x.double() @ s_gate.double().t(), x.double() @ s_up.double().t(), shared_limit, alpha, shift)
+    got = s_hidden[:n, :shared].double()
+    assert (got - want).norm(dim=1).le(4e-3 * want.norm(dim=1)).all()
+    y = got @ s_down.double().t()
+    assert (s_out[:n].double() - y).norm(dim=1).le(1e-5 * y.norm(dim=1) + 1e-6).all()
+    assert bool((out[-1] == 7.0).all()) and bool((s_out[n] == 7.0).all()) and bool((s_hidden[:, shared:] == 7.0).all()) and bool((s_hidden[n] == 7.0).all())
