@@ -15,6 +15,12 @@
 // consumer warps take every eighth 16-wide k step of a stage (`mma.sync.m16n8k16`: 16 weight rows x
 // 8 tokens), add their partial tiles through shared memory in warp order and apply the epilogue.
 //
+// An accumulating product may lead to an RMS norm (hfee_gemm_ring_then_norm): its epilogue, which has the new rows of the residual
+// stream in registers, also leaves them times the norm's weight in bfloat16 and each CTA's sum of their squares per token; the
+// product that follows (hfee_gemm_stream_scaled) adds the CTAs' sums in order and scales its float32 results by the row's
+// 1/sqrt(mean + eps).  The norm as a kernel between the two, over a few rows, was all latency: 2.0 us twice a layer at 8 tokens and
+// 2,048 columns, against the sums' loads, which the product issues with its first weights (16 layers: 843 -> 817 us a step).
+//
 // Every wait has a time limit; a wait that runs out sets the status word.
 #include "tcgen05.cuh"
 
@@ -47,6 +53,9 @@ struct RingArgs {
   int resident;                                    // 1: all tokens are loaded once and stay in shared memory
   int token_bytes;                                 // size of the token region
   int* status;
+  __nv_bfloat16* next; long long ld_next;          // null, or: the new rows times next_w, rounded (EPI_ACCUM only)
+  const float* next_w; int next_unit;              // next_unit: times 1 + next_w
+  float* next_sums;                                // [MAX_TOKENS][grid] the CTAs' sums of squares
 };
 
 // A box [8 slabs][rows][64 k] of a matrix seen as (k in slab, row, slab): coordinates (0, row, slab).
@@ -162,6 +171,7 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     OutT* C = reinterpret_cast<OutT*>(a.C);
     if (EPI == EPI_ACCUM) pdl_wait();                               // what is added to is an earlier kernel's output
     if (a.resident && r0 < r1) ok = __all_sync(0xffffffffu, mbar_wait(a_full, 0, &abort_flag));
+    float squares = 0.f;
 
     for (int row0 = r0; row0 < r1 && ok; row0 += a.tile) {
       const int rows = min(a.tile, r1 - row0);
@@ -170,7 +180,8 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       // ahead of its use
       const int e_row = ct / MAX_TOKENS, e_m = ct % MAX_TOKENS;
       const bool e_mine = ct < TILE_ROWS * MAX_TOKENS && e_m < a.M && e_row < rows;
-      float old = 0.f;
+      float old = 0.f, next_w = 0.f;
+      if (EPI == EPI_ACCUM && e_mine && a.next != nullptr) next_w = __ldg(a.next_w + row0 + e_row) + (a.next_unit ? 1.f : 0.f);
       if (EPI == EPI_ACCUM && e_mine) old = __ldcg(reinterpret_cast<const float*>(a.C) + (long long)e_m * a.ldc + row0 + e_row);
       for (int k0 = 0; k0 < a.K; k0 += KC, ++it) {
         const int s = it % S, ts = it % T_STAGES;
@@ -227,7 +238,12 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (EPI == EPI_STORE) {
           C[(long long)m * a.ldc + row0 + row] = to_out<OutT>(total(row));
         } else if (EPI == EPI_ACCUM) {
-          C[(long long)m * a.ldc + row0 + row] = to_out<OutT>(old + total(row));
+          const float y = old + total(row);
+          C[(long long)m * a.ldc + row0 + row] = to_out<OutT>(y);
+          if (a.next != nullptr) {
+            a.next[(long long)m * a.ld_next + row0 + row] = __float2bfloat16_rn(y * next_w);
+            squares = fmaf(y, y, squares);
+          }
         } else if ((row & 7) < 4) {
           // rows 8u .. 8u+3 are gate rows, 8u+4 .. 8u+7 the up rows of the same four outputs
           const float gate = total(row), up = total(row + 4);
@@ -236,6 +252,19 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
       }
       consumer_sync();
+    }
+    if (EPI == EPI_ACCUM && a.next != nullptr) {
+      // lane = (row mod 4, token): rows of a warp, then the four warps that hold the tile's rows, in order
+      squares += __shfl_xor_sync(0xffffffffu, squares, 8);
+      squares += __shfl_xor_sync(0xffffffffu, squares, 16);
+      if (cw < 4 && lane < MAX_TOKENS) red[cw * MAX_TOKENS + lane] = squares;
+      consumer_sync();
+      if (ct < a.M) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) v += red[w * MAX_TOKENS + ct];
+        a.next_sums[ct * gridDim.x + blockIdx.x] = v;
+      }
     }
   }
 
@@ -309,10 +338,11 @@ HFEE_API int hfee_gemm_ring_supports(int M, int N, int K, int epilogue) {
   return 1;
 }
 
-// epilogue: 0 store, 1 accumulate into float32 C, 2 SwiGLU (C is [M, N/2]; rows of W in groups of
-// 4 gate rows and 4 up rows).  out_dtype: 0 float32, 1 bfloat16.
-HFEE_API int hfee_gemm_ring(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
-                            int out_dtype, int epilogue, int M, int N, int K, int* status, cudaStream_t stream) {
+namespace {
+struct NextNorm { void* rows; long long ld; const float* weight; int add_unit; float* sums; };
+
+int ring_any(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
+             int out_dtype, int epilogue, int M, int N, int K, int* status, const NextNorm& next, cudaStream_t stream) {
   if (M == 0 || N == 0) return HFEE_OK;
   HFEE_REQUIRE(hfee_gemm_ring_supports(M, N, K, epilogue),
                "gemm_ring: takes 1..%d tokens, K a multiple of 64 and, for SwiGLU, N a multiple of 8 (got M=%d N=%d K=%d epilogue=%d)",
@@ -334,6 +364,8 @@ HFEE_API int hfee_gemm_ring(const void* A, long long lda, const void* W, long lo
   a.token_bytes = token_region_bytes(K);
   a.resident = (K + KC - 1) / KC * T_BYTES <= RESIDENT_MAX ? 1 : 0;
   a.status = status;
+  a.next = (__nv_bfloat16*)next.rows; a.ld_next = next.ld;
+  a.next_w = next.weight; a.next_unit = next.add_unit; a.next_sums = next.sums;
   CUtensorMap mw, ma;
   int rc;
   if ((rc = make_slab_map(&mw, W, N, K, ldw, a.tile)) != HFEE_OK) return rc;
@@ -345,4 +377,27 @@ HFEE_API int hfee_gemm_ring(const void* A, long long lda, const void* W, long lo
   if (out_dtype == HFEE_F32) HFEE_RING(EPI_SWIGLU, float);
   HFEE_RING(EPI_SWIGLU, __nv_bfloat16);
 #undef HFEE_RING
+}
+}  // namespace
+
+// epilogue: 0 store, 1 accumulate into float32 C, 2 SwiGLU (C is [M, N/2]; rows of W in groups of
+// 4 gate rows and 4 up rows).  out_dtype: 0 float32, 1 bfloat16.
+HFEE_API int hfee_gemm_ring(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
+                            int out_dtype, int epilogue, int M, int N, int K, int* status, cudaStream_t stream) {
+  return ring_any(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, status, NextNorm{nullptr, 0, nullptr, 0, nullptr}, stream);
+}
+
+// C += A W^T in float32, and for the RMS norm that reads C next: next [M, N] bfloat16 = the new rows times next_weight (one plus it
+// with add_unit), sums [8][hfee_gemm_ring_parts(N)] = parts of each row's sum of squares.
+HFEE_API int hfee_gemm_ring_then_norm(const void* A, long long lda, const void* W, long long ldw, float* C, long long ldc, int M, int N,
+                                      int K, void* next, long long ld_next, const float* next_weight, int add_unit, float* sums,
+                                      int* status, cudaStream_t stream) {
+  HFEE_REQUIRE(next != nullptr && next_weight != nullptr && sums != nullptr && ld_next >= N, "gemm_ring_then_norm: no place for the norm's input");
+  return ring_any(A, lda, W, ldw, C, ldc, HFEE_F32, EPI_ACCUM, M, N, K, status, NextNorm{next, ld_next, next_weight, add_unit, sums}, stream);
+}
+
+// CTAs of an accumulating product of N weight rows: the parts of a row's sum of squares.
+HFEE_API int hfee_gemm_ring_parts(int N) {
+  const int sms = hfee_sm_count();
+  return N < sms ? N : sms;
 }

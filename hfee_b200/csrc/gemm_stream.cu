@@ -84,7 +84,10 @@ struct NormArgs {
   const float* weight;   // [K]
   float eps;
   int add_unit;          // scale by 1 + weight
+  const float* sums;     // NORM_SCALED: [8][parts] parts of each token's sum of squares; the rows in A carry the weight already
+  int parts;
 };
+enum { NORM_NONE = 0, NORM_ROWS = 1, NORM_SCALED = 2 };
 
 template <int MT, int NT, int NW, int EPI, typename TOut>
 __global__ void __launch_bounds__(NW * 32, 2048 / (NW * 32) >= 4 ? 2 : 1)
@@ -367,8 +370,10 @@ gemm_stream_rows_kernel(const __nv_bfloat16* __restrict__ A, long long lda, cons
 // contiguous range of 8-row tiles (the ranges differ by at most one tile, whatever N is); the
 // warps' partial sums of a group of up to 8 tiles meet in shared memory (pass after pass in pass
 // order, then added in warp order: one fixed order whatever M is) and are written 64 columns wide.
-// NORM (K of at most one pass) makes the token fragments from float32 rows: the RMS norm fused in
-// front, computed once per CTA from the very loads that fill the fragments.
+// NORM_ROWS (K of at most one pass) makes the token fragments from float32 rows: the RMS norm fused in
+// front, computed once per CTA from the very loads that fill the fragments.  NORM_SCALED reads rows that
+// the product before left in bfloat16, weight included, and multiplies the float32 results by each row's
+// 1/sqrt(mean square + eps): half the bytes of the float32 rows, which every CTA reads, and any K.
 constexpr int SL_WARPS = 8;
 constexpr int SL_STEPS = 8;                              // k32 steps per warp and pass
 constexpr int SL_SLICE = SL_STEPS * 32;                  // 256 columns per warp and pass
@@ -376,13 +381,14 @@ constexpr int SL_PASS = SL_WARPS * SL_SLICE;             // 2048 columns per pas
 constexpr int SL_GROUP = 8;                              // row tiles whose sums are added together
 constexpr int SL_TOKEN_PITCH = SL_GROUP * 8 + 8;         // floats per token row of the partial sums (padded)
 
-template <int EPI, bool NORM, typename TOut>
+template <int EPI, int NORM, typename TOut>
 __global__ void __launch_bounds__(SL_WARPS * 32, 2)
 gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const __nv_bfloat16* __restrict__ W,
                           long long ldw, TOut* __restrict__ C, long long ldc, int M, int N, int K, GluArgs glu, NormArgs norm) {
   __shared__ __align__(16) float red[2][SL_WARPS][8][SL_TOKEN_PITCH];
-  __shared__ __align__(16) float norm_w[NORM ? SL_PASS : 4];       // NORM: the scales of this pass, staged before the wait
+  __shared__ __align__(16) float norm_w[NORM == NORM_ROWS ? SL_PASS : 4];       // NORM: the scales of this pass, staged before the wait
   __shared__ float sq_part[SL_WARPS][8];
+  __shared__ float token_scale[8];                                 // NORM_SCALED
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, c = lane & 3;
   const int n_tiles = (N + 7) / 8;
@@ -414,7 +420,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
   load_unit(total > 0, cur, wv[0]);
   const bool tok_ok = g < M;            // this lane's token: row g of the MMA's A tile; rows 8-15 stay zero
   const float* xrow = nullptr;
-  if constexpr (NORM) {
+  if constexpr (NORM == NORM_ROWS) {
     // NORM covers K <= one pass.  The scales do not come from the previous kernel: warp w stages the
     // 256 of its columns before the wait.
 #pragma unroll
@@ -432,7 +438,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
   const __nv_bfloat16* arow = A + (long long)(tok_ok ? g : 0) * lda;
   uint4 a_lo[SL_STEPS];
   int a_pass = -1;
-  if constexpr (NORM) {
+  if constexpr (NORM == NORM_ROWS) {
     // This lane's 64 values of token g (all requested at once), their squares summed over the quad,
     // the warps' sums added in warp order: one fixed order whatever the batch is.  Then
     // a = bf16(x * rsqrt(mean(x^2) + eps) * w), as the norm kernel computes it.
@@ -482,6 +488,24 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
     a_pass = pass;
   };
 
+  if constexpr (NORM == NORM_SCALED) {
+    static_assert(SL_WARPS == 8, "a warp per token adds its parts");
+    load_tokens(0);
+    float v = 0.f;
+    for (int i0 = 0; i0 < norm.parts; i0 += 8 * 32) {       // a token's parts are asked for together: one trip to memory
+      float part[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j * 32 + lane;
+        part[j] = warp < M && i < norm.parts ? norm.sums[warp * norm.parts + i] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v += part[j];
+    }
+    v = warp_sum(v);
+    if (lane == 0) token_scale[warp] = 1.0f / sqrtf(v / (float)K + norm.eps);       // read behind the first group's barrier
+  }
+
   // sums of a finished group: warps in warp order, then the epilogue, 64 (SwiGLU: 32) columns per token
   auto finish_group = [&](int grp) {
     const int gs = group_size(grp);
@@ -496,6 +520,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
         float gate = 0.f, up = 0.f;
 #pragma unroll
         for (int w = 0; w < SL_WARPS; ++w) { gate += part[w][t][tile * 8 + i]; up += part[w][t][tile * 8 + 4 + i]; }
+        if constexpr (NORM == NORM_SCALED) { gate *= token_scale[t]; up *= token_scale[t]; }
         C[(long long)t * ldc + col] = from_f32<TOut>(gated_out<EPI>(gate, up, glu));
       }
     } else {
@@ -507,6 +532,7 @@ gemm_stream_slices_kernel(const __nv_bfloat16* __restrict__ A, long long lda, co
           float v = 0.f;
 #pragma unroll
           for (int w = 0; w < SL_WARPS; ++w) v += part[w][t][o];
+          if constexpr (NORM == NORM_SCALED) v *= token_scale[t];
           const long long at = (long long)t * ldc + col;
           if constexpr (EPI == EPI_ACCUM) C[at] = to_f32<TOut>(C[at]) + v;
           else C[at] = from_f32<TOut>(stored_out<EPI>(v));
@@ -702,7 +728,7 @@ int launch_wide(const void* A, long long lda, const void* W, long long ldw, void
   return hfee_check_launch("gemm_stream_wide");
 }
 
-template <bool NORM>
+template <int NORM>
 int launch_slices(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype,
                   int epilogue, int M, int N, int K, const GluArgs& glu, const NormArgs& norm, cudaStream_t stream) {
   const __nv_bfloat16* a = (const __nv_bfloat16*)A;
@@ -786,8 +812,8 @@ int stream_any(const void* A, long long lda, const void* W, long long ldw, void*
   if (rc != HFEE_OK) return rc;
   HFEE_REQUIRE(lda % 8 == 0 && lda >= K && (uintptr_t)A % 16 == 0,
                "gemm_stream: the tokens' leading dimension %lld must be a multiple of 8, at least K, and 16-byte aligned", lda);
-  NormArgs none{nullptr, 0, nullptr, nullptr, 0.f, 0};
-  if (M <= 8) return launch_slices<false>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, none, stream);
+  NormArgs none{nullptr, 0, nullptr, nullptr, 0.f, 0, nullptr, 0};
+  if (M <= 8) return launch_slices<NORM_NONE>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, none, stream);
   if (M <= 16 && K <= WD_WARPS * WD_SLICE) return launch_wide(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
   if ((N + 7) / 8 >= ROWS_MIN_TILES && M <= 32) {
     if (M <= 16) return launch_rows<1>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, glu, stream);
@@ -825,6 +851,19 @@ HFEE_API int hfee_gemm_stream_norm(const float* X, long long ldx, const int* row
   HFEE_REQUIRE(ldx % 4 == 0 && ldx >= K && (uintptr_t)X % 16 == 0 && (uintptr_t)norm_weight % 16 == 0,
                "gemm_stream_norm: float32 rows need a leading dimension %% 4 == 0 and 16-byte alignment");
   HFEE_REQUIRE(epilogue != EPI_CLAMPED, "gemm_stream_norm: the clamped activation takes normed rows");
-  NormArgs norm{X, ldx, rows, norm_weight, eps, add_unit};
-  return launch_slices<true>(nullptr, 0, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, GluArgs{0.f, 0.f, 0.f}, norm, stream);
+  NormArgs norm{X, ldx, rows, norm_weight, eps, add_unit, nullptr, 0};
+  return launch_slices<NORM_ROWS>(nullptr, 0, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, GluArgs{0.f, 0.f, 0.f}, norm, stream);
+}
+
+// The same behind hfee_gemm_ring_then_norm: rows A [M, K] bfloat16 with the norm's weight in them, and `sums` [8][parts].
+HFEE_API int hfee_gemm_stream_scaled(const void* A, long long lda, const float* sums, int parts, float eps, const void* W, long long ldw,
+                                     void* C, long long ldc, int out_dtype, int epilogue, int M, int N, int K, cudaStream_t stream) {
+  if (M == 0 || N == 0) return HFEE_OK;
+  int rc = check_common(W, ldw, ldc, epilogue, M, N, K);
+  if (rc != HFEE_OK) return rc;
+  HFEE_REQUIRE(M <= 8 && epilogue != EPI_CLAMPED, "gemm_stream_scaled: takes at most 8 tokens (got %d) and no clamped activation", M);
+  HFEE_REQUIRE(lda % 8 == 0 && lda >= K && (uintptr_t)A % 16 == 0 && sums != nullptr && parts > 0,
+               "gemm_stream_scaled: rows need a leading dimension %% 8 == 0, 16-byte alignment and their sums of squares");
+  NormArgs norm{nullptr, 0, nullptr, nullptr, eps, 0, sums, parts};
+  return launch_slices<NORM_SCALED>(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, GluArgs{0.f, 0.f, 0.f}, norm, stream);
 }

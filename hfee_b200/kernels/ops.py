@@ -44,6 +44,9 @@ _SIGNATURES = {
     "hfee_gemm_skinny_splits": [_I, _I, _I, _L],
     "hfee_gemm_ring": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _P],
     "hfee_gemm_ring_supports": [_I, _I, _I, _I],
+    "hfee_gemm_ring_then_norm": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _L, _P, _I, _P, _P, _P],
+    "hfee_gemm_ring_parts": [_I],
+    "hfee_gemm_stream_scaled": [_P, _L, _P, _I, _F, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
     "hfee_attention_tc": [_P, _I, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "hfee_attention_tc_general": [_P, _I, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _F, _P, _F, _P, _P],
     "hfee_attention_tc_supports": [_I, _I, _I, _I],
@@ -634,11 +637,66 @@ def _norm_fusable(inp, w: torch.Tensor) -> bool:
             and p[0].data_ptr() % 16 == 0)
 
 
+def gemm_ring_then_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, add_unit: bool, rows: torch.Tensor,
+                        sums: torch.Tensor) -> torch.Tensor:
+    """out += a @ w.T in float32 (:func:`gemm_ring`), and for the RMS norm that reads ``out`` next: ``rows`` = bf16(out * weight) and,
+    returned, a view [8, parts] of ``sums`` with the parts of each row's sum of squares (see :func:`gemm_stream_scaled`)."""
+    lib = library()
+    m, k = a.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and a.dtype == w.dtype == rows.dtype == torch.bfloat16 and out.dtype == weight.dtype == sums.dtype == torch.float32
+    assert tuple(out.shape) == tuple(rows.shape) == (m, n) and weight.numel() == n
+    parts = lib.hfee_gemm_ring_parts(n)
+    sums = sums[:8 * parts].view(8, parts)
+    _check(lib.hfee_gemm_ring_then_norm(a.data_ptr(), _rows(a, "gemm a"), w.data_ptr(), _rows(w, "gemm w"), out.data_ptr(),
+                                        _rows(out, "gemm out"), m, n, k, rows.data_ptr(), _rows(rows, "rows"), weight.data_ptr(),
+                                        int(add_unit), sums.data_ptr(), _status().data_ptr(), _stream()), lib)
+    return sums
+
+
+def gemm_stream_scaled(rows: torch.Tensor, sums: torch.Tensor, eps: float, w: torch.Tensor, out: torch.Tensor,
+                       epilogue: int = EPI_STORE) -> None:
+    """:func:`gemm_stream` of RMS-normed rows that only lack their scale (:func:`gemm_ring_then_norm`): the float32 results are
+    multiplied by 1/sqrt(sum(sums) / width + eps) of their row.  At most 8 rows."""
+    lib = library()
+    m, k = rows.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and rows.dtype == w.dtype == torch.bfloat16 and sums.dtype == torch.float32 and sums.is_contiguous()
+    assert tuple(out.shape) == (m, n // 2 if epilogue in EPI_GATED else n) and sums.shape[0] == 8
+    _check(lib.hfee_gemm_stream_scaled(rows.data_ptr(), _rows(rows, "rows"), sums.data_ptr(), sums.shape[1], float(eps), w.data_ptr(),
+                                       _rows(w, "gemm w"), out.data_ptr(), _rows(out, "gemm out"), _dt(out), epilogue, m, n, k,
+                                       _stream()), lib)
+
+
+def _leads_to_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, then) -> bool:
+    """out += a @ w.T together with the norm ``then`` that reads ``out`` (parts/norm.py: LazyNormed); False, and nothing done, where the
+    plain product and a norm of its own are to run."""
+    p = then.fused_params()
+    if (p is None or then.rows is not None or then.out_dtype != torch.bfloat16 or then.source.data_ptr() != out.data_ptr()
+            or then.buffer.shape != out.shape or then.source.stride() != out.stride() or not _streamable(a, w)):
+        return False
+    weight, eps, add_unit = p
+    (m, k), n = a.shape, w.shape[0]
+    if then.sums is not None and _ring_rule(m, n, k, EPI_ACCUM):
+        then.scaled = gemm_ring_then_norm(a, w, out, weight, add_unit, then.buffer, then.sums)
+        return True
+    return False
+
+
+def _scaled_rows(inp, w: torch.Tensor):
+    """(rows, sums, eps) where ``inp`` holds rows that only lack their scale and the streaming product takes them, else None."""
+    if inp.scaled is None or inp.n > 8 or not _streamable(inp.buffer, w):
+        return None
+    return inp.buffer, inp.scaled, inp.fused_params()[1]
+
+
 def linear_normed(inp, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> None:
     """out (+)= norm(x) @ w.T where ``inp`` is a lazily normed input: the norm runs inside the
     product when a kernel that can do so fits, else ``inp`` is materialised first."""
     if isinstance(inp, torch.Tensor):
         linear(inp, w, out, accumulate)
+    elif (scaled := _scaled_rows(inp, w)) is not None:
+        gemm_stream_scaled(scaled[0], scaled[1], scaled[2], w, out, EPI_ACCUM if accumulate else EPI_STORE)
     elif _norm_fusable(inp, w):
         weight, eps, add_unit = inp.fused_params()
         gemm_stream_norm(inp.source, weight, eps, w, out, EPI_ACCUM if accumulate else EPI_STORE, inp.rows, add_unit)
@@ -650,6 +708,8 @@ def linear_swiglu_normed(inp, w_gate_up: torch.Tensor, out: torch.Tensor, granul
     """:func:`linear_swiglu` on a lazily normed input."""
     if isinstance(inp, torch.Tensor):
         linear_swiglu(inp, w_gate_up, out, granule, scratch)
+    elif granule == SWIGLU_GRANULE and w_gate_up.shape[0] % 8 == 0 and (scaled := _scaled_rows(inp, w_gate_up)) is not None:
+        gemm_stream_scaled(scaled[0], scaled[1], scaled[2], w_gate_up, out, EPI_SWIGLU)
     elif granule == SWIGLU_GRANULE and w_gate_up.shape[0] % 8 == 0 and _norm_fusable(inp, w_gate_up):
         weight, eps, add_unit = inp.fused_params()
         gemm_stream_norm(inp.source, weight, eps, w_gate_up, out, EPI_SWIGLU, inp.rows, add_unit)
@@ -713,6 +773,13 @@ def _small_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
 def _ring_rule(m: int, n: int, k: int, epilogue: int) -> bool:
     return (epilogue in RING_EPILOGUES and RING_MIN_TOKENS <= m <= RING_MAX_TOKENS and USE_TCGEN05
             and n <= 16 * sm_count() and ring_takes(m, n, k, epilogue))
+
+
+def linear_then_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, then) -> None:
+    """out += a @ w.T where ``then``, the lazily normed rows (parts/norm.py) of a norm, reads ``out`` next: they are computed along with
+    the product where a kernel does that, else when they are asked for."""
+    if not _leads_to_norm(a, w, out, then):
+        linear(a, w, out, accumulate=True)
 
 
 def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> None:
@@ -2365,7 +2432,7 @@ def argmax(logits: torch.Tensor, out: torch.Tensor, scratch: torch.Tensor, slots
 # the entry points the parts and the sampler launch through can be left out by class (see tag())
 for _name in ("rmsnorm_add_norm", "latent_attention", "linear_act", "attention_simt_general", "rope_norm_cache", "latent_norm_rope_cache", "head_linear", "head_linear_parts", "conv_act", "delta_rule",
               "head_norm_gate", "unary_act", "head_gate", "attention_simt_masked", "short_conv", "linear_attention", "rmsnorm_add", "norm_gate", "gated_act", "scale_", "cast_rows", "sigmoid_attention",
-              "qk_norm_rope_cache", "embed", "rmsnorm", "rope_table", "rope_cache_write", "swiglu", "linear", "linear_normed", "linear_swiglu", "linear_rope_cache",
+              "qk_norm_rope_cache", "embed", "rmsnorm", "rope_table", "rope_cache_write", "swiglu", "linear", "linear_then_norm", "linear_normed", "linear_swiglu", "linear_rope_cache",
               "linear_swiglu_normed", "paged_attention", "paged_attention_rope", "sample", "argmax", "sample_chain",
               "mingru", "selective_scan", "distance_attention", "moe_route", "moe_plan", "moe_experts", "moe_experts_grouped", "moe_experts_few", "moe_combine",
               "clamped_glu", "linear_clamped_glu", "depth_average", "scaled_add_norm", "scaled_add", "add_sinusoid", "softcap_",

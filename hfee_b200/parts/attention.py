@@ -25,6 +25,7 @@ class PagedAttention(Mixer):
     (None = head_dim**-0.5, internal/llm/forward.go:149)."""
 
     accepts_lazy_input = True        # the input norm may be fused into the q/k/v projection
+    leads_to_norm = True             # the norm that reads the residual next may leave with the output projection (``then``)
 
     @property
     def graph_safe(self) -> bool:    # every launch reads the batch from device buffers; the position part decides
@@ -57,7 +58,7 @@ class PagedAttention(Mixer):
     def cache_need(self) -> PagedKV:
         return PagedKV(self.kv_heads, self.head_dim, self.window)
 
-    def forward(self, xn: torch.Tensor, residual: torch.Tensor, step: Any, cache: Any, writes_cache: bool) -> None:
+    def forward(self, xn: torch.Tensor, residual: torch.Tensor, step: Any, cache: Any, writes_cache: bool, then=None) -> None:
         n, rt = step.n, self.rt
         cs = self.position.table(step)
         q = rt.scratch("attn_q", (rt.max_tokens, self.q_cols))[:n]
@@ -84,7 +85,10 @@ class PagedAttention(Mixer):
                                      self.kv_heads, self.head_dim, self.scale, int(self.window or 0), step,
                                      self.split_scratch)
             ops.tag("o")
-            ops.linear(att, self.w_o, residual, accumulate=True)
+            if then is not None:
+                ops.linear_then_norm(att, self.w_o, residual, then)
+            else:
+                ops.linear(att, self.w_o, residual, accumulate=True)
             return
         if not fused_qkv:
             ops.tag("rope")

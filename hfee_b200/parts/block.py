@@ -1,7 +1,7 @@
 """Arrangement of norm, mixer and feed-forward in one layer."""
 from __future__ import annotations
 
-from typing import Any
+from typing import Any, Optional
 
 import torch
 
@@ -29,21 +29,51 @@ class PreNormBlock(Block):
         import inspect
         self.takes_residual_add = "residual_add" in inspect.signature(self.mixer_norm.forward).parameters
 
-    def forward(self, residual: torch.Tensor, step: Any, cache: Any, writes_cache: bool, residual_add=None) -> None:
+    @property
+    def takes_entry(self) -> bool:
+        """The norm in front of this layer may be computed by whatever writes the residual before it (:meth:`entry`): by bfloat16
+        products; in float32 every norm has a kernel of its own."""
+        return self.rt.dtype == torch.bfloat16 and bool(getattr(self.mixer, "accepts_lazy_input", False))
+
+    def entry(self, residual: torch.Tensor, step: Any) -> LazyNormed:
+        """The normed input of the mixer, for the product in front of this layer and then for :meth:`forward`."""
+        return LazyNormed(self.mixer_norm, residual, self.rt.scratch("block_normed", (self.rt.max_tokens, self.width))[:step.n],
+                          sums=self._sums())
+
+    def _sums(self) -> Optional[torch.Tensor]:
+        """Room for the parts of a few rows' sums of squares: written by a product, read by the next one on the same stream."""
+        if self.rt.device.type != "cuda":
+            return None
+        return self.rt.scratch("norm_sums", (8 * ops.sm_count(),), torch.float32)
+
+    def forward(self, residual: torch.Tensor, step: Any, cache: Any, writes_cache: bool, residual_add=None, entry=None, then=None) -> None:
+        """``entry``: what :meth:`entry` gave for this step; ``then``: the next layer's."""
         xn = self.rt.scratch("block_normed", (self.rt.max_tokens, self.width))[:step.n]
+        ffn_in, middle = None, {}
+        if self.feed_forward is None:
+            middle = self._handed(self.mixer, then)
+        else:
+            lead = self.rt.dtype == torch.bfloat16 and getattr(self.mixer, "leads_to_norm", False)
+            ffn_in = LazyNormed(self.ffn_norm, residual, xn, sums=self._sums() if lead else None)
+            if lead and getattr(self.feed_forward, "accepts_lazy_input", False):
+                middle = self._handed(self.mixer, ffn_in)
         if residual_add is not None:
             self.mixer_norm.forward(residual, xn, residual_add=residual_add)
-            self.mixer.forward(xn, residual, step, cache, writes_cache)
+            self.mixer.forward(xn, residual, step, cache, writes_cache, **middle)
         else:
-            self.mixer.forward(self._normed(self.mixer, self.mixer_norm, residual, xn), residual, step, cache, writes_cache)
+            lazy = entry if entry is not None else LazyNormed(self.mixer_norm, residual, xn)
+            self.mixer.forward(self._input(self.mixer, lazy), residual, step, cache, writes_cache, **middle)
         if self.feed_forward is not None:
-            self.feed_forward.forward(self._normed(self.feed_forward, self.ffn_norm, residual, xn), residual, step)
+            self.feed_forward.forward(self._input(self.feed_forward, ffn_in), residual, step, **self._handed(self.feed_forward, then))
 
     @staticmethod
-    def _normed(consumer, norm, residual, buffer):
+    def _handed(part, then) -> dict:
+        return {"then": then} if then is not None and getattr(part, "leads_to_norm", False) else {}
+
+    @staticmethod
+    def _input(consumer, lazy):
         """The consumer's input: a lazily normed one if it says it can take it (and may fuse the
         norm into its first product), else the normed tensor."""
-        lazy = LazyNormed(norm, residual, buffer)
         return lazy if getattr(consumer, "accepts_lazy_input", False) else lazy.tensor()
 
 

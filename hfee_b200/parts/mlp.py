@@ -20,6 +20,7 @@ class SwiGLUFeedForward(Part):
     category = "feed_forward"
     graph_safe = True
     accepts_lazy_input = True        # the input norm may be fused into the gate/up projection
+    leads_to_norm = True             # the norm that reads the residual next may leave with the down projection (``then``)
 
     @staticmethod
     def tensor_needs(spec: PartSpec) -> Dict[str, TensorNeed]:
@@ -45,7 +46,7 @@ class SwiGLUFeedForward(Part):
             self.w_gate_up = torch.cat([gate, up], dim=0).contiguous()
         self.w_down = tensors["down"]
 
-    def forward(self, xn: torch.Tensor, residual: torch.Tensor, step: Any, accumulate: bool = True) -> None:
+    def forward(self, xn: torch.Tensor, residual: torch.Tensor, step: Any, accumulate: bool = True, then=None) -> None:
         n, rt = step.n, self.rt
         gu = rt.scratch("ffn_gate_up", (rt.max_tokens, 2 * self.inner))[:n]
         h = rt.scratch("ffn_hidden", (rt.max_tokens, self.inner))[:n]
@@ -55,7 +56,10 @@ class SwiGLUFeedForward(Part):
         else:
             ops.linear_gated_normed(xn, self.w_gate_up, h, self.granule, gu, self.activation)
         ops.tag("down")
-        ops.linear(h, self.w_down, residual, accumulate=accumulate)
+        if then is not None and accumulate:
+            ops.linear_then_norm(h, self.w_down, residual, then)
+        else:
+            ops.linear(h, self.w_down, residual, accumulate=accumulate)
 
 
 class DenseFeedForward(Part):

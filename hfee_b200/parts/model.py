@@ -131,7 +131,9 @@ class DecoderModel:
             embedded.copy_(residual)
         if self.streams is not None:
             residual = ResidualStreams(rt, residual, self.streams)
-        for run in self.spec.schedule:
+        entry = None                     # the normed input of the next layer, which the layer before may have computed
+        schedule = self.spec.schedule
+        for i, run in enumerate(schedule):
             block = self.blocks[run.layer]
             if run.adds_embedding:
                 if getattr(block, "takes_residual_add", False):      # the block's first norm does the sum as well
@@ -140,7 +142,15 @@ class DecoderModel:
                 from ..kernels import ops
                 ops.tag("norm")
                 ops.scaled_add(embedded, 1.0, residual)
-            block.forward(residual, step, caches.get(run.cache), run.writes_cache)
+            if not getattr(block, "takes_entry", False):
+                block.forward(residual, step, caches.get(run.cache), run.writes_cache)
+                continue
+            then = None
+            if i + 1 < len(schedule) and not schedule[i + 1].adds_embedding:
+                after = self.blocks[schedule[i + 1].layer]
+                then = after.entry(residual, step) if getattr(after, "takes_entry", False) else None
+            block.forward(residual, step, caches.get(run.cache), run.writes_cache, entry=entry, then=then)
+            entry = then
         m = step.n_logits
         if m == 0:
             return None

@@ -111,13 +111,22 @@ class LazyNormed:
     A part that can fuse the norm into its first matrix product hands this object to
     ``ops.linear_normed``; any other use calls :meth:`tensor`, which runs the norm once into
     ``buffer`` and returns it.  ``rows`` gathers source rows (the head norms only the rows whose
-    logits are wanted)."""
+    logits are wanted).  The product that writes ``source`` may be handed this object too
+    (``ops.linear_then_norm``) and leave the normed rows in ``buffer`` itself, or (``scaled``) the rows times the norm's
+    weight there and the sums of their squares, which a product that scales its results takes."""
 
-    def __init__(self, norm, source: torch.Tensor, buffer: torch.Tensor, rows: Optional[torch.Tensor] = None):
+    def __init__(self, norm, source: torch.Tensor, buffer: torch.Tensor, rows: Optional[torch.Tensor] = None,
+                 sums: Optional[torch.Tensor] = None):
         self.norm, self.source, self.buffer, self.rows = norm, source, buffer, rows
         self.n = buffer.shape[0]
         self.out_dtype = buffer.dtype
         self._done = False
+        self.sums = sums             # room for the parts of eight rows' sums, a part for each SM; without it nothing is left unscaled
+        self.scaled = None           # the sums of squares [8, parts] where ``buffer`` holds rows that only lack their scale
+
+    def in_buffer(self) -> None:
+        """The normed rows are in ``buffer``: a kernel has left them there."""
+        self._done = True
 
     def fused_params(self):
         f = getattr(self.norm, "fused_params", None)
@@ -126,7 +135,7 @@ class LazyNormed:
     def tensor(self) -> torch.Tensor:
         if not self._done:
             self.norm.forward(self.source, self.buffer, rows=self.rows)
-            self._done = True
+            self._done, self.scaled = True, None
         return self.buffer
 
 

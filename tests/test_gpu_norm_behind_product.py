@@ -1,0 +1,76 @@
+"""A norm that leaves with the accumulating product in front of it, of a few tokens: the product behind it scales its results."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+EPS = 1e-5
+
+
+class _Norm:
+    def __init__(self, weight, add_unit):
+        self.weight, self.add_unit = weight, add_unit
+
+    def fused_params(self):
+        return self.weight, EPS, self.add_unit
+
+    def forward(self, x, out, rows=None):
+        from hfee_b200.kernels import ops
+        ops.rmsnorm(x, self.weight, out, EPS, rows=rows, add_unit=self.add_unit)
+
+
+def _rand(shape, seed, scale=1.0):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale
+
+
+def _case(m, n, k, add_unit):
+    from hfee_b200.kernels import ops
+    from hfee_b200.parts.norm import LazyNormed
+    a, w = _rand((m, k), 1).to(torch.bfloat16).to(DEV), _rand((n, k), 2, 0.05).to(torch.bfloat16).to(DEV)
+    residual = _rand((m + 1, n), 3, 4.0).to(DEV)
+    residual[0] *= 1e3                                                   # rows of very different size
+    weight = (_rand((n,), 4, 0.1) + (0.0 if add_unit else 1.0)).to(DEV)
+    want = residual[:m].double() + a.double() @ w.double().t()
+    scale = torch.rsqrt((want * want).mean(1, keepdim=True) + EPS)
+    normed = want * scale * (weight.double() + (1.0 if add_unit else 0.0))
+    buffer = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    sums = torch.full((8 * ops.sm_count(),), float("nan"), device=DEV)
+    return a, w, residual, LazyNormed(_Norm(weight, add_unit), residual[:m], buffer, sums=sums), want, normed
+
+
+# parts of a row's sum: one CTA's single column up to all of 16; a K of one slab, one pass and several
+@pytest.mark.parametrize("m,n,k", [(3, 8, 64), (8, 2048, 2048), (5, 2048, 8192), (4, 152, 192), (7, 2368, 512), (8, 72, 4096)])
+@pytest.mark.parametrize("add_unit", [False, True])
+def test_few_tokens(m, n, k, add_unit):
+    from hfee_b200.kernels import ops
+    a, w, residual, lazy, want, normed = _case(m, n, k, add_unit)
+    last = residual[m].clone()
+    ops.linear_then_norm(a, w, residual[:m], lazy)
+    assert lazy.scaled is not None and bool((residual[m] == last).all())
+    assert (residual[:m].double() - want).norm(dim=1).le(1e-5 * want.norm(dim=1)).all()
+    for out_rows, epilogue in ((24, "plain"), (4104, "plain"), (48, "gated")):
+        w2 = _rand((out_rows, n), 5, 0.05).to(torch.bfloat16).to(DEV)
+        y = normed @ w2.double().t()
+        if epilogue == "plain":
+            out = torch.empty(m, out_rows, dtype=torch.float32, device=DEV)
+            ops.linear_normed(lazy, w2, out)
+        else:
+            out = torch.empty(m, out_rows // 2, dtype=torch.bfloat16, device=DEV)
+            ops.linear_swiglu_normed(lazy, w2, out, ops.SWIGLU_GRANULE, None)
+            y = y.reshape(m, -1, 2, 4)
+            y = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(m, -1)
+        assert lazy.scaled is not None                                   # no norm kernel ran
+        # the operand is rounded to bfloat16 (2^-9 each, averaged over the sum), a gated result once more
+        assert (out.double() - y).norm(dim=1).le(8e-3 * y.norm(dim=1)).all()
+    ops.check_status()
+    assert (lazy.tensor().double() - normed).norm(dim=1).le(4e-3 * normed.norm(dim=1)).all() and lazy.scaled is None
+
+
+def test_what_has_no_such_kernel_takes_the_plain_product():
+    from hfee_b200.kernels import ops
+    for m, n, k in ((1, 2048, 2048), (12, 2048, 2048), (65, 256, 512), (4, 4096, 512), (8, 100, 72)):
+        a, w, residual, lazy, want, normed = _case(m, n, k, False)
+        ops.linear_then_norm(a, w, residual[:m], lazy)
+        assert lazy.scaled is None and not lazy._done
+        assert (residual[:m].double() - want).norm(dim=1).le(1e-5 * want.norm(dim=1)).all()
+        assert (lazy.tensor().double() - normed).norm(dim=1).le(4e-3 * normed.norm(dim=1)).all()
