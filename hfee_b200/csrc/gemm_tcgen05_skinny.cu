@@ -277,6 +277,69 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, TOut* __restr
   }
 }
 
+// The same sum into a float32 C whose rows an RMS norm reads next: a block has a token, so the norm of the new row leaves from the
+// same kernel (out = bf16(row * 1/sqrt(mean square + eps) * weight)).  Both are latency, not bytes: at 64 tokens and 2,048 columns the
+// two kernels took 3.1 and 2.4 us of a decode step, this one 4.1 to 4.5 (with the parts of 16 splits asked for together, which is more
+// registers than it has use for: 5.9 to 7.0).  VEC float4 a thread; the weights are asked for before the wait.
+constexpr int RN_THREADS = 512, RN_VEC_MAX = 4;
+
+template <int VEC>
+__global__ void __launch_bounds__(RN_THREADS)
+splitk_reduce_norm_kernel(const float* __restrict__ ws, float* __restrict__ C, long long ldc, int M, int N, int splits,
+                          const float* __restrict__ weight, float eps, int add_unit, __nv_bfloat16* __restrict__ out, long long ld_out) {
+  __shared__ float part_sum[RN_THREADS / 32];
+  const int t = blockIdx.x, n4 = N / 4;
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 w[VEC], v[VEC];
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    const int c = threadIdx.x + j * RN_THREADS;
+    w[j] = c < n4 ? __ldg(reinterpret_cast<const float4*>(weight) + c) : none;
+    if (add_unit) { w[j].x += 1.f; w[j].y += 1.f; w[j].z += 1.f; w[j].w += 1.f; }
+    v[j] = none;
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  const long long split_pitch = (long long)M * n4;
+  const float4* p = reinterpret_cast<const float4*>(ws) + (long long)t * n4;
+  float4* row = reinterpret_cast<float4*>(C + (long long)t * ldc);
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    const int c = threadIdx.x + j * RN_THREADS;
+    if (c >= n4) continue;
+    const float4 old = row[c];
+    for (int s0 = 0; s0 < splits; s0 += RED_BATCH) {
+      float4 part[RED_BATCH];
+#pragma unroll
+      for (int i = 0; i < RED_BATCH; ++i) part[i] = s0 + i < splits ? p[(s0 + i) * split_pitch + c] : none;
+#pragma unroll
+      for (int i = 0; i < RED_BATCH; ++i) { v[j].x += part[i].x; v[j].y += part[i].y; v[j].z += part[i].z; v[j].w += part[i].w; }
+    }
+    v[j].x += old.x; v[j].y += old.y; v[j].z += old.z; v[j].w += old.w;
+    row[c] = v[j];
+    ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) part_sum[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int i = 0; i < RN_THREADS / 32; ++i) total += part_sum[i];
+  const float scale = 1.0f / sqrtf(total / (float)N + eps);
+  __nv_bfloat16* dst = out + (long long)t * ld_out;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    const int c = threadIdx.x + j * RN_THREADS;
+    if (c >= n4) continue;
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v[j].x * scale * w[j].x, v[j].y * scale * w[j].y);
+    __nv_bfloat162 hi = __floats2bfloat162_rn(v[j].z * scale * w[j].z, v[j].w * scale * w[j].w);
+    *reinterpret_cast<uint2*>(dst + 4 * c) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  }
+}
+
+struct NextNorm { const float* weight; float eps; int add_unit; __nv_bfloat16* out; long long ld_out; };
+
 int device_sms() { return hfee_sm_count(); }
 
 // K split for N weight rows and K: as many CTAs as SMs, at least 4 K blocks each.
@@ -297,7 +360,8 @@ void plan_split(int N, int K, int M, long long workspace_floats, int* splits, in
 }
 
 template <int TN, int EPI, typename TOut>
-int launch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, const SkinnyArgs& a, int* status, cudaStream_t stream) {
+int launch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, const SkinnyArgs& a, int* status, cudaStream_t stream,
+           const NextNorm* next = nullptr) {
   using Cfg = SkinnyCfg<TN>;
   static bool configured = false;
   if (!configured) {
@@ -311,6 +375,15 @@ int launch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, const SkinnyAr
               stream, mw, ma, (TOut*)C, a, status);
   int rc = hfee_check_launch("gemm_skinny");
   if (rc != HFEE_OK || a.splits == 1) return rc;
+  if constexpr (EPI == EPI_ACCUM) {
+    if (next != nullptr) {
+      const int vec = (a.N / 4 + RN_THREADS - 1) / RN_THREADS;
+      auto kernel = vec <= 1 ? splitk_reduce_norm_kernel<1> : vec <= 2 ? splitk_reduce_norm_kernel<2> : splitk_reduce_norm_kernel<RN_VEC_MAX>;
+      hfee_launch(kernel, dim3((unsigned)a.M), dim3(RN_THREADS), 0, stream, (const float*)a.workspace, (float*)C, a.ldc, a.M, a.N, a.splits,
+                  next->weight, next->eps, next->add_unit, next->out, next->ld_out);
+      return hfee_check_launch("splitk_reduce_norm");
+    }
+  }
   const long long outs = (long long)a.M * ((EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_REGLU) ? a.N / 2 : a.N);
   hfee_launch(splitk_reduce_kernel<EPI, TOut>, dim3((unsigned)((outs + 255) / 256)), dim3(256), 0, stream,
               (const float*)a.workspace, (TOut*)C, a.ldc, a.M, a.N, a.splits);
@@ -319,10 +392,10 @@ int launch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, const SkinnyAr
 
 template <int TN>
 int dispatch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, int out_dtype, int epilogue, const SkinnyArgs& a,
-             int* status, cudaStream_t stream) {
+             int* status, cudaStream_t stream, const NextNorm* next) {
   if (epilogue == EPI_ACCUM) {
     if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_skinny: accumulate needs a float32 output");
-    return launch<TN, EPI_ACCUM, float>(mw, ma, C, a, status, stream);
+    return launch<TN, EPI_ACCUM, float>(mw, ma, C, a, status, stream, next);
   }
   if (epilogue == EPI_GEGLU) {
     if (out_dtype == HFEE_BF16) return launch<TN, EPI_GEGLU, __nv_bfloat16>(mw, ma, C, a, status, stream);
@@ -350,11 +423,9 @@ HFEE_API int hfee_gemm_skinny_splits(int M, int N, int K, long long workspace_fl
   return s;
 }
 
-// A [M,K], W [N,K]: bfloat16, 16-byte aligned, leading dimensions multiples of 8; M <= 64.
-// `workspace` holds splits*M*N floats when the shape is split along K (may be null: no split).
-HFEE_API int hfee_gemm_skinny(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
-                              int out_dtype, int epilogue, int M, int N, int K, float* workspace,
-                              long long workspace_floats, int* status, cudaStream_t stream) {
+namespace {
+int skinny_any(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, int out_dtype, int epilogue, int M, int N,
+               int K, float* workspace, long long workspace_floats, int* status, const NextNorm* next, cudaStream_t stream) {
   if (M == 0 || N == 0) return HFEE_OK;
   HFEE_REQUIRE(M > 0 && M <= 64, "gemm_skinny: M=%d is outside 1..64", M);
   HFEE_REQUIRE(N > 0 && K > 0 && K % 8 == 0, "gemm_skinny: K=%d must be a positive multiple of 8", K);
@@ -371,13 +442,35 @@ HFEE_API int hfee_gemm_skinny(const void* A, long long lda, const void* W, long 
   plan_split(N, K, M, workspace ? workspace_floats : 0, &a.splits, &a.kb_per_split);
   a.ldc = ldc;
   a.workspace = workspace;
+  HFEE_REQUIRE(next == nullptr || a.splits > 1, "gemm_skinny_then_norm: this product is not split along K");
   const int tn = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   CUtensorMap mw, ma;
   int rc = make_map(&mw, W, N, K, ldw, WM);
   if (rc != HFEE_OK) return rc;
   rc = make_map(&ma, A, M, K, lda, tn);
   if (rc != HFEE_OK) return rc;
-  if (tn == 16) return dispatch<16>(mw, ma, C, out_dtype, epilogue, a, status, stream);
-  if (tn == 32) return dispatch<32>(mw, ma, C, out_dtype, epilogue, a, status, stream);
-  return dispatch<64>(mw, ma, C, out_dtype, epilogue, a, status, stream);
+  if (tn == 16) return dispatch<16>(mw, ma, C, out_dtype, epilogue, a, status, stream, next);
+  if (tn == 32) return dispatch<32>(mw, ma, C, out_dtype, epilogue, a, status, stream, next);
+  return dispatch<64>(mw, ma, C, out_dtype, epilogue, a, status, stream, next);
+}
+}  // namespace
+
+// A [M,K], W [N,K]: bfloat16, 16-byte aligned, leading dimensions multiples of 8; M <= 64.
+// `workspace` holds splits*M*N floats when the shape is split along K (may be null: no split).
+HFEE_API int hfee_gemm_skinny(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
+                              int out_dtype, int epilogue, int M, int N, int K, float* workspace,
+                              long long workspace_floats, int* status, cudaStream_t stream) {
+  return skinny_any(A, lda, W, ldw, C, ldc, out_dtype, epilogue, M, N, K, workspace, workspace_floats, status, nullptr, stream);
+}
+
+// C += A W^T in float32 by a product split along K (hfee_gemm_skinny_splits > 1), and out [M, N] bfloat16 = the RMS norm of the new rows.
+HFEE_API int hfee_gemm_skinny_then_norm(const void* A, long long lda, const void* W, long long ldw, float* C, long long ldc, int M, int N, int K,
+                                        float* workspace, long long workspace_floats, const float* weight, float eps, int add_unit,
+                                        void* out, long long ld_out, int* status, cudaStream_t stream) {
+  HFEE_REQUIRE(N % 4 == 0 && N <= 4 * RN_THREADS * RN_VEC_MAX && ldc % 4 == 0 && ld_out % 4 == 0 && ld_out >= N,
+               "gemm_skinny_then_norm: takes rows of at most %d numbers in whole pieces of four (N=%d)", 4 * RN_THREADS * RN_VEC_MAX, N);
+  HFEE_REQUIRE((uintptr_t)C % 16 == 0 && (uintptr_t)workspace % 16 == 0 && (uintptr_t)weight % 16 == 0 && (uintptr_t)out % 8 == 0,
+               "gemm_skinny_then_norm: rows must start on 16-byte boundaries");
+  NextNorm next{weight, eps, add_unit, (__nv_bfloat16*)out, ld_out};
+  return skinny_any(A, lda, W, ldw, C, ldc, HFEE_F32, EPI_ACCUM, M, N, K, workspace, workspace_floats, status, &next, stream);
 }

@@ -46,6 +46,7 @@ _SIGNATURES = {
     "hfee_gemm_ring_supports": [_I, _I, _I, _I],
     "hfee_gemm_ring_then_norm": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _L, _P, _I, _P, _P, _P],
     "hfee_gemm_ring_parts": [_I],
+    "hfee_gemm_skinny_then_norm": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _L, _P, _F, _I, _P, _L, _P, _P],
     "hfee_gemm_stream_scaled": [_P, _L, _P, _I, _F, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P],
     "hfee_attention_tc": [_P, _I, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "hfee_attention_tc_general": [_P, _I, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _F, _P, _F, _P, _P],
@@ -668,6 +669,24 @@ def gemm_stream_scaled(rows: torch.Tensor, sums: torch.Tensor, eps: float, w: to
                                        _stream()), lib)
 
 
+def gemm_skinny_then_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, eps: float, add_unit: bool,
+                          normed: torch.Tensor) -> None:
+    """out += a @ w.T in float32 (:func:`gemm_skinny`, split along K) and ``normed`` = bf16 of the RMS norm of the new rows."""
+    lib = library()
+    m, k = a.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and a.dtype == w.dtype == normed.dtype == torch.bfloat16 and out.dtype == weight.dtype == torch.float32
+    assert tuple(out.shape) == tuple(normed.shape) == (m, n) and weight.numel() == n
+    ws = _skinny_workspace()
+    _check(lib.hfee_gemm_skinny_then_norm(a.data_ptr(), _rows(a, "gemm a"), w.data_ptr(), _rows(w, "gemm w"), out.data_ptr(),
+                                          _rows(out, "gemm out"), m, n, k, ws.data_ptr(), ws.numel(), weight.data_ptr(), float(eps),
+                                          int(add_unit), normed.data_ptr(), _rows(normed, "normed"), _status().data_ptr(), _stream()), lib)
+    count_launches(1)
+
+
+NORM_BEHIND_SKINNY_MAX_WIDTH = 8192      # a block keeps a row in registers
+
+
 def _leads_to_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, then) -> bool:
     """out += a @ w.T together with the norm ``then`` that reads ``out`` (parts/norm.py: LazyNormed); False, and nothing done, where the
     plain product and a norm of its own are to run."""
@@ -679,6 +698,13 @@ def _leads_to_norm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, then) ->
     (m, k), n = a.shape, w.shape[0]
     if then.sums is not None and _ring_rule(m, n, k, EPI_ACCUM):
         then.scaled = gemm_ring_then_norm(a, w, out, weight, add_unit, then.buffer, then.sums)
+        return True
+    if (m > STREAM_BEST_TOKENS and USE_TCGEN05 and _skinny_rule(m, n, k, EPI_ACCUM, out, a, w) and n % 4 == 0
+            and n <= NORM_BEHIND_SKINNY_MAX_WIDTH and weight.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and _rows(out, "out") % 4 == 0
+            and then.buffer.data_ptr() % 8 == 0 and _rows(then.buffer, "normed") % 4 == 0
+            and library().hfee_gemm_skinny_splits(m, n, k, SKINNY_WS_FLOATS) > 1):
+        gemm_skinny_then_norm(a, w, out, weight, eps, add_unit, then.buffer)
+        then.in_buffer()
         return True
     return False
 
@@ -761,13 +787,17 @@ def _small_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
         gemm_ring(a, w, out, epilogue)
     elif m <= STREAM_BEST_TOKENS or not USE_TCGEN05:
         gemm_stream(a, w, out, epilogue)
-    elif m > 32 and 64 * 128 <= n <= 256 * 128 and a.shape[1] <= 4096 and _tensor_core_ok(a, w) and (
-            epilogue not in EPI_GATED or out.dtype == torch.bfloat16):
-        # 64-256 narrow tiles of the large-tile kernel fill the SMs about once, and their epilogues are cheaper than the
-        # swapped one: measured at 64 tokens, N = 16,384, K = 2,048: 16.3 us against 18.9 us
-        gemm_tcgen05(a, w, out, epilogue)
-    else:
+    elif _skinny_rule(m, n, a.shape[1], epilogue, out, a, w):
         gemm_skinny(a, w, out, epilogue)
+    else:
+        gemm_tcgen05(a, w, out, epilogue)
+
+
+def _skinny_rule(m: int, n: int, k: int, epilogue: int, out: torch.Tensor, a: torch.Tensor, w: torch.Tensor) -> bool:
+    """More than STREAM_BEST_TOKENS tokens: the swapped-operand kernel, unless 64-256 narrow tiles of the large-tile kernel fill the SMs
+    about once: their epilogues are cheaper than the swapped one (64 tokens, N = 16,384, K = 2,048: 16.3 us against 18.9 us)."""
+    return not (m > 32 and 64 * 128 <= n <= 256 * 128 and k <= 4096 and _tensor_core_ok(a, w)
+                and (epilogue not in EPI_GATED or out.dtype == torch.bfloat16))
 
 
 def _ring_rule(m: int, n: int, k: int, epilogue: int) -> bool:

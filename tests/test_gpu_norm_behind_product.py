@@ -1,4 +1,5 @@
-"""A norm that leaves with the accumulating product in front of it, of a few tokens: the product behind it scales its results."""
+"""A norm that leaves with the accumulating product in front of it: few tokens (the product behind it scales its results) and
+products split along K (the kernel that adds the parts norms the row)."""
 import pytest
 import torch
 
@@ -64,6 +65,20 @@ def test_few_tokens(m, n, k, add_unit):
         assert (out.double() - y).norm(dim=1).le(8e-3 * y.norm(dim=1)).all()
     ops.check_status()
     assert (lazy.tensor().double() - normed).norm(dim=1).le(4e-3 * normed.norm(dim=1)).all() and lazy.scaled is None
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 2048, 8192), (64, 2048, 2048), (33, 132, 1024), (20, 8192, 4096), (64, 4100, 8192), (48, 128, 512)])
+@pytest.mark.parametrize("add_unit", [False, True])
+def test_products_split_along_k(m, n, k, add_unit):
+    from hfee_b200.kernels import ops
+    a, w, residual, lazy, want, normed = _case(m, n, k, add_unit)
+    last = residual[m].clone()
+    splits = ops.library().hfee_gemm_skinny_splits(m, n, k, ops.SKINNY_WS_FLOATS)
+    ops.linear_then_norm(a, w, residual[:m], lazy)
+    ops.check_status()
+    assert (lazy._done or splits == 1 or not ops._skinny_rule(m, n, k, ops.EPI_ACCUM, residual, a, w)) and bool((residual[m] == last).all())
+    assert (residual[:m].double() - want).norm(dim=1).le(1e-5 * want.norm(dim=1)).all()
+    assert (lazy.tensor().double() - normed).norm(dim=1).le(4e-3 * normed.norm(dim=1)).all()       # rounded to bfloat16: 2^-9 an element
 
 
 def test_what_has_no_such_kernel_takes_the_plain_product():
