@@ -59,7 +59,7 @@ attention_sigmoid_mma_kernel(const bf16* __restrict__ q, long long ld_q, const b
   if (window > 0) key_lo = max(key_lo, p_first + 1 - window);
   // A block's keys and values wait in registers for the block before to be used up; the first block's are asked for before the wait for
   // the kernel in front where earlier steps wrote them all (a decode step sees a block or two, and their trip to memory was half of it:
-  // 9.5 -> 6.6 us; a prompt of 500 tokens 34 -> 29).
+  // 9.5 -> 6.6 us; prompts of 2,000 tokens 34 -> 29).
   constexpr int PIECES = SA_KEYS * (HD / 8) / (SA_WARPS * 32);
   static_assert(PIECES * SA_WARPS * 32 == SA_KEYS * (HD / 8) && (SA_WARPS * 32) % SA_KEYS == 0, "whole pieces, one key a thread");
   uint4 k_next[PIECES], v_next[PIECES];

@@ -5,9 +5,11 @@
 // bytes in flight: a TMA warp streams 128 x 64 weight tiles (and the small token tile) through a
 // ring of 8-10 shared-memory stages, far more than registers could hold, while one thread issues
 // the MMAs into tensor memory.  The grid is persistent over work items (weight tile, K split);
-// K is split among CTAs when there are fewer weight tiles than SMs.  A split writes its partial
-// tile to a float32 workspace and a second kernel adds the splits in split order, so the sum
-// order is fixed; without a split the epilogue writes C directly (transposed: a thread holds one
+// K is split among CTAs when there are fewer weight tiles than SMs.  The splits of a tile are a
+// cluster where 2, 4 or 8 of them nearly fill the chip: they leave their partial tiles in shared
+// memory, and each adds a share of the tile's tokens from all of them.  Otherwise a split writes
+// its partial tile to a float32 workspace and a second kernel adds them.  Either way in split
+// order, so the sum order is fixed; without a split the epilogue writes C directly (transposed: a thread holds one
 // weight row for all tokens).  Epilogues: store, accumulate into float32 C, SwiGLU over rows
 // interleaved [4 gate | 4 up].  Every barrier wait is bounded (see tcgen05.cuh).
 // Reference: out[t*Rows+r] = Dot(W[r,:], x[t,:]), hostfog/hfee internal/ggml/ops.go:54-70
@@ -47,7 +49,18 @@ struct SkinnyArgs {
   int w_tiles, splits, kb_per_split, k_blocks;
   long long ldc;
   float* workspace;        // [splits][M][N] float32 partial tiles (splits > 1)
+  int cluster;             // the splits of a tile are a cluster: CTA splits * tile + split, one item each
 };
+
+__device__ __forceinline__ float4 ld_peer4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void skinny_cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // One 16-token column group of a thread's weight row: direct epilogue or partial write.
 template <int EPI, typename TOut, int COLS>
@@ -131,7 +144,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       // ring (all stages are free) are requested before the wait, their token tiles after it.
       uint32_t pre = 0;
       for (int i = blockIdx.x; i < items && pre < (uint32_t)STAGES; i += gridDim.x) {
-        const int n0 = (i % a.w_tiles) * WM, split = i / a.w_tiles;
+        const int n0 = (a.cluster ? i / a.splits : i % a.w_tiles) * WM, split = a.cluster ? i % a.splits : i / a.w_tiles;
         const int kb0 = split * a.kb_per_split, kb1 = min(a.k_blocks, kb0 + a.kb_per_split);
         for (int kb = kb0; kb < kb1 && pre < (uint32_t)STAGES; ++kb, ++pre) {
           mbar_expect_tx(&full_bar[pre], Cfg::STAGE_BYTES);
@@ -142,7 +155,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       uint32_t it = 0;
       bool ok = true;
       for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
-        const int n0 = (i % a.w_tiles) * WM, split = i / a.w_tiles;
+        const int n0 = (a.cluster ? i / a.splits : i % a.w_tiles) * WM, split = a.cluster ? i % a.splits : i / a.w_tiles;
         const int kb0 = split * a.kb_per_split, kb1 = min(a.k_blocks, kb0 + a.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
@@ -165,7 +178,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     bool ok = true;
     const uint64_t desc0 = make_desc(smem_u32(tiles));
     for (int i = blockIdx.x; i < items && ok; i += gridDim.x, ++acc_it) {
-      const int split = i / a.w_tiles;
+      const int split = a.cluster ? i % a.splits : i / a.w_tiles;
       const int kb0 = split * a.kb_per_split, kb1 = min(a.k_blocks, kb0 + a.kb_per_split);
       const uint32_t buf = acc_it & 1u;
       ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty_bar[buf], ((acc_it >> 1) & 1u) ^ 1u, &abort_flag));
@@ -196,7 +209,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     uint32_t acc_it = 0;
     bool ok = true;
     for (int i = blockIdx.x; i < items && ok; i += gridDim.x, ++acc_it) {
-      const int n0 = (i % a.w_tiles) * WM, split = i / a.w_tiles;
+      const int n0 = (a.cluster ? i / a.splits : i % a.w_tiles) * WM, split = a.cluster ? i % a.splits : i / a.w_tiles;
       const uint32_t buf = acc_it & 1u;
       ok = mbar_wait(&tmem_full_bar[buf], (acc_it >> 1) & 1u, &abort_flag);
       tc_fence_after();
@@ -208,7 +221,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t v[16];
         tc_ld16(taddr + (uint32_t)c0, v);
         tc_wait_ld();
-        write_columns<EPI, TOut, 16>(v, c0, w_row, lane, split, C, a);
+        if (a.cluster) {       // all products of this CTA's one tile are done: the ring's memory takes the partial tile, [token][row]
+          float* part = reinterpret_cast<float*>(tiles) + quad * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) part[(c0 + j) * WM] = __uint_as_float(v[j]);
+        } else {
+          write_columns<EPI, TOut, 16>(v, c0, w_row, lane, split, C, a);
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -216,6 +235,33 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
   }
   pdl_launch_dependents();
+  if (EPI <= EPI_ACCUM && a.cluster) {
+    skinny_cluster_sync();
+    const int n0 = (int)blockIdx.x / a.splits * WM, rank = (int)blockIdx.x % a.splits;
+    const int share = (a.M + a.splits - 1) / a.splits, t0 = rank * share, t1 = min(a.M, t0 + share);
+    for (int e = threadIdx.x; e < (t1 - t0) * (WM / 4); e += SK_THREADS) {
+      const int t = t0 + e / (WM / 4), row = e % (WM / 4) * 4;
+      uint32_t mine = smem_u32(reinterpret_cast<float*>(tiles) + t * WM + row);
+      float4 part[8], v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        uint32_t at = 0;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(q < a.splits ? q : 0));
+        part[q] = q < a.splits ? ld_peer4(at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) { v.x += part[q].x; v.y += part[q].y; v.z += part[q].z; v.w += part[q].w; }
+      const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (n0 + row + j >= a.N) continue;
+        TOut* dst = C + (long long)t * a.ldc + n0 + row + j;
+        if constexpr (EPI == EPI_ACCUM) *dst = from_f32<TOut>(to_f32<TOut>(*dst) + x[j]);
+        else *dst = from_f32<TOut>(x[j]);
+      }
+    }
+    skinny_cluster_sync();                 // no CTA of the cluster ends while another reads its tile
+  }
 
   tc_fence_before();
   __syncthreads();
@@ -371,10 +417,10 @@ int launch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, const SkinnyAr
   }
   const int items = a.w_tiles * a.splits;
   const int sms = device_sms();
-  hfee_launch(gemm_skinny_kernel<TN, EPI, TOut>, dim3((unsigned)(items < sms ? items : sms)), dim3(SK_THREADS), Cfg::SMEM,
-              stream, mw, ma, (TOut*)C, a, status);
+  hfee_launch_with(hfee_carveout(), a.cluster ? dim3((unsigned)a.splits, 1, 1) : dim3(0, 0, 0), gemm_skinny_kernel<TN, EPI, TOut>,
+                   dim3((unsigned)(items < sms ? items : sms)), dim3(SK_THREADS), Cfg::SMEM, stream, mw, ma, (TOut*)C, a, status);
   int rc = hfee_check_launch("gemm_skinny");
-  if (rc != HFEE_OK || a.splits == 1) return rc;
+  if (rc != HFEE_OK || a.splits == 1 || a.cluster) return rc;
   if constexpr (EPI == EPI_ACCUM) {
     if (next != nullptr) {
       const int vec = (a.N / 4 + RN_THREADS - 1) / RN_THREADS;
@@ -415,6 +461,22 @@ int dispatch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, int out_dtyp
 
 }  // namespace
 
+namespace {
+// Splits of a tile that are a cluster, or 0: the most of 8, 4 and 2 that the chip holds, with at least 4 K blocks each, if that is at least
+// three fifths of the SMs (64 tokens, N = 3,072, K = 2,048: 96 CTAs that add their own tiles 7.4 us, 144 and a kernel behind them 10.2).
+int cluster_splits(int N, int K, int epilogue) {
+  if (epilogue != EPI_STORE && epilogue != EPI_ACCUM) return 0;
+  const int w_tiles = (N + WM - 1) / WM, k_blocks = (K + BK - 1) / BK, sms = device_sms();
+  for (int s = 8; s >= 2; s /= 2)
+    if (w_tiles * s <= sms && k_blocks >= 4 * s)       // and no split without K blocks
+      return w_tiles * s * 5 >= sms * 3 && (s - 1) * ((k_blocks + s - 1) / s) < k_blocks ? s : 0;
+  return 0;
+}
+}  // namespace
+
+// 1 when hfee_gemm_skinny adds the splits of this shape in one launch.
+HFEE_API int hfee_gemm_skinny_in_cluster(int N, int K, int epilogue) { return cluster_splits(N, K, epilogue) > 0 ? 1 : 0; }
+
 // How many K splits hfee_gemm_skinny uses for this shape given `workspace_floats` of workspace
 // (1 = none, no workspace needed, one launch; otherwise two launches).
 HFEE_API int hfee_gemm_skinny_splits(int M, int N, int K, long long workspace_floats) {
@@ -442,6 +504,14 @@ int skinny_any(const void* A, long long lda, const void* W, long long ldw, void*
   plan_split(N, K, M, workspace ? workspace_floats : 0, &a.splits, &a.kb_per_split);
   a.ldc = ldc;
   a.workspace = workspace;
+  a.cluster = 0;
+  if (next == nullptr) {
+    if (const int s = cluster_splits(N, K, epilogue)) {
+      a.kb_per_split = (a.k_blocks + s - 1) / s;
+      a.splits = s;
+      a.cluster = 1;
+    }
+  }
   HFEE_REQUIRE(next == nullptr || a.splits > 1, "gemm_skinny_then_norm: this product is not split along K");
   const int tn = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   CUtensorMap mw, ma;

@@ -42,6 +42,7 @@ _SIGNATURES = {
     "hfee_gemm_tcgen05_rope_supports": [_I, _I],
     "hfee_gemm_skinny": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "hfee_gemm_skinny_splits": [_I, _I, _I, _L],
+    "hfee_gemm_skinny_in_cluster": [_I, _I, _I],
     "hfee_gemm_ring": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _P, _P],
     "hfee_gemm_ring_supports": [_I, _I, _I, _I],
     "hfee_gemm_ring_then_norm": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _P, _L, _P, _I, _P, _P, _P],
@@ -768,7 +769,7 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
     _check(lib.hfee_gemm_skinny(a.data_ptr(), _rows(a, "gemm a"), w.data_ptr(), _rows(w, "gemm w"), out.data_ptr(),
                                 _rows(out, "gemm out"), _dt(out), epilogue, m, n, k, ws.data_ptr(), ws.numel(),
                                 _status().data_ptr(), _stream()), lib)
-    if lib.hfee_gemm_skinny_splits(m, n, k, ws.numel()) > 1:
+    if lib.hfee_gemm_skinny_splits(m, n, k, ws.numel()) > 1 and not lib.hfee_gemm_skinny_in_cluster(n, k, epilogue):
         count_launches(1)
 
 
@@ -2096,7 +2097,7 @@ def qk_norm_rope_cache(qk: torch.Tensor, q_weight: Optional[torch.Tensor], k_wei
         assert v_pool is None or (v_pool.dtype == qk.dtype and v_pool.is_contiguous() and v_pool.shape == k_pool.shape)
     assert cs is None or (cs.dtype == torch.float32 and cs.is_contiguous() and cs.numel() == n * rope_dim)
     if v_pool is not None and (heads + 2 * kv_heads) * head_dim * 4 <= PREPARE_MAX_BYTES:
-        # the kernels of attention_prepare take a row in 16-byte pieces: in a decode step 5.9 -> 4.0 us, in a prompt of 500 tokens 21 -> 14.7
+        # the kernels of attention_prepare take a row in 16-byte pieces: in a decode step 5.9 -> 4.0 us, in prompts of 2,000 tokens 21 -> 14.7
         _check(lib.hfee_attention_prepare(qk.data_ptr(), _rows(qk, "qk"), _dt(qk), n, 0, heads * head_dim,
                                           heads * head_dim if v_offset < 0 else int(v_offset), None, None, None, _ptr(q_weight), _ptr(k_weight),
                                           float(eps), _ptr(cs), int(rope_dim) if cs is not None else 0, 0, positions.data_ptr(),

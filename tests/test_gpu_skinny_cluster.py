@@ -1,0 +1,27 @@
+"""Products of 17 to 64 tokens whose splits along K are a cluster and add their tiles themselves."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# clusters of 8, 4 and 2; rows that end inside a tile and a piece of four, tokens fewer than a cluster's CTAs and no multiple of them
+@pytest.mark.parametrize("m,n,k", [(64, 2048, 2048), (17, 2047, 2048), (33, 3072, 2048), (5, 4601, 1032), (64, 6149, 2048), (3, 1925, 8192)])
+@pytest.mark.parametrize("epilogue", ["store", "accumulate"])
+def test_cluster_of_splits(m, n, k, epilogue):
+    from hfee_b200.kernels import ops
+    g = torch.Generator().manual_seed(m + n + k)
+    a, w = (torch.randn(r, k, generator=g).to(torch.bfloat16).to(DEV) for r in (m, n))
+    epi = ops.EPI_STORE if epilogue == "store" else ops.EPI_ACCUM
+    assert ops.library().hfee_gemm_skinny_in_cluster(n, k, epi)
+    before = ops.launch_count()
+    want = a.double() @ w.double().t()
+    for dtype in (torch.float32, torch.bfloat16) if epilogue == "store" else (torch.float32,):
+        out = torch.full((m + 1, n), 3.0, dtype=dtype, device=DEV)
+        ops.gemm_skinny(a, w, out[:m], epi)
+        ops.check_status()
+        ref = want if epilogue == "store" else want + 3.0
+        assert (out[:m].double() - ref).norm() <= (1e-5 if dtype == torch.float32 else 4e-3) * ref.norm()
+        assert bool((out[m] == 3.0).all())
+    assert ops.launch_count() == before + (2 if epilogue == "store" else 1)
