@@ -73,6 +73,9 @@ struct RecurrenceArgs {
   const float* a_log;
   const float* d_skip;
   int qk_share;
+  // the states were written before the kernel in front of this one began (an engine step: a copy of the step's integers lies between
+  // two steps): the walk asks for them under that kernel's end (a decode step of two requests: 5.2 -> 3.6 us)
+  int settled;
 };
 
 __device__ __forceinline__ float softplus_f32(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
@@ -126,9 +129,7 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
     count = min(GC_T, count - run * GC_T);
   }
   const int slot = p.slots[req];
-  pdl_wait();
-  pdl_launch_dependents();
-  if (count <= 0) return;
+  if (PASS != PASS_WHOLE || !p.settled) pdl_wait();   // a run's states are the kernel in front's
 
   // where the state comes from and goes to: the request's slot, or the run's place in the workspace
   const long long place = PASS == PASS_WHOLE ? (long long)slot * heads + head : (long long)blockIdx.y * heads + head;
@@ -143,7 +144,7 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int row = g * ROWS + 2 * i + e;
-        at[e] = (PASS != PASS_LOCAL && row < dim && col + c * GR_LANES < vdim) ? S_g[(long long)row * vdim + col + c * GR_LANES] : 0.f;
+        at[e] = (PASS != PASS_LOCAL && count > 0 && row < dim && col + c * GR_LANES < vdim) ? S_g[(long long)row * vdim + col + c * GR_LANES] : 0.f;
       }
       S[c][i] = pair_of(at[0], at[1]);
     }
@@ -151,9 +152,12 @@ gated_recurrence_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   float decay_own = 1.f;                              // PASS_LOCAL: product of the run's decays of that row
   const int own_row = g * ROWS + (j < ROWS ? j : 0);
   if constexpr (MODE == MODE_EXP_GATES) {
-    if (PASS != PASS_LOCAL && j < ROWS && own_row < dim) n_own = n_g[own_row];
-    if (PASS == PASS_WHOLE && tid == 0) m_cur = p.max_state[(long long)slot * heads + head];
+    if (PASS != PASS_LOCAL && count > 0 && j < ROWS && own_row < dim) n_own = n_g[own_row];
+    if (PASS == PASS_WHOLE && count > 0 && tid == 0) m_cur = p.max_state[(long long)slot * heads + head];
   }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (count <= 0) return;
   // A block has SHARE threads for each (padded) key channel of a staged token: a thread brings its channel of every SHARE-th
   // token of a stage, and its share of the stage's values.
   const int ch = SHARE == 1 ? tid : tid % dim_pad, first_t = SHARE == 1 ? 0 : tid / dim_pad;
@@ -562,7 +566,7 @@ HFEE_API int hfee_gated_recurrence(int mode, const void* q, const void* k, const
                                    const float* pre, long long ld_pre, const float* bias, float p0, float q_scale,
                                    float* state, float* norm_state, float* max_state, const int* cu_tokens,
                                    const int* slots, float* out, long long ld_o, int requests, int heads, int dim,
-                                   int vdim, int write_state, cudaStream_t stream) {
+                                   int vdim, int write_state, int settled, cudaStream_t stream) {
   if (requests == 0) return HFEE_OK;
   HFEE_REQUIRE(mode == MODE_CHANNEL_DECAY || mode == MODE_EXP_GATES, "gated_recurrence: unknown mode %d", mode);
   HFEE_REQUIRE(heads > 0 && dim > 0 && vdim > 0 && dim <= GR_MAX_DIM, "gated_recurrence: key size %d is outside 1..%d", dim, GR_MAX_DIM);
@@ -573,6 +577,7 @@ HFEE_API int hfee_gated_recurrence(int mode, const void* q, const void* k, const
   HFEE_REQUIRE(p0 > 0.f, "gated_recurrence: the temperature or cap must be positive");
   RecurrenceArgs p{ld, pre, ld_pre, bias, p0, q_scale, state, norm_state, max_state, cu_tokens, slots, out, ld_o, heads, dim, vdim, write_state,
                    requests, nullptr, nullptr, nullptr, nullptr, 0, 0};
+  p.settled = settled;
   if (dtype == HFEE_F32) return launch_recurrence<float, PASS_WHOLE>(mode, q, k, v, p, requests, stream);
   if (dtype == HFEE_BF16) return launch_recurrence<__nv_bfloat16, PASS_WHOLE>(mode, q, k, v, p, requests, stream);
   return hfee_fail(HFEE_ERR_ARG, "gated_recurrence: unknown dtype %d", dtype);
@@ -624,14 +629,14 @@ HFEE_API int hfee_head_scan(const void* x, const void* bmat, const void* cmat, l
                             int dtype, const float* dt_bias, const float* a_log, const float* d_skip, float* state,
                             const int* cu_tokens, const int* slots, float* out, long long ld_o, int requests, int n_tokens,
                             int heads, int groups, int state_dim, int vdim, int write_state, float* workspace,
-                            long long workspace_floats, cudaStream_t stream) {
+                            long long workspace_floats, int settled, cudaStream_t stream) {
   if (requests == 0 || n_tokens == 0) return HFEE_OK;
   HFEE_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0 && vdim > 0, "head_scan: heads %d must be a multiple of groups %d", heads, groups);
   HFEE_REQUIRE(state_dim > 0 && state_dim <= GR_MAX_DIM, "head_scan: state size %d is outside 1..%d", state_dim, GR_MAX_DIM);
   HFEE_REQUIRE(requests <= 65535 && (vdim + GR_COLS - 1) / GR_COLS <= 65535, "head_scan: too many requests or columns for one grid");
   HFEE_REQUIRE(ld_o >= (long long)heads * vdim && ld_step >= heads, "head_scan: a row stride is too small");
   RecurrenceArgs p{ld, nullptr, 0, dt_bias, 1.f, 1.f, state, nullptr, nullptr, cu_tokens, slots, out, ld_o, heads, state_dim, vdim, write_state,
-                   requests, nullptr, nullptr, nullptr, nullptr, 0, 0, step, ld_step, a_log, d_skip, heads / groups};
+                   requests, nullptr, nullptr, nullptr, nullptr, 0, 0, step, ld_step, a_log, d_skip, heads / groups, settled};
   if (workspace == nullptr) {
     if (dtype == HFEE_F32) return launch_recurrence<float, PASS_WHOLE>(MODE_STEP, cmat, bmat, x, p, requests, stream);
     if (dtype == HFEE_BF16) return launch_recurrence<__nv_bfloat16, PASS_WHOLE>(MODE_STEP, cmat, bmat, x, p, requests, stream);

@@ -109,6 +109,7 @@ class ModelRunner:
         cache.sync()
         step = Step(entries, cache.length, self.buffers)
         step.feedback = self.feedback
+        step.states_settled = True             # the upload lies between what the last step launched and this one
         if self.device.type == "cuda":
             # in effect until the next step: what runs between steps (sampling) belongs to the chain too
             from ..kernels import ops

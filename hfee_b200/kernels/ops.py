@@ -61,7 +61,7 @@ _SIGNATURES = {
     "hfee_attention_sigmoid_mma_supports": [_I, _I, _I],
     "hfee_short_conv": [_P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
     "hfee_short_conv_launches": [_I, _I, _I],
-    "hfee_linear_attention": [_P, _P, _P, _L, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
+    "hfee_linear_attention": [_P, _P, _P, _L, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P],
     "hfee_linear_attention_chunked": [_P, _P, _P, _L, _I, _P, _P, _P, _P, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "hfee_rmsnorm_add": [_P, _L, _P, _P, _I, _I, _F, _I, _P, _L, _I, _P],
     "hfee_rmsnorm_add_norm": [_P, _L, _P, _P, _I, _I, _F, _I, _P, _F, _I, _P, _L, _I, _P],
@@ -116,7 +116,7 @@ _SIGNATURES = {
     "hfee_gate_parts_norm": [_P, _L, _P, _L, _P, _F, _P, _L, _I, _I, _I, _F, _I, _P],
     "hfee_head_scan_mma": [_P, _P, _P, _L, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _L, _P],
     "hfee_head_scan_mma_supports": [_I, _I],
-    "hfee_head_scan": [_P, _P, _P, _L, _P, _L, _I, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _L, _P],
+    "hfee_head_scan": [_P, _P, _P, _L, _P, _L, _I, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _L, _I, _P],
     "hfee_attention_prepare": [_P, _L, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _F, _P, _I, _I, _P, _P, _P, _L, _P, _P, _P, _I, _I,
                                _I, _I, _I, _I, _P, _L, _I, _F, _P],
     "hfee_attention_simt_capped": [_P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P, _L, _I,
@@ -125,7 +125,7 @@ _SIGNATURES = {
                                  _P, _P, _F, _P, _I, _P],
     "hfee_attention_mma_general": [_P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P, _F, _I,
                                    _I, _F, _I, _P, _P],
-    "hfee_gated_recurrence": [_I, _P, _P, _P, _L, _I, _P, _L, _P, _F, _F, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _P],
+    "hfee_gated_recurrence": [_I, _P, _P, _P, _L, _I, _P, _L, _P, _F, _F, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
     "hfee_gated_recurrence_chunked": [_I, _P, _P, _P, _L, _I, _P, _L, _P, _F, _F, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P, _L, _P],
     "hfee_head_norm_gate_scaled": [_P, _L, _P, _I, _F, _P, _L, _P, _L, _I, _I, _I, _I, _F, _I, _P],
     "hfee_moe_combine_extra": [_P, _P, _P, _I, _I, _P, _I, _I, _P, _P, _L, _P],
@@ -1084,6 +1084,12 @@ def short_conv(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor, step,
 LINEAR_ATTENTION_CHUNKED_MIN = 8
 
 
+def _settled(step) -> int:
+    """1 in a step of the runner: the requests' states were written before the kernel in front began, since the copy of a step's integers
+    lies between two steps.  Whoever calls an op by itself may have called it just before, on the same state."""
+    return int(getattr(step, "states_settled", False))
+
+
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                      step, out: torch.Tensor, heads: int, dim: int, vdim: int, activation: str = "none",
                      write_state: bool = True, workspace: Optional[torch.Tensor] = None,
@@ -1116,7 +1122,7 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
         return
     _check(lib.hfee_linear_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), _dt(q), decay.data_ptr(),
                                      state.data_ptr(), step.cu_tokens.data_ptr(), step.slots.data_ptr(), out.data_ptr(),
-                                     _rows(out, "out"), step.r, heads, dim, vdim, act, int(write_state), _stream()), lib)
+                                     _rows(out, "out"), step.r, heads, dim, vdim, act, int(write_state), _settled(step), _stream()), lib)
 
 
 def linear_attention_workspace(requests: int, tokens: int, heads: int, dim: int, vdim: int) -> int:
@@ -2299,7 +2305,7 @@ def gated_recurrence(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
     _check(lib.hfee_gated_recurrence(int(mode), q.data_ptr(), k.data_ptr(), v.data_ptr(), ld, _dt(q), pre.data_ptr(), pre.stride(0),
                                      _ptr(bias), float(p0), float(q_scale), state.data_ptr(), _ptr(norm_state), _ptr(max_state),
                                      step.cu_tokens.data_ptr(), step.slots.data_ptr(), out.data_ptr(), _rows(out, "out"), step.r,
-                                     heads, dim, vdim, int(write_state), _stream()), lib)
+                                     heads, dim, vdim, int(write_state), _settled(step), _stream()), lib)
 
 
 HEAD_SCAN_RUNS_MIN = 65            # from this many new tokens of one request on, runs of 64 tokens work side by side
@@ -2348,7 +2354,8 @@ def head_scan(x: torch.Tensor, bmat: torch.Tensor, cmat: torch.Tensor, step_size
     _check(lib.hfee_head_scan(x.data_ptr(), bmat.data_ptr(), cmat.data_ptr(), ld, step_size.data_ptr(), _rows(step_size, "step"), _dt(x),
                               dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), step.cu_tokens.data_ptr(),
                               step.slots.data_ptr(), out.data_ptr(), _rows(out, "out"), step.r, n, heads, groups, state_dim, vdim,
-                              int(write_state), _ptr(workspace) if runs else None, workspace.numel() if runs else 0, _stream()), lib)
+                              int(write_state), _ptr(workspace) if runs else None, workspace.numel() if runs else 0, _settled(step),
+                              _stream()), lib)
     if runs:
         count_launches(3)
 
