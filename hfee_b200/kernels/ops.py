@@ -886,8 +886,9 @@ def attention_splits(requests: int, kv_heads: int, max_context: int, sms: Option
 
     One or two requests take clusters of eight instead, which need no combine kernel (decode step of one request at 1,024 keys 684 us
     against 706 with 32 splits and the combine kernel, at 3,900 keys 736 against 725; of two requests at 2,048 keys 710 against 720;
-    clusters of 16 at 1,024 / 3,900: 690 / 710, and at 80 keys no faster than the combine kernel, which eights beat by 12 us).  More clusters than the chip holds at once wait for room among the kernels around them: eight
-    requests at 2,048 keys 848 us against 833, 64 requests 1,565 against 1,532."""
+    clusters of 16 at 1,024 / 3,900: 690 / 710, and at 80 keys no faster than the combine kernel, which eights beat by 12 us).  More
+    clusters than the chip holds at once wait for room among the kernels around them: eight requests at 2,048 keys 848 us against 833, 64
+    requests 1,565 against 1,532."""
     pairs = max(1, requests * kv_heads)
     per_sm = 2 if pairs <= FEW_PAIRS else 4
     sms = sms or sm_count()
