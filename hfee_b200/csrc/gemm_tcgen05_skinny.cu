@@ -105,7 +105,8 @@ __device__ __forceinline__ void write_columns(const uint32_t (&v)[COLS], int tok
   }
 }
 
-template <int TN, int EPI, typename TOut>
+// CLUSTER: the splits of a tile are a cluster (a kernel of its own: the test for it in the other cost them 0.2 us).
+template <int TN, int EPI, typename TOut, bool CLUSTER>
 __global__ void __launch_bounds__(SK_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                    TOut* __restrict__ C, SkinnyArgs a, int* __restrict__ status) {
@@ -144,7 +145,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       // ring (all stages are free) are requested before the wait, their token tiles after it.
       uint32_t pre = 0;
       for (int i = blockIdx.x; i < items && pre < (uint32_t)STAGES; i += gridDim.x) {
-        const int n0 = (a.cluster ? i / a.splits : i % a.w_tiles) * WM, split = a.cluster ? i % a.splits : i / a.w_tiles;
+        const int n0 = (CLUSTER ? i / a.splits : i % a.w_tiles) * WM, split = CLUSTER ? i % a.splits : i / a.w_tiles;
         const int kb0 = split * a.kb_per_split, kb1 = min(a.k_blocks, kb0 + a.kb_per_split);
         for (int kb = kb0; kb < kb1 && pre < (uint32_t)STAGES; ++kb, ++pre) {
           mbar_expect_tx(&full_bar[pre], Cfg::STAGE_BYTES);
@@ -155,7 +156,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       uint32_t it = 0;
       bool ok = true;
       for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
-        const int n0 = (a.cluster ? i / a.splits : i % a.w_tiles) * WM, split = a.cluster ? i % a.splits : i / a.w_tiles;
+        const int n0 = (CLUSTER ? i / a.splits : i % a.w_tiles) * WM, split = CLUSTER ? i % a.splits : i / a.w_tiles;
         const int kb0 = split * a.kb_per_split, kb1 = min(a.k_blocks, kb0 + a.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
@@ -178,7 +179,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     bool ok = true;
     const uint64_t desc0 = make_desc(smem_u32(tiles));
     for (int i = blockIdx.x; i < items && ok; i += gridDim.x, ++acc_it) {
-      const int split = a.cluster ? i % a.splits : i / a.w_tiles;
+      const int split = CLUSTER ? i % a.splits : i / a.w_tiles;
       const int kb0 = split * a.kb_per_split, kb1 = min(a.k_blocks, kb0 + a.kb_per_split);
       const uint32_t buf = acc_it & 1u;
       ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty_bar[buf], ((acc_it >> 1) & 1u) ^ 1u, &abort_flag));
@@ -209,7 +210,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     uint32_t acc_it = 0;
     bool ok = true;
     for (int i = blockIdx.x; i < items && ok; i += gridDim.x, ++acc_it) {
-      const int n0 = (a.cluster ? i / a.splits : i % a.w_tiles) * WM, split = a.cluster ? i % a.splits : i / a.w_tiles;
+      const int n0 = (CLUSTER ? i / a.splits : i % a.w_tiles) * WM, split = CLUSTER ? i % a.splits : i / a.w_tiles;
       const uint32_t buf = acc_it & 1u;
       ok = mbar_wait(&tmem_full_bar[buf], (acc_it >> 1) & 1u, &abort_flag);
       tc_fence_after();
@@ -221,7 +222,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t v[16];
         tc_ld16(taddr + (uint32_t)c0, v);
         tc_wait_ld();
-        if (a.cluster) {       // all products of this CTA's one tile are done: the ring's memory takes the partial tile, [token][row]
+        if constexpr (CLUSTER) {       // all products of this CTA's one tile are done: the ring's memory takes the partial tile, [token][row]
           float* part = reinterpret_cast<float*>(tiles) + quad * 32 + lane;
 #pragma unroll
           for (int j = 0; j < 16; ++j) part[(c0 + j) * WM] = __uint_as_float(v[j]);
@@ -235,7 +236,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
   }
   pdl_launch_dependents();
-  if (EPI <= EPI_ACCUM && a.cluster) {
+  if constexpr (CLUSTER) {
     skinny_cluster_sync();
     const int n0 = (int)blockIdx.x / a.splits * WM, rank = (int)blockIdx.x % a.splits;
     const int share = (a.M + a.splits - 1) / a.splits, t0 = rank * share, t1 = min(a.M, t0 + share);
@@ -405,22 +406,22 @@ void plan_split(int N, int K, int M, long long workspace_floats, int* splits, in
   *kb_per_split = kbs;
 }
 
-template <int TN, int EPI, typename TOut>
+template <int TN, int EPI, typename TOut, bool CLUSTER = false>
 int launch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, const SkinnyArgs& a, int* status, cudaStream_t stream,
            const NextNorm* next = nullptr) {
   using Cfg = SkinnyCfg<TN>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TN, EPI, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<TN, EPI, TOut, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
     if (e != cudaSuccess) return hfee_fail(HFEE_ERR_CUDA, "gemm_skinny: cannot get %d bytes of shared memory: %s", Cfg::SMEM, cudaGetErrorString(e));
     configured = true;
   }
   const int items = a.w_tiles * a.splits;
   const int sms = device_sms();
-  hfee_launch_with(hfee_carveout(), a.cluster ? dim3((unsigned)a.splits, 1, 1) : dim3(0, 0, 0), gemm_skinny_kernel<TN, EPI, TOut>,
+  hfee_launch_with(hfee_carveout(), CLUSTER ? dim3((unsigned)a.splits, 1, 1) : dim3(0, 0, 0), gemm_skinny_kernel<TN, EPI, TOut, CLUSTER>,
                    dim3((unsigned)(items < sms ? items : sms)), dim3(SK_THREADS), Cfg::SMEM, stream, mw, ma, (TOut*)C, a, status);
   int rc = hfee_check_launch("gemm_skinny");
-  if (rc != HFEE_OK || a.splits == 1 || a.cluster) return rc;
+  if (rc != HFEE_OK || a.splits == 1 || CLUSTER) return rc;
   if constexpr (EPI == EPI_ACCUM) {
     if (next != nullptr) {
       const int vec = (a.N / 4 + RN_THREADS - 1) / RN_THREADS;
@@ -441,7 +442,8 @@ int dispatch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, int out_dtyp
              int* status, cudaStream_t stream, const NextNorm* next) {
   if (epilogue == EPI_ACCUM) {
     if (out_dtype != HFEE_F32) return hfee_fail(HFEE_ERR_ARG, "gemm_skinny: accumulate needs a float32 output");
-    return launch<TN, EPI_ACCUM, float>(mw, ma, C, a, status, stream, next);
+    return a.cluster ? launch<TN, EPI_ACCUM, float, true>(mw, ma, C, a, status, stream)
+                     : launch<TN, EPI_ACCUM, float>(mw, ma, C, a, status, stream, next);
   }
   if (epilogue == EPI_GEGLU) {
     if (out_dtype == HFEE_BF16) return launch<TN, EPI_GEGLU, __nv_bfloat16>(mw, ma, C, a, status, stream);
@@ -455,6 +457,9 @@ int dispatch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, int out_dtyp
     if (out_dtype == HFEE_BF16) return launch<TN, EPI_SWIGLU, __nv_bfloat16>(mw, ma, C, a, status, stream);
     return launch<TN, EPI_SWIGLU, float>(mw, ma, C, a, status, stream);
   }
+  if (a.cluster)
+    return out_dtype == HFEE_BF16 ? launch<TN, EPI_STORE, __nv_bfloat16, true>(mw, ma, C, a, status, stream)
+                                  : launch<TN, EPI_STORE, float, true>(mw, ma, C, a, status, stream);
   if (out_dtype == HFEE_BF16) return launch<TN, EPI_STORE, __nv_bfloat16>(mw, ma, C, a, status, stream);
   return launch<TN, EPI_STORE, float>(mw, ma, C, a, status, stream);
 }
@@ -464,11 +469,14 @@ int dispatch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, int out_dtyp
 namespace {
 // Splits of a tile that are a cluster, or 0: the most of 8, 4 and 2 that the chip holds, with at least 4 K blocks each, if that is at least
 // three fifths of the SMs (64 tokens, N = 3,072, K = 2,048: 96 CTAs that add their own tiles 7.4 us, 144 and a kernel behind them 10.2).
+// A cluster lies within a GPC, and each of the nine or so leaves half a cluster's SMs over on average: what does not fit beside them runs
+// as a second round (20 tokens, K = 2,048, us with a cluster and without: 14 tiles of 8 CTAs 5.4 and 6.3, 16 of 8 9.2 and 6.4, 32 of 4 7.5
+// and 8.6, 36 of 4 11.8 and 9.0).
 int cluster_splits(int N, int K, int epilogue) {
   if (epilogue != EPI_STORE && epilogue != EPI_ACCUM) return 0;
   const int w_tiles = (N + WM - 1) / WM, k_blocks = (K + BK - 1) / BK, sms = device_sms();
   for (int s = 8; s >= 2; s /= 2)
-    if (w_tiles * s <= sms && k_blocks >= 4 * s)       // and no split without K blocks
+    if (w_tiles * s <= sms - 9 * s / 2 && k_blocks >= 4 * s)       // and no split without K blocks
       return w_tiles * s * 5 >= sms * 3 && (s - 1) * ((k_blocks + s - 1) / s) < k_blocks ? s : 0;
   return 0;
 }

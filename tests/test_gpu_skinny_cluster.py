@@ -7,7 +7,7 @@ DEV = "cuda:0"
 
 
 # clusters of 8, 4 and 2; rows that end inside a tile and a piece of four, tokens fewer than a cluster's CTAs and no multiple of them
-@pytest.mark.parametrize("m,n,k", [(64, 2048, 2048), (17, 2047, 2048), (33, 3072, 2048), (5, 4601, 1032), (64, 6149, 2048), (3, 1925, 8192)])
+@pytest.mark.parametrize("m,n,k", [(64, 1792, 2048), (17, 1663, 2048), (33, 3072, 2048), (5, 4091, 1032), (64, 6149, 2048), (3, 1541, 8192)])
 @pytest.mark.parametrize("epilogue", ["store", "accumulate"])
 def test_cluster_of_splits(m, n, k, epilogue):
     from hfee_b200.kernels import ops
@@ -25,3 +25,10 @@ def test_cluster_of_splits(m, n, k, epilogue):
         assert (out[:m].double() - ref).norm() <= (1e-5 if dtype == torch.float32 else 4e-3) * ref.norm()
         assert bool((out[m] == 3.0).all())
     assert ops.launch_count() == before + (2 if epilogue == "store" else 1)
+
+
+@pytest.mark.parametrize("n", [2048, 2304, 4608, 9472])
+def test_clusters_that_would_run_in_two_rounds_are_not_taken(n):
+    from hfee_b200.kernels import ops
+    if ops.sm_count() == 148:
+        assert not ops.library().hfee_gemm_skinny_in_cluster(n, 2048, ops.EPI_STORE)

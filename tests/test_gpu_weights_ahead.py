@@ -1,0 +1,25 @@
+"""Large-tile products of one tile of tokens ask for their first weight blocks before the wait for the kernel in front."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# a round of the ring over several tiles of a CTA (one K block each), within one tile, K split among CTAs, ragged ends, more tokens than a tile
+@pytest.mark.parametrize("m,n,k", [(65, 60000, 64), (128, 40960, 136), (100, 2048, 8192), (33, 8200, 1032), (1, 256, 8), (128, 128, 64),
+                                   (129, 8192, 512)])
+def test_products_behind_a_kernel_that_writes_their_tokens(m, n, k):
+    from hfee_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    x = torch.randn((m, k), generator=gen, device=DEV) * 3
+    w = (torch.randn((n, k), generator=gen, device=DEV) * 0.05).bfloat16()
+    a, out = torch.full((m, k), float("nan"), device=DEV, dtype=torch.bfloat16), torch.empty((m, n), device=DEV)
+    weight = torch.ones(k, device=DEV)
+    for scale in (1.0, -2.0):
+        ops.rmsnorm(x * scale, weight, a, 1e-5)
+        ops.gemm_tcgen05(a, w, out, ops.EPI_STORE)
+        want = a.double() @ w.double().t()
+        # sums of k products of bfloat16 numbers in float32: 2^-24 a step
+        assert ((out.double() - want).abs() <= 1e-6 * k ** 0.5 * (a.double().abs() @ w.double().abs().t()) + 1e-6).all()
+    ops.check_status()
