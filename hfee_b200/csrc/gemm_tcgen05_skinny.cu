@@ -105,7 +105,7 @@ __device__ __forceinline__ void write_columns(const uint32_t (&v)[COLS], int tok
   }
 }
 
-// CLUSTER: the splits of a tile are a cluster (a kernel of its own: the test for it in the other cost them 0.2 us).
+// CLUSTER: the splits of a tile are a cluster (a kernel of its own: a test at run time cost the other products 0.2 us).
 template <int TN, int EPI, typename TOut, bool CLUSTER>
 __global__ void __launch_bounds__(SK_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
@@ -468,7 +468,7 @@ int dispatch(const CUtensorMap& mw, const CUtensorMap& ma, void* C, int out_dtyp
 
 namespace {
 // Splits of a tile that are a cluster, or 0: the most of 8, 4 and 2 that the chip holds, with at least 4 K blocks each, if that is at least
-// three fifths of the SMs (64 tokens, N = 3,072, K = 2,048: 96 CTAs that add their own tiles 7.4 us, 144 and a kernel behind them 10.2).
+// three fifths of the SMs (64 tokens, N = 3,072, K = 2,048: 96 CTAs that add their own tiles 7.0 us, 144 and a kernel behind them 10.2).
 // A cluster lies within a GPC, and each of the nine or so leaves half a cluster's SMs over on average: what does not fit beside them runs
 // as a second round (20 tokens, K = 2,048, us with a cluster and without: 14 tiles of 8 CTAs 5.4 and 6.3, 16 of 8 9.2 and 6.4, 32 of 4 7.5
 // and 8.6, 36 of 4 11.8 and 9.0).
